@@ -253,6 +253,14 @@ int check_linear_args(kq_ctx* ctx, const Weight* w, uint64_t x, int x_dtype, uin
   return KQ_OK;
 }
 
+// The many-row kernel of kq_qgemm_exact.cu runs this call: more than 16 rows, weights of one kind,
+// and not a case of the bf16 GEMM (bf16 activations on a tiled weight, whose operands are rounded).
+bool takes_exact_gemm(const kq_ctx* ctx, int count, const kq::LinearTarget* targets, int x_dtype, uint32_t m) {
+  for (int i = 0; i < count; ++i)
+    if (kq::qgemm_i4_supports(*targets[i].w, x_dtype, m) || kq::qgemm_i8_supports(*targets[i].w, x_dtype, m)) return false;
+  return kq::qgemm_exact_supports(count, targets, m, ctx->workspace ? ctx->workspace_bytes : 0);
+}
+
 int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x, int x_dtype,
                const uint64_t* bias, const uint64_t* out, uint32_t m, const kq::LinearFusion* fusion = nullptr) {
   if (count < 1 || count > (uint32_t)kq::kMaxMulti)
@@ -294,19 +302,13 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
     }
     return KQ_OK;
   }
-  bool x32 = all_tiled;
-  for (uint32_t i = 0; i < count && x32; ++i)
-    x32 = targets[i].w->n == 0 || kq::qgemm_i4_x32_supports(*targets[i].w, x_dtype, m, ctx->workspace ? ctx->workspace_bytes : 0);
-  if (x32) {
-    // Prefill with f32 / binary16 activations: the split-operand tcgen05 GEMM, one weight at a time.
-    for (uint32_t i = 0; i < count; ++i) {
-      if (targets[i].w->n == 0) continue;
-      int launched = 0;
-      cudaError_t e = kq::launch_qgemm_i4_x32(env, targets[i], reinterpret_cast<const void*>(x), x_dtype, m, ctx->gemm_status_dev,
-                                              &launched);
-      if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemm_i4_x32 launch");
-      ctx->launches += launched;
-    }
+  if (takes_exact_gemm(ctx, static_cast<int>(count), targets, x_dtype, m)) {
+    // Many rows, and not the bf16 GEMM: weights as exact integers on the tensor cores, one launch
+    // for all weights of the call.
+    int launched = 0;
+    cudaError_t e = kq::launch_qgemm_exact(env, static_cast<int>(count), targets, reinterpret_cast<const void*>(x), x_dtype, m, &launched);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemm_exact launch");
+    ctx->launches += launched;
     return KQ_OK;
   }
   if (all_tiled && same_scale) {
@@ -328,6 +330,13 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
   // Everything else: one generic launch per weight.
   for (uint32_t i = 0; i < count; ++i) {
     const Weight& w = *targets[i].w;
+    if (w.n != 0 && takes_exact_gemm(ctx, 1, &targets[i], x_dtype, m)) {
+      int launched = 0;
+      cudaError_t e = kq::launch_qgemm_exact(env, 1, &targets[i], reinterpret_cast<const void*>(x), x_dtype, m, &launched);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemm_exact launch");
+      ctx->launches += launched;
+      continue;
+    }
     if (w.layout == kq::kLayoutTiledI4) {
       kq::LinearTarget one = targets[i];
       for (uint32_t m0 = 0; m0 < m; m0 += 16) {
@@ -847,6 +856,15 @@ int kq_linear_a8(kq_ctx* ctx, kq_weight h, uint64_t xq_dptr, uint64_t xs_dptr, u
     return fail(ctx, KQ_ERR_UNSUPPORTED, "kq_linear_a8: k=%u exceeds the int32 reduction gate 131072", w->k);
   if (m == 0 || w->n == 0) return KQ_OK;
   DeviceGuard guard(ctx->device);
+  if (kq::qgemm_exact_a8_supports(*w, reinterpret_cast<const int8_t*>(xq_dptr), m, ctx->workspace ? ctx->workspace_bytes : 0)) {
+    const kq::LinearTarget target{w, reinterpret_cast<const float*>(bias_dptr), reinterpret_cast<float*>(out_dptr)};
+    int n_launched = 0;
+    cudaError_t e = kq::launch_qgemm_exact_a8(env_of(ctx), target, reinterpret_cast<const int8_t*>(xq_dptr),
+                                              reinterpret_cast<const float*>(xs_dptr), m, &n_launched);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "linear_a8 launch");
+    ctx->launches += n_launched;
+    return KQ_OK;
+  }
   const bool tiled = w->layout == kq::kLayoutTiledI4 || w->layout == kq::kLayoutTiledI8;
   int* row_sum = nullptr;
   int* group_sum = nullptr;
@@ -1063,8 +1081,9 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
   }
   if (m == 0) return KQ_OK;
   DeviceGuard guard(ctx->device);
-  // Outside a plan: the same arithmetic as a sequence of kernels — except where the GEMV takes
-  // the norm and the residual into its own launches (five and more rows, tiled int4 weights).
+  // Outside a plan: the same arithmetic as a sequence of kernels — except where the linear takes
+  // the norm and the residual into its own launches (five to sixteen rows on tiled int4 weights,
+  // and the many-row kernel).
   {
     kq::LinearTarget probe[kq::kMaxMulti];
     bool known = true;
@@ -1072,8 +1091,9 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
       probe[i] = kq::LinearTarget{find_weight(ctx, w[i]), nullptr, nullptr};
       known = known && probe[i].w != nullptr;
     }
-    if (known && !reduce &&
-        kq::qgemv_i4_fuses_neighbours(static_cast<int>(count), probe, x_dtype, m) && (norm_weight_dptr || residual_dptr)) {
+    if (known && !reduce && (norm_weight_dptr || residual_dptr) &&
+        (kq::qgemv_i4_fuses_neighbours(static_cast<int>(count), probe, x_dtype, m) ||
+         takes_exact_gemm(ctx, static_cast<int>(count), probe, x_dtype, m))) {
       int rc;
       if (swiglu) {
         const uint64_t each = static_cast<uint64_t>(m) * w0->n;

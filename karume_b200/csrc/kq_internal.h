@@ -128,10 +128,16 @@ bool qgemm_i4_supports(const Weight& w, int x_dtype, uint32_t m);
 bool qgemm_i8_supports(const Weight& w, int x_dtype, uint32_t m);
 cudaError_t launch_qgemm_i4(const LaunchEnv& env, const LinearTarget& target, const void* x, uint32_t m,
                             int* status_word, int* extra_launches);
-// The same for f32 and binary16 activations (kq_qgemm_i4_x32.cu): both operands as two bf16 numbers.
-bool qgemm_i4_x32_supports(const Weight& w, int x_dtype, uint32_t m, uint64_t workspace_bytes);
-cudaError_t launch_qgemm_i4_x32(const LaunchEnv& env, const LinearTarget& target, const void* x, int x_dtype, uint32_t m,
-                                int* status_word, int* launches);
+// Every other many-row linear (kq_qgemm_exact.cu): f32 / binary16 / bf16 activations on any packed
+// storage, weights as exact integers.  All targets of one call share storage, layout, k, group
+// size and scale type.  env.norm_weight (f32 activations) and env.residual (one target) are applied.
+bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, uint64_t workspace_bytes);
+cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,
+                               int* launches);
+// ... and the integer-dot form: int8 activations [m, k] with row scales xs (bit-exact contract).
+bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes);
+cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& target, const int8_t* xq, const float* xs, uint32_t m,
+                                  int* launches);
 }  // namespace kq
 
 // ---- error reporting shared with kq_container.cu (kq_api.cu) ------------------------------

@@ -1,0 +1,1112 @@
+// qgemm_exact — the linear for many activation rows (m > 16) whose weights enter the tensor
+// core as EXACT small integers:  out[m, n] = x[m, k] . W[n, k]^T + bias.
+//
+// Replaces the reference's large-M linear variants that compute in f32
+// (linear:v2:f32:reg64x32r4x4w8 and reg128x128r8x8w16 —
+// packages/runtime/src/kernels/gemm-geometry.ts:243-267) for every packed storage, and its
+// integer-dot GEMMs (packages/runtime/src/kernels/linear-i8a8.ts:21-72).
+//
+// A stored int4 / int8 weight is an integer q of at most 8 bits, exact in binary16, so nothing
+// has to be rounded and nothing has to be multiplied by a scale on its way to the tensor core:
+//     y[m, n] = sum_groups s[n, g] * ( sum_{k in g} x[m, k] * q[n, k] )
+// The inner sum is a short MMA chain into a tensor-memory accumulator; every group the "drain"
+// warps read that accumulator and add it, times the group's scale, to f32 sums they keep in
+// registers.  An activation is carried exactly (binary16 input, int8 input of the integer-dot
+// form) or as two binary16 parts of its power-of-two pre-scaled value (f32, bf16: 22 bits).  So
+//   * binary16 activations cost ONE product and f32 activations two, where splitting both
+//     operands costs three;
+//   * an accumulator chain is one group long (at most kMaxChain k), so the tensor core's f32
+//     accumulation never gets the chance to drift;
+//   * the integer-dot form of int4 weights is the same kernel: its per-group sums are integers
+//     below 2^24, exact in the f32 accumulator, and the contract's one fma per group in
+//     ascending order IS the drain (bit-identical).  Int8 weights with int8 activations run on
+//     kind::i8 with an int32 accumulator over the whole of k.
+//
+// The weights are the M side (256 output channels per CTA pair, 128 per CTA), the activation
+// rows the N side (NT <= 256 of them), so a lane of the accumulator is one output channel: its
+// scale and bias are per-lane scalars and a store instruction writes 32 consecutive outputs.
+//
+//   warps 0-7    drain: tcgen05.ld, one fma per sum, then the epilogue
+//   warps 8-11   producers: raw packed weights (shared memory) -> integers in the K-major,
+//                128-byte-swizzled tile the MMA reads.  Shared memory to shared memory only: a
+//                global load still in flight when a thread runs its proxy fence would hold the
+//                fence, and with it the stage, for a trip to memory.
+//   warp 12      starts every copy: the activation tile (tensor map), the raw weights (bulk)
+//   warps 14-15  the group scales, a few chains ahead, as f32 into shared memory
+//   warp 13      tensor memory; in the CTA of cluster rank 0 one thread issues the MMAs
+//                (cta_group::2: the pair shares the activation tile, half from each CTA)
+// Register split (setmaxnreg): 2 x 128 x 184 + 2 x 128 x 72 = 512 x 128.
+//
+// Every mbarrier wait is bounded; a wait that gives up sets a status word and a CTA-wide abort
+// flag that makes all later waits return at once, so tensor memory is always released.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "kq_common.cuh"
+#include "kq_gemv_core.cuh"
+#include "kq_internal.h"
+#include "kq_umma.cuh"
+
+namespace kq {
+namespace {
+
+using namespace umma;
+
+enum WeightKind : int { kI4Tiled = 0, kI4Rows = 1, kI8Tiled = 2, kI8Rows = 3 };
+enum MathKind : int { kHalf1 = 1, kHalf2 = 2, kInt8 = 3 };  // one binary16 part, two, or int8 x int8
+
+constexpr int kDrainWarps = 8, kProdWarps = 4, kCopyWarp = 12, kMmaWarp = 13, kScaleWarp = 14, kExThreads = 512;
+constexpr uint32_t kRows = 128;                 // output channels per CTA
+constexpr uint32_t kATile = kRows * 128;        // 16 KB: 128 rows x 128 bytes of k
+constexpr uint32_t kMaxNT = 256;                // activation rows per tile
+constexpr uint32_t kMaxStages = 8;
+constexpr uint32_t kSmemLimit = 227 * 1024;
+constexpr uint32_t kScaleBatch = 8;             // accumulator chains per slot of the scale ring (two slots)
+constexpr uint32_t kTailRowScale = 320, kTailScales = kTailRowScale + kMaxNT * 4;
+constexpr uint32_t kSmemTail = kTailScales + 2 * kScaleBatch * kRows * 4;  // barriers, the tile's row scales, the scale ring
+constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain
+
+struct ExTarget {
+  const uint8_t* w;
+  const void* scale;      // rows layouts: [n, k / group]; int8: [n]; tiled int4: inside the chunks
+  const float* bias;
+  float* out;
+  const float* residual;  // null, or [m, n] added after the bias (may alias out)
+  uint32_t n;
+  uint32_t pair0;         // first column pair (256 channels) of this weight
+};
+
+struct ExParams {
+  ExTarget t[kMaxMulti];
+  uint32_t count;
+  uint32_t m, k;
+  uint32_t ksteps;         // k-steps of 128 bytes (64 binary16 or 128 int8 values)
+  uint32_t nt;             // activation rows per tile, a multiple of 32
+  uint32_t drain16;        // k16 slices per accumulator chain
+  uint32_t drains_per_group_shift;  // accumulator chains per scale group, log2 (groups longer than kMaxChain)
+  uint32_t groups;         // scale groups per row
+  uint32_t scale_f16;
+  uint32_t stages, stage_bytes, raw_off, raw_bytes, raw_box;
+  const float* row_scale;  // [m]: undoes the pre-scale (2^-e), or the activation scale of the integer-dot form; null: 1
+  uint32_t splits, ksteps_per_split;
+  float* partial;          // [splits][m][n of all weights] raw sums when splits > 1
+  uint32_t n_total;
+  int* status;
+};
+
+__device__ __forceinline__ float load_scale_dyn(const void* base, size_t index, uint32_t f16) {
+  return f16 ? __half2float(reinterpret_cast<const __half*>(base)[index]) : reinterpret_cast<const float*>(base)[index];
+}
+
+// ---- integers -> binary16 -----------------------------------------------------------------
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) { return (a & mask) | bits; }
+
+// 8 nibbles u (k ascending) -> 8 binary16 values u - 8, exact.  (w & 0x000F000F) | 0x6400.. is
+// the pair 1024 + u of nibbles 0 and 4; (w & 0x00F000F0) | 0x6400.. the pair 1024 + 16 u of
+// nibbles 1 and 5, brought down by one exact fused multiply-add.
+__device__ __forceinline__ uint4 nibbles_to_half(uint32_t w) {
+  const __half2 k1032 = __half2half2(__ushort_as_half(0x6408)), k16th = __half2half2(__ushort_as_half(0x2C00)),
+                km72 = __half2half2(__ushort_as_half(0xD480));
+  const uint32_t w8 = w >> 8;
+  uint32_t r[4] = {and_or(w, 0x000F000Fu, 0x64006400u), and_or(w, 0x00F000F0u, 0x64006400u),
+                   and_or(w8, 0x000F000Fu, 0x64006400u), and_or(w8, 0x00F000F0u, 0x64006400u)};
+  __half2 h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 v = *reinterpret_cast<const __half2*>(&r[i]);
+    h[i] = (i & 1) ? __hfma2(v, k16th, km72) : __hsub2(v, k1032);
+    r[i] = *reinterpret_cast<const uint32_t*>(&h[i]);
+  }
+  return make_uint4(__byte_perm(r[0], r[1], 0x5410), __byte_perm(r[2], r[3], 0x5410), __byte_perm(r[0], r[1], 0x7632),
+                    __byte_perm(r[2], r[3], 0x7632));
+}
+
+// 4 bytes q + 128 -> 4 binary16 values q, exact: a byte under the exponent of 1024 is 1024 + byte.
+__device__ __forceinline__ uint2 bytes_to_half(uint32_t w) {
+  const __half2 k1152 = __half2half2(__ushort_as_half(0x6480));
+  uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
+  const __half2 ha = __hsub2(*reinterpret_cast<const __half2*>(&a), k1152), hb = __hsub2(*reinterpret_cast<const __half2*>(&b), k1152);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts64(uint32_t addr, uint2 v) {
+  asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// ---- tensor memory ---------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// kind::f16 with binary16 operands / kind::i8 with signed operands; f32 / s32 accumulate, M 256
+template <int kMath>
+__host__ __device__ constexpr uint32_t exact_idesc(uint32_t nt) {
+  return (kMath == kInt8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((nt >> 3) << 17) | ((256u >> 4) << 24);
+}
+// Descriptors by their low words (address, leading offset); the high word is the layout's constant.
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+// One lane of a warp, the same one every time.  What a single thread has to do below is a predicated
+// instruction of a converged warp, never a branch: in a divergent lane-0 region the barrier tests and
+// MMA issues took two to three times as long (700 - 850 clocks a k-step whatever its width).
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+template <int kMath, bool kAccumulate>
+__device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
+  if constexpr (kMath == kInt8)
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+                 "@q tcgen05.mma.cta_group::2.kind::i8 [%0], a, b, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHigh), "r"(leader) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+                 "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHigh), "r"(leader) : "memory");
+}
+// arrives on the barrier at this address in BOTH CTAs of the pair once the MMAs issued so far are done
+__device__ __forceinline__ void commit_both(uint32_t leader, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+               ::"r"(bar), "h"(static_cast<uint16_t>(3)), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void arrive_if(uint32_t leader, uint32_t cluster_bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}"
+               ::"r"(cluster_bar), "r"(leader) : "memory");
+}
+
+// ---- copies ---------------------------------------------------------------------------------
+__device__ __forceinline__ void expect_tx(uint32_t leader, uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
+               ::"r"(bar), "r"(bytes), "r"(leader) : "memory");
+}
+// reports to a barrier of either CTA of the pair
+__device__ __forceinline__ void copy_tile_3d(uint32_t leader, uint32_t dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t z, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void copy_tile_2d(uint32_t leader, uint32_t dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "r"(leader) : "memory");
+}
+
+// Bytes of raw weights one 16-row block (tiled layouts) or one row (rows layouts) brings per k-step.
+template <int kW, int kMath>
+__host__ __device__ constexpr uint32_t raw_unit_bytes(uint32_t scale_f16) {
+  return kW == kI4Tiled ? kChunkWeightBytes + (scale_f16 ? 64u : 128u)
+         : kW == kI4Rows ? 32u
+         : kW == kI8Tiled ? (kMath == kInt8 ? 2048u : 1024u)
+                          : (kMath == kInt8 ? 128u : 64u);
+}
+
+template <int kW, int kMath>
+__global__ void __launch_bounds__(kExThreads, 1)
+qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map0,
+                   const __grid_constant__ CUtensorMap w_map1, const __grid_constant__ CUtensorMap w_map2,
+                   const __grid_constant__ CUtensorMap w_map3) {
+  constexpr bool kTiled = kW == kI4Tiled || kW == kI8Tiled;
+  constexpr bool kGroupScales = kW == kI4Tiled || kW == kI4Rows;
+  constexpr uint32_t kParts = kMath == kHalf2 ? 2u : 1u;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t raw_base = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
+  const uint32_t tiles = (raw_base + 1023u) & ~1023u;
+  const uint32_t bars = tiles + p.stages * p.stage_bytes;
+  uint8_t* tail = smem_raw + (tiles - raw_base) + p.stages * p.stage_bytes;
+  const uint32_t full = bars, empty = bars + kMaxStages * 8, rawfull = empty + kMaxStages * 8, dfull = rawfull + kMaxStages * 8,
+                 dempty = dfull + 32, sfull = dempty + 32, sempty = sfull + 16;
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(tail + 296);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 304);
+  float* row_scale_s = reinterpret_cast<float*>(tail + kTailRowScale);
+  float* scale_ring = reinterpret_cast<float*>(tail + kTailScales);
+  const uint32_t cta_rank = cluster_ctarank();
+  // Accumulators in tensor memory: four of up to 128 columns or two of up to 256.  From an MMA's issue
+  // to its drain and back are three barrier hops (about 700 clocks), so the narrow form keeps four
+  // chains in flight.
+  const uint32_t acc_shift = p.nt <= kMaxNT / 2 ? 2u : 1u, acc_mask = (1u << acc_shift) - 1u, acc_cols = 512u >> acc_shift;
+
+  // which weight, which channels, which activation rows, which k-steps
+  const uint32_t pair = blockIdx.x >> 1;
+  uint32_t wi = 0;
+#pragma unroll
+  for (int i = 1; i < kMaxMulti; ++i)
+    if (i < static_cast<int>(p.count) && pair >= p.t[i].pair0) wi = i;
+  // (the weight's pointers are read from the parameters where they are used: kept in registers from
+  // here on they would spill beside the drain warps' sums)
+  const uint32_t n0 = (pair - p.t[wi].pair0) * (2 * kRows) + cta_rank * kRows;  // this CTA's first output channel
+  const uint32_t m0 = blockIdx.y * p.nt;
+  const uint32_t ks_begin = blockIdx.z * p.ksteps_per_split;
+  const uint32_t ks_count = min(ks_begin + p.ksteps_per_split, p.ksteps) - ks_begin;
+
+  if (warp == kMmaWarp) {
+    if (lane == 0) {
+      for (uint32_t s = 0; s < p.stages; ++s) {
+        mbar_init(full + s * 8, 2 + 1);               // the producer warp of each CTA; + the activation tiles' bytes
+        mbar_init(empty + s * 8, 1);                  // one tcgen05.commit
+        mbar_init(rawfull + s * 8, 1);                // the raw weights' bytes
+      }
+      for (uint32_t b = 0; b < 4; ++b) {
+        mbar_init(dfull + b * 8, 1);
+        mbar_init(dempty + b * 8, 2 * kDrainWarps);
+      }
+      for (uint32_t b = 0; b < 2; ++b) {
+        mbar_init(sfull + b * 8, 2);
+        mbar_init(sempty + b * 8, kDrainWarps);
+      }
+      *abort_flag = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars + 296), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  pdl_wait_prior_grid();  // the converted activations come from the launch before
+  for (uint32_t i = threadIdx.x; i < p.nt; i += kExThreads)
+    row_scale_s[i] = p.row_scale != nullptr && m0 + i < p.m ? p.row_scale[m0 + i] : 1.0f;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster_sync_all();  // barriers of both CTAs are initialised
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot_ptr;
+  pdl_launch_dependents();
+
+  const uint32_t leader = elect_lane();
+
+  if (warp < kDrainWarps) {
+    // ---------------- drain ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+    const uint32_t quarter = warp & 3u, half = warp >> 2;
+    const uint32_t cols = p.nt / 2, col0 = half * cols;  // this warp's share of the tile's activation rows
+    const uint32_t row = n0 + quarter * 32u + lane;      // this lane's output channel
+    const uint32_t taddr = tmem + ((quarter * 32u) << 16) + col0;
+    // The finished sums go through this thread's own words of shared memory (the stages are free
+    // then): the stores to `out` can be a short loop, where 128 unrolled copies of it are 24 KB of
+    // instructions that every CTA fetches cold (13 us instead of 3 for 256 x 18944 outputs).
+    const uint32_t park = tiles + warp * (cols * 128u) + lane * 4u;
+    if constexpr (kMath == kInt8) {
+      wait_bounded(dfull, 0, abort_flag, p.status, 23);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+      for (uint32_t b = 0; b * 16u < cols; ++b) {
+        uint32_t v[16];
+        tmem_ld16(taddr + b * 16u, v);
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) sts32(park + (b * 16u + j) * 128u, v[j]);
+      }
+    } else {
+      const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16;
+      const uint32_t dempty_0 = map_to_cta(dempty, 0);
+      const float* my_scale = scale_ring + quarter * 32u + lane;
+      // kBatches x 16 columns per warp, a constant: a branch around every batch (a runtime width) takes
+      // the 450-clock drain of 256 columns to 1,400
+      auto drain_all = [&](auto batches) {
+        constexpr int kBatches = decltype(batches)::value;
+        float acc[kBatches][16];
+#pragma unroll
+        for (int b = 0; b < kBatches; ++b)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc[b][j] = 0.0f;
+#pragma unroll 1
+        for (uint32_t d = 0; d < drains; ++d) {
+          const uint32_t buf = d & acc_mask, batch = d / kScaleBatch;
+          float s = 1.0f;
+          if constexpr (kGroupScales) {
+            if (d % kScaleBatch == 0) wait_bounded(sfull + (batch & 1u) * 8, (batch >> 1) & 1u, abort_flag, p.status, 25);
+            s = my_scale[((batch & 1u) * kScaleBatch + d % kScaleBatch) * kRows];
+          }
+          wait_bounded(dfull + buf * 8, (d >> acc_shift) & 1u, abort_flag, p.status, 23);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int b = 0; b < kBatches; ++b) {
+            uint32_t v[16];
+            tmem_ld16(taddr + buf * acc_cols + b * 16u, v);
+            // scalar fused multiply-adds: the packed form (fma.rn.f32x2) needs register pairs the
+            // allocator does not find beside 128 sums (measured 460 - 800 clocks a chain against 335)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if constexpr (kGroupScales) acc[b][j] = fmaf(__uint_as_float(v[j]), s, acc[b][j]);
+              else acc[b][j] += __uint_as_float(v[j]);
+            }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          arrive_if(leader, dempty_0 + buf * 8);
+          if (kGroupScales) arrive_if(d % kScaleBatch == kScaleBatch - 1 ? leader : 0u, sempty + (batch & 1u) * 8);
+        }
+#pragma unroll
+        for (int b = 0; b < kBatches; ++b)
+#pragma unroll
+          for (uint32_t j = 0; j < 16; ++j) sts32(park + (b * 16u + j) * 128u, __float_as_uint(acc[b][j]));
+      };
+      switch (p.nt / 32) {
+        case 1: drain_all(std::integral_constant<int, 1>{}); break;
+        case 2: drain_all(std::integral_constant<int, 2>{}); break;
+        case 3: drain_all(std::integral_constant<int, 3>{}); break;
+        case 4: drain_all(std::integral_constant<int, 4>{}); break;
+        case 6: drain_all(std::integral_constant<int, 6>{}); break;
+        default: drain_all(std::integral_constant<int, 8>{}); break;
+      }
+    }
+    // ---------------- epilogue ----------------
+    const ExTarget tg = p.t[wi];
+    const bool row_live = row < tg.n;
+    const uint32_t mm0 = m0 + col0;
+    const uint32_t live_cols = row_live && mm0 < p.m ? min(cols, p.m - mm0) : 0u;
+    if (p.splits == 1) {
+      const float bias = row_live ? tg.bias[row] : 0.0f;
+      float ws = 1.0f;
+      if constexpr (!kGroupScales) ws = row_live ? load_scale_dyn(tg.scale, row, p.scale_f16) : 0.0f;
+      float* dst = tg.out + static_cast<size_t>(mm0) * tg.n + row;
+      const float* res = tg.residual != nullptr ? tg.residual + static_cast<size_t>(mm0) * tg.n + row : nullptr;
+#pragma unroll 4
+      for (uint32_t c = 0; c < live_cols; ++c) {
+        const uint32_t v = lds32(park + c * 128u);
+        const float rs = row_scale_s[col0 + c];
+        float o;
+        if constexpr (kMath == kInt8) o = fmaf(__int2float_rn(static_cast<int>(v)), __fmul_rn(rs, ws), bias);
+        else if constexpr (kGroupScales) o = fmaf(__uint_as_float(v), rs, bias);
+        else o = fmaf(__uint_as_float(v) * ws, rs, bias);
+        if (res != nullptr) {
+          o = __fadd_rn(o, *res);
+          res += tg.n;
+        }
+        *dst = o;
+        dst += tg.n;
+      }
+    } else {
+      uint32_t before = 0;
+#pragma unroll
+      for (int i = 0; i < kMaxMulti; ++i)
+        if (static_cast<uint32_t>(i) < wi) before += p.t[i].n;
+      uint32_t* dst = reinterpret_cast<uint32_t*>(p.partial) + (static_cast<size_t>(blockIdx.z) * p.m + mm0) * p.n_total + before + row;
+#pragma unroll 4
+      for (uint32_t c = 0; c < live_cols; ++c) {
+        *dst = lds32(park + c * 128u);
+        dst += p.n_total;
+      }
+    }
+  } else if (warp < kDrainWarps + kProdWarps) {
+    // ---------------- producers ----------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    // One warp converts the whole weight tile of a k-step, and the four warps take stages in turn: what
+    // a k-step costs in latency (wait, loads, fence, arrival) then overlaps other k-steps.  A stage
+    // belongs to ONE warp: it waits for that barrier's phases one after the other, so a parity can
+    // never be mistaken for the one two phases away (copies of different stages finish in any order).
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), full_0 = map_to_cta(full, 0);
+    uint32_t s = 0, phase = 0;
+    for (uint32_t ks = 0; ks < ks_count; ++ks, s = s + 1 == p.stages ? 0u : s + 1u, phase ^= s == 0 ? 1u : 0u) {
+      if ((s & (kProdWarps - 1u)) != warp - kDrainWarps) continue;
+      wait_bounded(rawfull + s * 8, phase, abort_flag, p.status, 21);
+      const uint32_t a_tile = tiles + s * p.stage_bytes, raw = a_tile + p.raw_off;
+      if constexpr (kW == kI4Tiled) {
+        // words: row g group 0 | row g+8 group 0 | row g group 1 | row g+8 group 1, each k 8t..8t+7 of
+        // the group: 16-byte piece t / 4 + t of the tile row.  Odd g stores group 1 first, so the 8
+        // lanes of a shared-memory phase hit 8 different pieces of the swizzled rows.
+        const bool odd = (g & 1u) != 0;
+        const uint32_t p0 = odd ? 4u + t : t, p1 = odd ? t : 4u + t;
+        uint4 q = lds128(raw + lane * 16u);
+#pragma unroll 4
+        for (uint32_t c = 0; c < 8; ++c) {
+          const uint4 now = q;
+          if (c < 7) q = lds128(raw + (c + 1u) * unit + lane * 16u);
+          const uint32_t r_a = c * 16u + g, r_b = r_a + 8u;
+          sts128(a_tile + swz(r_a, p0), nibbles_to_half(odd ? now.z : now.x));
+          sts128(a_tile + swz(r_a, p1), nibbles_to_half(odd ? now.x : now.z));
+          sts128(a_tile + swz(r_b, p0), nibbles_to_half(odd ? now.w : now.y));
+          sts128(a_tile + swz(r_b, p1), nibbles_to_half(odd ? now.y : now.w));
+        }
+      } else if constexpr (kW == kI4Rows) {
+        // a row's k-step is 32 bytes: lane = (row, half), 16 bytes = 32 k = four pieces
+#pragma unroll 4
+        for (uint32_t c = 0; c < 8; ++c) {
+          const uint32_t r = c * 16u + (lane >> 1), h = lane & 1u;
+          const uint4 q = lds128(raw + r * 32u + h * 16u);
+          sts128(a_tile + swz(r, h * 4u + 0u), nibbles_to_half(q.x));
+          sts128(a_tile + swz(r, h * 4u + 1u), nibbles_to_half(q.y));
+          sts128(a_tile + swz(r, h * 4u + 2u), nibbles_to_half(q.z));
+          sts128(a_tile + swz(r, h * 4u + 3u), nibbles_to_half(q.w));
+        }
+      } else if constexpr (kW == kI8Tiled && kMath != kInt8) {
+        // chunk j, words: row g k 4t.. | row g+8 same k | row g k 16+4t.. | row g+8: four weights = 8
+        // bytes = half (t & 1) of piece 4j + 2h + (t >> 1).  The order in which a lane walks its four
+        // (j, h) pairs is XORed with a value that differs where the rows' swizzle term does not, so
+        // the 16 lanes of a phase hit 8 different pieces.
+#pragma unroll 2
+        for (uint32_t rb = 0; rb < 8; ++rb) {
+          const uint32_t r_a = rb * 16u + g, r_b = r_a + 8u;
+          const uint32_t flip = (g & 1u) * 2u, sub = t >> 1, byte = (t & 1u) * 8u;
+          uint4 q[2];
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j) q[j] = lds128(raw + rb * unit + (j ^ (flip >> 1)) * 512u + lane * 16u);
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j) {
+            const uint32_t o = (2u * j) ^ flip;
+            sts64(a_tile + swz(r_a, o * 2u + sub) + byte, bytes_to_half(q[j].x));
+            sts64(a_tile + swz(r_b, o * 2u + sub) + byte, bytes_to_half(q[j].y));
+            sts64(a_tile + swz(r_a, (o + 1u) * 2u + sub) + byte, bytes_to_half(q[j].z));
+            sts64(a_tile + swz(r_b, (o + 1u) * 2u + sub) + byte, bytes_to_half(q[j].w));
+          }
+        }
+      } else if constexpr (kW == kI8Rows && kMath != kInt8) {
+        // a row's k-step is 64 bytes: lane = (row, quarter), 16 bytes = 16 k = two pieces
+#pragma unroll 4
+        for (uint32_t c = 0; c < 16; ++c) {
+          const uint32_t r = c * 8u + (lane >> 2), qd = lane & 3u;
+          const uint4 q = lds128(raw + r * 64u + qd * 16u);
+          const uint2 a = bytes_to_half(q.x ^ 0x80808080u), b = bytes_to_half(q.y ^ 0x80808080u);
+          const uint2 d = bytes_to_half(q.z ^ 0x80808080u), e = bytes_to_half(q.w ^ 0x80808080u);
+          sts128(a_tile + swz(r, qd * 2u), make_uint4(a.x, a.y, b.x, b.y));
+          sts128(a_tile + swz(r, qd * 2u + 1u), make_uint4(d.x, d.y, e.x, e.y));
+        }
+      } else if constexpr (kW == kI8Tiled) {
+        // int8 tile: four chunks (32 k each) of a row block; a word is 4 bytes of piece 2j + h, the sign
+        // bit flipped back.  Eight rows x four words hit 32 different banks.
+#pragma unroll 2
+        for (uint32_t rb = 0; rb < 8; ++rb) {
+          const uint32_t r_a = rb * 16u + g, r_b = r_a + 8u;
+          uint4 qs[4];
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j) qs[j] = lds128(raw + rb * unit + j * 512u + lane * 16u);
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j) {
+            const uint4 q = qs[j];
+            sts32(a_tile + swz(r_a, 2u * j) + 4u * t, q.x ^ 0x80808080u);
+            sts32(a_tile + swz(r_b, 2u * j) + 4u * t, q.y ^ 0x80808080u);
+            sts32(a_tile + swz(r_a, 2u * j + 1u) + 4u * t, q.z ^ 0x80808080u);
+            sts32(a_tile + swz(r_b, 2u * j + 1u) + 4u * t, q.w ^ 0x80808080u);
+          }
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // -> visible to the tensor core
+      __syncwarp();
+      arrive_if(leader, full_0 + s * 8);  // the issuing CTA's barrier
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == kCopyWarp) {
+      // ---------------- copies ----------------
+      // One thread, two or three tensor copies per k-step: a bulk copy per 16-row block (eight of
+      // them) took 700 - 1000 clocks to start, more than the k-step's MMAs.
+      {
+        const uint32_t half_rows = p.nt / 2, b_bytes = half_rows * 128u, raw_bytes = p.raw_bytes;
+        const CUtensorMap* w_map = wi == 0 ? &w_map0 : wi == 1 ? &w_map1 : wi == 2 ? &w_map2 : &w_map3;
+        const uint32_t full_0 = map_to_cta(full, 0), raw_off = kW == kI8Rows && kMath == kInt8 ? 0u : p.raw_off;
+        const uint32_t w_row = kTiled ? n0 / 16u : n0, w_step = p.raw_box;  // tensor-map rows and columns of the raw weights
+        uint32_t s = 0, phase = 0;
+        for (uint32_t ks = 0; ks < ks_count; ++ks) {
+          wait_bounded(empty + s * 8, phase ^ 1u, abort_flag, p.status, 20);
+          const uint32_t a_tile = tiles + s * p.stage_bytes, kstep = ks_begin + ks;
+          expect_tx(cta_rank == 0 ? leader : 0u, full + s * 8, kParts * 2u * b_bytes);
+          expect_tx(leader, rawfull + s * 8, raw_bytes);
+          copy_tile_2d(leader, a_tile + raw_off, w_map, kstep * w_step, w_row, rawfull + s * 8);
+#pragma unroll
+          for (uint32_t part = 0; part < kParts; ++part)
+            copy_tile_3d(leader, a_tile + kATile + part * b_bytes, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), m0 + cta_rank * half_rows, part,
+                         full_0 + s * 8);
+          if (++s == p.stages) { s = 0; phase ^= 1u; }
+        }
+      }
+      __syncwarp();
+    } else if (warp == kMmaWarp && cta_rank == 0) {
+      // ---------------- MMA issuer: one thread, nothing converges in its loop ----------------
+      {
+        const uint32_t idesc = exact_idesc<kMath>(p.nt);
+        const uint32_t b_step = (p.nt / 2 * 128u) >> 4, stage_step = p.stage_bytes >> 4;
+        const uint32_t desc_a0 = static_cast<uint32_t>(umma_desc(tiles)), desc_b0 = static_cast<uint32_t>(umma_desc(tiles + kATile));
+        // kSlices: k16 slices per accumulator chain when chains end inside a k-step or with it; 0: longer
+        // chains, of p.drain16 slices.  A barrier test takes the thread some 230 clocks even when the
+        // barrier is long complete, so the next stage's is asked for before this stage's MMAs are issued
+        // and its answer read after them.
+        auto issue = [&](auto slices) {
+          constexpr uint32_t kSlices = decltype(slices)::value;
+          uint32_t s = 0, phase = 0, d = 0, in_chain = 0;
+          bool ready = mbar_try_wait(full, 0);
+          for (uint32_t ks = 0; ks < ks_count; ++ks) {
+            if (!ready && !wait_bounded(full + s * 8, phase, abort_flag, p.status, 22)) return;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t desc_a = desc_a0 + s * stage_step, desc_b = desc_b0 + s * stage_step, this_empty = empty + s * 8;
+            if (++s == p.stages) { s = 0; phase ^= 1u; }
+            ready = mbar_try_wait(full + s * 8, phase);  // (past the last k-step: an answer nobody reads)
+#pragma unroll
+            for (uint32_t kk = 0; kk < 4; ++kk) {
+              const bool starts = kSlices != 0 ? kk % (kSlices == 0 ? 1u : kSlices) == 0 : kk == 0 && in_chain == 0;
+              if (kMath != kInt8 && starts && d > acc_mask) {  // both CTAs have read the accumulator's previous sums
+                if (!wait_bounded(dempty + (d & acc_mask) * 8, ((d >> acc_shift) - 1u) & 1u, abort_flag, p.status, 24)) return;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              }
+              const uint32_t dst = tmem + (d & acc_mask) * acc_cols;
+              if (starts) mma_pair<kMath, false>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
+              else mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
+              if constexpr (kParts == 2) mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + b_step + kk * 2u, idesc);
+              if (kMath != kInt8 && kSlices != 0 && (kk + 1) % (kSlices == 0 ? 1u : kSlices) == 0) {
+                commit_both(leader, dfull + (d & acc_mask) * 8);
+                ++d;
+              }
+            }
+            if constexpr (kSlices == 0) {
+              in_chain += 4;
+              if (kMath != kInt8 && in_chain == p.drain16) {
+                commit_both(leader, dfull + (d & acc_mask) * 8);
+                ++d;
+                in_chain = 0;
+              }
+            }
+            commit_both(leader, this_empty);  // the stage is free, in both CTAs, once these MMAs have read it
+          }
+          if (kSlices == 0 && in_chain != 0) commit_both(leader, dfull + (d & acc_mask) * 8);  // a last, short chain
+        };
+        if (kGroupScales && p.drain16 == 1) issue(std::integral_constant<uint32_t, 1>{});
+        else if (kGroupScales && p.drain16 == 2) issue(std::integral_constant<uint32_t, 2>{});
+        else if (kGroupScales && p.drain16 == 4) issue(std::integral_constant<uint32_t, 4>{});
+        else issue(std::integral_constant<uint32_t, 0>{});
+      }
+      __syncwarp();
+    } else if (kGroupScales && warp >= kScaleWarp) {
+      // ---------------- scales: global memory -> f32 ring, eight accumulator chains at a time ----------------
+      const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16, drain0 = ks_begin * 4 / p.drain16;
+      const uint32_t each = p.scale_f16 ? 2u : 4u;
+      const ExTarget tg = p.t[wi];
+      for (uint32_t d0 = 0, batch = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
+        if (batch >= 2) wait_bounded(sempty + (batch & 1u) * 8, ((batch >> 1) - 1u) & 1u, abort_flag, p.status, 26);
+#pragma unroll 1
+        for (uint32_t rr = 0; rr < 2; ++rr) {
+          const uint32_t r = (warp - kScaleWarp) * 64u + rr * 32u + lane, row = n0 + r;
+          const uint8_t* base;
+          if constexpr (kW == kI4Tiled)
+            base = tg.w + static_cast<size_t>(row >> 4) * (p.k / kChunkK) * raw_unit_bytes<kW, kMath>(p.scale_f16) + kChunkWeightBytes +
+                   ((row & 7u) * 4u + ((row >> 3) & 1u)) * each;
+          else
+            base = static_cast<const uint8_t*>(tg.scale) + static_cast<size_t>(row) * p.groups * each;
+          float v[kScaleBatch];
+#pragma unroll
+          for (uint32_t i = 0; i < kScaleBatch; ++i) {
+            const uint32_t grp = (drain0 + d0 + i) >> p.drains_per_group_shift;
+            v[i] = 0.0f;
+            if (row < tg.n && grp < p.groups && d0 + i < drains) {
+              const uint8_t* a = kW == kI4Tiled ? base + static_cast<size_t>(grp >> 1) * raw_unit_bytes<kW, kMath>(p.scale_f16) + (grp & 1u) * 2u * each
+                                                : base + static_cast<size_t>(grp) * each;
+              v[i] = p.scale_f16 ? __half2float(*reinterpret_cast<const __half*>(a)) : *reinterpret_cast<const float*>(a);
+            }
+          }
+#pragma unroll
+          for (uint32_t i = 0; i < kScaleBatch; ++i) scale_ring[((batch & 1u) * kScaleBatch + i) * kRows + r] = v[i];
+        }
+        __syncwarp();
+        arrive_if(leader, sfull + (batch & 1u) * 8);
+      }
+    }
+  }
+
+  if (*abort_flag)  // a wait gave up: copies may still be in flight towards this CTA's shared memory
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  cluster_sync_all();  // neither CTA leaves, or frees tensor memory, while the other still works
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// ---- activations -> binary16 parts -----------------------------------------------------------
+// One CTA per row.  [rms_norm ->] power-of-two pre-scale of the whole row (pow2_prescale) -> hi = RN_f16(v),
+// lo = RN_f16(v - hi); inv[row] = 2^-e undoes the scale in the epilogue.  A row is read once from
+// memory and again from the cache.
+template <typename XT>
+__global__ void __launch_bounds__(256)
+split_half_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, __half* __restrict__ parts, float* __restrict__ inv,
+                  const float* __restrict__ norm_weight, float norm_eps) {
+  const uint32_t row = blockIdx.x;
+  const XT* xr = x + static_cast<size_t>(row) * k;
+  __shared__ float part[8];
+  pdl_wait_prior_grid();
+  float r_inv = 1.0f;
+  if (norm_weight != nullptr) {
+    // sum of squares in a fixed order: thread-strided, shuffle tree, warps in order
+    float sq = 0.0f;
+    for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
+      float v[8];
+      load_x8<XT>(xr + i, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sq = fmaf(v[e], v[e], sq);
+    }
+    sq = warp_sum(sq);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    float total = 0.0f;
+    for (int w = 0; w < 8; ++w) total += part[w];
+    r_inv = rsqrtf(total * (1.0f / static_cast<float>(k)) + norm_eps);
+    __syncthreads();
+  }
+  auto load = [&](uint32_t i, float (&v)[8]) {
+    load_x8<XT>(xr + i, v);
+    if (norm_weight != nullptr) {
+      const float4 w0 = __ldg(reinterpret_cast<const float4*>(norm_weight + i)), w1 = __ldg(reinterpret_cast<const float4*>(norm_weight + i + 4));
+      const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = __fmul_rn(__fmul_rn(v[e], r_inv), wv[e]);
+    }
+  };
+  float amax = 0.0f;
+  for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {  // k is a multiple of 16
+    float v[8];
+    load(i, v);
+    amax = fmaxf(amax, absmax8(v));
+  }
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
+  if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = part[0];
+  for (int w = 1; w < 8; ++w) amax = fmaxf(amax, part[w]);
+  const Pow2 ps = pow2_prescale(amax);
+  if (threadIdx.x == 0) inv[row] = ps.inv;
+  __half* hi = parts + static_cast<size_t>(row) * k;
+  __half* lo = hi + static_cast<size_t>(m) * k;
+  for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
+    float v[8];
+    load(i, v);
+    uint4 oh, ol;
+    uint32_t* ph = reinterpret_cast<uint32_t*>(&oh);
+    uint32_t* pl = reinterpret_cast<uint32_t*>(&ol);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float a = v[2 * j] * ps.scale, b = v[2 * j + 1] * ps.scale;
+      const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
+      ph[j] = pack_half2(ha, hb);
+      pl[j] = pack_half2(__float2half_rn(a - __half2float(ha)), __float2half_rn(b - __half2float(hb)));
+    }
+    *reinterpret_cast<uint4*>(hi + i) = oh;
+    *reinterpret_cast<uint4*>(lo + i) = ol;
+  }
+  pdl_launch_dependents();
+}
+
+// int8 activations -> binary16 (exact), 16 values per thread
+__global__ void __launch_bounds__(256)
+bytes_to_half_kernel(const int8_t* __restrict__ q, uint64_t sixteens, __half* __restrict__ out) {
+  pdl_wait_prior_grid();
+  for (uint64_t i = blockIdx.x * 256ull + threadIdx.x; i < sixteens; i += static_cast<uint64_t>(gridDim.x) * 256ull) {
+    const uint4 v = reinterpret_cast<const uint4*>(q)[i];
+    const uint2 a = bytes_to_half(v.x ^ 0x80808080u), b = bytes_to_half(v.y ^ 0x80808080u);
+    const uint2 c = bytes_to_half(v.z ^ 0x80808080u), d = bytes_to_half(v.w ^ 0x80808080u);
+    reinterpret_cast<uint4*>(out)[2 * i] = make_uint4(a.x, a.y, b.x, b.y);
+    reinterpret_cast<uint4*>(out)[2 * i + 1] = make_uint4(c.x, c.y, d.x, d.y);
+  }
+  pdl_launch_dependents();
+}
+
+// The K slices of a split launch, added in ascending order, then the epilogue.
+struct ExReduceParams {
+  ExTarget t[kMaxMulti];
+  uint32_t count, m, n_total, splits, scale_f16, per_channel;
+  const float* row_scale;
+  const void* partial;
+};
+template <bool kInt8Sums>
+__global__ void __launch_bounds__(256) exact_reduce_kernel(const ExReduceParams p) {
+  pdl_wait_prior_grid();
+  pdl_launch_dependents();
+  const size_t slice = static_cast<size_t>(p.m) * p.n_total;
+  for (size_t i = blockIdx.x * static_cast<size_t>(256) + threadIdx.x; i < slice; i += static_cast<size_t>(gridDim.x) * 256) {
+    const uint32_t mm = static_cast<uint32_t>(i / p.n_total);
+    uint32_t col = static_cast<uint32_t>(i - static_cast<size_t>(mm) * p.n_total);
+    uint32_t wi = 0;
+#pragma unroll
+    for (int j = 1; j < kMaxMulti; ++j)
+      if (j < static_cast<int>(p.count) && wi + 1 == static_cast<uint32_t>(j) && col >= p.t[j - 1].n) { col -= p.t[j - 1].n; wi = j; }
+    const ExTarget& tg = p.t[wi];
+    const float rs = p.row_scale != nullptr ? p.row_scale[mm] : 1.0f;
+    float o;
+    if constexpr (kInt8Sums) {
+      const int* src = static_cast<const int*>(p.partial) + i;
+      int acc = 0;
+      for (uint32_t z = 0; z < p.splits; ++z) acc += src[z * slice];
+      o = fmaf(__int2float_rn(acc), __fmul_rn(rs, load_scale_dyn(tg.scale, col, p.scale_f16)), tg.bias[col]);
+    } else {
+      const float* src = static_cast<const float*>(p.partial) + i;
+      float acc = 0.0f;
+      for (uint32_t z = 0; z < p.splits; ++z) acc += src[z * slice];
+      if (p.per_channel) acc *= load_scale_dyn(tg.scale, col, p.scale_f16);
+      o = fmaf(acc, rs, tg.bias[col]);
+    }
+    const size_t at = static_cast<size_t>(mm) * tg.n + col;
+    if (tg.residual != nullptr) o = __fadd_rn(o, tg.residual[at]);
+    tg.out[at] = o;
+  }
+}
+
+// ---- host ---------------------------------------------------------------------------------------
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled tensor_map_encoder() {
+  static EncodeTiled encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<EncodeTiled>(fn);
+  }();
+  return encode;
+}
+
+// Activations [parts][m][k] (binary16 or int8), box 128 bytes x `rows` rows, 128-byte swizzle; what lies
+// past k or m reads as zero.
+cudaError_t encode_x_map(const void* x, bool int8, uint32_t m, uint32_t k, uint32_t parts, uint32_t rows, CUtensorMap* map) {
+  EncodeTiled encode = tensor_map_encoder();
+  if (encode == nullptr) return cudaErrorNotSupported;
+  const cuuint64_t each = int8 ? 1 : 2;
+  const cuuint64_t dims[3] = {k, m, parts}, strides[2] = {k * each, static_cast<cuuint64_t>(m) * k * each};
+  const cuuint32_t box[3] = {int8 ? 128u : 64u, rows, 1}, ones[3] = {1, 1, 1};
+  const CUresult r = encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims,
+                            strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+// The packed weights as rows of bytes, one copy per k-step and CTA: rows layouts [n][row_bytes], box
+// `bytes` x 128 rows (128-byte swizzled when it is the MMA's tile itself); tiled layouts [n / 16][row_bytes]
+// of 16-row blocks, box `bytes` x 8.  `elem` bytes per element keep the box within 256 elements.
+cudaError_t encode_w_map(const void* w, uint32_t rows, uint64_t row_bytes, uint32_t bytes, uint32_t elem, uint32_t box_rows, bool swizzle,
+                         CUtensorMap* map) {
+  EncodeTiled encode = tensor_map_encoder();
+  if (encode == nullptr) return cudaErrorNotSupported;
+  const cuuint64_t dims[2] = {row_bytes / elem, rows}, strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {bytes / elem, box_rows}, ones[2] = {1, 1};
+  const CUtensorMapDataType type = elem == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT64;
+  const CUresult r = encode(map, type, 2, const_cast<void*>(w), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <typename Kernel, typename... Args>
+cudaError_t launch_dependent(Kernel kernel, dim3 grid, uint32_t threads, size_t smem, uint32_t cluster, const LaunchEnv& env, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = env.stream;
+  cudaLaunchAttribute attr[2];
+  unsigned int na = 0;
+  if (env.overlap) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  if (cluster > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = cluster;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+WeightKind kind_of(const Weight& w) {
+  if (w.layout == kLayoutTiledI4) return kI4Tiled;
+  if (w.layout == kLayoutTiledI8) return kI8Tiled;
+  return w.storage == KQ_STORAGE_I4 ? kI4Rows : kI8Rows;
+}
+// The packed rows of the untiled layouts are read through a tensor map: 16-byte row strides.
+bool kind_ok(const Weight& w) {
+  switch (kind_of(w)) {
+    case kI4Tiled: return true;
+    case kI8Tiled: return w.k % 16 == 0;
+    case kI4Rows: return w.k % 32 == 0;
+    default: return w.k % 16 == 0;
+  }
+}
+
+template <int kW, int kMath>
+cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, uint32_t pairs, uint32_t m_tiles, const CUtensorMap& xm,
+                        const CUtensorMap (&wm)[kMaxMulti]) {
+  auto kernel = qgemm_exact_kernel<kW, kMath>;
+  static PerDevice<bool> configured_on;
+  bool* configured = configured_on.slot();
+  if (configured == nullptr) return cudaErrorInvalidDevice;
+  if (!*configured) {
+    // the register split adds up to 512 x 128: refuse to run a build whose launch holds fewer
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    if (fa.numRegs < 128) return cudaErrorInvalidKernelImage;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
+    if (e != cudaSuccess) return e;
+    *configured = true;
+  }
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + kSmemTail;
+  return launch_dependent(kernel, dim3(pairs * 2, m_tiles, p.splits), kExThreads, smem, 2, env, p, xm, wm[0], wm[1], wm[2], wm[3]);
+}
+
+template <int kW>
+cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, uint32_t pairs, uint32_t m_tiles, const CUtensorMap& xm,
+                        const CUtensorMap (&wm)[kMaxMulti]) {
+  if (math == kHalf1) return launch_main<kW, kHalf1>(env, p, pairs, m_tiles, xm, wm);
+  if (math == kHalf2) return launch_main<kW, kHalf2>(env, p, pairs, m_tiles, xm, wm);
+  if constexpr (kW == kI8Tiled || kW == kI8Rows) return launch_main<kW, kInt8>(env, p, pairs, m_tiles, xm, wm);
+  return cudaErrorInvalidValue;
+}
+
+// Clocks of one k-step of a tile of `nt` activation rows, as measured (full machine, one tile per pair):
+// the slowest of the tensor core, the thread that issues (100 an MMA, 350 a chain's barrier), the
+// drain (300 and two a column a chain) and the conversion of the weight tile.
+uint32_t kstep_clocks(uint32_t nt, uint32_t parts, uint32_t drains_x4, bool int8) {
+  const uint32_t mma = 4 * parts * std::max(nt / 2, 48u);
+  const uint32_t thread = 400 + 400 * parts + (int8 ? 0u : drains_x4 * 350 / 4);
+  const uint32_t drain = int8 ? 0u : drains_x4 * (nt * 2 + 300) / 4;
+  return std::max({mma, thread, drain, 500u});
+}
+
+struct Geometry { uint32_t nt, m_tiles, splits; };
+// Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
+// loads, epilogue) plus its k-steps; a split adds the reduce launch and the partial sums' traffic.
+Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t ksteps, uint32_t parts, uint32_t drain16, bool int8,
+                         uint32_t slice_unit, bool may_split, uint32_t sm_pairs, uint64_t partial_room) {
+  Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1};
+  uint64_t best_cost = ~0ull;
+  const uint32_t drains_x4 = std::max(1u, 16 / drain16);  // accumulator chains per k-step, times four
+  const uint32_t most = (m + 31) / 32;
+  for (uint32_t mt = (m + kMaxNT - 1) / kMaxNT; mt <= most; ++mt) {
+    uint32_t nt = ((m + mt - 1) / mt + 31) / 32 * 32;
+    if (nt > 128) nt = (nt + 63) / 64 * 64;
+    if ((m + nt - 1) / nt != mt) continue;
+    const uint32_t per = kstep_clocks(nt, parts, drains_x4, int8);
+    for (uint32_t splits = 1; splits <= (may_split ? 16u : 1u); splits *= 2) {
+      if (splits > 1 && (ksteps / splits < 4 || static_cast<uint64_t>(splits) * m * n_total * 4 > partial_room)) break;
+      uint32_t each = (ksteps + splits - 1) / splits;
+      each = (each + slice_unit - 1) / slice_unit * slice_unit;
+      const uint64_t waves = (static_cast<uint64_t>(pairs) * mt * splits + sm_pairs - 1) / sm_pairs;
+      uint64_t cost = waves * (5000 + nt * 30 + static_cast<uint64_t>(each) * per);
+      if (splits > 1) cost += 4000 + static_cast<uint64_t>(m) * n_total * (splits + 1) * 4 / 4000;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {nt, mt, splits};
+      }
+    }
+    if (mt >= 8 * sm_pairs) break;
+  }
+  return best;
+}
+
+// x: binary16 (kHalf1, `x` used in place), parts already split (kHalf1 / kHalf2) or int8 (kInt8).
+cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const float* residual, const void* x, int math,
+                      uint32_t m, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, int* launches) {
+  const Weight& w0 = *targets[0].w;
+  const WeightKind kind = kind_of(w0);
+  ExParams p = {};
+  ExReduceParams rp = {};
+  CUtensorMap xm, wm[kMaxMulti] = {};
+  const bool int8 = math == kInt8;
+  uint32_t pairs = 0, n_total = 0;
+  uint32_t used = 0;
+  const uint32_t unit = kind == kI4Tiled ? raw_unit_bytes<kI4Tiled, kHalf1>(w0.scale_dtype == KQ_F16)
+                        : kind == kI4Rows ? 32u
+                        : kind == kI8Tiled ? (int8 ? 2048u : 1024u) : (int8 ? 128u : 64u);
+  const bool tiled = kind == kI4Tiled || kind == kI8Tiled;
+  const uint32_t elem = !tiled ? 1u : unit > 1024 ? 8u : 4u;
+  for (int i = 0; i < count; ++i) {
+    const Weight& w = *targets[i].w;
+    if (w.n == 0) continue;
+    p.t[used] = ExTarget{static_cast<const uint8_t*>(w.data), w.scale, targets[i].bias, targets[i].out, residual, w.n, pairs};
+    const uint64_t row_bytes = kind == kI4Tiled ? static_cast<uint64_t>(w.k / kChunkK) * unit
+                               : kind == kI8Tiled ? static_cast<uint64_t>(w.k) * 16 : kind == kI4Rows ? w.k / 2 : w.k;
+    cudaError_t e = tiled ? encode_w_map(w.data, w.n / 16, row_bytes, unit, elem, 8, false, &wm[used])
+                          : encode_w_map(w.data, w.n, row_bytes, unit, elem, kRows, kind == kI8Rows && int8, &wm[used]);
+    if (e != cudaSuccess) return e;
+    pairs += (w.n + 2 * kRows - 1) / (2 * kRows);
+    n_total += w.n;
+    ++used;
+  }
+  if (used == 0) return cudaSuccess;
+  p.count = used;
+  p.m = m;
+  p.k = w0.k;
+  const uint32_t step_k = int8 ? 128 : 64;
+  p.ksteps = (w0.k + step_k - 1) / step_k;
+  p.scale_f16 = w0.scale_dtype == KQ_F16;
+  const bool i4 = kind == kI4Tiled || kind == kI4Rows;
+  const uint32_t group = i4 ? w0.group_size : kMaxChain;
+  const uint32_t chain = std::min(group, kMaxChain);
+  p.drain16 = chain / 16;
+  p.drains_per_group_shift = 0;
+  while ((chain << p.drains_per_group_shift) < group) ++p.drains_per_group_shift;
+  p.groups = i4 ? w0.k / w0.group_size : ~0u;
+  p.row_scale = row_scale;
+  p.n_total = n_total;
+  p.status = env.status;
+  p.partial = static_cast<float*>(scratch);
+  const uint32_t parts = math == kHalf2 ? 2 : 1;
+  // a K slice is a whole number of int4 accumulator chains (an int8 chain may end anywhere)
+  const uint32_t align = i4 && p.drain16 > 4 ? p.drain16 / 4 : 1;
+  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, parts, p.drain16, int8, align, may_split && scratch != nullptr,
+                                       std::max(1, env.sm_count / 2), scratch_bytes);
+  p.nt = geo.nt;
+  p.ksteps_per_split = ((p.ksteps + geo.splits - 1) / geo.splits + align - 1) / align * align;
+  p.splits = (p.ksteps + p.ksteps_per_split - 1) / p.ksteps_per_split;
+  // stage: weight tile, activation parts, raw weights
+  p.raw_bytes = (tiled ? 8 : kRows) * unit;
+  p.raw_box = unit / elem;
+  const uint32_t raw_bytes = kind == kI8Rows && int8 ? 0 : p.raw_bytes;  // straight into the weight tile
+  p.raw_off = kATile + parts * p.nt / 2 * 128;
+  p.stage_bytes = (p.raw_off + raw_bytes + 1023) / 1024 * 1024;
+  p.stages = std::min<uint32_t>(kMaxStages, (kSmemLimit - 1024 - kSmemTail) / p.stage_bytes);
+  cudaError_t e = encode_x_map(x, int8, m, w0.k, parts, p.nt / 2, &xm);
+  if (e != cudaSuccess) return e;
+  switch (kind) {
+    case kI4Tiled: e = launch_math<kI4Tiled>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
+    case kI4Rows: e = launch_math<kI4Rows>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
+    case kI8Tiled: e = launch_math<kI8Tiled>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
+    default: e = launch_math<kI8Rows>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
+  }
+  if (e != cudaSuccess) return e;
+  if (launches) *launches += 1;
+  if (p.splits > 1) {
+    for (uint32_t i = 0; i < used; ++i) rp.t[i] = p.t[i];
+    rp.count = used;
+    rp.m = m;
+    rp.n_total = n_total;
+    rp.splits = p.splits;
+    rp.scale_f16 = p.scale_f16;
+    rp.per_channel = i4 ? 0u : 1u;
+    rp.row_scale = row_scale;
+    rp.partial = scratch;
+    const uint64_t outs = static_cast<uint64_t>(m) * n_total;
+    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>((outs + 255) / 256, static_cast<uint64_t>(env.sm_count) * 8));
+    e = int8 ? launch_dependent(exact_reduce_kernel<true>, dim3(grid), 256, 0, 1, env, rp)
+             : launch_dependent(exact_reduce_kernel<false>, dim3(grid), 256, 0, 1, env, rp);
+    if (e != cudaSuccess) return e;
+    if (launches) *launches += 1;
+  }
+  return cudaSuccess;
+}
+
+uint64_t align256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
+
+}  // namespace
+
+bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, uint64_t workspace_bytes) {
+  if (count < 1 || count > kMaxMulti || m <= 16) return false;
+  const Weight& w0 = *targets[0].w;
+  for (int i = 0; i < count; ++i) {
+    const Weight& w = *targets[i].w;
+    if (w.layout != w0.layout || w.storage != w0.storage || w.k != w0.k || w.group_size != w0.group_size ||
+        w.scale_dtype != w0.scale_dtype || w.k == 0 || !kind_ok(w))
+      return false;
+  }
+  // one row panel of 32 rows of split activations has to fit the scratch
+  return align256(static_cast<uint64_t>(w0.k) * 4 * 32) + 256 <= workspace_bytes;
+}
+
+cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,
+                               int* launches) {
+  const Weight& w0 = *targets[0].w;
+  const uint32_t k = w0.k;
+  const bool direct = x_dtype == KQ_F16 && env.norm_weight == nullptr;  // binary16 rows are the operand
+  uint8_t* ws = static_cast<uint8_t*>(env.workspace);
+  const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
+  // row panels whose split activations take at most half of the scratch (the rest: partial sums)
+  const uint64_t per_row = static_cast<uint64_t>(k) * 4 + 4;
+  uint32_t panel = m;
+  if (!direct && per_row * m > room / 2) {
+    panel = static_cast<uint32_t>(std::min<uint64_t>(m, std::max<uint64_t>(32, room / 2 / per_row)));
+    if (panel >= 256) panel = panel / 256 * 256;
+  }
+  for (uint32_t r0 = 0; r0 < m; r0 += panel) {
+    const uint32_t pm = std::min(panel, m - r0);
+    LinearTarget t[kMaxMulti];
+    for (int i = 0; i < count; ++i)
+      t[i] = LinearTarget{targets[i].w, targets[i].bias, targets[i].out + static_cast<size_t>(r0) * targets[i].w->n};
+    const float* residual = env.residual != nullptr ? env.residual + static_cast<size_t>(r0) * w0.n : nullptr;
+    const uint32_t xb = x_dtype == KQ_F32 ? 4 : 2;
+    const uint8_t* xp = static_cast<const uint8_t*>(x) + static_cast<size_t>(r0) * k * xb;
+    cudaError_t e;
+    if (direct) {
+      e = run_exact(env, count, t, residual, xp, kHalf1, pm, nullptr, ws, room, true, launches);
+    } else {
+      float* inv = reinterpret_cast<float*>(ws);
+      __half* parts = reinterpret_cast<__half*>(ws + align256(static_cast<uint64_t>(pm) * 4));
+      const uint64_t taken = align256(static_cast<uint64_t>(pm) * 4) + align256(static_cast<uint64_t>(pm) * k * 4);
+      if (taken > room) return cudaErrorMemoryAllocation;
+      if (x_dtype == KQ_F32)
+        e = launch_dependent(split_half_kernel<float>, dim3(pm), 256, 0, 1, env, reinterpret_cast<const float*>(xp), pm, k, parts, inv,
+                             env.norm_weight, env.norm_eps);
+      else if (x_dtype == KQ_F16)
+        e = launch_dependent(split_half_kernel<__half>, dim3(pm), 256, 0, 1, env, reinterpret_cast<const __half*>(xp), pm, k, parts, inv,
+                             env.norm_weight, env.norm_eps);
+      else
+        e = launch_dependent(split_half_kernel<__nv_bfloat16>, dim3(pm), 256, 0, 1, env, reinterpret_cast<const __nv_bfloat16*>(xp), pm, k,
+                             parts, inv, env.norm_weight, env.norm_eps);
+      if (e != cudaSuccess) return e;
+      if (launches) *launches += 1;
+      e = run_exact(env, count, t, residual, parts, kHalf2, pm, inv, ws + taken, room - taken, true, launches);
+    }
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// Integer-dot form: int8 activations xq [m, k] with row scales xs.
+bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes) {
+  if (m <= 16 || w.k == 0 || !kind_ok(w) || w.k % 16 != 0 || (reinterpret_cast<uintptr_t>(xq) & 15u) != 0) return false;
+  if (w.storage == KQ_STORAGE_I8) return true;
+  return w.group_size <= kMaxChain && align256(static_cast<uint64_t>(w.k) * 2 * 32) <= workspace_bytes;
+}
+
+cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& target, const int8_t* xq, const float* xs, uint32_t m,
+                                  int* launches) {
+  const Weight& w = *target.w;
+  uint8_t* ws = static_cast<uint8_t*>(env.workspace);
+  const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
+  if (w.storage == KQ_STORAGE_I8) return run_exact(env, 1, &target, nullptr, xq, kInt8, m, xs, ws, room, true, launches);
+  // int4: per-group sums as binary16 products (exact), flushed in ascending order: no K slices
+  const uint64_t per_row = static_cast<uint64_t>(w.k) * 2;
+  uint32_t panel = static_cast<uint32_t>(std::min<uint64_t>(m, room / per_row));
+  if (panel < m && panel >= 256) panel = panel / 256 * 256;
+  if (panel == 0) return cudaErrorMemoryAllocation;
+  for (uint32_t r0 = 0; r0 < m; r0 += panel) {
+    const uint32_t pm = std::min(panel, m - r0);
+    const uint64_t sixteens = static_cast<uint64_t>(pm) * w.k / 16;
+    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>((sixteens + 255) / 256, static_cast<uint64_t>(env.sm_count) * 16));
+    cudaError_t e = launch_dependent(bytes_to_half_kernel, dim3(grid), 256, 0, 1, env, xq + static_cast<size_t>(r0) * w.k, sixteens,
+                                     reinterpret_cast<__half*>(ws));
+    if (e != cudaSuccess) return e;
+    if (launches) *launches += 1;
+    const LinearTarget t{target.w, target.bias, target.out + static_cast<size_t>(r0) * w.n};
+    e = run_exact(env, 1, &t, nullptr, ws, kHalf1, pm, xs + r0, nullptr, 0, false, launches);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace kq

@@ -517,13 +517,12 @@ __device__ __forceinline__ void qgemm_body(const GemmParams& p, const CUtensorMa
     for (uint32_t f = 0; f < frag_count; ++f) {
     select_fragment(f);
     if (f != 0) {  // both CTAs have read the previous fragment's sums out of TMEM
-      wait_bounded_cluster(tmem_free, (f - 1u) & 1u, abort_flag, p.status, 7);
+      wait_bounded(tmem_free, (f - 1u) & 1u, abort_flag, p.status, 7);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     for (uint32_t ks = 0; ks < ksteps; ++ks) {
       const uint32_t it = it_base + ks, s = it % kStagesG, phase = (it / kStagesG) & 1u;
-      const bool ok = kPair ? wait_bounded_cluster(bars + s * 8, phase, abort_flag, p.status, 2)
-                            : wait_bounded(bars + s * 8, phase, abort_flag, p.status, 2);
+      const bool ok = wait_bounded(bars + s * 8, phase, abort_flag, p.status, 2);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (lane == 0) {
         const uint32_t a_tile = tiles + s * kStageBytes, b_tile = a_tile + kATileBytes;

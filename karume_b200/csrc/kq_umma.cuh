@@ -1,4 +1,4 @@
-// Helpers shared by the tcgen05 GEMM kernels (kq_qgemm_i4.cu, kq_qgemm_i4_x32.cu): mbarriers with
+// Helpers shared by the tcgen05 GEMM kernels (kq_qgemm_i4.cu, kq_qgemm_exact.cu): mbarriers with
 // bounded waits, shared-memory matrix descriptors for the K-major 128-byte-swizzled layout, the
 // kind::f16 MMA with bf16 operands, and the swizzled tile addressing.
 #pragma once
@@ -77,26 +77,12 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
+// Arrives on a barrier of either CTA of the pair.  What such an arrival hands over is read by the
+// tensor core (a tile behind fence.proxy.async, an accumulator behind tcgen05.fence), never by a
+// load of the other CTA's threads, so the default CTA-scope release is enough; a cluster-scope one
+// waits for the thread's whole memory traffic (500 - 1500 clocks per arrival beside running copies).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done != 0;
-}
-// wait_bounded for a barrier that threads of the peer CTA arrive on
-__device__ __forceinline__ bool wait_bounded_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                                     int code) {
-  for (uint32_t spins = 0; spins < kWaitLimit; ++spins) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((spins & 1023u) == 1023u && *abort_flag) return false;
-  }
-  *abort_flag = 1;
-  *reinterpret_cast<volatile int*>(status) = code;
-  return false;
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // M 256 (128 rows per CTA) x N: A and D are each CTA's own rows, B is read half from each CTA.
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,

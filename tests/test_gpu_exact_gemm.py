@@ -1,0 +1,114 @@
+"""The many-row linear with weights as exact integers (kq_qgemm_exact.cu): every packed layout,
+activation type and accumulator-chain length at the edges of its tiles, against the f64 oracle;
+the integer-dot form bit for bit."""
+import numpy as np
+import pytest
+
+import oracle
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    import karume_b200 as kb
+    g = kb.acquire_gpu(0)
+    yield g
+    g.destroy()
+
+
+def dev(a):
+    import torch
+    t = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    torch.cuda.synchronize()
+    return t
+
+
+# (storage, group, m, n, k): one and several row tiles, ragged rows and channels, k tails of half a
+# k-step, groups of one k16 slice up to longer than an accumulator chain, K slices
+SHAPES = [("i4", 32, 17, 16, 64), ("i4", 32, 257, 272, 512), ("i4", 32, 40, 130, 96), ("i4", 16, 65, 304, 1152),
+          ("i4", 64, 33, 250, 320), ("i4", 128, 300, 512, 4096), ("i4", 2048, 18, 144, 4096), ("i8", 0, 40, 64, 96),
+          ("i8", 0, 257, 512, 1536), ("i8", 0, 66, 131, 80), ("i8", 0, 600, 784, 4096)]
+
+
+@pytest.mark.parametrize("xdt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("storage,group,m,n,k", SHAPES)
+def test_matches_the_f64_oracle(gpu, xdt, storage, group, m, n, k):
+    import torch
+    if xdt == "bf16" and n % 16 == 0 and k % 64 == 0 and group in (0, 32):
+        pytest.skip("the bf16 GEMM's case")
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[m // 2] *= np.float32(1e30) if xdt != "f16" else np.float32(1e3)  # a row of another magnitude
+    x[m - 1] *= np.float32(1e-30) if xdt != "f16" else np.float32(1e-3)
+    x = {"f32": lambda v: v, "f16": oracle.round_to_f16, "bf16": oracle.round_to_bf16}[xdt](x)
+    bias = rng.standard_normal(n).astype(np.float32)
+    bias[n // 2:] = 0.0
+    if storage == "i4":
+        data, scale = cases.synth_i4(n, k, seed=n, group_size=group, scale_dtype="f32" if m % 2 else "f16")
+        ref = oracle.linear_i4(x, data, scale.astype(np.float32), bias, n, k, group)
+    else:
+        data, scale = cases.synth_i8(n, k, seed=n)
+        ref = oracle.linear_i8(x, data, scale.astype(np.float32), bias, n, k)
+    w = gpu.upload_weight(storage, data, scale, (n, k), group)
+    xd = dev(x).to({"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[xdt])
+    out = torch.full((m, n), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    gpu.linear(xd, w, dev(bias), out=out)
+    gpu.sync()
+    got = out.cpu().numpy()
+    for rows in (slice(m // 2, m // 2 + 1), slice(m - 1, m), np.setdiff1d(np.arange(m), [m // 2, m - 1])):
+        rms = float(np.sqrt(np.mean(ref[rows].astype(np.float64) ** 2)))
+        rep = oracle.allclose(got[rows], ref[rows], atol=1e-5 * max(1.0, rms), rtol=1e-4)
+        assert rep["pass"], rep
+    again = gpu.linear(xd, w, dev(bias))
+    gpu.sync()
+    assert torch.equal(out, again)
+    w.free()
+
+
+@pytest.mark.parametrize("storage,group,m,n,k", [s for s in SHAPES if s[1] <= 1024] + [("i4", 16, 129, 67, 48), ("i8", 0, 300, 528, 8960)])
+def test_integer_dot_is_bit_exact(gpu, storage, group, m, n, k):
+    rng = np.random.default_rng(m)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    if storage == "i4":
+        data, scale = cases.synth_i4(n, k, seed=n, group_size=group, scale_dtype="f32" if m % 2 else "f16")
+        u = np.stack([data & 15, data >> 4], axis=1).reshape(n, k).astype(np.int16) - 8
+        want = oracle.linear_w4a8(x, u.astype(np.int8), scale.astype(np.float32), bias, group)
+    else:
+        data, scale = cases.synth_i8(n, k, seed=n)
+        want = oracle.linear_w8a8(x, data, scale.astype(np.float32), bias)
+    w = gpu.upload_weight(storage, data, scale, (n, k), group)
+    xq, xs = gpu.quantize_rows(dev(x))
+    out = gpu.linear_a8(xq, xs, w, dev(bias))
+    gpu.sync()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), np.asarray(want, np.float32).view(np.uint32))
+    w.free()
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 64, 128), (130, 544, 1536)])
+def test_norm_gate_and_residual_around_it(gpu, m, n, k):
+    import torch
+    rng = np.random.default_rng(k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    g = (1 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    ws, refs = [], []
+    xn = oracle.rms_norm(x, g, 1e-5)
+    zero = np.zeros(n, np.float32)
+    for s in (1, 2):
+        data, scale = cases.synth_i4(n, k, seed=s)
+        ws.append(gpu.upload_weight("i4", data, scale, (n, k), 32))
+        refs.append(oracle.linear_i4(xn, data, scale.astype(np.float32), zero, n, k, 32))
+    bias = dev(zero)
+    res = rng.standard_normal((m, n)).astype(np.float32)
+    (act,) = gpu.linear_fused(dev(x), ws, [bias, bias], norm_weight=dev(g), eps=1e-5, swiglu=True)
+    (added,) = gpu.linear_fused(dev(x), ws[:1], [bias], norm_weight=dev(g), eps=1e-5, residual=dev(res))
+    both = gpu.linear_multi(dev(xn), ws, [bias, bias])
+    gpu.sync()
+    for got, want in ((act, oracle.silu_mul(refs[0], refs[1])), (added, oracle.add(refs[0], res)), (both[0], refs[0]), (both[1], refs[1])):
+        rep = oracle.allclose(got.cpu().numpy(), want, atol=1e-5, rtol=1e-3)
+        assert rep["pass"], rep
+    for w in ws:
+        w.free()
