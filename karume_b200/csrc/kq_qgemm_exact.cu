@@ -1016,8 +1016,14 @@ uint64_t align256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
 }  // namespace
 
 bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, uint64_t workspace_bytes) {
-  if (count < 1 || count > kMaxMulti || m <= 16) return false;
+  if (count < 1 || count > kMaxMulti || m == 0) return false;
   const Weight& w0 = *targets[0].w;
+  // Tiled layouts have GEMVs of their own up to 16 rows.  The untiled ones only have the generic kernel
+  // (one warp per channel), which is faster while the launch is: 13.5 us for anything up to 1 x 4096 ->
+  // 1000, then 26 us for 1 x 4096 -> 4096 int4 (here 22) or 35 us int8 (here 19), and 242 us at 16 rows (here 25).
+  uint64_t work = 0;
+  for (int i = 0; i < count; ++i) work += static_cast<uint64_t>(m) * targets[i].w->n * w0.k;
+  if (w0.layout != kLayoutNative ? m <= 16 : work < (w0.storage == KQ_STORAGE_I4 ? 12u << 20 : 8u << 20)) return false;
   for (int i = 0; i < count; ++i) {
     const Weight& w = *targets[i].w;
     if (w.layout != w0.layout || w.storage != w0.storage || w.k != w0.k || w.group_size != w0.group_size ||
@@ -1078,7 +1084,11 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
 
 // Integer-dot form: int8 activations xq [m, k] with row scales xs.
 bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes) {
-  if (m <= 16 || w.k == 0 || !kind_ok(w) || w.k % 16 != 0 || (reinterpret_cast<uintptr_t>(xq) & 15u) != 0) return false;
+  // At most eight rows of a tiled int4 weight run faster on the mma.sync kernel (4096 -> 11008: 31 us, here 43:
+  // the ascending fma chain over the groups allows no K split); a tiled int8 one only with a short k
+  // (k = 4096: 25 us, here 17); the generic kernel of the untiled layouts (0.09 us per k) only below k = 128.
+  if (w.layout == kLayoutTiledI4 ? m <= 8 : w.layout == kLayoutTiledI8 ? m <= 8 && w.k < 512 : w.k < 128) return false;
+  if (m == 0 || w.k == 0 || !kind_ok(w) || w.k % 16 != 0 || (reinterpret_cast<uintptr_t>(xq) & 15u) != 0) return false;
   if (w.storage == KQ_STORAGE_I8) return true;
   return w.group_size <= kMaxChain && align256(static_cast<uint64_t>(w.k) * 2 * 32) <= workspace_bytes;
 }
