@@ -19,6 +19,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 OUT = os.path.join(HERE, "libkq.so")
+TORCH_SRC = os.path.join(CSRC, "kq_torch.cpp")
+TORCH_OUT = os.path.join(HERE, "_kqtorch.so")  # the Python calls on torch tensors (a CPython extension module)
 
 SOURCES = ["kq_api.cu", "kq_generic.cu", "kq_qgemv_i4.cu", "kq_qgemv_i4_tc.cu", "kq_plan.cu", "kq_qgemm_i4.cu", "kq_qgemm_exact.cu", "kq_qgemv_i8.cu",
            "kq_comm.cu", "kq_idot.cu", "kq_fused_ops.cu", "kq_container.cu"]
@@ -85,5 +87,29 @@ def build(force: bool = False, verbose: bool = False, extra_flags=(), out: str =
     return out
 
 
+def build_torch_calls(force: bool = False) -> str:
+    """Compiles kq_torch.cpp against the torch of this interpreter (host code only)."""
+    if not force and os.path.exists(TORCH_OUT) and os.path.getmtime(TORCH_OUT) >= max(os.path.getmtime(TORCH_SRC), os.path.getmtime(os.path.abspath(__file__))):
+        return TORCH_OUT
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), sysconfig.get_paths()["include"]]
+    lib = os.path.join(root, "lib")
+    cmd = [shutil.which("g++") or "/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for i in include:
+        cmd += ["-isystem", i]
+    cmd += ["-o", TORCH_OUT, TORCH_SRC, "-L" + lib, "-Wl,-rpath," + lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        sys.stderr.write(proc.stdout + proc.stderr)
+        raise RuntimeError(f"g++ failed ({proc.returncode}): {' '.join(cmd)}")
+    return TORCH_OUT
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_torch_calls(force="--force" in sys.argv))

@@ -45,6 +45,20 @@ def _torch():
     return torch
 
 
+_fast = None  # the native form of the serving calls (csrc/kq_torch.cpp), loaded with the first context
+
+
+def _load_fast() -> None:
+    """Loads the extension module and hands it the library's entry points; raises if it is not built."""
+    global _fast
+    if _fast is None:
+        _torch()
+        from . import _kqtorch
+        _kqtorch.bind(*[ctypes.cast(f, ctypes.c_void_p).value
+                        for f in (L.kq_linear, L.kq_linear_fused, L.kq_quantize_rows, L.kq_linear_a8, L.kq_embedding)])
+        _fast = _kqtorch
+
+
 def _tensor_dtype_code(t) -> int:
     torch = _torch()
     table = {torch.float32: KQ_F32, torch.float16: KQ_F16, torch.bfloat16: KQ_BF16}
@@ -95,10 +109,18 @@ class Gpu:
         if rc != 0:
             raise KqError(rc, (L.kq_last_error(None) or b"").decode())
         self._ctx = ctx
+        self._ctx_addr = ctx.value
+        _load_fast()
         if use_torch_stream:
             self.use_stream(torch.cuda.current_stream(self.device))
 
     # -- plumbing -----------------------------------------------------------
+    def _done(self, result):
+        """What a native call returned: its result, or the status of a call the library refused."""
+        if result.__class__ is int:
+            self._check(result)
+        return result
+
     def _check(self, rc: int) -> None:
         if rc != 0:
             raise KqError(rc, (L.kq_last_error(self._ctx) or b"").decode())
@@ -119,7 +141,7 @@ class Gpu:
     def destroy(self) -> None:
         if self._ctx:
             L.kq_destroy(self._ctx)
-            self._ctx = None
+            self._ctx = self._ctx_addr = None
 
     # -- weights ------------------------------------------------------------
     def upload_weight(self, storage: str, payload, scale, shape, group_size: int = 0,
@@ -150,6 +172,9 @@ class Gpu:
 
     def embedding(self, index, weight: Weight, out=None):
         """Rows index[...] (CUDA int32) of a resident weight [vocab, hidden], dequantised to f32."""
+        done = _fast.embedding(self._ctx_addr, weight.handle, weight.k, index, out)
+        if done is not None:
+            return self._done(done)
         torch = _torch()
         if index.dtype != torch.int32 or not index.is_cuda or not index.is_contiguous():
             raise ValueError("index must be a contiguous CUDA int32 tensor")
@@ -162,6 +187,9 @@ class Gpu:
     def quantize_rows(self, x):
         """Per-row symmetric int8 quantisation of a CUDA f32 tensor [..., dim]:
         returns (q int8 [..., dim], scale f32 [...])."""
+        done = _fast.quantize_rows(self._ctx_addr, x)
+        if done is not None:
+            return self._done(done)
         torch = _torch()
         if x.dtype != torch.float32 or not x.is_cuda or not x.is_contiguous():
             raise ValueError("quantize_rows takes a contiguous CUDA f32 tensor")
@@ -175,6 +203,9 @@ class Gpu:
     def linear_a8(self, xq, xs, weight: Weight, bias, out=None):
         """Integer-dot linear: xq int8 [..., k] and xs f32 [...] from quantize_rows against a
         resident int8 (w8a8) or int4 (w4a8) weight.  Returns f32 [..., n]."""
+        done = _fast.linear_a8(self._ctx_addr, weight.handle, weight.n, weight.k, xq, xs, bias, out)
+        if done is not None:
+            return self._done(done)
         torch = _torch()
         if xq.dtype != torch.int8 or xq.shape[-1] != weight.k or not xq.is_contiguous():
             raise ValueError("xq must be a contiguous int8 tensor [..., k]")
@@ -193,6 +224,9 @@ class Gpu:
     def linear(self, x, weight: Weight, bias, out=None):
         """out[..., n] = x[..., k] @ W[n, k]^T + bias[n]; x is a CUDA tensor (f32/f16/bf16),
         bias a CUDA f32 tensor [n] (required: the op's arity is 3).  Returns f32."""
+        done = _fast.linear(self._ctx_addr, weight.handle, weight.n, weight.k, x, bias, out)
+        if done is not None:
+            return self._done(done)
         torch = _torch()
         if x.shape[-1] != weight.k:
             raise KqError(2, f"linear: x[..., {x.shape[-1]}] does not match W[{weight.n},{weight.k}]")
@@ -276,6 +310,11 @@ class Gpu:
                      swiglu: bool = False, reduce: bool = False):
         """[rms_norm ->] linear(s) [-> silu(gate) * up] [-> sum over ranks] [-> + residual] (kq_linear_fused).
         `weights` / `biases` are lists; with swiglu=True they are (gate, up) and there is one output."""
+        if outs is not None:
+            done = _fast.linear_fused(self._ctx_addr, [w.handle for w in weights], weights[0].k, x, biases, outs, norm_weight, float(eps),
+                                      residual, (1 if swiglu else 0) | (2 if reduce else 0))
+            if done is not None:
+                return self._done(done)
         torch = _torch()
         x = x.contiguous()
         k = weights[0].k
