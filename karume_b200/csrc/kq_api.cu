@@ -321,7 +321,9 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
                                     targets[i].out + static_cast<size_t>(m0) * targets[i].w->n};
       int launched = 0;
       const void* xp = reinterpret_cast<const uint8_t*>(x) + static_cast<size_t>(m0) * targets[0].w->k * xb;
-      cudaError_t e = kq::launch_qgemv_i4(env, static_cast<int>(count), panel, xp, x_dtype, mm, &launched);
+      cudaError_t e = kq::qgemv_i4_xs_preferred(static_cast<int>(count), panel, x_dtype, mm, false, false)
+                          ? kq::launch_qgemv_i4_xs(env, static_cast<int>(count), panel, xp, x_dtype, mm, false, &launched)
+                          : kq::launch_qgemv_i4(env, static_cast<int>(count), panel, xp, x_dtype, mm, &launched);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_i4 launch");
       ctx->launches += launched;
     }
@@ -344,7 +346,9 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
         kq::LinearTarget panel{one.w, one.bias, one.out + static_cast<size_t>(m0) * w.n};
         int launched = 0;
         const void* xp = reinterpret_cast<const uint8_t*>(x) + static_cast<size_t>(m0) * w.k * xb;
-        cudaError_t e = kq::launch_qgemv_i4(env, 1, &panel, xp, x_dtype, mm, &launched);
+        cudaError_t e = kq::qgemv_i4_xs_preferred(1, &panel, x_dtype, mm, false, false)
+                            ? kq::launch_qgemv_i4_xs(env, 1, &panel, xp, x_dtype, mm, false, &launched)
+                            : kq::launch_qgemv_i4(env, 1, &panel, xp, x_dtype, mm, &launched);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_i4 launch");
         ctx->launches += launched;
       }
@@ -1090,6 +1094,26 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
     for (uint32_t i = 0; i < count; ++i) {
       probe[i] = kq::LinearTarget{find_weight(ctx, w[i]), nullptr, nullptr};
       known = known && probe[i].w != nullptr;
+    }
+    if (known && !reduce && (norm_weight_dptr || residual_dptr || swiglu) &&
+        kq::qgemv_i4_xs_preferred(static_cast<int>(count), probe, x_dtype, m, norm_weight_dptr || residual_dptr, swiglu)) {
+      // Up to sixteen rows on tiled int4 weights: one launch does it all.
+      for (uint32_t i = 0; i < count; ++i) {
+        const uint64_t out_i = swiglu ? out_dptr[0] : out_dptr[i];
+        const int rc = check_linear_args(ctx, probe[i].w, x_dptr, x_dtype, bias_dptr[i], out_i);
+        if (rc != KQ_OK) return rc;
+        probe[i].bias = reinterpret_cast<const float*>(bias_dptr[i]);
+        probe[i].out = reinterpret_cast<float*>(out_i);
+      }
+      kq::LaunchEnv env = env_of(ctx);
+      env.norm_weight = reinterpret_cast<const float*>(norm_weight_dptr);
+      env.norm_eps = norm_eps;
+      env.residual = reinterpret_cast<const float*>(residual_dptr);
+      int launched = 0;
+      cudaError_t e = kq::launch_qgemv_i4_xs(env, static_cast<int>(count), probe, reinterpret_cast<const void*>(x_dptr), x_dtype, m, swiglu, &launched);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_i4_xs launch");
+      ctx->launches += launched;
+      return KQ_OK;
     }
     if (known && !reduce && (norm_weight_dptr || residual_dptr) &&
         (kq::qgemv_i4_fuses_neighbours(static_cast<int>(count), probe, x_dtype, m) ||

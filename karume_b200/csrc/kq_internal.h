@@ -113,6 +113,13 @@ bool qgemv_i4_fuses_neighbours(int count, const LinearTarget* targets, int x_dty
 cudaError_t launch_qgemv_i4(const LaunchEnv& env, int count, const LinearTarget* targets,
                             const void* x, int x_dtype, uint32_t m, int* launches);
 
+// The same with the activations in registers (kq_qgemv_i4_xs.cu), one launch with its neighbours: env.norm_weight
+// (f32 activations), env.residual (one weight) and, for two weights (gate, up) of one shape, the SiLU gate.
+bool qgemv_i4_xs_supports(int count, const LinearTarget* targets, int x_dtype, uint32_t m);
+bool qgemv_i4_xs_preferred(int count, const LinearTarget* targets, int x_dtype, uint32_t m, bool norm_or_residual, bool swiglu);
+cudaError_t launch_qgemv_i4_xs(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,
+                               bool swiglu, int* launches);
+
 // The same on the tcgen05 tensor cores (kq_qgemv_i4_tc.cu): 5..16 binary16 rows or 5..8 f32 /
 // bf16 rows.  Needs env.status.
 bool qgemv_i4_tc_supports(int count, const LinearTarget* targets, int x_dtype, uint32_t m, int sm_count);

@@ -11,7 +11,7 @@
 //     4.6 KB through its private shared-memory ring with cp.async.bulk + mbarrier.  The
 //     copies for the next op are issued before the warp waits for the previous op to
 //     finish, so HBM keeps streaming through the dependency barriers;
-//   * the math per 64-k chunk is the same as in qgemv_i4_kernel (kq_gemv_core.cuh): nibble
+//   * the math per 64-k chunk is the same as in kq_qgemv_i4.cu (kq_gemv_core.cuh): nibble
 //     pairs as binary16 subnormals into mma.sync, hi/lo activation columns, f32 group scale;
 //   * an op with few output rows splits K over the warps of ONE CTA (S slabs x 16/S row
 //     blocks per CTA round); the S partial sums meet in shared memory and are added in slab
@@ -251,7 +251,7 @@ plan_kernel(const PlanParams p) {
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) produce();
 
-  // Persistent per-lane state of the MMA operands (see qgemv_i4_kernel).
+  // Persistent per-lane state of the MMA operands (see kq_qgemv_i4.cu).
   uint4 bfrag[kTiles];
   float cterm[kTiles][kCorrPerTile], cinv[kTiles][kCorrPerTile];
   bool load_b[kTiles], load_c[kTiles][kCorrPerTile];

@@ -1,5 +1,7 @@
 // qgemv_i4 — the decode-path kernel of libkq: y[m, n] = x[m, k] . W[n, k]^T + b for
-// 1 <= m <= 16 with W in the tiled int4 / group-32 layout (kq_common.cuh).
+// W in the tiled int4 / group-32 layout (kq_common.cuh): the group-packed kernel for one or two f32 rows
+// (up to four binary16 ones) and the wide kernel for five and more rows of a very large matrix; the rest
+// of 1 <= m <= 16 is kq_qgemv_i4_xs.cu (the rule: qgemv_i4_xs_preferred).
 //
 // Replaces the reference's small-M linear variant with in-kernel int4 dequant
 // (pipeline key linear:v2:f32:reg16x16r1x4w4:wi4g32 — packages/runtime/src/kernels/
@@ -249,235 +251,8 @@ struct ChunkRegs {
   uint4 w;  // row g grp 0 | row g+8 grp 0 | row g grp 1 | row g+8 grp 1
   typename std::conditional<kScaleF16, uint2, uint4>::type s;
 };
-template <typename XT, bool kScaleF16, int kCols, int kRB>
-__global__ void __launch_bounds__(kWarps * 32)
-qgemv_i4_kernel(const GemvParams p) {
-  constexpr bool kHasLo = !std::is_same<XT, __half>::value;
-  constexpr uint32_t kScaleBytes = kScaleF16 ? 2u : 4u;
-  constexpr uint32_t kCB = kChunkWeightBytes + 32u * kScaleBytes;  // chunk bytes
-  constexpr int kTiles = kCols / 8;
-  constexpr int kAccPerTile = kHasLo ? 2 : 4;
-  constexpr int kCorrPerTile = kHasLo ? 1 : 2;
-  constexpr int kCorrStride = kHasLo ? kCols / 2 : kCols;
-  constexpr uint32_t kTileRowsCta = kWarps * kRB * 16;
-
-  extern __shared__ __align__(16) uint8_t smem[];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t g = lane >> 2, t = lane & 3u;
-
-  pdl_launch_dependents();
-
-  // which weight of the launch this CTA's row tile belongs to
-  uint32_t wi = 0;
-#pragma unroll
-  for (int i = 1; i < kMaxMulti; ++i)
-    if (i < static_cast<int>(p.count) && blockIdx.x >= p.tile_begin[i]) wi = i;
-  const uint8_t* w_base = p.w[0];
-  const float* bias = p.bias[0];
-  float* out = p.out[0];
-  uint32_t n = p.n[0], tile0 = p.tile_begin[0];
-#pragma unroll
-  for (int i = 1; i < kMaxMulti; ++i)
-    if (wi == static_cast<uint32_t>(i)) {
-      w_base = p.w[i]; bias = p.bias[i]; out = p.out[i]; n = p.n[i]; tile0 = p.tile_begin[i];
-    }
-  const uint32_t tile = blockIdx.x - tile0;
-  const uint32_t row_block0 = (tile * kWarps + warp) * kRB;
-
-  const uint32_t chunks_per_row = p.k / kChunkK;
-  const uint32_t split = blockIdx.y;  // == rank in the cluster when splits > 1
-  const uint32_t cbeg = min(split * p.chunks_per_split, chunks_per_row);
-  const uint32_t cend = min(cbeg + p.chunks_per_split, chunks_per_row);
-  const uint32_t nch = cend - cbeg;
-
-  const uint32_t active_cols = kHasLo ? 2 * p.m : p.m;
-  const uint32_t xs_stride = active_cols * 64;  // bytes of staged activations per group
-  uint8_t* xs = smem;
-  float* corr = reinterpret_cast<float*>(smem + 2 * p.slab_chunks * xs_stride);
-
-  bool active[kRB];
-  const uint8_t* next[kRB];  // address this lane loads for the chunk kDepth ahead of the current block
-#pragma unroll
-  for (int r = 0; r < kRB; ++r) {
-    active[r] = (row_block0 + r) * 16u < n;
-    next[r] = w_base + (static_cast<size_t>(row_block0 + r) * chunks_per_row + cbeg) * kCB + lane * 16;
-  }
-  const uint32_t scale_off = kChunkWeightBytes - lane * 16 + g * (4 * kScaleBytes);
-
-  ChunkRegs<kScaleF16> ring[kDepth][kRB];
-  auto fetch = [&](ChunkRegs<kScaleF16>& dst, const uint8_t* src) {
-    dst.w = ldg_stream_v4(src);
-    if constexpr (kScaleF16) dst.s = ldg_stream_v2(src + scale_off);
-    else dst.s = ldg_stream_v4(src + scale_off);
-  };
-
-  // Weights do not depend on the previous kernel: start streaming before the wait.
-#pragma unroll
-  for (int d = 0; d < kDepth; ++d)
-#pragma unroll
-    for (int r = 0; r < kRB; ++r) {
-      ring[d][r].w = make_uint4(0, 0, 0, 0);
-      if constexpr (kScaleF16) ring[d][r].s = make_uint2(0, 0);
-      else ring[d][r].s = make_uint4(0, 0, 0, 0);
-      if (active[r] && static_cast<uint32_t>(d) < nch) fetch(ring[d][r], next[r] + d * kCB);
-    }
-#pragma unroll
-  for (int r = 0; r < kRB; ++r) next[r] += kDepth * kCB;
-
-  pdl_wait_prior_grid();
-
-  float acc[kRB][kTiles][kAccPerTile];
-#pragma unroll
-  for (int r = 0; r < kRB; ++r)
-#pragma unroll
-    for (int i = 0; i < kTiles; ++i)
-#pragma unroll
-      for (int j = 0; j < kAccPerTile; ++j) acc[r][i][j] = 0.0f;
-
-  const XT* x = static_cast<const XT*>(p.x);
-  constexpr uint32_t kMask0 = 0x000F000Fu;  // nibbles 0 and 4 of a word: u * 2^-24 as binary16
-  constexpr uint32_t kMask1 = 0x00F000F0u;  // nibbles 1 and 5 of a word: u * 2^-20 as binary16
-
-  // B fragments and "-8 sum x" terms live in registers that only lanes with a real
-  // column / activation row ever load into; everybody else keeps the initial zeros.
-  uint4 bfrag[kTiles];
-  float cterm[kTiles][kCorrPerTile], cinv[kTiles][kCorrPerTile];  // {-8 sum x, 2^-e} of the lane's activation rows
-  bool load_b[kTiles], load_c[kTiles][kCorrPerTile];
-#pragma unroll
-  for (int tile_m = 0; tile_m < kTiles; ++tile_m) {
-    bfrag[tile_m] = make_uint4(0, 0, 0, 0);
-    load_b[tile_m] = tile_m * 8 + g < active_cols;
-#pragma unroll
-    for (int j = 0; j < kCorrPerTile; ++j) {
-      cterm[tile_m][j] = 0.0f;
-      cinv[tile_m][j] = 0.0f;
-      const uint32_t mm = kHasLo ? tile_m * 4 + t : tile_m * 8 + 2 * t + j;
-      load_c[tile_m][j] = mm < p.m;
-    }
-  }
-  const uint32_t xs_lane = static_cast<uint32_t>(__cvta_generic_to_shared(xs)) + lane * 16;
-  const uint32_t corr_lane = static_cast<uint32_t>(__cvta_generic_to_shared(corr)) + (kHasLo ? t : 2 * t) * 8;
-
-  // One chunk (64 k = two scale groups) of every row block of the warp, out of ring
-  // slot d; then the slot is refilled with the chunk kDepth further on.
-  auto process = [&](const int d, uint32_t xs_addr, uint32_t corr_addr, bool refill) {
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj) {
-#pragma unroll
-      for (int tile_m = 0; tile_m < kTiles; ++tile_m) {
-        lds_v4_if(bfrag[tile_m], xs_addr + jj * xs_stride + tile_m * 512, load_b[tile_m]);
-#pragma unroll
-        for (int j = 0; j < kCorrPerTile; ++j)
-          lds_v2f_if(cterm[tile_m][j], cinv[tile_m][j], corr_addr + (jj * kCorrStride + tile_m * (kHasLo ? 4 : 8) + j) * 8,
-                     load_c[tile_m][j]);
-      }
-#pragma unroll
-      for (int r = 0; r < kRB; ++r) {
-        const uint32_t wa = jj ? ring[d][r].w.z : ring[d][r].w.x;  // row g
-        const uint32_t wb = jj ? ring[d][r].w.w : ring[d][r].w.y;  // row g + 8
-        const uint32_t wa8 = wa >> 8, wb8 = wb >> 8;
-        const uint32_t a0[4] = {wa & kMask0, wb & kMask0, wa & kMask1, wb & kMask1};
-        const uint32_t a1[4] = {wa8 & kMask0, wb8 & kMask0, wa8 & kMask1, wb8 & kMask1};
-        float2 s;  // .x = row g, .y = row g + 8
-        if constexpr (kScaleF16) {
-          s = __half22float2(*reinterpret_cast<const __half2*>(jj ? &ring[d][r].s.y : &ring[d][r].s.x));
-        } else {
-          s = jj ? make_float2(__uint_as_float(ring[d][r].s.z), __uint_as_float(ring[d][r].s.w))
-                 : make_float2(__uint_as_float(ring[d][r].s.x), __uint_as_float(ring[d][r].s.y));
-        }
-#pragma unroll
-        for (int tile_m = 0; tile_m < kTiles; ++tile_m) {
-          float cf[4];
-          mma_f16_zero(cf, a0, bfrag[tile_m].x, bfrag[tile_m].y);
-          mma_f16(cf, a1, bfrag[tile_m].z, bfrag[tile_m].w);
-          if constexpr (kHasLo) {
-            acc[r][tile_m][0] = fmaf(s.x, fmaf(cf[0] + cf[1], cinv[tile_m][0], cterm[tile_m][0]), acc[r][tile_m][0]);
-            acc[r][tile_m][1] = fmaf(s.y, fmaf(cf[2] + cf[3], cinv[tile_m][0], cterm[tile_m][0]), acc[r][tile_m][1]);
-          } else {
-            acc[r][tile_m][0] = fmaf(s.x, fmaf(cf[0], cinv[tile_m][0], cterm[tile_m][0]), acc[r][tile_m][0]);
-            acc[r][tile_m][1] = fmaf(s.x, fmaf(cf[1], cinv[tile_m][1], cterm[tile_m][1]), acc[r][tile_m][1]);
-            acc[r][tile_m][2] = fmaf(s.y, fmaf(cf[2], cinv[tile_m][0], cterm[tile_m][0]), acc[r][tile_m][2]);
-            acc[r][tile_m][3] = fmaf(s.y, fmaf(cf[3], cinv[tile_m][1], cterm[tile_m][1]), acc[r][tile_m][3]);
-          }
-        }
-      }
-    }
-    if (refill) {
-#pragma unroll
-      for (int r = 0; r < kRB; ++r)
-        if (active[r]) fetch(ring[d][r], next[r] + d * kCB);
-    }
-  };
-
-  for (uint32_t done = 0; done < nch;) {
-    const uint32_t slab_n = min(p.slab_chunks, nch - done);
-    if (done != 0) __syncthreads();  // everyone is done reading the previous slab
-    stage_x<XT, kHasLo, kCorrStride>(x, p.m, p.k, 2 * (cbeg + done), 2 * slab_n, xs, xs_stride, corr);
-    __syncthreads();
-    uint32_t xs_addr = xs_lane, corr_addr = corr_lane;
-    uint32_t i = 0;
-    for (; i + kDepth <= slab_n; i += kDepth) {
-#pragma unroll
-      for (int d = 0; d < kDepth; ++d) {
-        process(d, xs_addr, corr_addr, done + i + d + kDepth < nch);
-        xs_addr += 2 * xs_stride;
-        corr_addr += 2 * kCorrStride * 8;
-      }
-#pragma unroll
-      for (int r = 0; r < kRB; ++r) next[r] += kDepth * kCB;
-    }
-#pragma unroll
-    for (int d = 0; d < kDepth - 1; ++d) {  // the last, short block of the split
-      if (i + d < slab_n) {
-        process(d, xs_addr, corr_addr, false);
-        xs_addr += 2 * xs_stride;
-        corr_addr += 2 * kCorrStride * 8;
-      }
-    }
-    done += slab_n;
-  }
-
-  // ---- epilogue -----------------------------------------------------------------
-  // lane owns, per row block and tile: rows g and g+8 of the block and activation rows
-  //   with hi/lo columns : mm = 4*tile + t             (acc[..][0] row g, [1] row g+8)
-  //   binary16 input     : mm = 8*tile + 2t, 2t+1      (acc[..][0,1] row g, [2,3] row g+8)
-  float* red = reinterpret_cast<float*>(smem);  // [m][kTileRowsCta], aliases the x slab
-  if (p.splits > 1) __syncthreads();            // the slab is dead from here on
-#pragma unroll
-  for (int r = 0; r < kRB; ++r) {
-    if (!active[r]) continue;
-    const uint32_t row_a = (row_block0 + r) * 16u + g;
-    const uint32_t tr_a = (warp * kRB + r) * 16u + g;  // row inside the CTA tile
-    float bias_a = 0.0f, bias_b = 0.0f;
-    if (p.splits == 1) {
-      bias_a = bias[row_a];
-      bias_b = bias[row_a + 8];
-    }
-#pragma unroll
-    for (int tile_m = 0; tile_m < kTiles; ++tile_m) {
-#pragma unroll
-      for (int j = 0; j < (kHasLo ? 1 : 2); ++j) {
-        const uint32_t mm = kHasLo ? tile_m * 4 + t : tile_m * 8 + 2 * t + j;
-        if (mm >= p.m) continue;
-        const float va = acc[r][tile_m][kHasLo ? 0 : j];
-        const float vb = acc[r][tile_m][kHasLo ? 1 : 2 + j];
-        if (p.splits == 1) {
-          out[static_cast<size_t>(mm) * n + row_a] = fmaf(va, kUnscale, bias_a);
-          out[static_cast<size_t>(mm) * n + row_a + 8] = fmaf(vb, kUnscale, bias_b);
-        } else {
-          red[mm * kTileRowsCta + tr_a] = va;
-          red[mm * kTileRowsCta + tr_a + 8] = vb;
-        }
-      }
-    }
-  }
-  if (p.splits == 1) return;
-
-  cluster_reduce_store(p, red, kTileRowsCta, tile, split, n, out, bias);
-}
-
 // ---- group-packed variant: at most 4 of the 8 MMA columns are needed -----------------
-// With one or two activation rows the block above would leave most of each MMA tile empty
+// With one or two activation rows a tile of one group would leave most of each MMA tile empty
 // and, worse, make every lane apply every group's scale.  Here the spare columns carry
 // OTHER scale groups: a unit is kG consecutive groups, group j of the unit owns columns
 // [j * kCpg, (j + 1) * kCpg) of the tile (its activations are zero in every other column),
@@ -695,75 +470,6 @@ qgemv_i4_gp_kernel(const GemvParams p) {
   }
   if (p.splits == 1) return;
   cluster_reduce_store(p, red, kTileRowsCta, tile, split, n, out, bias);
-}
-
-template <typename XT, int kCols>
-uint32_t group_smem_bytes(uint32_t m) {
-  constexpr bool kHasLo = !std::is_same<XT, __half>::value;
-  return (kHasLo ? 2 * m : m) * 64 + (kHasLo ? kCols / 2 : kCols) * 8;  // staged halves + {corr, 2^-e} pairs
-}
-
-template <typename XT, bool kScaleF16, int kCols, int kRB>
-cudaError_t launch_typed(const LaunchEnv& env, GemvParams& p, int count, const LinearTarget* targets) {
-  auto kernel = qgemv_i4_kernel<XT, kScaleF16, kCols, kRB>;
-  static PerDevice<bool> configured_on;
-  bool* configured = configured_on.slot();
-  if (configured == nullptr) return cudaErrorInvalidDevice;
-  if (!*configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (e != cudaSuccess) return e;
-    *configured = true;
-  }
-  constexpr uint32_t kTileRowsCta = kWarps * kRB * 16;
-  uint32_t tiles = 0;
-  for (int i = 0; i < count; ++i) {
-    p.tile_begin[i] = tiles;
-    tiles += (targets[i].w->n + kTileRowsCta - 1) / kTileRowsCta;
-  }
-  for (int i = count; i <= kMaxMulti; ++i) p.tile_begin[i] = tiles;
-
-  const uint32_t chunks_per_row = p.k / kChunkK;
-
-  // Split K over a cluster until the grid fills the machine (about four CTAs per SM);
-  // a pure function of the shape, never autotuned.
-  const uint32_t want_ctas = static_cast<uint32_t>(env.sm_count) * kWantCtasPerSm;
-  uint32_t splits = 1;
-  while (splits < static_cast<uint32_t>(kMaxCluster) && tiles * splits < want_ctas &&
-         splits * 2 <= chunks_per_row)
-    splits *= 2;
-  p.splits = splits;
-  p.chunks_per_split = (chunks_per_row + splits - 1) / splits;
-  // Activations are staged at most ~32 KB at a time; a slab that is not the last one of
-  // its split must be a whole number of ring rounds.
-  const uint32_t per_chunk = 2 * group_smem_bytes<XT, kCols>(p.m);
-  uint32_t slab_cap = std::max<uint32_t>(kDepth, (32768u / per_chunk) / kDepth * kDepth);
-  p.slab_chunks = std::max<uint32_t>(1u, std::min(p.chunks_per_split, slab_cap));
-
-  const size_t slab_bytes = static_cast<size_t>(p.slab_chunks) * per_chunk;
-  const size_t red_bytes = splits > 1 ? static_cast<size_t>(p.m) * kTileRowsCta * sizeof(float) : 0;
-
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles, splits, 1);
-  cfg.blockDim = dim3(kWarps * 32, 1, 1);
-  cfg.dynamicSmemBytes = std::max(slab_bytes, red_bytes);
-  cfg.stream = env.stream;
-  cudaLaunchAttribute attr[2];
-  unsigned int na = 0;
-  if (env.overlap) {
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
-  if (splits > 1) {
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = 1;
-    attr[na].val.clusterDim.y = splits;
-    attr[na].val.clusterDim.z = 1;
-    ++na;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 // How many CTAs of a launch configuration fit on the device at the same time (0 when the
@@ -1330,8 +1036,6 @@ cudaError_t launch_x(const LaunchEnv& env, GemvParams& p, int count, const Linea
   if (cols <= 4)
     return f16s ? launch_typed_gp<XT, true, 2>(env, p, count, t) : launch_typed_gp<XT, false, 2>(env, p, count, t);
   if (env.fused != nullptr) return cudaErrorNotSupported;  // only the group-packed kernel exchanges in its epilogue
-  if (kHasLo && p.m <= 4)  // three or four f32 / bf16 rows: hi and lo in adjacent columns of one tile
-    return f16s ? launch_typed<XT, true, 8, 1>(env, p, count, t) : launch_typed<XT, false, 8, 1>(env, p, count, t);
   // Five or more rows.  Two row blocks per warp (sharing the activation loads) pay off when a
   // row block costs many MMAs (hi + lo parts, or two column tiles) and the matrix has rows to
   // spare; otherwise one row block per warp and a deeper ring keep more CTAs in flight.  A pure

@@ -3,7 +3,7 @@
 // dequant (pipeline key linear:v2:f32:reg16x16r1x4w4:wi8 —
 // packages/runtime/src/kernels/weight-storage.ts:191-209 inside gemm.ts:1187-1237).
 //
-// Same construction as qgemv_i4_kernel (see that file): the stored bytes (q + 128) reach
+// Same construction as the int4 kernels (kq_qgemv_i4.cu): the stored bytes (q + 128) reach
 // mma.sync.m16n8k16 as binary16 subnormals b * 2^-24 after one mask per pair, the
 // activations are the B operand staged once per CTA (hi / lo binary16 columns for f32 and
 // bf16 input), weights stream through a register ring, K can be split over a cluster and
