@@ -16,9 +16,9 @@
 // the weight past them.  Per 576-byte chunk that leaves the weight load, the unpack, the MMAs and
 // the scale.
 //   * The power-of-two pre-scale is per (row, slab), so it costs one multiply per partial sum.
-//   * rms_norm: the warp multiplies x by the norm weight and adds the squares of its slab; the
-//     row's rsqrt multiplies the finished sums, (sum_k (x g) w) r instead of sum_k ((x r) g) w.
-//   * The slabs of a CTA meet in shared memory, four row blocks at a time, in slab order; a k
+//   * rms_norm: the CTAs of a cluster share out the rows' sums of squares while the first weights are on
+//     their way; what is staged is (x r) g as the reference computes it.
+//   * The slabs of a CTA meet in shared memory, a batch of row blocks at a time, in slab order; a k
 //     longer than a CTA's 16 slabs is spread over a thread-block cluster, whose CTAs add their
 //     sums over distributed shared memory in rank order once per launch (and over several passes
 //     where that is not enough).  No atomics: the same bits every time.
@@ -37,14 +37,25 @@ namespace {
 
 constexpr int kXsWarps = 16, kXsThreads = kXsWarps * 32;
 constexpr int kXsAhead = 4;            // row blocks a warp has in flight, in registers (two: 15 % slower on a large matrix)
-constexpr int kXsBatch = 4;            // row blocks per reduction
 constexpr uint32_t kXsMaxCluster = 8;
-constexpr uint32_t kXsHead = 2048;     // sums of squares, row factors
+constexpr uint32_t kXsHead = 1024;     // sums of squares, row factors
 constexpr uint32_t kXsSmem = 227 * 1024;
-// [buffer][block][warp][tile][128 sums]
-__host__ __device__ constexpr uint32_t red_bytes(uint32_t tiles) { return 2u * kXsBatch * kXsWarps * tiles * 512u; }
-// row blocks whose finished sums a CTA can hold
-__host__ __device__ constexpr uint32_t part_blocks(uint32_t tiles) { return (kXsSmem - kXsHead - red_bytes(tiles)) / (tiles * 512u); }
+
+// How the columns of a warp's MMA tiles are used:
+//   kPacked  up to four f32 / bf16 rows: columns 2r and 2r + 1 = the high and the low part of row r (one MMA carries
+//            both, one lane holds both sums); a warp's slab is 128 k
+//   kEight   up to eight rows, column c = row c, the low parts a second B operand; 128 k
+//   kSixteen up to sixteen rows, two tiles: the nibbles are unpacked once for both; 64 k, so that the fragments
+//            take the same registers
+enum XsForm : int { kPacked, kEight, kSixteen };
+template <int kForm>
+struct XsShape {
+  static constexpr uint32_t tiles = kForm == kSixteen ? 2 : 1, slab_chunks = kForm == kSixteen ? 1 : 2;
+  static constexpr uint32_t sums = kForm == kPacked ? 64 : 128 * tiles;  // finished sums of a 16-row block
+  static constexpr uint32_t batch = kForm == kPacked ? 8 : 4;            // row blocks per reduction
+  static constexpr uint32_t red_bytes = 2u * batch * kXsWarps * sums * 4u;  // [buffer][block][warp][sums]
+  static constexpr uint32_t part_blocks = (kXsSmem - kXsHead - red_bytes) / (sums * 4u);  // row blocks a CTA can hold the sums of
+};
 
 struct XsParams {
   const uint8_t* w[kMaxMulti];
@@ -105,36 +116,28 @@ struct XsChunk {
   typename std::conditional<kScaleF16, uint2, uint4>::type s;
 };
 
-// How the columns of a warp's MMA tiles are used:
-//   kPacked  up to four f32 / bf16 rows: column c < 4 = the high part of row c, column 4 + c its low part (one MMA
-//            carries both); a warp's slab is 128 k
-//   kEight   up to eight rows, column c = row c, the low parts a second B operand; 128 k
-//   kSixteen up to sixteen rows, two tiles: the nibbles are unpacked once for both; 64 k, so that the fragments
-//            take the same registers
-enum XsForm : int { kPacked, kEight, kSixteen };
-
 template <typename XT, bool kScaleF16, int kForm>
 __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsParams p) {
   constexpr bool kHasLo = !std::is_same<XT, __half>::value;
   constexpr bool kPackLo = kForm == kPacked, kLoSet = kHasLo && !kPackLo;
-  constexpr uint32_t kTiles = kForm == kSixteen ? 2 : 1, kSlabChunks = kForm == kSixteen ? 1 : 2;
-  constexpr int kGroups = 2 * kSlabChunks;
+  using Shape = XsShape<kForm>;
+  constexpr uint32_t kTiles = Shape::tiles, kSlabChunks = Shape::slab_chunks, kSums = Shape::sums;
+  constexpr int kGroups = 2 * kSlabChunks, kBatch = Shape::batch;
   static_assert(kHasLo || !kPackLo, "binary16 activations have no low part");
-  static_assert(kXsThreads == kXsBatch * 128 && kXsBatch % kXsAhead == 0, "the reduction's thread layout");
+  static_assert(kXsThreads * kTiles == kBatch * kSums && kBatch % kXsAhead == 0, "the reduction's thread layout");
   constexpr uint32_t kCB = kChunkWeightBytes + 32u * (kScaleF16 ? 2u : 4u);
   constexpr uint32_t kMask0 = 0x000F000Fu, kMask1 = 0x00F000F0u;
   extern __shared__ __align__(16) uint8_t smem[];
-  float* squares = reinterpret_cast<float*>(smem);           // [16 warps][16] sums of squares of a warp's rows
-  float* row_squares = squares + kXsWarps * 16;              // [16] the CTA's sums
-  float* row_factor = row_squares + 16;                      // [16] rsqrt of the whole row's
+  float* squares = reinterpret_cast<float*>(smem);           // [18 rows][8 warps] sums of squares
+  float* row_factor = squares + 18 * 8;                      // [16] the rows' rsqrt
   float* red = reinterpret_cast<float*>(smem + kXsHead);
-  float* part = reinterpret_cast<float*>(smem + kXsHead + red_bytes(kTiles));  // [block][tile][128]
+  float* part = reinterpret_cast<float*>(smem + kXsHead + Shape::red_bytes);  // [block][sums]
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
   const uint32_t rank = p.cluster > 1 ? xs_rank() : 0u, cluster_id = blockIdx.x / p.cluster;
   const uint32_t chunks = p.k / kChunkK, per_unit = p.swiglu ? 2u : 1u;
   const uint32_t unit_first = static_cast<uint32_t>(static_cast<uint64_t>(p.units) * cluster_id / p.clusters);
   const uint32_t unit_last = static_cast<uint32_t>(static_cast<uint64_t>(p.units) * (cluster_id + 1) / p.clusters);
-  const uint32_t round_units = part_blocks(kTiles) / per_unit;
+  const uint32_t round_units = Shape::part_blocks / per_unit;
 
   pdl_launch_dependents();
 
@@ -193,44 +196,88 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
       if (pass == 0 && u0 == unit_first) pdl_wait_prior_grid();
 
       // ---- the slab's activations as B fragments ----
-      uint4 bhi[kTiles][kGroups], blo[kTiles][kLoSet ? kGroups : 1];
-      float cterm[kTiles][kGroups][4], inv[kTiles][2];  // the MMA's C operand (rows g and g + 8 alike); 2^-e of the C columns
-#pragma unroll
-      for (uint32_t tl = 0; tl < kTiles; ++tl) {
-        const uint32_t row = kPackLo ? (g & 3u) : tl * 8u + g;
-        const bool row_live = row < p.m;
-        const XT* xr = static_cast<const XT*>(p.x) + static_cast<size_t>(row_live ? row : 0u) * p.k + chunk0 * kChunkK + t * 8u;
-        const float* gr = p.norm_weight + chunk0 * kChunkK + t * 8u;
-        float v[kGroups][8];
-        float amax = 0.0f, sq = 0.0f;
+      // lane (g, t) prepares B column g (k-octet t of every group) of each tile
+      auto row_of = [&](uint32_t tl) { return kPackLo ? g >> 1 : tl * 8u + g; };
+      float v[kTiles][kGroups][8];
+      auto load_slab = [&](uint32_t tl, uint32_t chunk, uint32_t chunks_live, float (&dst)[kGroups][8]) {
+        const uint32_t row = row_of(tl);
+        const XT* xr = static_cast<const XT*>(p.x) + static_cast<size_t>(row < p.m ? row : 0u) * p.k + chunk * kChunkK + t * 8u;
 #pragma unroll
         for (int j = 0; j < kGroups; ++j) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[j][e] = 0.0f;
-          if (row_live && static_cast<uint32_t>(j) < 2 * live) load_x8<XT, true>(xr + j * 32, v[j]);
+          for (int e = 0; e < 8; ++e) dst[j][e] = 0.0f;
+          if (row < p.m && static_cast<uint32_t>(j) < 2 * chunks_live) load_x8<XT, true>(xr + j * 32, dst[j]);
         }
-        if (p.norm_weight != nullptr) {
+      };
 #pragma unroll
-          for (int j = 0; j < kGroups; ++j) {
-            if (static_cast<uint32_t>(j) < 2 * live) {
-              const float4 a = __ldg(reinterpret_cast<const float4*>(gr + j * 32)), b = __ldg(reinterpret_cast<const float4*>(gr + j * 32 + 4));
-              const float gw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      for (uint32_t tl = 0; tl < kTiles; ++tl) load_slab(tl, chunk0, live, v[tl]);
+      if (p.norm_weight != nullptr) {
+        if (pass == 0 && u0 == unit_first) {
+          // The rows' factors: rows are dealt to the cluster's CTAs, 256 threads a row (shuffle tree, warps in
+          // order), and the CTAs exchange the results.  One order whatever the cut of k, and that of the kernels
+          // which do the norm elsewhere (rms_norm_kernel up to four rows, stage_x_global_kernel above): the same
+          // bits.  A norm factor one ulp off is an error common to a whole row, which a chain of layers amplifies.
+          const uint32_t half = threadIdx.x >> 8, th = threadIdx.x & 255u;
+          for (uint32_t r0 = rank * 2u; r0 < p.m; r0 += p.cluster * 2u) {
+            const uint32_t row = r0 + half;
+            float sq = 0.0f;
+            const XT* xr = static_cast<const XT*>(p.x) + static_cast<size_t>(row) * p.k;
+            if (row < p.m && kPackLo) {
+#pragma unroll 8
+              for (uint32_t i = th; i < p.k; i += 256u) {
+                const float u = to_f32(xr[i]);
+                sq = fmaf(u, u, sq);
+              }
+            } else if (row < p.m) {
+#pragma unroll 2
+              for (uint32_t i = th * 8u; i < p.k; i += 2048u) {
+                float u[8];
+                load_x8<XT, true>(xr + i, u);
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                sq = fmaf(v[j][e], v[j][e], sq);
-                v[j][e] = __fmul_rn(v[j][e], gw[e]);
+                for (int e = 0; e < 8; ++e) sq = fmaf(u[e], u[e], sq);
               }
             }
+            sq = warp_sum(sq);
+            if (lane == 0) squares[row * 8u + (warp & 7u)] = sq;  // rows up to m rounded up: 18 at most
           }
-          sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-          sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-          if (u0 == unit_first && t == 0) {
-            float* mine = squares + warp * 16 + tl * 8 + g;
-            *mine = pass == 0 ? sq : *mine + sq;
+          __syncthreads();
+          const uint32_t mine = (threadIdx.x >> 1) % p.cluster;  // rows 2r, 2r + 1 belong to rank r % cluster
+          if (threadIdx.x < p.m && mine == rank) {
+            float total = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) total += squares[threadIdx.x * 8 + w];
+            row_factor[threadIdx.x] = rsqrtf(total * (1.0f / static_cast<float>(p.k)) + p.norm_eps);
+          }
+          if (p.cluster > 1) {
+            xs_cluster_sync();
+            if (threadIdx.x < p.m && mine != rank)
+              row_factor[threadIdx.x] = xs_ld_rank(static_cast<uint32_t>(__cvta_generic_to_shared(row_factor + threadIdx.x)), mine);
+          }
+          __syncthreads();
+        }
+        const float* gr = p.norm_weight + chunk0 * kChunkK + t * 8u;
+#pragma unroll
+        for (int j = 0; j < kGroups; ++j) {
+          if (static_cast<uint32_t>(j) < 2 * live) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(gr + j * 32)), b = __ldg(reinterpret_cast<const float4*>(gr + j * 32 + 4));
+            const float gw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (uint32_t tl = 0; tl < kTiles; ++tl) {
+              const float r = row_of(tl) < p.m ? row_factor[row_of(tl)] : 0.0f;
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[tl][j][e] = __fmul_rn(__fmul_rn(v[tl][j][e], r), gw[e]);
+            }
           }
         }
+      }
+      uint4 bhi[kTiles][kGroups], blo[kTiles][kLoSet ? kGroups : 1];
+      // -8 sum x of the lane's C columns: the MMA's C operand (rows g and g + 8 alike); packed: one value, added in f32
+      float cterm[kTiles][kGroups][kPackLo ? 1 : 4], inv[kTiles][2];  // ... and the columns' 2^-e
 #pragma unroll
-        for (int j = 0; j < kGroups; ++j) amax = fmaxf(amax, absmax8(v[j]));
+      for (uint32_t tl = 0; tl < kTiles; ++tl) {
+        float amax = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kGroups; ++j) amax = fmaxf(amax, absmax8(v[tl][j]));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         const Pow2 ps = pow2_prescale(amax);
@@ -241,17 +288,13 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
           float sum = 0.0f;
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const float staged = v[j][e] * ((e & 1) ? odd_scale : ps.scale);
+            const float staged = v[tl][j][e] * ((e & 1) ? odd_scale : ps.scale);
             h[e] = __float2half_rn(staged);
             float used = __half2float(h[e]);
             if constexpr (kHasLo) {
               l[e] = __float2half_rn(staged - used);
-              if constexpr (kPackLo) {
-                if (g >= 4u) h[e] = l[e];
-                used = __half2float(h[e]);
-              } else {
-                used += __half2float(l[e]);
-              }
+              used += __half2float(l[e]);
+              if (kPackLo && (g & 1u)) h[e] = l[e];
             }
             sum = fmaf(used, (e & 1) ? 16.0f : 1.0f, sum);
           }
@@ -261,18 +304,23 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
           sum += __shfl_xor_sync(0xffffffffu, sum, 1);
           sum += __shfl_xor_sync(0xffffffffu, sum, 2);
           // column c's sum sits in the lanes of g == c; this lane's C columns are 2t and 2t + 1
-          cterm[tl][j][0] = cterm[tl][j][2] = __shfl_sync(0xffffffffu, sum, 8 * t) * (-8.0f / kUnscale);
-          cterm[tl][j][1] = cterm[tl][j][3] = __shfl_sync(0xffffffffu, sum, 8 * t + 4) * (-8.0f / kUnscale);
+          const float c0 = __shfl_sync(0xffffffffu, sum, 8 * t) * (-8.0f / kUnscale);
+          if constexpr (kPackLo) {
+            cterm[tl][j][0] = c0;
+          } else {
+            cterm[tl][j][0] = cterm[tl][j][2] = c0;
+            cterm[tl][j][1] = cterm[tl][j][3] = __shfl_sync(0xffffffffu, sum, 8 * t + 4) * (-8.0f / kUnscale);
+          }
         }
         inv[tl][0] = __shfl_sync(0xffffffffu, ps.inv, 8 * t);
         inv[tl][1] = __shfl_sync(0xffffffffu, ps.inv, 8 * t + 4);
       }
 
       // ---- stream the row blocks ----
-      for (uint32_t b0 = 0; b0 < blocks; b0 += kXsBatch) {
-        float* red_now = red + ((b0 / kXsBatch) & 1u) * (kXsBatch * kXsWarps * kTiles * 128);
+      for (uint32_t b0 = 0; b0 < blocks; b0 += kBatch) {
+        float* red_now = red + ((b0 / kBatch) & 1u) * (kBatch * kXsWarps * kSums);
 #pragma unroll
-        for (int i = 0; i < kXsBatch; ++i) {
+        for (int i = 0; i < kBatch; ++i) {
           const uint32_t b = b0 + i;
           if (b >= blocks) break;
           float acc[kTiles][4];
@@ -296,37 +344,50 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
 #pragma unroll
               for (uint32_t tl = 0; tl < kTiles; ++tl) {
                 float cf[4];
-                xs_mma_from(cf, a0, bhi[tl][j].x, bhi[tl][j].y, cterm[tl][j]);
-                xs_mma_add(cf, a1, bhi[tl][j].z, bhi[tl][j].w);
-                if constexpr (kLoSet) {
-                  xs_mma_add(cf, a0, blo[tl][j].x, blo[tl][j].y);
-                  xs_mma_add(cf, a1, blo[tl][j].z, blo[tl][j].w);
+                if constexpr (kPackLo) {
+                  mma_f16_zero(cf, a0, bhi[tl][j].x, bhi[tl][j].y);
+                  xs_mma_add(cf, a1, bhi[tl][j].z, bhi[tl][j].w);
+                  acc[tl][0] = fmaf(s.x, (cf[0] + cf[1]) + cterm[tl][j][0], acc[tl][0]);
+                  acc[tl][1] = fmaf(s.y, (cf[2] + cf[3]) + cterm[tl][j][0], acc[tl][1]);
+                } else {
+                  xs_mma_from(cf, a0, bhi[tl][j].x, bhi[tl][j].y, cterm[tl][j]);
+                  xs_mma_add(cf, a1, bhi[tl][j].z, bhi[tl][j].w);
+                  if constexpr (kLoSet) {
+                    xs_mma_add(cf, a0, blo[tl][j].x, blo[tl][j].y);
+                    xs_mma_add(cf, a1, blo[tl][j].z, blo[tl][j].w);
+                  }
+                  acc[tl][0] = fmaf(s.x, cf[0], acc[tl][0]);
+                  acc[tl][1] = fmaf(s.x, cf[1], acc[tl][1]);
+                  acc[tl][2] = fmaf(s.y, cf[2], acc[tl][2]);
+                  acc[tl][3] = fmaf(s.y, cf[3], acc[tl][3]);
                 }
-                acc[tl][0] = fmaf(s.x, cf[0], acc[tl][0]);
-                acc[tl][1] = fmaf(s.x, cf[1], acc[tl][1]);
-                acc[tl][2] = fmaf(s.y, cf[2], acc[tl][2]);
-                acc[tl][3] = fmaf(s.y, cf[3], acc[tl][3]);
               }
             }
           }
           if (b + kXsAhead < blocks) fetch(ring[i % kXsAhead], p.swiglu && (i & 1));
+          float* mine = red_now + (i * kXsWarps + warp) * kSums;
+          if constexpr (kPackLo) {
+            reinterpret_cast<float2*>(mine)[lane] = make_float2(acc[0][0] * inv[0][0], acc[0][1] * inv[0][0]);
+          } else {
 #pragma unroll
-          for (uint32_t tl = 0; tl < kTiles; ++tl)
-            reinterpret_cast<float4*>(red_now + ((i * kXsWarps + warp) * kTiles + tl) * 128)[lane] =
-                make_float4(acc[tl][0] * inv[tl][0], acc[tl][1] * inv[tl][1], acc[tl][2] * inv[tl][0], acc[tl][3] * inv[tl][1]);
+            for (uint32_t tl = 0; tl < kTiles; ++tl)
+              reinterpret_cast<float4*>(mine + tl * 128)[lane] =
+                  make_float4(acc[tl][0] * inv[tl][0], acc[tl][1] * inv[tl][1], acc[tl][2] * inv[tl][0], acc[tl][3] * inv[tl][1]);
+          }
         }
         __syncthreads();
         // the slabs' sums meet, in slab order; the next batch goes to the other buffer
-        // (thread = one of the 128 sums of block warp / 4 of the batch, in every tile)
-        const uint32_t bi = threadIdx.x >> 7, o = threadIdx.x & 127u;
+        // (thread = one of a tile's sums of one block of the batch, in every tile)
+        constexpr uint32_t kTileSums = kSums / kTiles;
+        const uint32_t bi = threadIdx.x / kTileSums, o = threadIdx.x % kTileSums;
         if (b0 + bi < blocks) {
-          const float* src = red_now + bi * (kXsWarps * kTiles * 128) + o;
-          float* dst = part + (b0 + bi) * kTiles * 128 + o;
+          const float* src = red_now + bi * (kXsWarps * kSums) + o;
+          float* dst = part + (b0 + bi) * kSums + o;
 #pragma unroll
           for (uint32_t tl = 0; tl < kTiles; ++tl) {
             float sum = 0.0f;
 #pragma unroll
-            for (int s = 0; s < kXsWarps; ++s) sum += src[(s * kTiles + tl) * 128];
+            for (int s = 0; s < kXsWarps; ++s) sum += src[s * kSums + tl * 128];
             dst[tl * 128] = pass == 0 ? sum : dst[tl * 128] + sum;
           }
         }
@@ -335,45 +396,21 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
     }
 
     // ---- the cluster's sums meet, in rank order, and leave with the neighbours applied ----
-    __syncthreads();
-    if (p.norm_weight != nullptr && u0 == unit_first && threadIdx.x < p.m) {
-      float total = 0.0f;
-      for (uint32_t s = 0; s < kXsWarps; ++s) total += squares[s * 16 + threadIdx.x];
-      row_squares[threadIdx.x] = total;
-    }
     if (p.cluster > 1) xs_cluster_sync();
     else __syncthreads();
-    if (p.norm_weight != nullptr && u0 == unit_first) {
-      if (threadIdx.x < p.m) {
-        const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(row_squares + threadIdx.x));
-        float total = 0.0f;
-        if (p.cluster > 1) for (uint32_t r = 0; r < p.cluster; ++r) total += xs_ld_rank(addr, r);
-        else total = row_squares[threadIdx.x];
-        row_factor[threadIdx.x] = rsqrtf(total * (1.0f / static_cast<float>(p.k)) + p.norm_eps);
-      }
-      __syncthreads();
-    }
     const uint32_t part_addr = static_cast<uint32_t>(__cvta_generic_to_shared(part));
     const uint32_t outs = units_now * p.m * 16u;
     for (uint32_t idx = rank * kXsThreads + threadIdx.x; idx < outs; idx += p.cluster * kXsThreads) {
       const uint32_t r = idx & 15u, um = idx >> 4, ul = um / p.m, mm = um - ul * p.m, unit = u0 + ul;
       const uint32_t col = mm & 7u, tl = mm >> 3;
-      // output (row r, column c) of a tile: lane (r & 7, c / 2), element 2 (r / 8) + c % 2
-      const uint32_t o = ((r & 7u) * 4u + (col >> 1)) * 4u + (r >> 3) * 2u + (col & 1u);
+      // output (row r, column c) of a tile: lane (r & 7, c / 2), element 2 (r / 8) + c % 2; packed: lane (r & 7, row), element r / 8
+      const uint32_t o = kPackLo ? ((r & 7u) * 4u + col) * 2u + (r >> 3) : tl * 128u + ((r & 7u) * 4u + (col >> 1)) * 4u + (r >> 3) * 2u + (col & 1u);
       auto total_of = [&](uint32_t block) {
-        const uint32_t addr = part_addr + ((block * kTiles + tl) * 128u + o) * 4u;
+        const uint32_t at = block * kSums + o;
+        if (p.cluster == 1) return part[at] * kUnscale;
         float sum = 0.0f;
-        for (uint32_t c = 0; c < p.cluster; ++c) {
-          if (p.cluster > 1) {
-            sum += xs_ld_rank(addr, c);
-            if constexpr (kPackLo) sum += xs_ld_rank(addr + 2u * 16u, c);  // column 4 + c: two lanes on
-          } else {
-            sum += part[(block * kTiles + tl) * 128u + o];
-            if constexpr (kPackLo) sum += part[(block * kTiles + tl) * 128u + o + 8u];
-          }
-        }
-        sum *= kUnscale;
-        return p.norm_weight != nullptr ? sum * row_factor[mm] : sum;
+        for (uint32_t c = 0; c < p.cluster; ++c) sum += xs_ld_rank(part_addr + at * 4u, c);
+        return sum * kUnscale;
       };
       if (p.swiglu) {
         const uint32_t row = unit * 16u + r;
@@ -422,7 +459,8 @@ uint32_t resident_clusters(Kernel kernel, uint32_t cluster, int sm_count) {
 template <typename XT, bool kScaleF16, int kForm>
 cudaError_t launch_xs(const LaunchEnv& env, XsParams& p) {
   auto kernel = qgemv_i4_xs_kernel<XT, kScaleF16, kForm>;
-  constexpr uint32_t kTiles = kForm == kSixteen ? 2 : 1, kSlabChunks = kForm == kSixteen ? 1 : 2;
+  using Shape = XsShape<kForm>;
+  constexpr uint32_t kSlabChunks = Shape::slab_chunks;
   struct Setup { bool done; uint32_t resident[kXsMaxCluster + 1]; };
   static PerDevice<Setup> setup_on;
   Setup* setup = setup_on.slot();
@@ -450,11 +488,11 @@ cudaError_t launch_xs(const LaunchEnv& env, XsParams& p) {
     }
   }
   if (best == ~0u) return cudaErrorInvalidConfiguration;
-  const uint32_t units_each = std::min((p.units + p.clusters - 1) / p.clusters, part_blocks(kTiles) / per_unit);
+  const uint32_t units_each = std::min((p.units + p.clusters - 1) / p.clusters, Shape::part_blocks / per_unit);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.clusters * p.cluster);
   cfg.blockDim = dim3(kXsThreads);
-  cfg.dynamicSmemBytes = kXsHead + red_bytes(kTiles) + static_cast<size_t>(units_each) * per_unit * kTiles * 512;
+  cfg.dynamicSmemBytes = kXsHead + Shape::red_bytes + static_cast<size_t>(units_each) * per_unit * Shape::sums * 4;
   cfg.stream = env.stream;
   cudaLaunchAttribute attr[2];
   unsigned int na = 0;
