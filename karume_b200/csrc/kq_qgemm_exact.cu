@@ -165,16 +165,6 @@ template <int kMath>
 __host__ __device__ constexpr uint32_t exact_idesc(uint32_t nt) {
   return (kMath == kInt8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((nt >> 3) << 17) | ((256u >> 4) << 24);
 }
-// Descriptors by their low words (address, leading offset); the high word is the layout's constant.
-constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
-// One lane of a warp, the same one every time.  What a single thread has to do below is a predicated
-// instruction of a converged warp, never a branch: in a divergent lane-0 region the barrier tests and
-// MMA issues took two to three times as long (700 - 850 clocks a k-step whatever its width).
-__device__ __forceinline__ uint32_t elect_lane() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-  return r;
-}
 template <int kMath, bool kAccumulate>
 __device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
   if constexpr (kMath == kInt8)
@@ -185,12 +175,6 @@ __device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t tmem_d, uint3
     asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
                  "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
                  ::"r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHigh), "r"(leader) : "memory");
-}
-// arrives on the barrier at this address in BOTH CTAs of the pair once the MMAs issued so far are done
-__device__ __forceinline__ void commit_both(uint32_t leader, uint32_t bar) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-               ::"r"(bar), "h"(static_cast<uint16_t>(3)), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void arrive_if(uint32_t leader, uint32_t cluster_bar) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}"

@@ -512,54 +512,49 @@ __device__ __forceinline__ void qgemm_body(const GemmParams& p, const CUtensorMa
     }
     }  // fragments
   } else if (cta_rank == 0) {
-    // ---------------- MMA issuer ----------------
+    // ---------------- MMA issuer: predicated instructions of a converged warp ----------------
     constexpr uint32_t kIdesc = umma_idesc(kPair ? 256 : 128, kBN);
+    const uint32_t leader = elect_lane();
+    const uint32_t desc_a0 = static_cast<uint32_t>(umma_desc(tiles));
+    auto mma = [&](auto accumulate, uint32_t acc, uint32_t a, uint32_t b) {
+      constexpr bool kAcc = decltype(accumulate)::value;
+      if constexpr (kPair) umma_bf16_pair<kAcc>(leader, acc, a, b, kIdesc);
+      else umma_bf16_single<kAcc>(leader, acc, a, b, kIdesc);
+    };
+    auto commit = [&](uint32_t bar) {
+      if constexpr (kPair) commit_both(leader, bar);
+      else commit_one(leader, bar);
+    };
+    uint32_t s = 0, phase = 0;
+    bool ready = mbar_try_wait(bars, 0);
     for (uint32_t f = 0; f < frag_count; ++f) {
-    select_fragment(f);
-    if (f != 0) {  // both CTAs have read the previous fragment's sums out of TMEM
-      wait_bounded(tmem_free, (f - 1u) & 1u, abort_flag, p.status, 7);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
-    for (uint32_t ks = 0; ks < ksteps; ++ks) {
-      const uint32_t it = it_base + ks, s = it % kStagesG, phase = (it / kStagesG) & 1u;
-      const bool ok = wait_bounded(bars + s * 8, phase, abort_flag, p.status, 2);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) {
-        const uint32_t a_tile = tiles + s * kStageBytes, b_tile = a_tile + kATileBytes;
+      select_fragment(f);
+      if (f != 0) {  // both CTAs have read the previous fragment's sums out of TMEM
+        wait_bounded(tmem_free, (f - 1u) & 1u, abort_flag, p.status, 7);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      for (uint32_t ks = 0; ks < ksteps; ++ks) {
+        const bool ok = ready || wait_bounded(bars + s * 8, phase, abort_flag, p.status, 2);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a_lo = desc_a0 + s * (kStageBytes >> 4), b_lo = a_lo + (kATileBytes >> 4), stage_empty = bars + (kStagesG + s) * 8;
+        if (++s == kStagesG) { s = 0; phase ^= 1u; }
+        ready = mbar_try_wait(bars + s * 8, phase);  // the next stage's answer is there after these MMAs are issued
         if (ok) {
 #pragma unroll
           for (uint32_t kk = 0; kk < kBK / 16; ++kk) {
-            const uint64_t db = umma_desc(b_tile + kk * 32u);
-            const uint32_t acc = (ks | kk) != 0 ? 1u : 0u;
-            if constexpr (kPair) {
-              umma_bf16_pair(tmem_base, umma_desc(a_tile + kk * 32u), db, kIdesc, acc);
-              umma_bf16_pair(tmem_base + kBN, umma_desc(a_tile + 128u * 128u + kk * 32u), db, kIdesc, acc);
+            if (kk == 0 && ks == 0) {
+              mma(std::false_type{}, tmem_base, a_lo, b_lo);
+              mma(std::false_type{}, tmem_base + kBN, a_lo + ((128u * 128u) >> 4), b_lo);
             } else {
-              umma_bf16(tmem_base, umma_desc(a_tile + kk * 32u), db, kIdesc, acc);
-              umma_bf16(tmem_base + kBN, umma_desc(a_tile + 128u * 128u + kk * 32u), db, kIdesc, acc);
+              mma(std::true_type{}, tmem_base, a_lo + kk * 2u, b_lo + kk * 2u);
+              mma(std::true_type{}, tmem_base + kBN, a_lo + ((128u * 128u) >> 4) + kk * 2u, b_lo + kk * 2u);
             }
           }
         }
-        // the stage is free once these MMAs have read it (in a pair: in both CTAs)
-        if constexpr (kPair) {
-          umma_commit_pair(bars + (kStagesG + s) * 8);
-          umma_commit_pair(map_to_cta(bars + (kStagesG + s) * 8, 1));
-        } else {
-          umma_commit(bars + (kStagesG + s) * 8);
-        }
+        commit(stage_empty);  // the stage is free once these MMAs have read it (in a pair: in both CTAs)
       }
+      commit(bars + 2 * kStagesG * 8);  // all MMAs done: accumulators are final
       __syncwarp();
-    }
-    if (lane == 0) {  // all MMAs done: accumulators are final
-      if constexpr (kPair) {
-        umma_commit_pair(bars + 2 * kStagesG * 8);
-        umma_commit_pair(map_to_cta(bars + 2 * kStagesG * 8, 1));
-      } else {
-        umma_commit(bars + 2 * kStagesG * 8);
-      }
-    }
-    __syncwarp();
-    it_base += ksteps;
     }  // fragments
   }
 

@@ -50,18 +50,6 @@ __host__ __device__ constexpr uint32_t umma_idesc(uint32_t mma_m, uint32_t mma_n
   return (1u << 4) | (1u << 7) | (1u << 10) | ((mma_n >> 3) << 17) | ((mma_m >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 // ---- CTA pairs (cta_group::2): one MMA spans the two CTAs of a cluster -------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -84,19 +72,38 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// M 256 (128 rows per CTA) x N: A and D are each CTA's own rows, B is read half from each CTA.
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+// One lane of a warp, the same one every time.  What a single thread has to do below is a predicated
+// instruction of a converged warp, never a branch: in a divergent lane-0 region the barrier tests and
+// MMA issues took two to three times as long (700 - 850 clocks a k-step whatever its width).
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
-// Arrives on `cluster_bar` (a shared::cluster address: this CTA's barrier, or the peer's through
-// map_to_cta) once the pair's MMAs issued so far are done.
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
+// Descriptors by their low words (address, leading offset); the high word is the layout's constant.
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+// bf16, M 128 x N in one CTA; or M 256 (128 rows per CTA) x N: A and D are each CTA's own rows, B is read half from each.
+template <bool kAccumulate>
+__device__ __forceinline__ void umma_bf16_single(uint32_t leader, uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
+               ::"r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHigh), "r"(leader) : "memory");
+}
+template <bool kAccumulate>
+__device__ __forceinline__ void umma_bf16_pair(uint32_t leader, uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
+               ::"r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHigh), "r"(leader) : "memory");
+}
+// arrives on the barrier at this address in BOTH CTAs of the pair once the MMAs issued so far are done
+__device__ __forceinline__ void commit_both(uint32_t leader, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+               ::"r"(bar), "h"(static_cast<uint16_t>(3)), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void commit_one(uint32_t leader, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+               ::"r"(bar), "r"(leader) : "memory");
 }
 
 // 8 nibbles of one 32-bit word -> 8 bf16 (16 bytes, k ascending), each
