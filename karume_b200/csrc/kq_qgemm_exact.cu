@@ -150,14 +150,24 @@ __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
 }
 
 // ---- tensor memory ---------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_ld16_begin(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
         "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr)
       : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Registers of a finished load: nothing that uses them may be scheduled in front of the wait.
+__device__ __forceinline__ void tmem_ld16_done(uint32_t (&v)[16]) {
+  asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                    "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]));
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  tmem_ld16_begin(taddr, v);
+  tmem_ld_wait();
+  tmem_ld16_done(v);
 }
 
 // kind::f16 with binary16 operands / kind::i8 with signed operands; f32 / s32 accumulate, M 256
@@ -224,16 +234,16 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   const uint32_t bars = tiles + p.stages * p.stage_bytes;
   uint8_t* tail = smem_raw + (tiles - raw_base) + p.stages * p.stage_bytes;
   const uint32_t full = bars, empty = bars + kMaxStages * 8, rawfull = empty + kMaxStages * 8, dfull = rawfull + kMaxStages * 8,
-                 dempty = dfull + 32, sfull = dempty + 32, sempty = sfull + 16;
+                 dempty = dfull + 16, sfull = dempty + 16, sempty = sfull + 16;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(tail + 296);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 304);
   float* row_scale_s = reinterpret_cast<float*>(tail + kTailRowScale);
   float* scale_ring = reinterpret_cast<float*>(tail + kTailScales);
   const uint32_t cta_rank = cluster_ctarank();
-  // Accumulators in tensor memory: four of up to 128 columns or two of up to 256.  From an MMA's issue
-  // to its drain and back are three barrier hops (about 700 clocks), so the narrow form keeps four
-  // chains in flight.
-  const uint32_t acc_shift = p.nt <= kMaxNT / 2 ? 2u : 1u, acc_mask = (1u << acc_shift) - 1u, acc_cols = 512u >> acc_shift;
+  // Tensor memory holds two sets of accumulators, the MMAs fill one while the drain reads the other.  A set is as
+  // many chains as fit half of the 512 columns (one of 256 columns, two of 128, four of 64, eight of 32): a
+  // hand-over costs about 390 clocks whatever it hands over (24 x 4096 -> 9472: 33 us with one chain of 32 columns each).
+  const uint32_t acc_cols = p.nt <= 32 ? 32u : p.nt <= 64 ? 64u : p.nt <= 128 ? 128u : 256u, per_set = 256u / acc_cols;
 
   // which weight, which channels, which activation rows, which k-steps
   const uint32_t pair = blockIdx.x >> 1;
@@ -255,11 +265,9 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         mbar_init(empty + s * 8, 1);                  // one tcgen05.commit
         mbar_init(rawfull + s * 8, 1);                // the raw weights' bytes
       }
-      for (uint32_t b = 0; b < 4; ++b) {
+      for (uint32_t b = 0; b < 2; ++b) {
         mbar_init(dfull + b * 8, 1);
         mbar_init(dempty + b * 8, 2 * kDrainWarps);
-      }
-      for (uint32_t b = 0; b < 2; ++b) {
         mbar_init(sfull + b * 8, 2);
         mbar_init(sempty + b * 8, kDrainWarps);
       }
@@ -316,31 +324,50 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
 #pragma unroll
           for (int j = 0; j < 16; ++j) acc[b][j] = 0.0f;
 #pragma unroll 1
-        for (uint32_t d = 0; d < drains; ++d) {
-          const uint32_t buf = d & acc_mask, batch = d / kScaleBatch;
-          float s = 1.0f;
+        for (uint32_t d0 = 0, set = 0; d0 < drains; d0 += per_set, ++set) {
+          const uint32_t batch = d0 / kScaleBatch, d_end = min(d0 + per_set, drains);  // a set lies inside a batch of scales
           if constexpr (kGroupScales) {
-            if (d % kScaleBatch == 0) wait_bounded(sfull + (batch & 1u) * 8, (batch >> 1) & 1u, abort_flag, p.status, 25);
-            s = my_scale[((batch & 1u) * kScaleBatch + d % kScaleBatch) * kRows];
+            if (d0 % kScaleBatch == 0) wait_bounded(sfull + (batch & 1u) * 8, (batch >> 1) & 1u, abort_flag, p.status, 25);
           }
-          wait_bounded(dfull + buf * 8, (d >> acc_shift) & 1u, abort_flag, p.status, 23);
+          wait_bounded(dfull + (set & 1u) * 8, (set >> 1) & 1u, abort_flag, p.status, 23);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-          for (int b = 0; b < kBatches; ++b) {
-            uint32_t v[16];
-            tmem_ld16(taddr + buf * acc_cols + b * 16u, v);
+          uint32_t at = taddr + (set & 1u) * kMaxNT;
+#pragma unroll 1
+          for (uint32_t d = d0; d < d_end; ++d, at += acc_cols) {
+            [[maybe_unused]] float s = 1.0f;
+            if constexpr (kGroupScales) s = my_scale[((batch & 1u) * kScaleBatch + d % kScaleBatch) * kRows];
             // scalar fused multiply-adds: the packed form (fma.rn.f32x2) needs register pairs the
             // allocator does not find beside 128 sums (measured 460 - 800 clocks a chain against 335)
+            auto add = [&](float (&sums)[16], const uint32_t (&v)[16]) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if constexpr (kGroupScales) acc[b][j] = fmaf(__uint_as_float(v[j]), s, acc[b][j]);
-              else acc[b][j] += __uint_as_float(v[j]);
+              for (int j = 0; j < 16; ++j) {
+                if constexpr (kGroupScales) sums[j] = fmaf(__uint_as_float(v[j]), s, sums[j]);
+                else sums[j] += __uint_as_float(v[j]);
+              }
+            };
+            if constexpr (kBatches <= 4) {  // the chain's columns in flight at once, one wait
+              uint32_t v[kBatches][16];
+#pragma unroll
+              for (int b = 0; b < kBatches; ++b) tmem_ld16_begin(at + b * 16u, v[b]);
+              tmem_ld_wait();
+#pragma unroll
+              for (int b = 0; b < kBatches; ++b) {
+                tmem_ld16_done(v[b]);
+                add(acc[b], v[b]);
+              }
+            } else {
+#pragma unroll
+              for (int b = 0; b < kBatches; ++b) {
+                uint32_t v[16];
+                tmem_ld16(at + b * 16u, v);
+                add(acc[b], v);
+              }
             }
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          arrive_if(leader, dempty_0 + buf * 8);
-          if (kGroupScales) arrive_if(d % kScaleBatch == kScaleBatch - 1 ? leader : 0u, sempty + (batch & 1u) * 8);
+          arrive_if(leader, dempty_0 + (set & 1u) * 8);
+          if (kGroupScales) arrive_if(d_end % kScaleBatch == 0 ? leader : 0u, sempty + (batch & 1u) * 8);
         }
 #pragma unroll
         for (int b = 0; b < kBatches; ++b)
@@ -524,46 +551,47 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         const uint32_t b_step = (p.nt / 2 * 128u) >> 4, stage_step = p.stage_bytes >> 4;
         const uint32_t desc_a0 = static_cast<uint32_t>(umma_desc(tiles)), desc_b0 = static_cast<uint32_t>(umma_desc(tiles + kATile));
         // kSlices: k16 slices per accumulator chain when chains end inside a k-step or with it; 0: longer
-        // chains, of p.drain16 slices.  A barrier test takes the thread some 230 clocks even when the
-        // barrier is long complete, so the next stage's is asked for before this stage's MMAs are issued
-        // and its answer read after them.
+        // chains, of p.drain16 slices
         auto issue = [&](auto slices) {
           constexpr uint32_t kSlices = decltype(slices)::value;
-          uint32_t s = 0, phase = 0, d = 0, in_chain = 0;
-          bool ready = mbar_try_wait(full, 0);
+          uint32_t s = 0, phase = 0, set = 0, in_set = 0, in_chain = 0;
+          auto chain_begins = [&]() {
+            if (in_set == 0 && set >= 2) {  // both CTAs have read the set's previous sums
+              wait_bounded(dempty + (set & 1u) * 8, ((set >> 1) - 1u) & 1u, abort_flag, p.status, 24);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+          };
+          auto chain_ends = [&](bool last) {
+            if (++in_set == per_set || last) {
+              commit_both(leader, dfull + (set & 1u) * 8);
+              ++set;
+              in_set = 0;
+            }
+          };
           for (uint32_t ks = 0; ks < ks_count; ++ks) {
-            if (!ready && !wait_bounded(full + s * 8, phase, abort_flag, p.status, 22)) return;
+            wait_bounded(full + s * 8, phase, abort_flag, p.status, 22);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t desc_a = desc_a0 + s * stage_step, desc_b = desc_b0 + s * stage_step, this_empty = empty + s * 8;
             if (++s == p.stages) { s = 0; phase ^= 1u; }
-            ready = mbar_try_wait(full + s * 8, phase);  // (past the last k-step: an answer nobody reads)
 #pragma unroll
             for (uint32_t kk = 0; kk < 4; ++kk) {
               const bool starts = kSlices != 0 ? kk % (kSlices == 0 ? 1u : kSlices) == 0 : kk == 0 && in_chain == 0;
-              if (kMath != kInt8 && starts && d > acc_mask) {  // both CTAs have read the accumulator's previous sums
-                if (!wait_bounded(dempty + (d & acc_mask) * 8, ((d >> acc_shift) - 1u) & 1u, abort_flag, p.status, 24)) return;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              }
-              const uint32_t dst = tmem + (d & acc_mask) * acc_cols;
+              if (kMath != kInt8 && starts) chain_begins();
+              const uint32_t dst = tmem + (set & 1u) * kMaxNT + in_set * acc_cols;
               if (starts) mma_pair<kMath, false>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
               else mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
               if constexpr (kParts == 2) mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + b_step + kk * 2u, idesc);
-              if (kMath != kInt8 && kSlices != 0 && (kk + 1) % (kSlices == 0 ? 1u : kSlices) == 0) {
-                commit_both(leader, dfull + (d & acc_mask) * 8);
-                ++d;
-              }
+              if (kMath != kInt8 && kSlices != 0 && (kk + 1) % (kSlices == 0 ? 1u : kSlices) == 0) chain_ends(kk == 3 && ks + 1 == ks_count);
             }
             if constexpr (kSlices == 0) {
               in_chain += 4;
-              if (kMath != kInt8 && in_chain == p.drain16) {
-                commit_both(leader, dfull + (d & acc_mask) * 8);
-                ++d;
+              if ((kMath != kInt8 && in_chain == p.drain16) || ks + 1 == ks_count) {  // the last chain may be short
+                chain_ends(ks + 1 == ks_count);
                 in_chain = 0;
               }
             }
             commit_both(leader, this_empty);  // the stage is free, in both CTAs, once these MMAs have read it
           }
-          if (kSlices == 0 && in_chain != 0) commit_both(leader, dfull + (d & acc_mask) * 8);  // a last, short chain
         };
         if (kGroupScales && p.drain16 == 1) issue(std::integral_constant<uint32_t, 1>{});
         else if (kGroupScales && p.drain16 == 2) issue(std::integral_constant<uint32_t, 2>{});

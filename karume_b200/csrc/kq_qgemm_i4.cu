@@ -526,7 +526,6 @@ __device__ __forceinline__ void qgemm_body(const GemmParams& p, const CUtensorMa
       else commit_one(leader, bar);
     };
     uint32_t s = 0, phase = 0;
-    bool ready = mbar_try_wait(bars, 0);
     for (uint32_t f = 0; f < frag_count; ++f) {
       select_fragment(f);
       if (f != 0) {  // both CTAs have read the previous fragment's sums out of TMEM
@@ -534,11 +533,10 @@ __device__ __forceinline__ void qgemm_body(const GemmParams& p, const CUtensorMa
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
       for (uint32_t ks = 0; ks < ksteps; ++ks) {
-        const bool ok = ready || wait_bounded(bars + s * 8, phase, abort_flag, p.status, 2);
+        const bool ok = wait_bounded(bars + s * 8, phase, abort_flag, p.status, 2);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a_lo = desc_a0 + s * (kStageBytes >> 4), b_lo = a_lo + (kATileBytes >> 4), stage_empty = bars + (kStagesG + s) * 8;
         if (++s == kStagesG) { s = 0; phase ^= 1u; }
-        ready = mbar_try_wait(bars + s * 8, phase);  // the next stage's answer is there after these MMAs are issued
         if (ok) {
 #pragma unroll
           for (uint32_t kk = 0; kk < kBK / 16; ++kk) {
