@@ -838,8 +838,7 @@ int kq_quantize_rows(kq_ctx* ctx, uint64_t x_dptr, uint32_t rows, uint32_t dim, 
   if (rows == 0 || dim == 0) return KQ_OK;
   DeviceGuard guard(ctx->device);
   cudaError_t e = kq::launch_quantize_rows(ctx->stream, reinterpret_cast<const float*>(x_dptr), rows, dim,
-                                           reinterpret_cast<int8_t*>(q_dptr), reinterpret_cast<float*>(scale_dptr),
-                                           nullptr, nullptr);
+                                           reinterpret_cast<int8_t*>(q_dptr), reinterpret_cast<float*>(scale_dptr));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "quantize_rows launch");
   ctx->launches += 1;
   return KQ_OK;

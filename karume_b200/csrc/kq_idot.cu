@@ -31,25 +31,47 @@ constexpr float kF32Tiny = 1.1754943508222875e-38f;
 
 __device__ __forceinline__ bool is_nan_bits(float v) { return (__float_as_uint(v) & 0x7fffffffu) > 0x7f800000u; }
 
-// One CTA per row.  Writes q[row, dim] (int8), scale[row], and the integer sums the
-// tensor-core kernels subtract: row_sum[row] = sum q, group_sum[row, dim/32] = sum q over each
-// 32-element group (written only when dim % 32 == 0).
+// clamp(round_ties_even(x / s), -127, 127), the quotient correctly rounded.  x * (1 / s) is within 2e-5 of the
+// quotient wherever the result is not clamped, so unless it lands that close to a tie it rounds to the same
+// integer; the correctly rounded division (some thirty instructions) runs only there, and for NaN.
+__device__ __forceinline__ int quantize_one(float x, float s, float inv) {
+  const float approx = fminf(fmaxf(x * inv, -200.0f), 200.0f);
+  float r = rintf(approx);
+  if (!(fabsf(fabsf(approx - r) - 0.5f) > 1e-4f) || is_nan_bits(x) || inv == 0.0f || !(inv < 1e38f)) r = rintf(__fdiv_rn(x, s));
+  if (!(r >= -127.0f)) r = -127.0f;  // also gives NaN, outside the contract, a fixed value
+  if (r > 127.0f) r = 127.0f;
+  return static_cast<int>(r);
+}
+
+// One CTA per row: q[row, dim] (int8) and scale[row].  Bound by memory: x is read once when a row fits the CTA's
+// registers (kHold float4 per thread), 128 bits at a time (4096 x 2048: 26 us element by element and in two passes).
+template <int kHold>
 __global__ void __launch_bounds__(256)
-quantize_rows_kernel(const float* __restrict__ x, uint32_t rows, uint32_t dim, int8_t* __restrict__ q,
-                     float* __restrict__ scale, int* __restrict__ row_sum, int* __restrict__ group_sum) {
+quantize_rows_kernel(const float* __restrict__ x, uint32_t rows, uint32_t dim, int8_t* __restrict__ q, float* __restrict__ scale) {
   __shared__ float s_max[8];
   __shared__ int s_nan[8];
-  __shared__ int s_sum[8];
-  __shared__ float s_scale;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* xr = x + static_cast<size_t>(row) * dim;
+    int8_t* qr = q + static_cast<size_t>(row) * dim;
+    float4 held[kHold > 0 ? kHold : 1];
     float amax = 0.0f;
     int saw_nan = 0;
-    for (uint32_t i = threadIdx.x; i < dim; i += blockDim.x) {
-      const float v = fabsf(xr[i]);
+    auto look = [&](float f) {
+      const float v = fabsf(f);
       if (is_nan_bits(v)) saw_nan = 1;
       else amax = fmaxf(amax, v);
+    };
+    if constexpr (kHold > 0) {
+#pragma unroll
+      for (int i = 0; i < kHold; ++i) {
+        const uint32_t at = threadIdx.x + i * 256u;
+        held[i] = at * 4u < dim ? __ldcs(reinterpret_cast<const float4*>(xr) + at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+#pragma unroll
+      for (int i = 0; i < kHold; ++i) { look(held[i].x); look(held[i].y); look(held[i].z); look(held[i].w); }
+    } else {
+      for (uint32_t i = threadIdx.x; i < dim; i += 256u) look(xr[i]);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -61,48 +83,30 @@ quantize_rows_kernel(const float* __restrict__ x, uint32_t rows, uint32_t dim, i
       s_nan[warp] = saw_nan;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float a = 0.0f;
-      int nan = 0;
-      for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
-        a = fmaxf(a, s_max[w]);
-        nan |= s_nan[w];
-      }
-      float s = __fmul_rn(a, kInv127);
-      if (s < kF32Tiny) s = kF32Tiny;
-      if (nan) s = __int_as_float(0x7fc00000);
-      s_scale = s;
-      scale[row] = s;
-    }
-    __syncthreads();
-    const float s = s_scale;
-    int local = 0;
-    const uint32_t groups = dim / 32;
-    const bool want_groups = group_sum != nullptr && dim % 32 == 0;
-    // consecutive threads take consecutive elements, so a warp covers exactly one 32-group per pass
-    for (uint32_t i = threadIdx.x; i < ((dim + 31u) & ~31u); i += blockDim.x) {
-      int v = 0;
-      if (i < dim) {
-        float r = rintf(__fdiv_rn(xr[i], s));
-        if (!(r >= -127.0f)) r = -127.0f;  // also gives NaN, outside the contract, a fixed value
-        if (r > 127.0f) r = 127.0f;
-        v = static_cast<int>(r);
-        q[static_cast<size_t>(row) * dim + i] = static_cast<int8_t>(v);
-      }
-      int gs = v;
+    amax = s_max[0];
+    int nan = s_nan[0];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, off);
-      if (want_groups && lane == 0 && i < dim) group_sum[static_cast<size_t>(row) * groups + (i >> 5)] = gs;
-      if (lane == 0) local += gs;
+    for (int w = 1; w < 8; ++w) {
+      amax = fmaxf(amax, s_max[w]);
+      nan |= s_nan[w];
     }
-    if (lane == 0) s_sum[warp] = local;
-    __syncthreads();
-    if (threadIdx.x == 0 && row_sum != nullptr) {
-      int total = 0;
-      for (uint32_t w = 0; w < blockDim.x / 32; ++w) total += s_sum[w];
-      row_sum[row] = total;
+    float s = __fmul_rn(amax, kInv127);
+    if (s < kF32Tiny) s = kF32Tiny;
+    if (nan) s = __int_as_float(0x7fc00000);
+    if (threadIdx.x == 0) scale[row] = s;
+    const float inv = __fdiv_rn(1.0f, s);
+    if constexpr (kHold > 0) {
+#pragma unroll
+      for (int i = 0; i < kHold; ++i) {
+        const uint32_t at = threadIdx.x + i * 256u;
+        if (at * 4u < dim)
+          reinterpret_cast<char4*>(qr)[at] = make_char4(quantize_one(held[i].x, s, inv), quantize_one(held[i].y, s, inv),
+                                                        quantize_one(held[i].z, s, inv), quantize_one(held[i].w, s, inv));
+      }
+    } else {
+      for (uint32_t i = threadIdx.x; i < dim; i += 256u) qr[i] = static_cast<int8_t>(quantize_one(xr[i], s, inv));
     }
-    __syncthreads();
+    __syncthreads();  // s_max / s_nan are rewritten by the next row
   }
 }
 
@@ -347,10 +351,16 @@ __global__ void __launch_bounds__(kIdotWarps * 32) idot_w4a8_tiled_kernel(const 
 
 }  // namespace
 
-cudaError_t launch_quantize_rows(cudaStream_t stream, const float* x, uint32_t rows, uint32_t dim, int8_t* q,
-                                 float* scale, int* row_sum, int* group_sum) {
+cudaError_t launch_quantize_rows(cudaStream_t stream, const float* x, uint32_t rows, uint32_t dim, int8_t* q, float* scale) {
   if (rows == 0) return cudaSuccess;
-  quantize_rows_kernel<<<std::min<uint32_t>(rows, 65535u), 256, 0, stream>>>(x, rows, dim, q, scale, row_sum, group_sum);
+  const uint32_t grid = std::min<uint32_t>(rows, 65535u);
+  const bool vector = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 3u) == 0;
+  if (vector && dim <= 1024u) quantize_rows_kernel<1><<<grid, 256, 0, stream>>>(x, rows, dim, q, scale);
+  else if (vector && dim <= 2048u) quantize_rows_kernel<2><<<grid, 256, 0, stream>>>(x, rows, dim, q, scale);
+  else if (vector && dim <= 4096u) quantize_rows_kernel<4><<<grid, 256, 0, stream>>>(x, rows, dim, q, scale);
+  else if (vector && dim <= 8192u) quantize_rows_kernel<8><<<grid, 256, 0, stream>>>(x, rows, dim, q, scale);
+  else if (vector && dim <= 16384u) quantize_rows_kernel<16><<<grid, 256, 0, stream>>>(x, rows, dim, q, scale);
+  else quantize_rows_kernel<0><<<grid, 256, 0, stream>>>(x, rows, dim, q, scale);
   return cudaGetLastError();
 }
 

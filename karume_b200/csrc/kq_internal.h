@@ -199,8 +199,7 @@ cudaError_t launch_add(const LaunchEnv& env, const float* a, const float* b, flo
 
 // ---- integer-dot linear (kq_idot.cu) ---------------------------------------------------
 namespace kq {
-cudaError_t launch_quantize_rows(cudaStream_t stream, const float* x, uint32_t rows, uint32_t dim, int8_t* q,
-                                 float* scale, int* row_sum, int* group_sum);
+cudaError_t launch_quantize_rows(cudaStream_t stream, const float* x, uint32_t rows, uint32_t dim, int8_t* q, float* scale);
 cudaError_t launch_xq_sums(cudaStream_t stream, const int8_t* q, uint32_t rows, uint32_t dim, int* row_sum,
                            int* group_sum);
 cudaError_t launch_linear_idot(cudaStream_t stream, const Weight& w, const int8_t* xq, const float* xs,

@@ -522,8 +522,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == kCopyWarp) {
       // ---------------- copies ----------------
-      // One thread, two or three tensor copies per k-step: a bulk copy per 16-row block (eight of
-      // them) took 700 - 1000 clocks to start, more than the k-step's MMAs.
+      // One thread, two tensor copies per k-step (both activation parts come with one): a copy takes it about
+      // 100 clocks, and a bulk copy per 16-row block, eight of them, 700 - 1000: more than the k-step's MMAs.
       {
         const uint32_t half_rows = p.nt / 2, b_bytes = half_rows * 128u, raw_bytes = p.raw_bytes;
         const CUtensorMap* w_map = wi == 0 ? &w_map0 : wi == 1 ? &w_map1 : wi == 2 ? &w_map2 : &w_map3;
@@ -536,10 +536,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           expect_tx(cta_rank == 0 ? leader : 0u, full + s * 8, kParts * 2u * b_bytes);
           expect_tx(leader, rawfull + s * 8, raw_bytes);
           copy_tile_2d(leader, a_tile + raw_off, w_map, kstep * w_step, w_row, rawfull + s * 8);
-#pragma unroll
-          for (uint32_t part = 0; part < kParts; ++part)
-            copy_tile_3d(leader, a_tile + kATile + part * b_bytes, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), m0 + cta_rank * half_rows, part,
-                         full_0 + s * 8);
+          copy_tile_3d(leader, a_tile + kATile, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), m0 + cta_rank * half_rows, 0, full_0 + s * 8);
           if (++s == p.stages) { s = 0; phase ^= 1u; }
         }
       }
@@ -790,14 +787,14 @@ EncodeTiled tensor_map_encoder() {
   return encode;
 }
 
-// Activations [parts][m][k] (binary16 or int8), box 128 bytes x `rows` rows, 128-byte swizzle; what lies
-// past k or m reads as zero.
+// Activations [parts][m][k] (binary16 or int8), box 128 bytes x `rows` rows of every part, 128-byte swizzle; what
+// lies past k or m reads as zero.
 cudaError_t encode_x_map(const void* x, bool int8, uint32_t m, uint32_t k, uint32_t parts, uint32_t rows, CUtensorMap* map) {
   EncodeTiled encode = tensor_map_encoder();
   if (encode == nullptr) return cudaErrorNotSupported;
   const cuuint64_t each = int8 ? 1 : 2;
   const cuuint64_t dims[3] = {k, m, parts}, strides[2] = {k * each, static_cast<cuuint64_t>(m) * k * each};
-  const cuuint32_t box[3] = {int8 ? 128u : 64u, rows, 1}, ones[3] = {1, 1, 1};
+  const cuuint32_t box[3] = {int8 ? 128u : 64u, rows, parts}, ones[3] = {1, 1, 1};
   const CUresult r = encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims,
                             strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
