@@ -598,36 +598,79 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       __syncwarp();
     } else if (kGroupScales && warp >= kScaleWarp) {
       // ---------------- scales: global memory -> f32 ring, eight accumulator chains at a time ----------------
+      // Each of the 64 lanes serves two rows.  A batch is fetched into registers as soon as the one before it has
+      // been stored: fetched only once its slot was free, a batch cost two trips to memory and the drain waited
+      // for it (4,600 clocks per eight chains; 24 x 4096 -> 9472: 30 us).
       const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16, drain0 = ks_begin * 4 / p.drain16;
-      const uint32_t each = p.scale_f16 ? 2u : 4u;
       const ExTarget tg = p.t[wi];
-      for (uint32_t d0 = 0, batch = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
-        if (batch >= 2) wait_bounded(sempty + (batch & 1u) * 8, ((batch >> 1) - 1u) & 1u, abort_flag, p.status, 26);
-#pragma unroll 1
-        for (uint32_t rr = 0; rr < 2; ++rr) {
-          const uint32_t r = (warp - kScaleWarp) * 64u + rr * 32u + lane, row = n0 + r;
-          const uint8_t* base;
-          if constexpr (kW == kI4Tiled)
-            base = tg.w + static_cast<size_t>(row >> 4) * (p.k / kChunkK) * raw_unit_bytes<kW, kMath>(p.scale_f16) + kChunkWeightBytes +
-                   ((row & 7u) * 4u + ((row >> 3) & 1u)) * each;
-          else
-            base = static_cast<const uint8_t*>(tg.scale) + static_cast<size_t>(row) * p.groups * each;
-          float v[kScaleBatch];
+      const uint32_t wl = (warp - kScaleWarp) * 32u + lane;
+      if constexpr (kW == kI4Tiled) {
+        // rows 16 (wl / 8) + wl % 8 and + 8: a chunk holds their scales of two groups side by side
+        const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), r = (wl >> 3) * 16u + (wl & 7u), row = n0 + r;
+        const uint8_t* base = tg.w + static_cast<size_t>(row >> 4) * (p.k / kChunkK) * unit + kChunkWeightBytes + (wl & 7u) * (p.scale_f16 ? 8u : 16u);
+        float4 v[kScaleBatch / 2];  // {row, group 0 | row + 8, group 0 | row, group 1 | row + 8, group 1}
+        auto load = [&](uint32_t d0) {
 #pragma unroll
-          for (uint32_t i = 0; i < kScaleBatch; ++i) {
-            const uint32_t grp = (drain0 + d0 + i) >> p.drains_per_group_shift;
-            v[i] = 0.0f;
-            if (row < tg.n && grp < p.groups && d0 + i < drains) {
-              const uint8_t* a = kW == kI4Tiled ? base + static_cast<size_t>(grp >> 1) * raw_unit_bytes<kW, kMath>(p.scale_f16) + (grp & 1u) * 2u * each
-                                                : base + static_cast<size_t>(grp) * each;
-              v[i] = p.scale_f16 ? __half2float(*reinterpret_cast<const __half*>(a)) : *reinterpret_cast<const float*>(a);
+          for (uint32_t i = 0; i < kScaleBatch / 2; ++i) {
+            const uint32_t chunk = (drain0 + d0) / 2 + i;
+            v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (row < tg.n && d0 + 2 * i < drains && chunk < p.k / kChunkK) {
+              const uint8_t* at = base + static_cast<size_t>(chunk) * unit;
+              if (p.scale_f16) {
+                const uint2 raw = __ldg(reinterpret_cast<const uint2*>(at));
+                const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+                v[i] = make_float4(lo.x, lo.y, hi.x, hi.y);
+              } else {
+                v[i] = __ldg(reinterpret_cast<const float4*>(at));
+              }
             }
           }
+        };
+        load(0);
+        for (uint32_t d0 = 0, batch = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
+          if (batch >= 2) wait_bounded(sempty + (batch & 1u) * 8, ((batch >> 1) - 1u) & 1u, abort_flag, p.status, 26);
+          float* ring = scale_ring + (batch & 1u) * (kScaleBatch * kRows) + r;
 #pragma unroll
-          for (uint32_t i = 0; i < kScaleBatch; ++i) scale_ring[((batch & 1u) * kScaleBatch + i) * kRows + r] = v[i];
+          for (uint32_t i = 0; i < kScaleBatch / 2; ++i) {
+            ring[2 * i * kRows] = v[i].x;
+            ring[2 * i * kRows + 8] = v[i].y;
+            ring[(2 * i + 1) * kRows] = v[i].z;
+            ring[(2 * i + 1) * kRows + 8] = v[i].w;
+          }
+          __syncwarp();
+          arrive_if(leader, sfull + (batch & 1u) * 8);
+          load(d0 + kScaleBatch);
         }
-        __syncwarp();
-        arrive_if(leader, sfull + (batch & 1u) * 8);
+      } else {
+        const uint32_t each = p.scale_f16 ? 2u : 4u;
+        float v[2][kScaleBatch];
+        auto load = [&](uint32_t d0) {
+#pragma unroll
+          for (uint32_t rr = 0; rr < 2; ++rr) {
+            const uint32_t row = n0 + wl + rr * 64u;
+            const uint8_t* base = static_cast<const uint8_t*>(tg.scale) + static_cast<size_t>(row) * p.groups * each;
+#pragma unroll
+            for (uint32_t i = 0; i < kScaleBatch; ++i) {
+              const uint32_t grp = (drain0 + d0 + i) >> p.drains_per_group_shift;
+              v[rr][i] = 0.0f;
+              if (row < tg.n && grp < p.groups && d0 + i < drains) {
+                const uint8_t* at = base + static_cast<size_t>(grp) * each;
+                v[rr][i] = p.scale_f16 ? __half2float(*reinterpret_cast<const __half*>(at)) : *reinterpret_cast<const float*>(at);
+              }
+            }
+          }
+        };
+        load(0);
+        for (uint32_t d0 = 0, batch = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
+          if (batch >= 2) wait_bounded(sempty + (batch & 1u) * 8, ((batch >> 1) - 1u) & 1u, abort_flag, p.status, 26);
+#pragma unroll
+          for (uint32_t rr = 0; rr < 2; ++rr)
+#pragma unroll
+            for (uint32_t i = 0; i < kScaleBatch; ++i) scale_ring[((batch & 1u) * kScaleBatch + i) * kRows + wl + rr * 64u] = v[rr][i];
+          __syncwarp();
+          arrive_if(leader, sfull + (batch & 1u) * 8);
+          load(d0 + kScaleBatch);
+        }
       }
     }
   }
