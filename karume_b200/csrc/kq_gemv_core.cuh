@@ -124,23 +124,30 @@ __device__ __forceinline__ void stage_octet(const float (&v)[8], bool valid, uin
   uint4 hi4 = make_uint4(0, 0, 0, 0), lo4 = make_uint4(0, 0, 0, 0);
   float sum = 0.0f;
   if (valid) {
-    __half h[8], l[8];
+    // (e, e + 4) share a register and are converted together: half the conversions of one at a time
+    float used[8];
+    uint32_t hw[4], lw[4];
+    const float odd_scale = ps.scale * 0.0625f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float staged = v[e] * ((e & 1) ? ps.scale * 0.0625f : ps.scale);
-      const float back = (e & 1) ? 16.0f : 1.0f;
-      h[e] = __float2half_rn(staged);
-      const float hf = __half2float(h[e]);
+    for (int e = 0; e < 4; ++e) {
+      const float s0 = v[e] * ((e & 1) ? odd_scale : ps.scale), s1 = v[e + 4] * ((e & 1) ? odd_scale : ps.scale);
+      const __half2 h = __floats2half2_rn(s0, s1);
+      const float2 hf = __half22float2(h);
+      hw[e] = *reinterpret_cast<const uint32_t*>(&h);
+      used[e] = hf.x;
+      used[e + 4] = hf.y;
       if constexpr (kHasLo) {
-        l[e] = __float2half_rn(staged - hf);
-        sum = fmaf(hf + __half2float(l[e]), back, sum);
-      } else {
-        sum = fmaf(hf, back, sum);
+        const __half2 l = __floats2half2_rn(s0 - hf.x, s1 - hf.y);
+        const float2 lf = __half22float2(l);
+        lw[e] = *reinterpret_cast<const uint32_t*>(&l);
+        used[e] += lf.x;
+        used[e + 4] += lf.y;
       }
     }
-    hi4 = make_uint4(pack_half2(h[0], h[4]), pack_half2(h[1], h[5]), pack_half2(h[2], h[6]), pack_half2(h[3], h[7]));
-    if constexpr (kHasLo)
-      lo4 = make_uint4(pack_half2(l[0], l[4]), pack_half2(l[1], l[5]), pack_half2(l[2], l[6]), pack_half2(l[3], l[7]));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sum = fmaf(used[e], (e & 1) ? 16.0f : 1.0f, sum);
+    hi4 = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+    if constexpr (kHasLo) lo4 = make_uint4(lw[0], lw[1], lw[2], lw[3]);
   }
   sum += __shfl_xor_sync(0xffffffffu, sum, 1);
   sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -174,7 +181,7 @@ __device__ __forceinline__ void stage_x(const XT* __restrict__ x, uint32_t m, ui
       for (int e = 0; e < 8; ++e) v[b][e] = 0.0f;
       if (item < items) {
         const uint32_t rest = item >> 2;
-        const uint32_t row = rest % m, lg = rest / m;
+        const uint32_t lg = m == 1 ? rest : rest / m, row = rest - lg * m;
         load_x8<XT, kFromL2>(x + static_cast<size_t>(row) * k + (static_cast<size_t>(group0 + lg) << 5) + ((item & 3u) << 3),
                              v[b]);
       }
@@ -183,9 +190,9 @@ __device__ __forceinline__ void stage_x(const XT* __restrict__ x, uint32_t m, ui
     for (int b = 0; b < kBatch; ++b) {
       const uint32_t item = base + b * blockDim.x;
       if (item >= items_padded) break;  // warp-uniform
-      const uint32_t rest = item >> 2;
-      stage_octet<kHasLo, kCorrStride, kPerGroup>(v[b], item < items, item & 3u, rest % m, rest / m, xs, xs_stride,
-                                                  corr, lo_offset, row_scale);
+      const uint32_t rest = item >> 2, lg = m == 1 ? rest : rest / m, row = rest - lg * m;
+      stage_octet<kHasLo, kCorrStride, kPerGroup>(v[b], item < items, item & 3u, row, lg, xs, xs_stride, corr, lo_offset,
+                                                  row_scale);
     }
   }
 }
@@ -195,17 +202,19 @@ __device__ __forceinline__ void stage_x(const XT* __restrict__ x, uint32_t m, ui
 // is what gets staged.  The sum of squares of a row is taken over the CTA: every thread adds
 // the squares of its own octets in ascending order, a warp adds its lanes with the shuffle
 // tree, and the warps' sums are added in warp order, so every CTA that stages the same x
-// computes the same bits.  `red` is [warps][m] floats of shared memory (`inv` is unused).
+// computes the same bits.  `red` is [kWarps][m] floats of shared memory.
 // When the block fits one round (items <= threads * kBatch, every decode shape) the octets
 // stay in registers between the two passes; otherwise x is read a second time.
-template <typename XT, bool kHasLo, int kCorrStride, bool kFromL2, int kBatch, int kMaxRows>
+// `wv0` holds the norm weights of the thread's first octet (load_first_norm_weights): nothing about
+// them depends on x, so the caller fetches them before it waits for x.
+template <int kWarps, typename XT, bool kHasLo, int kCorrStride, bool kFromL2, int kBatch, int kMaxRows>
 __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const float* __restrict__ weight, float eps,
                                                  uint32_t m, uint32_t k, uint8_t* xs, uint32_t xs_stride, float* corr,
-                                                 float* red, float* inv) {
+                                                 float* red, const float (&wv0)[8]) {
   const uint32_t groups = k >> 5;
   const uint32_t items = groups * m * 4;
   const uint32_t items_padded = (items + 31u) & ~31u;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const bool one_round = items_padded <= blockDim.x * kBatch;
   float v[kBatch][8];
   float sq[kMaxRows];  // m <= kMaxRows
@@ -219,7 +228,7 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
       for (int e = 0; e < 8; ++e) v[b][e] = 0.0f;
       if (item < items) {
         const uint32_t rest = item >> 2;
-        const uint32_t row = rest % m, lg = rest / m;
+        const uint32_t lg = m == 1 ? rest : rest / m, row = rest - lg * m;
         load_x8<XT, kFromL2>(x + static_cast<size_t>(row) * k + (static_cast<size_t>(lg) << 5) + ((item & 3u) << 3), v[b]);
         float s = 0.0f;
 #pragma unroll
@@ -230,15 +239,6 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
       }
     }
   }
-  // the norm weights of the thread's first octet travel while the sums of squares meet
-  float wv0[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (threadIdx.x < items) {
-    const uint32_t lg0 = (threadIdx.x >> 2) / m, q0 = threadIdx.x & 3u;
-    const float4 w0 = __ldg(reinterpret_cast<const float4*>(weight + (lg0 << 5) + (q0 << 3)));
-    const float4 w1 = __ldg(reinterpret_cast<const float4*>(weight + (lg0 << 5) + (q0 << 3) + 4));
-    wv0[0] = w0.x; wv0[1] = w0.y; wv0[2] = w0.z; wv0[3] = w0.w;
-    wv0[4] = w1.x; wv0[5] = w1.y; wv0[6] = w1.z; wv0[7] = w1.w;
-  }
 #pragma unroll
   for (int r = 0; r < kMaxRows; ++r) {
     if (static_cast<uint32_t>(r) < m) {  // uniform
@@ -247,7 +247,6 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
     }
   }
   __syncthreads();
-  (void)inv;
   for (uint32_t base = threadIdx.x; base < items_padded; base += blockDim.x * kBatch) {
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
@@ -255,14 +254,17 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
       if (item >= items_padded) break;  // warp-uniform
       const bool valid = item < items;
       const uint32_t rest = item >> 2;
-      const uint32_t row = rest % m, lg = rest / m, q = item & 3u;
+      const uint32_t lg = m == 1 ? rest : rest / m, row = rest - lg * m, q = item & 3u;
       if (valid) {
         if (!one_round)
           load_x8<XT, kFromL2>(x + static_cast<size_t>(row) * k + (static_cast<size_t>(lg) << 5) + (q << 3), v[b]);
         // every thread adds the warps' sums of its row itself, in warp order: the same bits in
         // every thread and in every CTA
-        float total = 0.0f;
-        for (uint32_t w = 0; w < warps; ++w) total += red[w * m + row];
+        float part[kWarps], total = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) part[w] = red[w * m + row];
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) total += part[w];
         const float r_inv = rsqrtf(total * (1.0f / static_cast<float>(k)) + eps);
         float wv[8];
         if (item == threadIdx.x) {
@@ -282,6 +284,17 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
   }
 }
 
+
+// The norm weights of the thread's first octet of a block staged by stage_x_rms_norm.
+__device__ __forceinline__ void load_first_norm_weights(const float* __restrict__ weight, uint32_t m, uint32_t k, float (&wv0)[8]) {
+  const uint32_t rest = threadIdx.x >> 2, lg = m == 1 ? rest : rest / m;
+  if (lg < k >> 5) {
+    const float4 w0 = __ldg(reinterpret_cast<const float4*>(weight + (lg << 5) + ((threadIdx.x & 3u) << 3)));
+    const float4 w1 = __ldg(reinterpret_cast<const float4*>(weight + (lg << 5) + ((threadIdx.x & 3u) << 3) + 4));
+    wv0[0] = w0.x; wv0[1] = w0.y; wv0[2] = w0.z; wv0[3] = w0.w;
+    wv0[4] = w1.x; wv0[5] = w1.y; wv0[6] = w1.z; wv0[7] = w1.w;
+  }
+}
 
 // Shared loads that leave the destination untouched where the predicate is false: the
 // registers of lanes whose MMA column holds no activation row stay zero for the whole

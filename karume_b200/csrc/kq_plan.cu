@@ -41,6 +41,9 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 // paired kernel, in the activation staging (norm) and in the epilogue (the rest).
 constexpr uint32_t kOpSwiglu = 1u;  // weights (gate, up): out[0] = silu(x.Wg^T + bg) * (x.Wu^T + bu)
 constexpr uint32_t kOpReduce = 2u;  // row-parallel shard: the outputs are added across ranks
+// No op of the plan writes this op's biases or norm weights: they are fetched while the CTA waits for the
+// previous op.
+constexpr uint32_t kOpEarlyParams = 4u;
 
 struct PlanOpDev {
   const uint8_t* w[kMaxMulti];
@@ -106,6 +109,16 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// The two copies of a piece and their byte count, by one lane of a converged warp (predicated: no branch).
+__device__ __forceinline__ void bulk_pair_g2s(bool leader, uint32_t dst0, const void* src0, uint32_t dst1, const void* src1,
+                                              uint32_t bytes_each, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t"
+               "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%6], %7;\n\t"
+               "@p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2], %5, [%6];\n\t"
+               "@p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%3], [%4], %5, [%6];\n\t}"
+               ::"r"(static_cast<uint32_t>(leader)), "r"(dst0), "l"(src0), "r"(dst1), "l"(src1), "r"(bytes_each), "r"(bar),
+               "r"(2u * bytes_each) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
@@ -801,13 +814,13 @@ plan_pair_kernel(const PlanParams p) {
   // there would sit on every warp's critical path.
   PlanOpDev* win = reinterpret_cast<PlanOpDev*>(
       (reinterpret_cast<uintptr_t>(red + 2 * kPlanWarps * 2 * p.m * 16) + 15) & ~static_cast<uintptr_t>(15));
-  auto fill_window = [&](uint32_t idx) {
+  auto fill_window = [&](uint32_t idx, uint32_t thread) {
     if (idx >= p.op_count) return;
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(p.ops + idx);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(win + idx % kOpWindow);
-    for (uint32_t i = threadIdx.x; i < sizeof(PlanOpDev) / 4; i += blockDim.x) dst[i] = __ldg(src + i);
+    static_assert(sizeof(PlanOpDev) / 4 <= (kPlanWarps - 1) * 32, "one word a thread, warp 0 left out");
+    if (thread < sizeof(PlanOpDev) / 4)
+      reinterpret_cast<uint32_t*>(win + idx % kOpWindow)[thread] = __ldg(reinterpret_cast<const uint32_t*>(p.ops + idx) + thread);
   };
-  for (uint32_t i = 0; i + 2 <= kOpWindow; ++i) fill_window(i);  // entries 0 .. kOpWindow - 2
+  for (uint32_t i = 0; i + 2 <= kOpWindow; ++i) fill_window(i, threadIdx.x);  // entries 0 .. kOpWindow - 2
   uint32_t cur_op = 0;  // the op this warp is working on; entries up to cur_op + kOpWindow - 2 are valid
   auto desc = [&](uint32_t idx) -> const PlanOpDev& {
     return idx + 2 <= cur_op + kOpWindow ? win[idx % kOpWindow] : p.ops[idx];
@@ -842,13 +855,10 @@ plan_pair_kernel(const PlanParams p) {
     }
     const uint32_t nc = min(static_cast<uint32_t>(kPiece), prod_left);
     const uint32_t slot = prod_q & (kNS - 1);
-    if (lane == 0) {
-      mbar_expect_tx(bars + slot * 8, 2u * nc * kCB);
-      bulk_copy_g2s(ring + slot * kSlotBytes, prod_src, nc * kCB, bars + slot * 8);
-      const long long delta = prod_stride16 != kStrideInDescriptor ? static_cast<long long>(prod_stride16) * 16
-                                                                   : desc(prod_op).gate_up_delta;
-      bulk_copy_g2s(ring + slot * kSlotBytes + kPiece * kCB, prod_src + delta, nc * kCB, bars + slot * 8);
-    }
+    const long long delta = prod_stride16 != kStrideInDescriptor ? static_cast<long long>(prod_stride16) * 16
+                                                                 : desc(prod_op).gate_up_delta;
+    bulk_pair_g2s(lane == 0, ring + slot * kSlotBytes, prod_src, ring + slot * kSlotBytes + kPiece * kCB, prod_src + delta, nc * kCB,
+                  bars + slot * 8);
     prod_src += nc * kCB;
     prod_left -= nc;
     prod_q += 1;
@@ -941,9 +951,21 @@ plan_pair_kernel(const PlanParams p) {
     // Nothing about the first item depends on the previous op: look it up before the wait.
     const PairItem first_item = pair_item_of<kCB>(win[op % kOpWindow], 0, warp, grid, cta);
     trace_stamp(p, op, kTraceOpBegin);
+    // What the op's parameters say is fetched before the wait as well.
+    const PlanOpDev& o = win[op % kOpWindow];
+    float bias_first = 0.0f, norm_first[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // the bias of a split op's pair: lane = row of the pair (SiLU gate: of the gate's, then of the up weight's block)
+    auto load_bias = [&](const PairItem& it, uint32_t local_row) {
+      if (!it.valid) return 0.0f;
+      const bool up = (o.flags & kOpSwiglu) != 0 && lane >= 16u;
+      return (up ? o.bias[1] - 16 : o.bias[it.wi])[local_row + lane];
+    };
+    auto load_early = [&]() {
+      if (o.slabs != 1) bias_first = load_bias(first_item, (first_item.rb - o.rb_begin[first_item.wi]) * 16u);
+      if (o.norm_weight != nullptr) load_first_norm_weights(o.norm_weight, p.m, o.k, norm_first);
+    };
+    if (o.flags & kOpEarlyParams) load_early();
     if (op > 0) {
-      // Slot (op - 2) % kOpWindow is dead: every warp passed the barrier of op - 1.
-      fill_window(op + kOpWindow - 2);
       // every output of the previous op must be complete and visible before x is read
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -958,17 +980,20 @@ plan_pair_kernel(const PlanParams p) {
             break;
           }
         }
+      } else if (warp != 0) {
+        // Slot (op - 2) % kOpWindow is dead: every warp passed the barrier of op - 1.
+        fill_window(op + kOpWindow - 2, threadIdx.x - 32u);
       }
       __syncthreads();
     }
+    if (!(o.flags & kOpEarlyParams)) load_early();
     cur_op = op;
-    const PlanOpDev& o = win[op % kOpWindow];
     trace_stamp(p, op, kTraceBarrier);
     if (o.norm_weight != nullptr) {
       // no reduction of the previous op is in flight any more: its buffers serve as scratch
       float* scratch = red + static_cast<size_t>(red_buf) * kPlanWarps * (2 * p.m * 16);
-      stage_x_rms_norm<XT, kHasLo, kCorrStride, true, 4, 4>(static_cast<const XT*>(o.x), o.norm_weight, o.norm_eps, p.m, o.k,
-                                                            xs, kXsStride, corr, scratch, scratch + kPlanWarps * p.m);
+      stage_x_rms_norm<kPlanWarps, XT, kHasLo, kCorrStride, true, 4, 4>(static_cast<const XT*>(o.x), o.norm_weight, o.norm_eps, p.m,
+                                                                        o.k, xs, kXsStride, corr, scratch, norm_first);
     } else {
       stage_x<XT, kHasLo, kCorrStride, true, 4>(static_cast<const XT*>(o.x), p.m, o.k, 0, o.k >> 5, xs, kXsStride, corr);
     }
@@ -982,22 +1007,22 @@ plan_pair_kernel(const PlanParams p) {
       for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int j = 0; j < kAcc; ++j) acc[r][j] = 0.0f;
-      // (1) the bias of the rows this lane will store, fetched while the weights are consumed
+      // the bias (and residual) of the rows this lane will store, fetched while the weights are consumed
       const uint32_t local_row = (it.rb - o.rb_begin[it.wi]) * 16u;  // first row of the pair inside its weight
-      float bias_pre[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      if (it.valid) {
-        const float* bias = o.bias[it.wi];
-        const float* bias2 = (o.flags & kOpSwiglu) ? o.bias[1] : bias + 16;  // bias of the pair's second block
-        if (o.slabs == 1) {
+      float bias_pre[4] = {bias_first, 0.0f, 0.0f, 0.0f};
+      if (slabs == 1) {
+        if (it.valid) {
+          const float* bias = o.bias[it.wi];
+          const float* bias2 = (o.flags & kOpSwiglu) ? o.bias[1] : bias + 16;  // bias of the pair's second block
           bias_pre[0] = bias[local_row + g];
           bias_pre[1] = bias[local_row + g + 8];
           bias_pre[2] = bias2[local_row + g];
           bias_pre[3] = bias2[local_row + g + 8];
-        } else if (!(o.flags & kOpSwiglu)) {
-          bias_pre[0] = bias[local_row + lane];  // the reducer's first pass covers rows lane of the pair
-          // ... and so does its residual (one activation row: output index == row)
-          if (p.m == 1 && o.residual[it.wi] != nullptr) bias_pre[1] = o.residual[it.wi][local_row + lane];
         }
+      } else {
+        if (round != 0) bias_pre[0] = load_bias(it, local_row);
+        // (one activation row: output index == row)
+        if (it.valid && p.m == 1 && o.residual[it.wi] != nullptr) bias_pre[1] = o.residual[it.wi][local_row + lane];
       }
 
       for (uint32_t first = 0; first < it.nck; first += kPiece) {
@@ -1042,7 +1067,7 @@ plan_pair_kernel(const PlanParams p) {
       const bool owner = jl == 0;
       // Ops with a SiLU gate, a residual or a cross-rank reduce finish in functions of their own
       // (not inlined: their registers must not weigh on the loop above); plain ops store here.
-      const bool plain = o.flags == 0 && o.residual[it.wi] == nullptr;
+      const bool plain = (o.flags & (kOpSwiglu | kOpReduce)) == 0 && o.residual[it.wi] == nullptr;
       if (slabs == 1) {
         if (it.nck != 0 && owner) {
 #pragma unroll
@@ -1081,7 +1106,25 @@ plan_pair_kernel(const PlanParams p) {
       __syncthreads();
       if ((warp & (slabs - 1u)) == 0 && it.valid) {
         const float* first_slab = mine;
-        if (plain) {
+        if (p.m == 1 && (o.flags & kOpReduce) == 0) {
+          // One activation row: lane = row of the pair.  Short and inline: the general function below is
+          // cold code in every op and cost 2,100 clocks of a 4096 x 4096 op's 12,000.
+          float v;
+          if (plain) {
+            v = first_slab[lane];
+            for (uint32_t sl = 1; sl < slabs; ++sl) v += first_slab[sl * 32u + lane];
+          } else {
+            v = sum_slabs(first_slab + lane, slabs, 32u);
+          }
+          v = fmaf(v, kUnscale, bias_pre[0]);
+          if (o.flags & kOpSwiglu) {
+            const float up = __shfl_down_sync(0xffffffffu, v, 16);
+            if (lane < 16u) o.out[0][local_row + lane] = silu_mul(v, up);
+          } else {
+            if (!plain) v = __fadd_rn(v, bias_pre[1]);
+            o.out[it.wi][local_row + lane] = v;
+          }
+        } else if (plain) {
           const uint32_t n_i = o.n[it.wi];
           float* out = o.out[it.wi];
           const float* bias = o.bias[it.wi];
@@ -1090,9 +1133,7 @@ plan_pair_kernel(const PlanParams p) {
             for (uint32_t sl = 0; sl < slabs; ++sl) total += first_slab[static_cast<size_t>(sl) * (2 * p.m * 16) + idx];
             const uint32_t r = idx / (p.m * 16), rem = idx - r * (p.m * 16);
             const uint32_t mm = rem >> 4, row = local_row + r * 16 + (rem & 15u);
-            // idx == lane in the first pass: row r * 16 + (lane & 15) of activation row 0 when m == 1
-            const float b = (idx == lane && p.m == 1) ? bias_pre[0] : bias[row];
-            out[static_cast<size_t>(mm) * n_i + row] = fmaf(total, kUnscale, b);
+            out[static_cast<size_t>(mm) * n_i + row] = fmaf(total, kUnscale, bias[row]);
           }
         } else {
           finish_fused_slabs(&o, it.wi, first_slab, slabs, p.m, local_row, lane, bias_pre[0], bias_pre[1], p.fcomm, p.status);
@@ -1295,6 +1336,34 @@ void shape_op(PlanOpDev& o, uint32_t grid, uint32_t unit_chunks, bool paired, ui
   *rot = (*rot + o.cta_items) % grid;  // the next op starts where this one left the grid idle
 }
 
+// Biases and norm weights are read ahead of the barrier unless some op of the plan writes them.
+void mark_early_params(Plan& plan) {
+  std::vector<std::pair<uintptr_t, uintptr_t>> written;  // merged, ascending [begin, end)
+  for (const PlanOpDev& o : plan.ops)
+    for (uint32_t i = 0; i < ((o.flags & kOpSwiglu) ? 1u : o.count); ++i) {
+      const uintptr_t at = reinterpret_cast<uintptr_t>(o.out[i]);
+      if (at != 0) written.emplace_back(at, at + static_cast<uintptr_t>(plan.m) * o.n[i] * sizeof(float));
+    }
+  std::sort(written.begin(), written.end());
+  size_t kept = 0;
+  for (const auto& r : written) {
+    if (kept != 0 && r.first <= written[kept - 1].second) written[kept - 1].second = std::max(written[kept - 1].second, r.second);
+    else written[kept++] = r;
+  }
+  written.resize(kept);
+  auto overlaps = [&](const float* p, size_t values) {
+    if (p == nullptr) return false;
+    const uintptr_t begin = reinterpret_cast<uintptr_t>(p), end = begin + values * sizeof(float);
+    auto next = std::lower_bound(written.begin(), written.end(), std::make_pair(end, uintptr_t{0}));  // first that begins at or past end
+    return next != written.begin() && std::prev(next)->second > begin;
+  };
+  for (PlanOpDev& o : plan.ops) {
+    bool safe = !overlaps(o.norm_weight, o.k);
+    for (uint32_t i = 0; i < o.count; ++i) safe = safe && !overlaps(o.bias[i], o.n[i]);
+    if (safe) o.flags |= kOpEarlyParams;
+  }
+}
+
 bool fill_op(PlanOpDev& o, int count, const LinearTarget* targets, const void* x, const LinearFusion& fusion,
              const char** why) {
   o = PlanOpDev{};
@@ -1438,6 +1507,7 @@ cudaError_t plan_finalize(Plan* plan, const LaunchEnv& env, const char** why) {
     }
     plan->fcomm = env.fused;
   }
+  mark_early_params(*plan);
   uint32_t rot = 0;
   for (PlanOpDev& o : plan->ops) shape_op(o, static_cast<uint32_t>(plan->grid), plan->unit_chunks, plan->paired, &rot);
   e = cudaMalloc(reinterpret_cast<void**>(&plan->ops_dev), plan->ops.size() * sizeof(PlanOpDev));
