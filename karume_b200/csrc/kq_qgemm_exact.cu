@@ -930,19 +930,21 @@ cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, uint3
   return cudaErrorInvalidValue;
 }
 
-// Clocks of one k-step of a tile of `nt` activation rows, as measured (full machine, one tile per pair):
-// the slowest of the tensor core, the thread that issues (100 an MMA, 350 a chain's barrier), the
-// drain (300 and two a column a chain) and the conversion of the weight tile.
+// Clocks of one k-step, fitted to timings of 30 shapes (17 to 1024 rows; within 15 % of them).  The
+// activation tile's copy and the MMAs grow with the tile and its parts, the conversion of the weights does
+// not; a drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step
+// (nt = 256, group 32: 1,900).  int4, group 32, two parts: 750 at nt = 32, 1,010 at 64, 1,250 at 128, 1,600 at 192, 2,060 at 256.
 uint32_t kstep_clocks(uint32_t nt, uint32_t parts, uint32_t drains_x4, bool int8) {
   const uint32_t mma = 4 * parts * std::max(nt / 2, 48u);
-  const uint32_t thread = 400 + 400 * parts + (int8 ? 0u : drains_x4 * 350 / 4);
-  const uint32_t drain = int8 ? 0u : drains_x4 * (nt * 2 + 300) / 4;
-  return std::max({mma, thread, drain, 500u});
+  const uint32_t step = (int8 ? 550 : 450) + 100 * parts + nt * parts + (int8 ? 0u : drains_x4 * (nt * 8 / 5 + 20) / 4);
+  const uint32_t drain = int8 ? 0u : drains_x4 * std::max(nt * 7 / 2 + 60, 330u) / 4;
+  return std::max({mma, step, drain});
 }
 
 struct Geometry { uint32_t nt, m_tiles, splits; };
 // Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
-// loads, epilogue) plus its k-steps; a split adds the reduce launch and the partial sums' traffic.
+// loads, epilogue) plus its k-steps; a split adds the reduce launch and the partial sums, written and read
+// at 2,200 bytes per clock.  (Priced at 4,000, 1024 x 4096 -> 6144 was cut in two at nt = 256: 174 us, 118 now.)
 Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t ksteps, uint32_t parts, uint32_t drain16, bool int8,
                          uint32_t slice_unit, bool may_split, uint32_t sm_pairs, uint64_t partial_room) {
   Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1};
@@ -960,7 +962,7 @@ Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t 
       each = (each + slice_unit - 1) / slice_unit * slice_unit;
       const uint64_t waves = (static_cast<uint64_t>(pairs) * mt * splits + sm_pairs - 1) / sm_pairs;
       uint64_t cost = waves * (5000 + nt * 30 + static_cast<uint64_t>(each) * per);
-      if (splits > 1) cost += 4000 + static_cast<uint64_t>(m) * n_total * (splits + 1) * 4 / 4000;
+      if (splits > 1) cost += 5500 + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
       if (cost < best_cost) {
         best_cost = cost;
         best = {nt, mt, splits};
