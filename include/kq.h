@@ -196,13 +196,12 @@ KQ_API int kq_model_tensor_info(kq_model model, const char* key, char* dtype8, u
  * The kernel is a pure function of (storage, shape, m, x_dtype) — never autotuned,
  * like the reference's geometry table
  * (packages/runtime/src/kernels/gemm-geometry.ts:243-267).
- * More than 16 rows on a tiled int4 weight run on the tcgen05 tensor cores: bf16 activations
- * with operands rounded to bf16 once (results within rtol 1e-3, atol 1e-4 * rms of the oracle
- * on bf16-rounded operands), f32 / binary16 activations with both operands carried as two bf16
- * numbers (the decode contract, atol 4e-5 * max(1, rms) for f32 activations).  A tiled int8
- * weight with k % 64 == 0 takes the same bf16 kernel and contract; its other cases, and
- * everything up to 16 rows, keep atol 1e-5 * max(1, rms), rtol 1e-3 against the f64-accumulate
- * reference. */
+ * More than 16 rows run on the tcgen05 tensor cores.  bf16 activations on a tiled weight
+ * (int4, or int8 with k % 64 == 0) have operands rounded to bf16 once (results within rtol
+ * 1e-3, atol 1e-4 * rms of the oracle on bf16-rounded operands).  Everything else enters with
+ * its weights as exact integers and its activations exact or as two binary16 parts, the group
+ * scales applied in f32: the decode contract.  That contract, for everything up to 16 rows
+ * too, is atol 1e-5 * max(1, rms), rtol 1e-3 against the f64-accumulate reference. */
 KQ_API int kq_linear(kq_ctx* ctx, kq_weight w, uint64_t x_dptr, int x_dtype, uint64_t bias_dptr,
                      uint64_t out_dptr, uint32_t m);
 
