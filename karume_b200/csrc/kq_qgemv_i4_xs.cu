@@ -341,25 +341,30 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
               float2 s;
               if constexpr (kScaleF16) s = __half22float2(*reinterpret_cast<const __half2*>(jj ? &ch.s.y : &ch.s.x));
               else s = jj ? make_float2(__uint_as_float(ch.s.z), __uint_as_float(ch.s.w)) : make_float2(__uint_as_float(ch.s.x), __uint_as_float(ch.s.y));
+              // (the tiles' chains side by side: each MMA of a chain waits for the one before it)
+              float cf[kTiles][4];
+              if constexpr (kPackLo) {
+                mma_f16_zero(cf[0], a0, bhi[0][j].x, bhi[0][j].y);
+                xs_mma_add(cf[0], a1, bhi[0][j].z, bhi[0][j].w);
+                acc[0][0] = fmaf(s.x, (cf[0][0] + cf[0][1]) + cterm[0][j][0], acc[0][0]);
+                acc[0][1] = fmaf(s.y, (cf[0][2] + cf[0][3]) + cterm[0][j][0], acc[0][1]);
+              } else {
 #pragma unroll
-              for (uint32_t tl = 0; tl < kTiles; ++tl) {
-                float cf[4];
-                if constexpr (kPackLo) {
-                  mma_f16_zero(cf, a0, bhi[tl][j].x, bhi[tl][j].y);
-                  xs_mma_add(cf, a1, bhi[tl][j].z, bhi[tl][j].w);
-                  acc[tl][0] = fmaf(s.x, (cf[0] + cf[1]) + cterm[tl][j][0], acc[tl][0]);
-                  acc[tl][1] = fmaf(s.y, (cf[2] + cf[3]) + cterm[tl][j][0], acc[tl][1]);
-                } else {
-                  xs_mma_from(cf, a0, bhi[tl][j].x, bhi[tl][j].y, cterm[tl][j]);
-                  xs_mma_add(cf, a1, bhi[tl][j].z, bhi[tl][j].w);
-                  if constexpr (kLoSet) {
-                    xs_mma_add(cf, a0, blo[tl][j].x, blo[tl][j].y);
-                    xs_mma_add(cf, a1, blo[tl][j].z, blo[tl][j].w);
-                  }
-                  acc[tl][0] = fmaf(s.x, cf[0], acc[tl][0]);
-                  acc[tl][1] = fmaf(s.x, cf[1], acc[tl][1]);
-                  acc[tl][2] = fmaf(s.y, cf[2], acc[tl][2]);
-                  acc[tl][3] = fmaf(s.y, cf[3], acc[tl][3]);
+                for (uint32_t tl = 0; tl < kTiles; ++tl) xs_mma_from(cf[tl], a0, bhi[tl][j].x, bhi[tl][j].y, cterm[tl][j]);
+#pragma unroll
+                for (uint32_t tl = 0; tl < kTiles; ++tl) xs_mma_add(cf[tl], a1, bhi[tl][j].z, bhi[tl][j].w);
+                if constexpr (kLoSet) {
+#pragma unroll
+                  for (uint32_t tl = 0; tl < kTiles; ++tl) xs_mma_add(cf[tl], a0, blo[tl][j].x, blo[tl][j].y);
+#pragma unroll
+                  for (uint32_t tl = 0; tl < kTiles; ++tl) xs_mma_add(cf[tl], a1, blo[tl][j].z, blo[tl][j].w);
+                }
+#pragma unroll
+                for (uint32_t tl = 0; tl < kTiles; ++tl) {
+                  acc[tl][0] = fmaf(s.x, cf[tl][0], acc[tl][0]);
+                  acc[tl][1] = fmaf(s.x, cf[tl][1], acc[tl][1]);
+                  acc[tl][2] = fmaf(s.y, cf[tl][2], acc[tl][2]);
+                  acc[tl][3] = fmaf(s.y, cf[tl][3], acc[tl][3]);
                 }
               }
             }
