@@ -88,6 +88,14 @@ __device__ __forceinline__ float absmax8(const float (&v)[8]) {
   return a;
 }
 
+// rest / m, where 1 <= m <= kMaxRows (a division by a variable is 20 instructions and a handful of registers)
+template <int kMaxRows>
+__device__ __forceinline__ uint32_t group_of(uint32_t rest, uint32_t m) {
+  if constexpr (kMaxRows == 1) return rest;
+  if constexpr (kMaxRows == 2) return rest >> (m - 1u);
+  return m == 1 ? rest : rest / m;
+}
+
 // Stages groups [group0, group0 + groups) of x into shared memory.
 //   xs   : [local group][active columns][32 halfs]; activation row r occupies column r
 //          (binary16 input) or columns 2r (hi) and 2r+1 (lo).  The 8 values of each
@@ -181,7 +189,7 @@ __device__ __forceinline__ void stage_x(const XT* __restrict__ x, uint32_t m, ui
       for (int e = 0; e < 8; ++e) v[b][e] = 0.0f;
       if (item < items) {
         const uint32_t rest = item >> 2;
-        const uint32_t lg = m == 1 ? rest : rest / m, row = rest - lg * m;
+        const uint32_t lg = group_of<kCorrStride>(rest, m), row = rest - lg * m;
         load_x8<XT, kFromL2>(x + static_cast<size_t>(row) * k + (static_cast<size_t>(group0 + lg) << 5) + ((item & 3u) << 3),
                              v[b]);
       }
@@ -228,7 +236,7 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
       for (int e = 0; e < 8; ++e) v[b][e] = 0.0f;
       if (item < items) {
         const uint32_t rest = item >> 2;
-        const uint32_t lg = m == 1 ? rest : rest / m, row = rest - lg * m;
+        const uint32_t lg = group_of<kMaxRows>(rest, m), row = rest - lg * m;
         load_x8<XT, kFromL2>(x + static_cast<size_t>(row) * k + (static_cast<size_t>(lg) << 5) + ((item & 3u) << 3), v[b]);
         float s = 0.0f;
 #pragma unroll
@@ -254,17 +262,21 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
       if (item >= items_padded) break;  // warp-uniform
       const bool valid = item < items;
       const uint32_t rest = item >> 2;
-      const uint32_t lg = m == 1 ? rest : rest / m, row = rest - lg * m, q = item & 3u;
+      const uint32_t lg = group_of<kMaxRows>(rest, m), row = rest - lg * m, q = item & 3u;
       if (valid) {
         if (!one_round)
           load_x8<XT, kFromL2>(x + static_cast<size_t>(row) * k + (static_cast<size_t>(lg) << 5) + (q << 3), v[b]);
         // every thread adds the warps' sums of its row itself, in warp order: the same bits in
         // every thread and in every CTA
-        float part[kWarps], total = 0.0f;
+        float total = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) part[w] = red[w * m + row];
+        for (int w = 0; w < kWarps; w += 4) {
+          float part[4];
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) total += part[w];
+          for (int i = 0; i < 4; ++i) part[i] = red[(w + i) * m + row];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) total += part[i];
+        }
         const float r_inv = rsqrtf(total * (1.0f / static_cast<float>(k)) + eps);
         float wv[8];
         if (item == threadIdx.x) {
@@ -286,8 +298,9 @@ __device__ __forceinline__ void stage_x_rms_norm(const XT* __restrict__ x, const
 
 
 // The norm weights of the thread's first octet of a block staged by stage_x_rms_norm.
+template <int kMaxRows>
 __device__ __forceinline__ void load_first_norm_weights(const float* __restrict__ weight, uint32_t m, uint32_t k, float (&wv0)[8]) {
-  const uint32_t rest = threadIdx.x >> 2, lg = m == 1 ? rest : rest / m;
+  const uint32_t lg = group_of<kMaxRows>(threadIdx.x >> 2, m);
   if (lg < k >> 5) {
     const float4 w0 = __ldg(reinterpret_cast<const float4*>(weight + (lg << 5) + ((threadIdx.x & 3u) << 3)));
     const float4 w1 = __ldg(reinterpret_cast<const float4*>(weight + (lg << 5) + ((threadIdx.x & 3u) << 3) + 4));

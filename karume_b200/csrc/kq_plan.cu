@@ -821,9 +821,9 @@ plan_pair_kernel(const PlanParams p) {
       reinterpret_cast<uint32_t*>(win + idx % kOpWindow)[thread] = __ldg(reinterpret_cast<const uint32_t*>(p.ops + idx) + thread);
   };
   for (uint32_t i = 0; i + 2 <= kOpWindow; ++i) fill_window(i, threadIdx.x);  // entries 0 .. kOpWindow - 2
-  uint32_t cur_op = 0;  // the op this warp is working on; entries up to cur_op + kOpWindow - 2 are valid
+  uint32_t op = 0;  // the op this warp is working on; entries up to op + kOpWindow - 2 are valid
   auto desc = [&](uint32_t idx) -> const PlanOpDev& {
-    return idx + 2 <= cur_op + kOpWindow ? win[idx % kOpWindow] : p.ops[idx];
+    return idx + 2 <= op + kOpWindow ? win[idx % kOpWindow] : p.ops[idx];
   };
 
   if (lane == 0) {
@@ -947,24 +947,27 @@ plan_pair_kernel(const PlanParams p) {
   };
 
   uint32_t cons_q = 0, red_buf = 0;
-  for (uint32_t op = 0; op < p.op_count; ++op) {
+  for (; op < p.op_count; ++op) {
     // Nothing about the first item depends on the previous op: look it up before the wait.
     const PairItem first_item = pair_item_of<kCB>(win[op % kOpWindow], 0, warp, grid, cta);
     trace_stamp(p, op, kTraceOpBegin);
     // What the op's parameters say is fetched before the wait as well.
     const PlanOpDev& o = win[op % kOpWindow];
     float bias_first = 0.0f, norm_first[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // the bias of a split op's pair: lane = row of the pair (SiLU gate: of the gate's, then of the up weight's block)
+    // the bias of the item's pair: lane = row of the pair (SiLU gate: of the gate's, then of the up weight's block)
     auto load_bias = [&](const PairItem& it, uint32_t local_row) {
       if (!it.valid) return 0.0f;
       const bool up = (o.flags & kOpSwiglu) != 0 && lane >= 16u;
       return (up ? o.bias[1] - 16 : o.bias[it.wi])[local_row + lane];
     };
     auto load_early = [&]() {
-      if (o.slabs != 1) bias_first = load_bias(first_item, (first_item.rb - o.rb_begin[first_item.wi]) * 16u);
-      if (o.norm_weight != nullptr) load_first_norm_weights(o.norm_weight, p.m, o.k, norm_first);
+      bias_first = load_bias(first_item, (first_item.rb - o.rb_begin[first_item.wi]) * 16u);
+      if (o.norm_weight != nullptr) load_first_norm_weights<kCorrStride>(o.norm_weight, p.m, o.k, norm_first);
     };
-    if (o.flags & kOpEarlyParams) load_early();
+    // (kG == 2 has no registers left to carry them over the barrier.  A spilled register costs more than its
+    // load here: the barrier's acquire empties L1, so the reload is a trip to L2, 700 clocks in every op.)
+    const bool early = kG == 4 && (o.flags & kOpEarlyParams) != 0;
+    if (early) load_early();
     if (op > 0) {
       // every output of the previous op must be complete and visible before x is read
       __syncthreads();
@@ -986,14 +989,13 @@ plan_pair_kernel(const PlanParams p) {
       }
       __syncthreads();
     }
-    if (!(o.flags & kOpEarlyParams)) load_early();
-    cur_op = op;
+    if (!early) load_early();
     trace_stamp(p, op, kTraceBarrier);
     if (o.norm_weight != nullptr) {
       // no reduction of the previous op is in flight any more: its buffers serve as scratch
       float* scratch = red + static_cast<size_t>(red_buf) * kPlanWarps * (2 * p.m * 16);
-      stage_x_rms_norm<kPlanWarps, XT, kHasLo, kCorrStride, true, 4, 4>(static_cast<const XT*>(o.x), o.norm_weight, o.norm_eps, p.m,
-                                                                        o.k, xs, kXsStride, corr, scratch, norm_first);
+      stage_x_rms_norm<kPlanWarps, XT, kHasLo, kCorrStride, true, 4, kCorrStride>(static_cast<const XT*>(o.x), o.norm_weight, o.norm_eps,
+                                                                                  p.m, o.k, xs, kXsStride, corr, scratch, norm_first);
     } else {
       stage_x<XT, kHasLo, kCorrStride, true, 4>(static_cast<const XT*>(o.x), p.m, o.k, 0, o.k >> 5, xs, kXsStride, corr);
     }
@@ -1002,28 +1004,18 @@ plan_pair_kernel(const PlanParams p) {
 
     const uint32_t slabs = o.slabs, rounds = o.rounds;
     for (uint32_t round = 0; round < rounds; ++round) {
-      const PairItem it = round == 0 ? first_item : pair_item_of<kCB>(o, round, warp, grid, cta);
+      // (looking the first item up again spares kG == 4 the registers, see above; kG == 2 spills less carrying it)
+      const PairItem it = kG == 2 && round == 0 ? first_item : pair_item_of<kCB>(o, round, warp, grid, cta);
 #pragma unroll
       for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int j = 0; j < kAcc; ++j) acc[r][j] = 0.0f;
       // the bias (and residual) of the rows this lane will store, fetched while the weights are consumed
       const uint32_t local_row = (it.rb - o.rb_begin[it.wi]) * 16u;  // first row of the pair inside its weight
-      float bias_pre[4] = {bias_first, 0.0f, 0.0f, 0.0f};
-      if (slabs == 1) {
-        if (it.valid) {
-          const float* bias = o.bias[it.wi];
-          const float* bias2 = (o.flags & kOpSwiglu) ? o.bias[1] : bias + 16;  // bias of the pair's second block
-          bias_pre[0] = bias[local_row + g];
-          bias_pre[1] = bias[local_row + g + 8];
-          bias_pre[2] = bias2[local_row + g];
-          bias_pre[3] = bias2[local_row + g + 8];
-        }
-      } else {
-        if (round != 0) bias_pre[0] = load_bias(it, local_row);
-        // (one activation row: output index == row)
-        if (it.valid && p.m == 1 && o.residual[it.wi] != nullptr) bias_pre[1] = o.residual[it.wi][local_row + lane];
-      }
+      const float bias_pre = round == 0 ? bias_first : load_bias(it, local_row);
+      float residual_pre = 0.0f;
+      // (one activation row: output index == row)
+      if (it.valid && p.m == 1 && slabs != 1 && o.residual[it.wi] != nullptr) residual_pre = o.residual[it.wi][local_row + lane];
 
       for (uint32_t first = 0; first < it.nck; first += kPiece) {
         const uint32_t nc = min(static_cast<uint32_t>(kPiece), it.nck - first);
@@ -1069,6 +1061,9 @@ plan_pair_kernel(const PlanParams p) {
       // (not inlined: their registers must not weigh on the loop above); plain ops store here.
       const bool plain = (o.flags & (kOpSwiglu | kOpReduce)) == 0 && o.residual[it.wi] == nullptr;
       if (slabs == 1) {
+        float bias_at[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bias_at[i] = __shfl_sync(0xffffffffu, bias_pre, g + 8 * i);
         if (it.nck != 0 && owner) {
 #pragma unroll
           for (int j = 0; j < (kHasLo ? 1 : 2); ++j) {
@@ -1078,13 +1073,13 @@ plan_pair_kernel(const PlanParams p) {
             const float b0 = acc[1][kHasLo ? 0 : j], b1 = acc[1][kHasLo ? 1 : 2 + j];
             if (plain) {
               float* dst = o.out[it.wi] + static_cast<size_t>(mm) * o.n[it.wi] + local_row + g;
-              dst[0] = fmaf(a0, kUnscale, bias_pre[0]);
-              dst[8] = fmaf(a1, kUnscale, bias_pre[1]);
-              dst[16] = fmaf(b0, kUnscale, bias_pre[2]);
-              dst[24] = fmaf(b1, kUnscale, bias_pre[3]);
+              dst[0] = fmaf(a0, kUnscale, bias_at[0]);
+              dst[8] = fmaf(a1, kUnscale, bias_at[1]);
+              dst[16] = fmaf(b0, kUnscale, bias_at[2]);
+              dst[24] = fmaf(b1, kUnscale, bias_at[3]);
             } else {
-              finish_fused_lane(&o, it.wi, mm, local_row + g, a0, a1, b0, b1, bias_pre[0], bias_pre[1], bias_pre[2],
-                                bias_pre[3], p.fcomm, p.status);
+              finish_fused_lane(&o, it.wi, mm, local_row + g, a0, a1, b0, b1, bias_at[0], bias_at[1], bias_at[2],
+                                bias_at[3], p.fcomm, p.status);
             }
           }
         }
@@ -1106,7 +1101,7 @@ plan_pair_kernel(const PlanParams p) {
       __syncthreads();
       if ((warp & (slabs - 1u)) == 0 && it.valid) {
         const float* first_slab = mine;
-        if (p.m == 1 && (o.flags & kOpReduce) == 0) {
+        if (kG == 4 && p.m == 1 && (o.flags & kOpReduce) == 0) {
           // One activation row: lane = row of the pair.  Short and inline: the general function below is
           // cold code in every op and cost 2,100 clocks of a 4096 x 4096 op's 12,000.
           float v;
@@ -1116,12 +1111,12 @@ plan_pair_kernel(const PlanParams p) {
           } else {
             v = sum_slabs(first_slab + lane, slabs, 32u);
           }
-          v = fmaf(v, kUnscale, bias_pre[0]);
+          v = fmaf(v, kUnscale, bias_pre);
           if (o.flags & kOpSwiglu) {
             const float up = __shfl_down_sync(0xffffffffu, v, 16);
             if (lane < 16u) o.out[0][local_row + lane] = silu_mul(v, up);
           } else {
-            if (!plain) v = __fadd_rn(v, bias_pre[1]);
+            if (!plain) v = __fadd_rn(v, residual_pre);
             o.out[it.wi][local_row + lane] = v;
           }
         } else if (plain) {
@@ -1136,7 +1131,7 @@ plan_pair_kernel(const PlanParams p) {
             out[static_cast<size_t>(mm) * n_i + row] = fmaf(total, kUnscale, bias[row]);
           }
         } else {
-          finish_fused_slabs(&o, it.wi, first_slab, slabs, p.m, local_row, lane, bias_pre[0], bias_pre[1], p.fcomm, p.status);
+          finish_fused_slabs(&o, it.wi, first_slab, slabs, p.m, local_row, lane, bias_pre, residual_pre, p.fcomm, p.status);
         }
       }
       red_buf ^= 1u;  // the next round writes the other buffer; this one is re-used two rounds on
