@@ -21,7 +21,7 @@ def cited_files():
     return [n for n in names if os.path.isfile(n) and n.endswith(keep) and os.sep + "build" + os.sep not in n]
 
 
-@pytest.mark.skipif(not os.path.isdir(REFERENCE), reason="reference tree not present")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REFERENCE, "packages")), reason="reference tree not present")
 def test_cited_reference_lines_exist():
     lengths, bad, seen = {}, [], 0
     for name in cited_files():
