@@ -199,9 +199,15 @@ KQ_API int kq_model_tensor_info(kq_model model, const char* key, char* dtype8, u
  * More than 16 rows run on the tcgen05 tensor cores.  bf16 activations on a tiled weight
  * (int4, or int8 with k % 64 == 0) have operands rounded to bf16 once (results within rtol
  * 1e-3, atol 1e-4 * rms of the oracle on bf16-rounded operands).  Everything else enters with
- * its weights as exact integers and its activations exact or as two binary16 parts, the group
- * scales applied in f32: the decode contract.  That contract, for everything up to 16 rows
- * too, is atol 1e-5 * max(1, rms), rtol 1e-3 against the f64-accumulate reference. */
+ * its weights as exact integers, the group scales applied in f32: the decode contract.  That
+ * contract, for everything up to 16 rows too, is atol 1e-5 * max(1, rms), rtol 1e-3 against the
+ * f64-accumulate reference.
+ * The activations of those many-row calls enter exactly (f32 ones as three bf16 parts), so a small
+ * value counts in full beside one many orders of magnitude larger, as in an f32 multiply-add;
+ * f32 ones on tiled int8 weights (k % 32 == 0, n % 16 == 0), and every row of the decode kernels,
+ * are resolved relative to the largest value of their block (2^-37 of it, or 2^-33), the decode
+ * kernels' sums to f32 relative to 8 (int4) or 128 (int8) times the sum of the block's
+ * activations. */
 KQ_API int kq_linear(kq_ctx* ctx, kq_weight w, uint64_t x_dptr, int x_dtype, uint64_t bias_dptr,
                      uint64_t out_dptr, uint32_t m);
 

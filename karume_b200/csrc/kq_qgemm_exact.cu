@@ -6,15 +6,20 @@
 // packages/runtime/src/kernels/gemm-geometry.ts:243-267) for every packed storage, and its
 // integer-dot GEMMs (packages/runtime/src/kernels/linear-i8a8.ts:21-72).
 //
-// A stored int4 / int8 weight is an integer q of at most 8 bits, exact in binary16, so nothing
-// has to be rounded and nothing has to be multiplied by a scale on its way to the tensor core:
+// A stored int4 / int8 weight is an integer q of at most 8 bits, exact in binary16 and in bf16, so
+// nothing has to be rounded and nothing has to be multiplied by a scale on its way to the tensor core:
 //     y[m, n] = sum_groups s[n, g] * ( sum_{k in g} x[m, k] * q[n, k] )
 // The inner sum is a short MMA chain into a tensor-memory accumulator; every group the "drain"
 // warps read that accumulator and add it, times the group's scale, to f32 sums they keep in
-// registers.  An activation is carried exactly (binary16 input, int8 input of the integer-dot
-// form) or as two binary16 parts of its power-of-two pre-scaled value (f32, bf16: 22 bits).  So
-//   * binary16 activations cost ONE product and f32 activations two, where splitting both
-//     operands costs three;
+// registers.  An activation is carried exactly: a binary16 or bf16 one as it is, an int8 one of the
+// integer-dot form as binary16, an f32 one as three bf16 parts (3 x 8 = 24 bits, each with f32's
+// exponents).  Only f32 ones on tiled int8 weights are two binary16 parts of the row's power-of-two
+// pre-scaled values, as in the int8 GEMV: 22 bits, down to 2^-37 of the row's largest value.  So
+//   * binary16 and bf16 activations cost ONE product, f32 ones three or two, where splitting both
+//     operands costs three for 16 bits.  (Two binary16 parts everywhere would lose what an f32
+//     multiply-add keeps: a small value of a row, on a channel without weight at the large ones.
+//     The third part costs 333 x 1536 -> 8960 int4 32.6 us against 32.1, 1024 x 4096 -> 6144 129
+//     against 118; 257 x 1536 -> 8960 int8 29 against 25.)
 //   * an accumulator chain is one group long (at most kMaxChain k), so the tensor core's f32
 //     accumulation never gets the chance to drift;
 //   * the integer-dot form of int4 weights is the same kernel: its per-group sums are integers
@@ -40,6 +45,7 @@
 // Every mbarrier wait is bounded; a wait that gives up sets a status word and a CTA-wide abort
 // flag that makes all later waits return at once, so tensor memory is always released.
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -56,7 +62,11 @@ namespace {
 using namespace umma;
 
 enum WeightKind : int { kI4Tiled = 0, kI4Rows = 1, kI8Tiled = 2, kI8Rows = 3 };
-enum MathKind : int { kHalf1 = 1, kHalf2 = 2, kInt8 = 3 };  // one binary16 part, two, or int8 x int8
+// one binary16 part or two, one bf16 part or three, or int8 x int8
+enum MathKind : int { kHalf1, kHalf2, kBf1, kBf3, kInt8 };
+template <int kMath>
+constexpr bool kIsBf = kMath == kBf1 || kMath == kBf3;
+__host__ __device__ constexpr uint32_t parts_of(int math) { return math == kBf3 ? 3u : math == kHalf2 ? 2u : 1u; }
 
 constexpr int kDrainWarps = 8, kProdWarps = 4, kCopyWarp = 12, kMmaWarp = 13, kScaleWarp = 14, kExThreads = 512;
 constexpr uint32_t kRows = 128;                 // output channels per CTA
@@ -101,7 +111,7 @@ __device__ __forceinline__ float load_scale_dyn(const void* base, size_t index, 
   return f16 ? __half2float(reinterpret_cast<const __half*>(base)[index]) : reinterpret_cast<const float*>(base)[index];
 }
 
-// ---- integers -> binary16 -----------------------------------------------------------------
+// ---- integers -> binary16 or bf16 ------------------------------------------------------------
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) { return (a & mask) | bits; }
 
 // 8 nibbles u (k ascending) -> 8 binary16 values u - 8, exact.  (w & 0x000F000F) | 0x6400.. is
@@ -123,6 +133,25 @@ __device__ __forceinline__ uint4 nibbles_to_half(uint32_t w) {
   return make_uint4(__byte_perm(r[0], r[1], 0x5410), __byte_perm(r[2], r[3], 0x5410), __byte_perm(r[0], r[1], 0x7632),
                     __byte_perm(r[2], r[3], 0x7632));
 }
+// ... -> 8 bf16 values u - 8, exact.  bf16 has seven bits behind the exponent of 128: 128 + u holds a
+// nibble in its lowest place only, so all four pairs are shifted there.
+__device__ __forceinline__ uint4 nibbles_to_bf16(uint32_t w) {
+  const __nv_bfloat162 k136 = __bfloat162bfloat162(__ushort_as_bfloat16(0x4308));
+  uint32_t r[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t v = and_or(w >> (4 * i), 0x000F000Fu, 0x43004300u);
+    const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), k136);
+    r[i] = *reinterpret_cast<const uint32_t*>(&d);
+  }
+  return make_uint4(__byte_perm(r[0], r[1], 0x5410), __byte_perm(r[2], r[3], 0x5410), __byte_perm(r[0], r[1], 0x7632),
+                    __byte_perm(r[2], r[3], 0x7632));
+}
+template <int kMath>
+__device__ __forceinline__ uint4 nibbles_to_operand(uint32_t w) {
+  if constexpr (kIsBf<kMath>) return nibbles_to_bf16(w);
+  else return nibbles_to_half(w);
+}
 
 // 4 bytes q + 128 -> 4 binary16 values q, exact: a byte under the exponent of 1024 is 1024 + byte.
 __device__ __forceinline__ uint2 bytes_to_half(uint32_t w) {
@@ -130,6 +159,25 @@ __device__ __forceinline__ uint2 bytes_to_half(uint32_t w) {
   uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
   const __half2 ha = __hsub2(*reinterpret_cast<const __half2*>(&a), k1152), hb = __hsub2(*reinterpret_cast<const __half2*>(&b), k1152);
   return make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
+}
+// ... -> 4 bf16 values q, exact.  With b = q + 128 under the exponent of 128 the seven low bits of b read as
+// 128 + (b & 127); the top bit, which would reach into the exponent, is taken out and says what to subtract:
+// 128 where it is set (q = b & 127), 256 = the bits of 128 with that one flipped where it is not.
+__device__ __forceinline__ uint2 bytes_to_bf16(uint32_t w) {
+  uint32_t r[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t t = __byte_perm(w, 0x43434343u, i ? 0x4342 : 0x4140);
+    const uint32_t low = t & 0xFF7FFF7Fu, off = (t & 0xFF80FF80u) ^ 0x00800080u;
+    const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&low), *reinterpret_cast<const __nv_bfloat162*>(&off));
+    r[i] = *reinterpret_cast<const uint32_t*>(&d);
+  }
+  return make_uint2(r[0], r[1]);
+}
+template <int kMath>
+__device__ __forceinline__ uint2 bytes_to_operand(uint32_t w) {
+  if constexpr (kIsBf<kMath>) return bytes_to_bf16(w);
+  else return bytes_to_half(w);
 }
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
@@ -170,10 +218,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   tmem_ld16_done(v);
 }
 
-// kind::f16 with binary16 operands / kind::i8 with signed operands; f32 / s32 accumulate, M 256
+// kind::f16 with binary16 or bf16 operands / kind::i8 with signed operands; f32 / s32 accumulate, M 256
 template <int kMath>
 __host__ __device__ constexpr uint32_t exact_idesc(uint32_t nt) {
-  return (kMath == kInt8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((nt >> 3) << 17) | ((256u >> 4) << 24);
+  return kIsBf<kMath> ? umma_idesc(256, nt)
+                      : (kMath == kInt8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((nt >> 3) << 17) | ((256u >> 4) << 24);
 }
 template <int kMath, bool kAccumulate>
 __device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
@@ -219,6 +268,12 @@ __host__ __device__ constexpr uint32_t raw_unit_bytes(uint32_t scale_f16) {
                           : (kMath == kInt8 ? 128u : 64u);
 }
 
+// Producer warps that convert a stage's weight tile together (each of them arrives on the stage's barrier).
+template <int kMath>
+__device__ __forceinline__ uint32_t stage_warps(uint32_t stages) {
+  return parts_of(kMath) == 3 && stages < kProdWarps ? kProdWarps : 1u;
+}
+
 template <int kW, int kMath>
 __global__ void __launch_bounds__(kExThreads, 1)
 qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map0,
@@ -226,7 +281,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
                    const __grid_constant__ CUtensorMap w_map3) {
   constexpr bool kTiled = kW == kI4Tiled || kW == kI8Tiled;
   constexpr bool kGroupScales = kW == kI4Tiled || kW == kI4Rows;
-  constexpr uint32_t kParts = kMath == kHalf2 ? 2u : 1u;
+  constexpr uint32_t kParts = parts_of(kMath);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t raw_base = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
@@ -261,7 +316,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   if (warp == kMmaWarp) {
     if (lane == 0) {
       for (uint32_t s = 0; s < p.stages; ++s) {
-        mbar_init(full + s * 8, 2 + 1);               // the producer warp of each CTA; + the activation tiles' bytes
+        mbar_init(full + s * 8, 2 * stage_warps<kMath>(p.stages) + 1);  // the producer warps of each CTA; + the activation tiles' bytes
         mbar_init(empty + s * 8, 1);                  // one tcgen05.commit
         mbar_init(rawfull + s * 8, 1);                // the raw weights' bytes
       }
@@ -424,15 +479,20 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   } else if (warp < kDrainWarps + kProdWarps) {
     // ---------------- producers ----------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-    // One warp converts the whole weight tile of a k-step, and the four warps take stages in turn: what
-    // a k-step costs in latency (wait, loads, fence, arrival) then overlaps other k-steps.  A stage
-    // belongs to ONE warp: it waits for that barrier's phases one after the other, so a parity can
-    // never be mistaken for the one two phases away (copies of different stages finish in any order).
+    // With four stages or more one warp converts the whole weight tile of a k-step, and the four warps take
+    // stages in turn: what a k-step costs in latency (wait, loads, fence, arrival) then overlaps other
+    // k-steps.  A stage belongs to ONE warp: it waits for that barrier's phases one after the other, so a
+    // parity can never be mistaken for the one two phases away (copies of different stages finish in any
+    // order).  Wide tiles of three-part activations leave three stages: a tile's conversion is then part of
+    // every third k-step's trip, and the four warps share it.
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), full_0 = map_to_cta(full, 0);
+    constexpr int kUnroll = kParts == 3 ? 2 : 4;
+    const bool shared_stage = stage_warps<kMath>(p.stages) != 1;
+    const uint32_t rb0 = shared_stage ? 2u * (warp - kDrainWarps) : 0u, rb1 = shared_stage ? rb0 + 2u : 8u;  // this warp's 16-row blocks
     uint32_t s = 0, phase = 0;
     for (uint32_t ks = 0; ks < ks_count; ++ks, s = s + 1 == p.stages ? 0u : s + 1u, phase ^= s == 0 ? 1u : 0u) {
-      if ((s & (kProdWarps - 1u)) != warp - kDrainWarps) continue;
+      if (!shared_stage && (s & (kProdWarps - 1u)) != warp - kDrainWarps) continue;
       wait_bounded(rawfull + s * 8, phase, abort_flag, p.status, 21);
       const uint32_t a_tile = tiles + s * p.stage_bytes, raw = a_tile + p.raw_off;
       if constexpr (kW == kI4Tiled) {
@@ -441,27 +501,27 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         // lanes of a shared-memory phase hit 8 different pieces of the swizzled rows.
         const bool odd = (g & 1u) != 0;
         const uint32_t p0 = odd ? 4u + t : t, p1 = odd ? t : 4u + t;
-        uint4 q = lds128(raw + lane * 16u);
-#pragma unroll 4
-        for (uint32_t c = 0; c < 8; ++c) {
+        uint4 q = lds128(raw + rb0 * unit + lane * 16u);
+#pragma unroll kUnroll
+        for (uint32_t c = rb0; c < rb1; ++c) {
           const uint4 now = q;
-          if (c < 7) q = lds128(raw + (c + 1u) * unit + lane * 16u);
+          if (c + 1u < rb1) q = lds128(raw + (c + 1u) * unit + lane * 16u);
           const uint32_t r_a = c * 16u + g, r_b = r_a + 8u;
-          sts128(a_tile + swz(r_a, p0), nibbles_to_half(odd ? now.z : now.x));
-          sts128(a_tile + swz(r_a, p1), nibbles_to_half(odd ? now.x : now.z));
-          sts128(a_tile + swz(r_b, p0), nibbles_to_half(odd ? now.w : now.y));
-          sts128(a_tile + swz(r_b, p1), nibbles_to_half(odd ? now.y : now.w));
+          sts128(a_tile + swz(r_a, p0), nibbles_to_operand<kMath>(odd ? now.z : now.x));
+          sts128(a_tile + swz(r_a, p1), nibbles_to_operand<kMath>(odd ? now.x : now.z));
+          sts128(a_tile + swz(r_b, p0), nibbles_to_operand<kMath>(odd ? now.w : now.y));
+          sts128(a_tile + swz(r_b, p1), nibbles_to_operand<kMath>(odd ? now.y : now.w));
         }
       } else if constexpr (kW == kI4Rows) {
         // a row's k-step is 32 bytes: lane = (row, half), 16 bytes = 32 k = four pieces
-#pragma unroll 4
-        for (uint32_t c = 0; c < 8; ++c) {
+#pragma unroll kUnroll
+        for (uint32_t c = rb0; c < rb1; ++c) {
           const uint32_t r = c * 16u + (lane >> 1), h = lane & 1u;
           const uint4 q = lds128(raw + r * 32u + h * 16u);
-          sts128(a_tile + swz(r, h * 4u + 0u), nibbles_to_half(q.x));
-          sts128(a_tile + swz(r, h * 4u + 1u), nibbles_to_half(q.y));
-          sts128(a_tile + swz(r, h * 4u + 2u), nibbles_to_half(q.z));
-          sts128(a_tile + swz(r, h * 4u + 3u), nibbles_to_half(q.w));
+          sts128(a_tile + swz(r, h * 4u + 0u), nibbles_to_operand<kMath>(q.x));
+          sts128(a_tile + swz(r, h * 4u + 1u), nibbles_to_operand<kMath>(q.y));
+          sts128(a_tile + swz(r, h * 4u + 2u), nibbles_to_operand<kMath>(q.z));
+          sts128(a_tile + swz(r, h * 4u + 3u), nibbles_to_operand<kMath>(q.w));
         }
       } else if constexpr (kW == kI8Tiled && kMath != kInt8) {
         // chunk j, words: row g k 4t.. | row g+8 same k | row g k 16+4t.. | row g+8: four weights = 8
@@ -469,7 +529,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         // (j, h) pairs is XORed with a value that differs where the rows' swizzle term does not, so
         // the 16 lanes of a phase hit 8 different pieces.
 #pragma unroll 2
-        for (uint32_t rb = 0; rb < 8; ++rb) {
+        for (uint32_t rb = rb0; rb < rb1; ++rb) {
           const uint32_t r_a = rb * 16u + g, r_b = r_a + 8u;
           const uint32_t flip = (g & 1u) * 2u, sub = t >> 1, byte = (t & 1u) * 8u;
           uint4 q[2];
@@ -478,20 +538,20 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
 #pragma unroll
           for (uint32_t j = 0; j < 2; ++j) {
             const uint32_t o = (2u * j) ^ flip;
-            sts64(a_tile + swz(r_a, o * 2u + sub) + byte, bytes_to_half(q[j].x));
-            sts64(a_tile + swz(r_b, o * 2u + sub) + byte, bytes_to_half(q[j].y));
-            sts64(a_tile + swz(r_a, (o + 1u) * 2u + sub) + byte, bytes_to_half(q[j].z));
-            sts64(a_tile + swz(r_b, (o + 1u) * 2u + sub) + byte, bytes_to_half(q[j].w));
+            sts64(a_tile + swz(r_a, o * 2u + sub) + byte, bytes_to_operand<kMath>(q[j].x));
+            sts64(a_tile + swz(r_b, o * 2u + sub) + byte, bytes_to_operand<kMath>(q[j].y));
+            sts64(a_tile + swz(r_a, (o + 1u) * 2u + sub) + byte, bytes_to_operand<kMath>(q[j].z));
+            sts64(a_tile + swz(r_b, (o + 1u) * 2u + sub) + byte, bytes_to_operand<kMath>(q[j].w));
           }
         }
       } else if constexpr (kW == kI8Rows && kMath != kInt8) {
         // a row's k-step is 64 bytes: lane = (row, quarter), 16 bytes = 16 k = two pieces
 #pragma unroll 4
-        for (uint32_t c = 0; c < 16; ++c) {
+        for (uint32_t c = 2u * rb0; c < 2u * rb1; ++c) {
           const uint32_t r = c * 8u + (lane >> 2), qd = lane & 3u;
           const uint4 q = lds128(raw + r * 64u + qd * 16u);
-          const uint2 a = bytes_to_half(q.x ^ 0x80808080u), b = bytes_to_half(q.y ^ 0x80808080u);
-          const uint2 d = bytes_to_half(q.z ^ 0x80808080u), e = bytes_to_half(q.w ^ 0x80808080u);
+          const uint2 a = bytes_to_operand<kMath>(q.x ^ 0x80808080u), b = bytes_to_operand<kMath>(q.y ^ 0x80808080u);
+          const uint2 d = bytes_to_operand<kMath>(q.z ^ 0x80808080u), e = bytes_to_operand<kMath>(q.w ^ 0x80808080u);
           sts128(a_tile + swz(r, qd * 2u), make_uint4(a.x, a.y, b.x, b.y));
           sts128(a_tile + swz(r, qd * 2u + 1u), make_uint4(d.x, d.y, e.x, e.y));
         }
@@ -499,7 +559,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         // int8 tile: four chunks (32 k each) of a row block; a word is 4 bytes of piece 2j + h, the sign
         // bit flipped back.  Eight rows x four words hit 32 different banks.
 #pragma unroll 2
-        for (uint32_t rb = 0; rb < 8; ++rb) {
+        for (uint32_t rb = rb0; rb < rb1; ++rb) {
           const uint32_t r_a = rb * 16u + g, r_b = r_a + 8u;
           uint4 qs[4];
 #pragma unroll
@@ -522,7 +582,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == kCopyWarp) {
       // ---------------- copies ----------------
-      // One thread, two tensor copies per k-step (both activation parts come with one): a copy takes it about
+      // One thread, two tensor copies per k-step (all activation parts come with one): a copy takes it about
       // 100 clocks, and a bulk copy per 16-row block, eight of them, 700 - 1000: more than the k-step's MMAs.
       {
         const uint32_t half_rows = p.nt / 2, b_bytes = half_rows * 128u, raw_bytes = p.raw_bytes;
@@ -577,7 +637,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
               const uint32_t dst = tmem + (set & 1u) * kMaxNT + in_set * acc_cols;
               if (starts) mma_pair<kMath, false>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
               else mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
-              if constexpr (kParts == 2) mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + b_step + kk * 2u, idesc);
+#pragma unroll
+              for (uint32_t part = 1; part < kParts; ++part) mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + part * b_step + kk * 2u, idesc);
               if (kMath != kInt8 && kSlices != 0 && (kk + 1) % (kSlices == 0 ? 1u : kSlices) == 0) chain_ends(kk == 3 && ks + 1 == ks_count);
             }
             if constexpr (kSlices == 0) {
@@ -686,14 +747,29 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   }
 }
 
-// ---- activations -> binary16 parts -----------------------------------------------------------
-// One CTA per row.  [rms_norm ->] power-of-two pre-scale of the whole row (pow2_prescale) -> hi = RN_f16(v),
-// lo = RN_f16(v - hi); inv[row] = 2^-e undoes the scale in the epilogue.  A row is read once from
-// memory and again from the cache.
-template <typename XT>
+// ---- f32 and bf16 activations -> parts ----------------------------------------------------------
+// One CTA per row.  [rms_norm ->] a power of two over the whole row -> parts that add up to the value: three
+// bf16 ones of an f32 value, the one of a bf16 value, or two binary16 ones (pow2_prescale); inv[row] = 2^-e
+// undoes the power in the epilogue.  A row is read once from memory and again from the cache.
+//
+// bf16 parts have f32's exponents, so their power of two is only there to keep the sums of up to 1024 products
+// with integers, and those times a group scale, away from both ends of the range: the row's largest value goes
+// to [2^40, 2^41).  A value then keeps all its bits down to 2^-150 of that one (a part of less than 2^-133
+// vanishes).  A row of zeros, or one whose largest value is not finite, keeps its values.
+__device__ __forceinline__ Pow2 pow2_row(float amax) {
+  const uint32_t bits = __float_as_uint(amax) & 0x7fffffffu;
+  int e = 0;
+  if (bits != 0u && bits < 0x7f800000u) e = min(126, 40 + 127 - static_cast<int>(bits >> 23));  // -87 .. 126
+  Pow2 r;
+  r.scale = __uint_as_float(static_cast<uint32_t>(e + 127) << 23);
+  r.inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+  return r;
+}
+template <typename XT, int kMath>
 __global__ void __launch_bounds__(256)
-split_half_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, __half* __restrict__ parts, float* __restrict__ inv,
-                  const float* __restrict__ norm_weight, float norm_eps) {
+split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restrict__ parts, float* __restrict__ inv,
+             const float* __restrict__ norm_weight, float norm_eps) {
+  constexpr uint32_t kParts = parts_of(kMath);
   const uint32_t row = blockIdx.x;
   const XT* xr = x + static_cast<size_t>(row) * k;
   __shared__ float part[8];
@@ -737,25 +813,35 @@ split_half_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, __half* __re
   __syncthreads();
   amax = part[0];
   for (int w = 1; w < 8; ++w) amax = fmaxf(amax, part[w]);
-  const Pow2 ps = pow2_prescale(amax);
+  const Pow2 ps = kIsBf<kMath> ? pow2_row(amax) : pow2_prescale(amax);
   if (threadIdx.x == 0) inv[row] = ps.inv;
-  __half* hi = parts + static_cast<size_t>(row) * k;
-  __half* lo = hi + static_cast<size_t>(m) * k;
   for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
     float v[8];
     load(i, v);
-    uint4 oh, ol;
-    uint32_t* ph = reinterpret_cast<uint32_t*>(&oh);
-    uint32_t* pl = reinterpret_cast<uint32_t*>(&ol);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float a = v[2 * j] * ps.scale, b = v[2 * j + 1] * ps.scale;
-      const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
-      ph[j] = pack_half2(ha, hb);
-      pl[j] = pack_half2(__float2half_rn(a - __half2float(ha)), __float2half_rn(b - __half2float(hb)));
+    for (int e = 0; e < 8; ++e) v[e] *= ps.scale;
+#pragma unroll
+    for (uint32_t part = 0; part < kParts; ++part) {
+      uint4 o;
+      uint32_t* po = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 f;
+        if constexpr (kIsBf<kMath>) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+          po[j] = *reinterpret_cast<const uint32_t*>(&h);
+          f = __bfloat1622float2(h);
+        } else {
+          const __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+          po[j] = *reinterpret_cast<const uint32_t*>(&h);
+          f = __half22float2(h);
+        }
+        // the rest is exact; an infinite value has none (Inf - Inf is a NaN)
+        v[2 * j] = isinf(f.x) ? 0.0f : v[2 * j] - f.x;
+        v[2 * j + 1] = isinf(f.y) ? 0.0f : v[2 * j + 1] - f.y;
+      }
+      *reinterpret_cast<uint4*>(parts + (static_cast<size_t>(part) * m + row) * k + i) = o;
     }
-    *reinterpret_cast<uint4*>(hi + i) = oh;
-    *reinterpret_cast<uint4*>(lo + i) = ol;
   }
   pdl_launch_dependents();
 }
@@ -830,7 +916,7 @@ EncodeTiled tensor_map_encoder() {
   return encode;
 }
 
-// Activations [parts][m][k] (binary16 or int8), box 128 bytes x `rows` rows of every part, 128-byte swizzle; what
+// Activations [parts][m][k] (binary16, bf16 or int8), box 128 bytes x `rows` rows of every part, 128-byte swizzle; what
 // lies past k or m reads as zero.
 cudaError_t encode_x_map(const void* x, bool int8, uint32_t m, uint32_t k, uint32_t parts, uint32_t rows, CUtensorMap* map) {
   EncodeTiled encode = tensor_map_encoder();
@@ -838,7 +924,7 @@ cudaError_t encode_x_map(const void* x, bool int8, uint32_t m, uint32_t k, uint3
   const cuuint64_t each = int8 ? 1 : 2;
   const cuuint64_t dims[3] = {k, m, parts}, strides[2] = {k * each, static_cast<cuuint64_t>(m) * k * each};
   const cuuint32_t box[3] = {int8 ? 128u : 64u, rows, parts}, ones[3] = {1, 1, 1};
-  const CUresult r = encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims,
+  const CUresult r = encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(x), dims,
                             strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -925,27 +1011,37 @@ template <int kW>
 cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, uint32_t pairs, uint32_t m_tiles, const CUtensorMap& xm,
                         const CUtensorMap (&wm)[kMaxMulti]) {
   if (math == kHalf1) return launch_main<kW, kHalf1>(env, p, pairs, m_tiles, xm, wm);
-  if (math == kHalf2) return launch_main<kW, kHalf2>(env, p, pairs, m_tiles, xm, wm);
+  if (math == kBf1) return launch_main<kW, kBf1>(env, p, pairs, m_tiles, xm, wm);
+  constexpr int kF32 = kW == kI8Tiled ? kHalf2 : kBf3;
+  if (math == kF32) return launch_main<kW, kF32>(env, p, pairs, m_tiles, xm, wm);
   if constexpr (kW == kI8Tiled || kW == kI8Rows) return launch_main<kW, kInt8>(env, p, pairs, m_tiles, xm, wm);
   return cudaErrorInvalidValue;
 }
 
-// Clocks of one k-step, fitted to timings of 30 shapes (17 to 1024 rows; within 15 % of them).  The
-// activation tile's copy and the MMAs grow with the tile and its parts, the conversion of the weights does
-// not; a drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step
-// (nt = 256, group 32: 1,900).  int4, group 32, two parts: 750 at nt = 32, 1,010 at 64, 1,250 at 128, 1,600 at 192, 2,060 at 256.
-uint32_t kstep_clocks(uint32_t nt, uint32_t parts, uint32_t drains_x4, bool int8) {
+// Clocks of one k-step, fitted to the difference between k = 4,096 and 12,288 at every tile width (1536
+// channels, one tile; within 25 % of it, and the choices below are the fastest of a sweep of 13 shapes, 24 to
+// 1,024 rows, within its noise).  The conversion of the weights does not grow with the tile, its copy and the
+// MMAs do; a drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step.
+// Measured at nt = 32, 64, 128, 192, 256:
+//   int4, group 32   binary16 685, 790, 1,010, 1,380, 1,765; f32 830, 1,090, 1,215, 1,510, 1,870
+//   int8             binary16 460, 525, 635, 650, 640; f32 tiled 635, 760, 665, 850, 1,190, untiled 900, 1,050,
+//                    1,075, 1,270, 1,680 (bytes take 9 instructions for four bf16 integers, 4 for binary16)
+// Three parts above 128 rows leave three stages: a k-step is a third of a stage's whole trip.
+uint32_t kstep_clocks(uint32_t nt, int math, uint32_t drains_x4, bool int8_weights) {
+  const bool int8 = math == kInt8, bytes_to_bf = int8_weights && (math == kBf1 || math == kBf3);
+  const uint32_t parts = parts_of(math);
   const uint32_t mma = 4 * parts * std::max(nt / 2, 48u);
-  const uint32_t step = (int8 ? 550 : 450) + 100 * parts + nt * parts + (int8 ? 0u : drains_x4 * (nt * 8 / 5 + 20) / 4);
+  const uint32_t step = int8 ? 650 + nt : 450 + (bytes_to_bf ? 200 : 0) + 100 * parts + nt + drains_x4 * (nt * 8 / 5 + 20) / 4;
+  const uint32_t trip = parts == 3 && nt > 128 ? nt * 15 / 2 + 100 : 0;
   const uint32_t drain = int8 ? 0u : drains_x4 * std::max(nt * 7 / 2 + 60, 330u) / 4;
-  return std::max({mma, step, drain});
+  return std::max({mma, step, trip, drain});
 }
 
 struct Geometry { uint32_t nt, m_tiles, splits; };
 // Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
 // loads, epilogue) plus its k-steps; a split adds the reduce launch and the partial sums, written and read
 // at 2,200 bytes per clock.  (Priced at 4,000, 1024 x 4096 -> 6144 was cut in two at nt = 256: 174 us, 118 now.)
-Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t ksteps, uint32_t parts, uint32_t drain16, bool int8,
+Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t ksteps, int math, bool int8_weights, uint32_t drain16,
                          uint32_t slice_unit, bool may_split, uint32_t sm_pairs, uint64_t partial_room) {
   Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1};
   uint64_t best_cost = ~0ull;
@@ -955,7 +1051,7 @@ Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t 
     uint32_t nt = ((m + mt - 1) / mt + 31) / 32 * 32;
     if (nt > 128) nt = (nt + 63) / 64 * 64;
     if ((m + nt - 1) / nt != mt) continue;
-    const uint32_t per = kstep_clocks(nt, parts, drains_x4, int8);
+    const uint32_t per = kstep_clocks(nt, math, drains_x4, int8_weights);
     for (uint32_t splits = 1; splits <= (may_split ? 16u : 1u); splits *= 2) {
       if (splits > 1 && (ksteps / splits < 4 || static_cast<uint64_t>(splits) * m * n_total * 4 > partial_room)) break;
       uint32_t each = (ksteps + splits - 1) / splits;
@@ -973,7 +1069,7 @@ Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t 
   return best;
 }
 
-// x: binary16 (kHalf1, `x` used in place), parts already split (kHalf1 / kHalf2) or int8 (kInt8).
+// x: binary16 (kHalf1), parts already split (kHalf2 / kBf1 / kBf3) or int8 (kInt8).
 cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const float* residual, const void* x, int math,
                       uint32_t m, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, int* launches) {
   const Weight& w0 = *targets[0].w;
@@ -1020,10 +1116,10 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   p.n_total = n_total;
   p.status = env.status;
   p.partial = static_cast<float*>(scratch);
-  const uint32_t parts = math == kHalf2 ? 2 : 1;
+  const uint32_t parts = parts_of(math);
   // a K slice is a whole number of int4 accumulator chains (an int8 chain may end anywhere)
   const uint32_t align = i4 && p.drain16 > 4 ? p.drain16 / 4 : 1;
-  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, parts, p.drain16, int8, align, may_split && scratch != nullptr,
+  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, math, !i4, p.drain16, align, may_split && scratch != nullptr,
                                        std::max(1, env.sm_count / 2), scratch_bytes);
   p.nt = geo.nt;
   p.ksteps_per_split = ((p.ksteps + geo.splits - 1) / geo.splits + align - 1) / align * align;
@@ -1084,22 +1180,25 @@ bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, ui
         w.scale_dtype != w0.scale_dtype || w.k == 0 || !kind_ok(w))
       return false;
   }
-  // one row panel of 32 rows of split activations has to fit the scratch
-  return align256(static_cast<uint64_t>(w0.k) * 4 * 32) + 256 <= workspace_bytes;
+  // a panel of 16 rows of split activations and its factors have to fit the scratch
+  return align256(static_cast<uint64_t>(w0.k) * 2 * parts_of(kBf3) * 16) + 256 <= workspace_bytes;
 }
 
 cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,
                                int* launches) {
   const Weight& w0 = *targets[0].w;
   const uint32_t k = w0.k;
-  const bool direct = x_dtype == KQ_F16 && env.norm_weight == nullptr;  // binary16 rows are the operand
+  const bool direct = x_dtype == KQ_F16;  // binary16 rows are the operand
+  if (direct && env.norm_weight != nullptr) return cudaErrorInvalidValue;
+  const int math = direct ? kHalf1 : x_dtype == KQ_BF16 ? kBf1 : kind_of(w0) == kI8Tiled ? kHalf2 : kBf3;
   uint8_t* ws = static_cast<uint8_t*>(env.workspace);
   const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
-  // row panels whose split activations take at most half of the scratch (the rest: partial sums)
-  const uint64_t per_row = static_cast<uint64_t>(k) * 4 + 4;
+  // row panels whose split activations take at most three quarters of the scratch (the rest: partial sums, which
+  // only calls of few tiles want)
+  const uint64_t part_bytes = static_cast<uint64_t>(k) * 2 * parts_of(math), per_row = part_bytes + 4, share = room / 4 * 3;
   uint32_t panel = m;
-  if (!direct && per_row * m > room / 2) {
-    panel = static_cast<uint32_t>(std::min<uint64_t>(m, std::max<uint64_t>(32, room / 2 / per_row)));
+  if (!direct && per_row * m > share) {
+    panel = static_cast<uint32_t>(std::min<uint64_t>(m, std::max<uint64_t>(16, share / per_row)));
     if (panel >= 256) panel = panel / 256 * 256;
   }
   for (uint32_t r0 = 0; r0 < m; r0 += panel) {
@@ -1112,24 +1211,21 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
     const uint8_t* xp = static_cast<const uint8_t*>(x) + static_cast<size_t>(r0) * k * xb;
     cudaError_t e;
     if (direct) {
-      e = run_exact(env, count, t, residual, xp, kHalf1, pm, nullptr, ws, room, true, launches);
+      e = run_exact(env, count, t, residual, xp, math, pm, nullptr, ws, room, true, launches);
     } else {
       float* inv = reinterpret_cast<float*>(ws);
-      __half* parts = reinterpret_cast<__half*>(ws + align256(static_cast<uint64_t>(pm) * 4));
-      const uint64_t taken = align256(static_cast<uint64_t>(pm) * 4) + align256(static_cast<uint64_t>(pm) * k * 4);
+      uint16_t* parts = reinterpret_cast<uint16_t*>(ws + align256(static_cast<uint64_t>(pm) * 4));
+      const uint64_t taken = align256(static_cast<uint64_t>(pm) * 4) + align256(pm * part_bytes);
       if (taken > room) return cudaErrorMemoryAllocation;
-      if (x_dtype == KQ_F32)
-        e = launch_dependent(split_half_kernel<float>, dim3(pm), 256, 0, 1, env, reinterpret_cast<const float*>(xp), pm, k, parts, inv,
-                             env.norm_weight, env.norm_eps);
-      else if (x_dtype == KQ_F16)
-        e = launch_dependent(split_half_kernel<__half>, dim3(pm), 256, 0, 1, env, reinterpret_cast<const __half*>(xp), pm, k, parts, inv,
-                             env.norm_weight, env.norm_eps);
-      else
-        e = launch_dependent(split_half_kernel<__nv_bfloat16>, dim3(pm), 256, 0, 1, env, reinterpret_cast<const __nv_bfloat16*>(xp), pm, k,
-                             parts, inv, env.norm_weight, env.norm_eps);
+      auto split = [&](auto kernel, auto* rows) {
+        return launch_dependent(kernel, dim3(pm), 256, 0, 1, env, rows, pm, k, parts, inv, env.norm_weight, env.norm_eps);
+      };
+      if (math == kBf1) e = split(split_kernel<__nv_bfloat16, kBf1>, reinterpret_cast<const __nv_bfloat16*>(xp));
+      else if (math == kBf3) e = split(split_kernel<float, kBf3>, reinterpret_cast<const float*>(xp));
+      else e = split(split_kernel<float, kHalf2>, reinterpret_cast<const float*>(xp));
       if (e != cudaSuccess) return e;
       if (launches) *launches += 1;
-      e = run_exact(env, count, t, residual, parts, kHalf2, pm, inv, ws + taken, room - taken, true, launches);
+      e = run_exact(env, count, t, residual, parts, math, pm, inv, ws + taken, room - taken, true, launches);
     }
     if (e != cudaSuccess) return e;
   }

@@ -116,3 +116,66 @@ def test_norm_gate_and_residual_around_it(gpu, m, n, k):
         assert rep["pass"], rep
     for w in ws:
         w.free()
+
+
+# Magnitudes that lie side by side in k: an f32 multiply-add gives a channel the sum of its own products
+# whatever else the row holds, so no value may be resolved relative to a larger one of its row.
+DECADES = (1e-9, 1.0, 1e9)
+
+
+@pytest.mark.parametrize("xdt", ["f32", "bf16"])
+@pytest.mark.parametrize("storage,group,m,n,k", [("i4", 32, 40, 144, 512), ("i4", 32, 300, 528, 2048), ("i4", 16, 65, 301, 1152), ("i4", 2048, 18, 202, 4096),
+                                                 ("i8", 0, 33, 330, 2800), ("i8", 0, 257, 130, 1536), ("i8", 0, 40, 144, 1056), ("i4", 64, 3, 3000, 4096)])
+def test_channels_that_only_see_the_small_values_of_a_row(gpu, xdt, storage, group, m, n, k):
+    """Channel c has weights only where k % 3 == c % 3, and those activations are 1e-9, 1 or 1e9 times
+    N(0, 1).  Each third of the channels has to meet the tolerance on its own scale: f32 sums of up to
+    4096 / 3 terms, 1e-5 of their rms (sqrt(k) 2^-24 is 4e-6) and 1e-4 relative."""
+    import torch
+    rng = np.random.default_rng(m + n)
+    which = np.arange(k) % 3
+    x = rng.standard_normal((m, k)).astype(np.float32) * np.asarray(DECADES, np.float32)[which]
+    x = {"f32": lambda v: v, "bf16": oracle.round_to_bf16}[xdt](x)
+    live = which[None, :] == (np.arange(n) % 3)[:, None]
+    bias = np.zeros(n, np.float32)
+    if storage == "i4":
+        if xdt == "bf16" and group == 32:
+            pytest.skip("the bf16 GEMM's case")
+        nibbles = np.where(live, rng.integers(0, 16, size=(n, k)), 8).astype(np.uint8)
+        data = cases.pack_nibbles(nibbles.reshape(-1))
+        scale = (np.abs(rng.standard_normal((n, k // group))) * 0.02 / 7 + 1e-6).astype(np.float32)
+        ref = oracle.linear_i4(x, data, scale, bias, n, k, group)
+    else:
+        if xdt == "f32" and n % 16 == 0 and k % 32 == 0:
+            pytest.skip("tiled int8 weights: resolved relative to the row's largest value, as in the int8 GEMV")
+        data = np.where(live, rng.integers(-127, 128, size=(n, k)), 0).astype(np.int8)
+        scale = (np.abs(rng.standard_normal(n)) * 0.02 / 127 + 1e-8).astype(np.float32)
+        ref = oracle.linear_i8(x, data, scale, bias, n, k)
+    w = gpu.upload_weight(storage, data, scale, (n, k), group)
+    got = gpu.linear(dev(x).to({"f32": torch.float32, "bf16": torch.bfloat16}[xdt]), w, dev(bias))
+    gpu.sync()
+    got = got.cpu().numpy()
+    for c in range(3):
+        mine, want = got[:, c::3], ref[:, c::3]
+        rep = oracle.allclose(mine, want, atol=1e-5 * float(np.sqrt(np.mean(want.astype(np.float64) ** 2))), rtol=1e-4)
+        assert rep["pass"], (DECADES[c], rep)
+    w.free()
+
+
+def test_an_infinite_activation_reaches_the_channels_that_multiply_it(gpu):
+    """Inf times a weight is an infinity of the product's sign, times a zero weight a NaN, and stays in its row."""
+    n, k, m = 144, 256, 20
+    rng = np.random.default_rng(2)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    q = rng.integers(-127, 128, size=(n, k)).astype(np.int8)
+    q[:, 100] = np.where(np.arange(n) % 3 == 0, 5, np.where(np.arange(n) % 3 == 1, -7, 0))
+    scale = np.full(n, 1e-3, np.float32)
+    clean = oracle.linear_i8(np.where(np.arange(m)[:, None] == 3, 0, x).astype(np.float32), q, scale, np.zeros(n, np.float32), n, k)
+    x[3, 100] = np.inf
+    w = gpu.upload_weight("i8", q, scale, (n, k), 0)
+    got = gpu.linear(dev(x), w, dev(np.zeros(n, np.float32)))
+    gpu.sync()
+    got = got.cpu().numpy()
+    assert np.all(got[3, 0::3] == np.inf) and np.all(got[3, 1::3] == -np.inf) and np.all(np.isnan(got[3, 2::3]))
+    rest = np.arange(m) != 3
+    assert oracle.allclose(got[rest], clean[rest], atol=1e-5, rtol=1e-4)["pass"]
+    w.free()
