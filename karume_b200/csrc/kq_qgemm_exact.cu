@@ -43,7 +43,9 @@
 // Register split (setmaxnreg): 2 x 128 x 184 + 2 x 128 x 72 = 512 x 128.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets a status word and a CTA-wide abort
-// flag that makes all later waits return at once, so tensor memory is always released.
+// flag that makes all later waits return at once, so tensor memory is always released.  Copies and
+// producers whose wait gave up leave their stage alone: an arrival on a barrier whose phase has all
+// its arrivals and still waits for bytes is undefined.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -493,7 +495,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     uint32_t s = 0, phase = 0;
     for (uint32_t ks = 0; ks < ks_count; ++ks, s = s + 1 == p.stages ? 0u : s + 1u, phase ^= s == 0 ? 1u : 0u) {
       if (!shared_stage && (s & (kProdWarps - 1u)) != warp - kDrainWarps) continue;
-      wait_bounded(rawfull + s * 8, phase, abort_flag, p.status, 21);
+      const uint32_t ready = wait_bounded(rawfull + s * 8, phase, abort_flag, p.status, 21) ? leader : 0u;
       const uint32_t a_tile = tiles + s * p.stage_bytes, raw = a_tile + p.raw_off;
       if constexpr (kW == kI4Tiled) {
         // words: row g group 0 | row g+8 group 0 | row g group 1 | row g+8 group 1, each k 8t..8t+7 of
@@ -576,7 +578,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // -> visible to the tensor core
       __syncwarp();
-      arrive_if(leader, full_0 + s * 8);  // the issuing CTA's barrier
+      arrive_if(ready, full_0 + s * 8);  // the issuing CTA's barrier
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -591,12 +593,12 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         const uint32_t w_row = kTiled ? n0 / 16u : n0, w_step = p.raw_box;  // tensor-map rows and columns of the raw weights
         uint32_t s = 0, phase = 0;
         for (uint32_t ks = 0; ks < ks_count; ++ks) {
-          wait_bounded(empty + s * 8, phase ^ 1u, abort_flag, p.status, 20);
+          const uint32_t free = wait_bounded(empty + s * 8, phase ^ 1u, abort_flag, p.status, 20) ? leader : 0u;
           const uint32_t a_tile = tiles + s * p.stage_bytes, kstep = ks_begin + ks;
-          expect_tx(cta_rank == 0 ? leader : 0u, full + s * 8, kParts * 2u * b_bytes);
-          expect_tx(leader, rawfull + s * 8, raw_bytes);
-          copy_tile_2d(leader, a_tile + raw_off, w_map, kstep * w_step, w_row, rawfull + s * 8);
-          copy_tile_3d(leader, a_tile + kATile, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), m0 + cta_rank * half_rows, 0, full_0 + s * 8);
+          expect_tx(cta_rank == 0 ? free : 0u, full + s * 8, kParts * 2u * b_bytes);
+          expect_tx(free, rawfull + s * 8, raw_bytes);
+          copy_tile_2d(free, a_tile + raw_off, w_map, kstep * w_step, w_row, rawfull + s * 8);
+          copy_tile_3d(free, a_tile + kATile, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), m0 + cta_rank * half_rows, 0, full_0 + s * 8);
           if (++s == p.stages) { s = 0; phase ^= 1u; }
         }
       }
