@@ -7,14 +7,17 @@
 //
 // Every function returns the result, an int (the kq_status of a call the library refused), or None
 // when an argument is not of the plain form it handles (then the Python method goes on with its
-// own checks and conversions, and raises what they raise).
+// own checks and conversions, and raises what they raise).  A C++ exception inside one (an output that
+// cannot be allocated, a tensor without memory) leaves as the Python exception torch makes of it.
 #define PY_SSIZE_T_CLEAN
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <Python.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
+#include <exception>
 
 namespace {
 
@@ -58,6 +61,16 @@ at::Tensor empty_like_lead(const at::Tensor& x, int64_t last, at::ScalarType typ
 PyObject* status_of(int rc) { return PyLong_FromLong(rc); }
 #define KQ_NONE Py_RETURN_NONE
 
+// The library call while other Python threads run; the lock is back before anything, an exception too, goes on.
+template <typename Call>
+int without_gil(Call call) {
+  struct Released {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
+  return call();
+}
+
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 5) {
     PyErr_SetString(PyExc_TypeError, "bind takes five addresses");
@@ -89,10 +102,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const uint64_t handle = PyLong_AsUnsignedLongLong(a[1]);
   const uint64_t px = ptr(*x), pb = ptr(*bias), po = ptr(out);
   const uint32_t m = static_cast<uint32_t>(x->numel() / k);
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = g_linear(ctx, handle, px, type, pb, po, m);
-  Py_END_ALLOW_THREADS
+  const int rc = without_gil([&] { return g_linear(ctx, handle, px, type, pb, po, m); });
   if (rc != 0) return status_of(rc);
   if (given != nullptr) return Py_NewRef(a[6]);
   return THPVariable_Wrap(std::move(made));
@@ -126,10 +136,7 @@ PyObject* linear_fused(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (PyErr_Occurred()) return nullptr;
   const uint64_t px = ptr(*x), pn = norm != nullptr ? ptr(*norm) : 0, pr = residual != nullptr ? ptr(*residual) : 0;
   const uint32_t m = static_cast<uint32_t>(x->numel() / k);
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = g_fused(ctx, static_cast<uint32_t>(count), w, px, type, pn, eps, b, pr, o, m, flags);
-  Py_END_ALLOW_THREADS
+  const int rc = without_gil([&] { return g_fused(ctx, static_cast<uint32_t>(count), w, px, type, pn, eps, b, pr, o, m, flags); });
   if (rc != 0) return status_of(rc);
   return Py_NewRef(outs);
 }
@@ -145,15 +152,12 @@ PyObject* quantize_rows(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   void* ctx = PyLong_AsVoidPtr(a[0]);
   const uint64_t px = ptr(*x), pq = ptr(q), ps = ptr(scale);
   const uint32_t rows = static_cast<uint32_t>(x->numel() / dim);
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = g_quantize(ctx, px, rows, static_cast<uint32_t>(dim), pq, ps);
-  Py_END_ALLOW_THREADS
+  const int rc = without_gil([&] { return g_quantize(ctx, px, rows, static_cast<uint32_t>(dim), pq, ps); });
   if (rc != 0) return status_of(rc);
-  PyObject* r = PyTuple_New(2);
-  if (r == nullptr) return nullptr;
-  PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(q)));
-  PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(std::move(scale)));
+  PyObject *pyq = THPVariable_Wrap(std::move(q)), *pys = THPVariable_Wrap(std::move(scale));
+  PyObject* r = pyq != nullptr && pys != nullptr ? PyTuple_Pack(2, pyq, pys) : nullptr;
+  Py_XDECREF(pyq);
+  Py_XDECREF(pys);
   return r;
 }
 
@@ -173,10 +177,7 @@ PyObject* linear_a8(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const uint64_t handle = PyLong_AsUnsignedLongLong(a[1]);
   const uint64_t pq = ptr(*xq), ps = ptr(*xs), pb = ptr(*bias), po = ptr(out);
   const uint32_t m = static_cast<uint32_t>(xq->numel() / k);
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = g_a8(ctx, handle, pq, ps, pb, po, m);
-  Py_END_ALLOW_THREADS
+  const int rc = without_gil([&] { return g_a8(ctx, handle, pq, ps, pb, po, m); });
   if (rc != 0) return status_of(rc);
   if (given != nullptr) return Py_NewRef(a[7]);
   return THPVariable_Wrap(std::move(made));
@@ -199,16 +200,24 @@ PyObject* embedding(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const uint64_t handle = PyLong_AsUnsignedLongLong(a[1]);
   const uint64_t pi = ptr(*index), po = ptr(out);
   const uint32_t rows = static_cast<uint32_t>(index->numel());
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = g_embedding(ctx, handle, pi, rows, po);
-  Py_END_ALLOW_THREADS
+  const int rc = without_gil([&] { return g_embedding(ctx, handle, pi, rows, po); });
   if (rc != 0) return status_of(rc);
   if (given != nullptr) return Py_NewRef(a[4]);
   return THPVariable_Wrap(std::move(made));
 }
 
-#define KQ_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+// CPython's frames have no handlers: what is thrown in a call must not leave it.
+template <PyObject* (*kCall)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t nargs) {
+  try {
+    return kCall(self, a, nargs);
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
+}
+
+#define KQ_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {KQ_METHOD(bind),      KQ_METHOD(linear),    KQ_METHOD(linear_fused), KQ_METHOD(quantize_rows),
                          KQ_METHOD(linear_a8), KQ_METHOD(embedding), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_kqtorch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
