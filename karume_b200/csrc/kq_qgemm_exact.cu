@@ -632,16 +632,26 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t desc_a = desc_a0 + s * stage_step, desc_b = desc_b0 + s * stage_step, this_empty = empty + s * 8;
             if (++s == p.stages) { s = 0; phase ^= 1u; }
+            // Low parts first: an accumulation truncates to the accumulator's size, so the fewer follow once the
+            // high parts are in, the better (through four layers of a decoder, 289
+            // rows: 1.8e-7 from f64 against 3.9e-7 with the high parts first).
+            constexpr uint32_t kRun = kSlices == 0 ? 4u : kSlices;  // slices of a chain in this k-step
 #pragma unroll
-            for (uint32_t kk = 0; kk < 4; ++kk) {
-              const bool starts = kSlices != 0 ? kk % (kSlices == 0 ? 1u : kSlices) == 0 : kk == 0 && in_chain == 0;
+            for (uint32_t run = 0; run < 4; run += kRun) {
+              const bool starts = kSlices != 0 || in_chain == 0;
               if (kMath != kInt8 && starts) chain_begins();
               const uint32_t dst = tmem + (set & 1u) * kMaxNT + in_set * acc_cols;
-              if (starts) mma_pair<kMath, false>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
-              else mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + kk * 2u, idesc);
 #pragma unroll
-              for (uint32_t part = 1; part < kParts; ++part) mma_pair<kMath, true>(leader, dst, desc_a + kk * 2u, desc_b + part * b_step + kk * 2u, idesc);
-              if (kMath != kInt8 && kSlices != 0 && (kk + 1) % (kSlices == 0 ? 1u : kSlices) == 0) chain_ends(kk == 3 && ks + 1 == ks_count);
+              for (uint32_t back = 1; back <= kParts; ++back) {
+                const uint32_t part = kParts - back;
+#pragma unroll
+                for (uint32_t kk = run; kk < run + kRun; ++kk) {
+                  const uint32_t a = desc_a + kk * 2u, b = desc_b + part * b_step + kk * 2u;
+                  if (back == 1 && kk == run && starts) mma_pair<kMath, false>(leader, dst, a, b, idesc);
+                  else mma_pair<kMath, true>(leader, dst, a, b, idesc);
+                }
+              }
+              if constexpr (kMath != kInt8 && kSlices != 0) chain_ends(run + kRun == 4 && ks + 1 == ks_count);
             }
             if constexpr (kSlices == 0) {
               in_chain += 4;
