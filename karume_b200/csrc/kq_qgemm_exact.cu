@@ -371,8 +371,9 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16;
       const uint32_t dempty_0 = map_to_cta(dempty, 0);
       const float* my_scale = scale_ring + quarter * 32u + lane;
-      // kBatches x 16 columns per warp, a constant: a branch around every batch (a runtime width) takes
-      // the 450-clock drain of 256 columns to 1,400
+      // kBatches x 16 columns per warp, a constant.  A chain of 256 columns takes 883 clocks from one to the next,
+      // hand-over included (group 32, binary16: two of them are the k-step of 1,765; 690 at 192 columns, 504 at
+      // 128); with a branch around every batch (a runtime width) it is 1,130, 1,043 and 728.
       auto drain_all = [&](auto batches) {
         constexpr int kBatches = decltype(batches)::value;
         float acc[kBatches][16];
@@ -393,8 +394,9 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           for (uint32_t d = d0; d < d_end; ++d, at += acc_cols) {
             [[maybe_unused]] float s = 1.0f;
             if constexpr (kGroupScales) s = my_scale[((batch & 1u) * kScaleBatch + d % kScaleBatch) * kRows];
-            // scalar fused multiply-adds: the packed form (fma.rn.f32x2) needs register pairs the
-            // allocator does not find beside 128 sums (measured 460 - 800 clocks a chain against 335)
+            // scalar fused multiply-adds: the packed form (fma.rn.f32x2) wants register pairs, which the
+            // allocator does not find beside 128 sums without spills (k-steps of 1,777 and 1,426 clocks at 256 and
+            // 192 columns against 1,765 and 1,380; narrower tiles, with sums to spare, gain 5 to 9 %)
             auto add = [&](float (&sums)[16], const uint32_t (&v)[16]) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
@@ -633,8 +635,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
             const uint32_t desc_a = desc_a0 + s * stage_step, desc_b = desc_b0 + s * stage_step, this_empty = empty + s * 8;
             if (++s == p.stages) { s = 0; phase ^= 1u; }
             // Low parts first: an accumulation truncates to the accumulator's size, so the fewer follow once the
-            // high parts are in, the better (through four layers of a decoder, 289
-            // rows: 1.8e-7 from f64 against 3.9e-7 with the high parts first).
+            // high parts are in, the better (289 rows through four layers of a decoder: 1.8e-7 from f64 against
+            // 3.9e-7 with the high parts first).
             constexpr uint32_t kRun = kSlices == 0 ? 4u : kSlices;  // slices of a chain in this k-step
 #pragma unroll
             for (uint32_t run = 0; run < 4; run += kRun) {
