@@ -20,8 +20,8 @@
 //     multiply-add keeps: a small value of a row, on a channel without weight at the large ones.
 //     The third part costs 333 x 1536 -> 8960 int4 32.6 us against 32.1, 1024 x 4096 -> 6144 129
 //     against 118; 257 x 1536 -> 8960 int8 29 against 25.)
-//   * an accumulator chain is one group long (at most kMaxChain k), so the tensor core's f32
-//     accumulation never gets the chance to drift;
+//   * an accumulator chain is at most one group long, and at most 64 to 256 k (chain_of), so the tensor
+//     core's f32 accumulation, which truncates, never gets the chance to drift;
 //   * the integer-dot form of int4 weights is the same kernel: its per-group sums are integers
 //     below 2^24, exact in the f32 accumulator, and the contract's one fma per group in
 //     ascending order IS the drain (bit-identical).  Int8 weights with int8 activations run on
@@ -79,7 +79,7 @@ constexpr uint32_t kSmemLimit = 227 * 1024;
 constexpr uint32_t kScaleBatch = 8;             // accumulator chains per slot of the scale ring (two slots)
 constexpr uint32_t kTailRowScale = 320, kTailScales = kTailRowScale + kMaxNT * 4;
 constexpr uint32_t kSmemTail = kTailScales + 2 * kScaleBatch * kRows * 4;  // barriers, the tile's row scales, the scale ring
-constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain
+constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
 
 struct ExTarget {
   const uint8_t* w;
@@ -98,7 +98,7 @@ struct ExParams {
   uint32_t ksteps;         // k-steps of 128 bytes (64 binary16 or 128 int8 values)
   uint32_t nt;             // activation rows per tile, a multiple of 32
   uint32_t drain16;        // k16 slices per accumulator chain
-  uint32_t drains_per_group_shift;  // accumulator chains per scale group, log2 (groups longer than kMaxChain)
+  uint32_t drains_per_group_shift;  // accumulator chains per scale group, log2 (groups longer than a chain)
   uint32_t groups;         // scale groups per row
   uint32_t scale_f16;
   uint32_t stages, stage_bytes, raw_off, raw_bytes, raw_box;
@@ -1083,9 +1083,24 @@ Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t 
   return best;
 }
 
+// Most k of an accumulator chain.  Each of a chain's accumulations truncates (half a unit of 2^-24 on average, all the
+// same way), while the sums of the drain round to nearest.  Relative error against f64 (2-norm, k = 4,096), and us for
+// 300 x 4096 -> 4090 int8, with chains of 64, 128, 256 and 1,024:
+//   f32, three parts        1.3, 2.7, 6.0, 26e-7   50, 47, 46, 46
+//   f32, two parts (tiled)  1.7, 2.5, 4.8, 21e-7   (1024 x 4096 -> 4096) 68, 63, 61.5, 60
+//   binary16, int8 weights  1.6, 1.5, 2.3, 9.7e-7  32, 30, 29, 29
+//   bf16, int8 weights      1.1, 1.0, 1.1, 3.3e-7  44, 42, 41, 40
+//   binary16, int4 weights  1.5, 1.1, 0.9, 2.1e-7  (300 x 8192 -> 4000) 52, 47, 45, 43
+// An f32 multiply-add per weight is 2.1e-7 from f64 there, the int8 GEMV 8 to 13e-7: each is kept below the path it
+// stands in for.
+uint32_t chain_of(int math, const Weight& w) {
+  if (math == kBf3) return 64;
+  return math == kHalf1 && w.storage == KQ_STORAGE_I8 ? 128 : 256;
+}
+
 // x: binary16 (kHalf1), parts already split (kHalf2 / kBf1 / kBf3) or int8 (kInt8).
 cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const float* residual, const void* x, int math,
-                      uint32_t m, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, int* launches) {
+                      uint32_t m, uint32_t max_chain, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, int* launches) {
   const Weight& w0 = *targets[0].w;
   const WeightKind kind = kind_of(w0);
   ExParams p = {};
@@ -1120,8 +1135,8 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   p.ksteps = (w0.k + step_k - 1) / step_k;
   p.scale_f16 = w0.scale_dtype == KQ_F16;
   const bool i4 = kind == kI4Tiled || kind == kI4Rows;
-  const uint32_t group = i4 ? w0.group_size : kMaxChain;
-  const uint32_t chain = std::min(group, kMaxChain);
+  const uint32_t group = i4 ? w0.group_size : max_chain;
+  const uint32_t chain = std::min(group, max_chain);
   p.drain16 = chain / 16;
   p.drains_per_group_shift = 0;
   while ((chain << p.drains_per_group_shift) < group) ++p.drains_per_group_shift;
@@ -1225,7 +1240,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
     const uint8_t* xp = static_cast<const uint8_t*>(x) + static_cast<size_t>(r0) * k * xb;
     cudaError_t e;
     if (direct) {
-      e = run_exact(env, count, t, residual, xp, math, pm, nullptr, ws, room, true, launches);
+      e = run_exact(env, count, t, residual, xp, math, pm, chain_of(math, w0), nullptr, ws, room, true, launches);
     } else {
       float* inv = reinterpret_cast<float*>(ws);
       uint16_t* parts = reinterpret_cast<uint16_t*>(ws + align256(static_cast<uint64_t>(pm) * 4));
@@ -1239,7 +1254,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
       else e = split(split_kernel<float, kHalf2>, reinterpret_cast<const float*>(xp));
       if (e != cudaSuccess) return e;
       if (launches) *launches += 1;
-      e = run_exact(env, count, t, residual, parts, math, pm, inv, ws + taken, room - taken, true, launches);
+      e = run_exact(env, count, t, residual, parts, math, pm, chain_of(math, w0), inv, ws + taken, room - taken, true, launches);
     }
     if (e != cudaSuccess) return e;
   }
@@ -1269,7 +1284,7 @@ cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& targ
   const Weight& w = *target.w;
   uint8_t* ws = static_cast<uint8_t*>(env.workspace);
   const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
-  if (w.storage == KQ_STORAGE_I8) return run_exact(env, 1, &target, nullptr, xq, kInt8, m, xs, ws, room, true, launches);
+  if (w.storage == KQ_STORAGE_I8) return run_exact(env, 1, &target, nullptr, xq, kInt8, m, kMaxChain, xs, ws, room, true, launches);
   // int4: per-group sums as binary16 products (exact), flushed in ascending order: no K slices
   const uint64_t per_row = static_cast<uint64_t>(w.k) * 2;
   uint32_t panel = static_cast<uint32_t>(std::min<uint64_t>(m, room / per_row));
@@ -1284,7 +1299,7 @@ cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& targ
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
     const LinearTarget t{target.w, target.bias, target.out + static_cast<size_t>(r0) * w.n};
-    e = run_exact(env, 1, &t, nullptr, ws, kHalf1, pm, xs + r0, nullptr, 0, false, launches);
+    e = run_exact(env, 1, &t, nullptr, ws, kHalf1, pm, kMaxChain, xs + r0, nullptr, 0, false, launches);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

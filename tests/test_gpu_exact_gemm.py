@@ -182,3 +182,30 @@ def test_an_infinite_activation_reaches_the_channels_that_multiply_it(gpu):
     rest = np.arange(m) != 3
     assert oracle.allclose(got[rest], clean[rest], atol=1e-5, rtol=1e-4)["pass"]
     w.free()
+
+
+@pytest.mark.parametrize("xdt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("storage,group,n", [("i8", 0, 515), ("i8", 0, 512), ("i4", 1024, 512), ("i4", 128, 512)])
+def test_long_sums_do_not_drift(gpu, xdt, storage, group, n):
+    """2-norm error against f64 of sums over 8192 k.  The tensor core truncates each accumulation of 16 k, half a unit of
+    2^-24 on average; chains of at most 256 k have 16: 16 x 2^-25 = 4.8e-7, and the rounding of 32 to 128 chains' sums,
+    sqrt(128) x 2^-25 at the most = 3.4e-7: together (at right angles) 6e-7.  (One chain of 1024 k: 1 to 2.6e-6.)"""
+    import torch
+    if xdt == "bf16" and storage == "i8" and n % 16 == 0:
+        pytest.skip("the bf16 GEMM's case")
+    m, k = 70, 8192
+    rng = np.random.default_rng(n + group)
+    x = {"f32": lambda v: v, "f16": oracle.round_to_f16, "bf16": oracle.round_to_bf16}[xdt](rng.standard_normal((m, k)).astype(np.float32))
+    bias = np.zeros(n, np.float32)
+    if storage == "i4":
+        data, scale = cases.synth_i4(n, k, seed=n, group_size=group, scale_dtype="f32")
+        ref = oracle.linear_i4(x, data, scale, bias, n, k, group)
+    else:
+        data, scale = cases.synth_i8(n, k, seed=n)
+        ref = oracle.linear_i8(x, data, scale.astype(np.float32), bias, n, k)
+    w = gpu.upload_weight(storage, data, scale, (n, k), group)
+    got = gpu.linear(dev(x).to({"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[xdt]), w, dev(bias))
+    gpu.sync()
+    diff = got.cpu().numpy().astype(np.float64) - ref
+    assert np.linalg.norm(diff) <= 6e-7 * np.linalg.norm(ref.astype(np.float64)), np.linalg.norm(diff) / np.linalg.norm(ref.astype(np.float64))
+    w.free()
