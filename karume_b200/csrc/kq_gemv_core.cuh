@@ -54,7 +54,8 @@ __device__ __forceinline__ void load_x8(const XT* p, float (&v)[8]) {
 // ---- power-of-two pre-scale of the activations -------------------------------------------
 // binary16 has a narrow exponent range, f32 activations do not.  Before an activation is split
 // into binary16 parts it is multiplied by 2^e, with e chosen from the largest magnitude of the
-// values that share it (a 32-k scale group of one activation row, or a whole activation row),
+// values that share it (a 32-k scale group of one activation row, a warp's slab of 64 or 128 k, or
+// a whole activation row),
 // so that this maximum lands in [2^13, 2^14).  The multiplication is exact, the matching
 // 2^-e is applied in f32 to the group's (or row's) partial sum, and the result no longer
 // depends on the magnitude of x: there is neither an upper limit at 65504 nor an absolute

@@ -1033,13 +1033,14 @@ cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, uint3
 }
 
 // Clocks of one k-step, fitted to the difference between k = 4,096 and 12,288 at every tile width (1536
-// channels, one tile; within 25 % of it, and the choices below are the fastest of a sweep of 13 shapes, 24 to
+// channels, one tile; within a third of it, and the choices below are the fastest of a sweep of 13 shapes, 24 to
 // 1,024 rows, within its noise).  The conversion of the weights does not grow with the tile, its copy and the
 // MMAs do; a drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step.
 // Measured at nt = 32, 64, 128, 192, 256:
-//   int4, group 32   binary16 685, 790, 1,010, 1,380, 1,765; f32 830, 1,090, 1,215, 1,510, 1,870
-//   int8             binary16 460, 525, 635, 650, 640; f32 tiled 635, 760, 665, 850, 1,190, untiled 900, 1,050,
-//                    1,075, 1,270, 1,680 (bytes take 9 instructions for four bf16 integers, 4 for binary16)
+//   int4, group 32   binary16 690, 785, 1,010, 1,375, 1,755; f32 805, 1,080, 1,275, 1,520, 1,880
+//   int8, tiled      binary16 475, 535, 650, 690, 775; f32 615, 720, 695, 860, 1,235
+//   int8, rows       binary16 625, 700, 835, 890, 985; f32 1,110, 1,325, 1,415, 1,580, 1,675 (bytes take 9
+//                    instructions for four bf16 integers, 4 for binary16)
 // Three parts above 128 rows leave three stages: a k-step is a third of a stage's whole trip.
 uint32_t kstep_clocks(uint32_t nt, int math, uint32_t drains_x4, bool int8_weights) {
   const bool int8 = math == kInt8, bytes_to_bf = int8_weights && (math == kBf1 || math == kBf3);

@@ -1,7 +1,7 @@
 """The linear op takes activations of ANY magnitude, as the reference's f32 multiply-add does
 (packages/runtime/src/kernels/gemm.ts:922-940).  The tensor-core GEMVs carry the activations
-as binary16 parts after an exact power-of-two pre-scale per 32-k group (per activation row
-for the wide and the int8 kernels); these tests drive every kernel family, the fused plan
+as binary16 parts after an exact power-of-two pre-scale per 32-k group (per 128 or 64 k of a row
+where they are held in registers, per activation row for the int8 kernels); these tests drive every kernel family, the fused plan
 and the static-scratch entry with activations scaled by 10^e, with rows that mix 1e-6 and
 1e3, with values beyond the binary16 range and with group scales near 1.
 
@@ -79,7 +79,7 @@ def activations(kind, m, k, seed):
 
 
 KINDS = [-6, -4, -2, 2, 4, "mixed", "beyond_f16"]
-# (m, dtype): group-packed (1, 2 rows), adjacent-column (3, 4 f32 rows), wide (5..16 rows)
+# (m, dtype): group-packed (1, 2 rows), activations in registers (3..16 rows; two parts of a row in adjacent columns up to 4)
 FAMILIES = [(1, "f32"), (2, "f32"), (3, "f32"), (4, "bf16"), (4, "f16"), (8, "f32"), (16, "f32"), (16, "f16")]
 
 
