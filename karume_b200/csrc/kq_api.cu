@@ -1,6 +1,7 @@
 // C ABI of libkq (see include/kq.h): context, buffers, weight residency, the linear
 // op's shape checks and kernel choice, CUDA-graph plans and timing.  There is no CPU
 // path anywhere in this file: a request no kernel covers is an error.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -47,13 +48,14 @@ struct kq_ctx {
   void* host_dev_out = nullptr;
   uint64_t host_x_bytes = 0, host_out_bytes = 0;
   float* zero_bias = nullptr;  // kq_linear_reduce's unfused path: ranks other than 0 add no bias
-  uint64_t zero_bias_count = 0;
+  uint64_t zero_bias_bytes = 0;
   int* idot_sums = nullptr;  // integer sums of the quantised activations (kq_linear_a8)
   uint64_t idot_sums_bytes = 0;
   float* fused_xn = nullptr;  // kq_linear_fused outside a plan: the normalised activations ...
   uint64_t fused_xn_bytes = 0;
   float* fused_gu = nullptr;  // ... and the gate / up outputs in front of the SiLU gate
   uint64_t fused_gu_bytes = 0;
+  std::vector<void*> outgrown;  // scratch that recorded graphs still point to
 };
 
 namespace {
@@ -239,6 +241,27 @@ int upload_checked(kq_ctx* ctx, int storage, const void* payload, uint64_t paylo
   const uint64_t handle = ctx->next_handle++;
   ctx->weights[handle] = w;
   *out = handle;
+  return KQ_OK;
+}
+
+// Grown scratch of a context (`buf` holds `have` bytes).  A recorded graph keeps the addresses of the scratch it
+// was recorded with, so while graphs exist an outgrown buffer stays until the last of them is freed; the new one is
+// then at least twice as large, which bounds what is kept to the size of what is in use.
+template <typename T>
+int grow_scratch(kq_ctx* ctx, T** buf, uint64_t* have, uint64_t need, const char* who) {
+  if (need <= *have) return KQ_OK;
+  if (ctx->capturing) return fail(ctx, KQ_ERR_STATE, "%s: scratch must grow; call once outside the recording first", who);
+  const bool keep = *buf && !ctx->graphs.empty();
+  if (keep) {
+    need = std::max(need, 2 * *have);
+    ctx->outgrown.push_back(*buf);
+  } else if (*buf) {
+    cudaFree(*buf);
+  }
+  *buf = nullptr;
+  *have = 0;
+  KQ_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(buf), need));
+  *have = need;
   return KQ_OK;
 }
 
@@ -455,6 +478,7 @@ void kq_destroy(kq_ctx* ctx) {
   if (ctx->host_x) cudaFreeHost(ctx->host_x);
   if (ctx->host_dev_x) cudaFree(ctx->host_dev_x);
   if (ctx->host_dev_out) cudaFree(ctx->host_dev_out);
+  for (void* p : ctx->outgrown) cudaFree(p);
   if (ctx->idot_sums) cudaFree(ctx->idot_sums);
   if (ctx->fused_xn) cudaFree(ctx->fused_xn);
   if (ctx->fused_gu) cudaFree(ctx->fused_gu);
@@ -762,6 +786,10 @@ int kq_graph_free(kq_ctx* ctx, kq_graph g) {
   cudaGraphExecDestroy(it->second);
   ctx->graphs.erase(it);
   ctx->graph_kernels.erase(g);
+  if (ctx->graphs.empty() && !ctx->capturing) {
+    for (void* p : ctx->outgrown) cudaFree(p);
+    ctx->outgrown.clear();
+  }
   return KQ_OK;
 }
 
@@ -874,14 +902,8 @@ int kq_linear_a8(kq_ctx* ctx, kq_weight h, uint64_t xq_dptr, uint64_t xs_dptr, u
   int launched = 0;
   if (tiled) {
     const uint64_t need = (static_cast<uint64_t>(m) * (w->k / 32) + m) * sizeof(int);
-    if (need > ctx->idot_sums_bytes) {
-      if (ctx->capturing) return fail(ctx, KQ_ERR_STATE, "kq_linear_a8: scratch must grow; call once outside the recording first");
-      if (ctx->idot_sums) cudaFree(ctx->idot_sums);
-      ctx->idot_sums = nullptr;
-      ctx->idot_sums_bytes = 0;
-      KQ_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->idot_sums), need));
-      ctx->idot_sums_bytes = need;
-    }
+    const int rc = grow_scratch(ctx, &ctx->idot_sums, &ctx->idot_sums_bytes, need, "kq_linear_a8");
+    if (rc != KQ_OK) return rc;
     row_sum = ctx->idot_sums;
     group_sum = ctx->idot_sums + m;
     cudaError_t e = kq::launch_xq_sums(ctx->stream, reinterpret_cast<const int8_t*>(xq_dptr), m, w->k, row_sum, group_sum);
@@ -967,15 +989,10 @@ int kq_linear_reduce(kq_ctx* ctx, kq_weight h, uint64_t x_dptr, int x_dtype, uin
   // Two steps: the linear with the bias on rank 0 only, then the all-reduce.
   uint64_t bias_here = bias_dptr;
   if (kq::comm_rank(ctx->comm) != 0) {
-    if (w->n > ctx->zero_bias_count) {
-      if (ctx->capturing) return fail(ctx, KQ_ERR_STATE, "kq_linear_reduce: scratch must grow; call once outside the recording first");
-      if (ctx->zero_bias) cudaFree(ctx->zero_bias);
-      ctx->zero_bias = nullptr;
-      ctx->zero_bias_count = 0;
-      KQ_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->zero_bias), static_cast<size_t>(w->n) * sizeof(float)));
-      KQ_CUDA(ctx, cudaMemset(ctx->zero_bias, 0, static_cast<size_t>(w->n) * sizeof(float)));
-      ctx->zero_bias_count = w->n;
-    }
+    const uint64_t had = ctx->zero_bias_bytes;
+    const int rc = grow_scratch(ctx, &ctx->zero_bias, &ctx->zero_bias_bytes, static_cast<uint64_t>(w->n) * sizeof(float), "kq_linear_reduce");
+    if (rc != KQ_OK) return rc;
+    if (ctx->zero_bias_bytes != had) KQ_CUDA(ctx, cudaMemsetAsync(ctx->zero_bias, 0, ctx->zero_bias_bytes, ctx->stream));
     bias_here = reinterpret_cast<uint64_t>(ctx->zero_bias);
   }
   const int rc2 = run_linear(ctx, 1, &h, x_dptr, x_dtype, &bias_here, &out_dptr, m);
@@ -983,18 +1000,6 @@ int kq_linear_reduce(kq_ctx* ctx, kq_weight h, uint64_t x_dptr, int x_dtype, uin
   cudaError_t e = kq::comm_all_reduce(ctx->comm, ctx->stream, reinterpret_cast<float*>(out_dptr), count);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "kq_linear_reduce: all-reduce launch");
   ctx->launches += 1;
-  return KQ_OK;
-}
-
-// Grows one of the context's lazily allocated scratch buffers (never during a graph capture).
-static int grow_scratch(kq_ctx* ctx, float** buf, uint64_t* have, uint64_t need, const char* who) {
-  if (need <= *have) return KQ_OK;
-  if (ctx->capturing) return fail(ctx, KQ_ERR_STATE, "%s: scratch must grow; call once outside the recording first", who);
-  if (*buf) cudaFree(*buf);
-  *buf = nullptr;
-  *have = 0;
-  KQ_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(buf), need));
-  *have = need;
   return KQ_OK;
 }
 

@@ -167,3 +167,47 @@ def test_int8_reduction_gate_fails_loudly(gpu):
     got = host(gpu, gpu.linear_a8(xq, xs, w4, zero_bias))
     assert np.array_equal(got, np.full((1, n), float(k), np.float32))
     w4.free()
+
+
+def test_a_graph_keeps_the_scratch_it_was_recorded_with():
+    """Scratch grown by later, larger calls leaves the buffers that a recorded graph points to in place."""
+    import torch
+    import karume_b200 as kb
+    gpu = kb.acquire_gpu(0)  # a context without scratch yet
+    n, k = 192, 512
+    rng = np.random.default_rng(4)
+    data, scale = cases.synth_i4(n, k, seed=3)
+    w = gpu.upload_weight("i4", data, scale, (n, k), 32)
+    w8 = gpu.upload_weight("i4", *cases.synth_i4(n, 8 * k, seed=5), (n, 8 * k), 32)
+    bias = torch.zeros(n, device="cuda")
+    x = torch.from_numpy(rng.standard_normal((2, k)).astype(np.float32)).cuda()
+    prompt = torch.from_numpy(rng.standard_normal((20, k)).astype(np.float32)).cuda()
+    out, act = torch.empty(2, n, device="cuda"), torch.empty(20, n, device="cuda")
+    torch.cuda.synchronize()
+
+    def step():
+        gpu.linear_a8(xq, xs, w, bias, out=out)
+        gpu.linear_fused(prompt, [w, w], [bias, bias], [act], swiglu=True)  # gate and up through scratch
+
+    xq, xs = gpu.quantize_rows(x)
+    step()
+    gpu.sync()
+    want = out.clone(), act.clone()
+    torch.cuda.synchronize()
+    gpu.graph_begin()
+    step()
+    g = gpu.graph_end()
+    for rows in (3, 8):  # the sums' scratch grows, twice
+        big, bigs = gpu.quantize_rows(torch.ones(rows, 8 * k, device="cuda"))
+        gpu.linear_a8(big, bigs, w8, bias)
+        gpu.linear_fused(torch.ones(rows * 64, k, device="cuda"), [w, w], [bias, bias], swiglu=True)
+    filler = [torch.full((1 << 18,), float("nan"), device="cuda") for _ in range(8)]  # takes what was given back
+    out.fill_(0)
+    act.fill_(0)
+    torch.cuda.synchronize()
+    gpu.graph_launch(g)
+    gpu.sync()
+    assert torch.equal(out, want[0]) and torch.equal(act, want[1])
+    gpu.graph_free(g)
+    del filler
+    gpu.destroy()
