@@ -887,7 +887,12 @@ int kq_linear_a8(kq_ctx* ctx, kq_weight h, uint64_t xq_dptr, uint64_t xs_dptr, u
     return fail(ctx, KQ_ERR_UNSUPPORTED, "kq_linear_a8: k=%u exceeds the int32 reduction gate 131072", w->k);
   if (m == 0 || w->n == 0) return KQ_OK;
   DeviceGuard guard(ctx->device);
-  if (kq::qgemm_exact_a8_supports(*w, reinterpret_cast<const int8_t*>(xq_dptr), m, ctx->workspace ? ctx->workspace_bytes : 0)) {
+  const bool tiled = w->layout == kq::kLayoutTiledI4 || w->layout == kq::kLayoutTiledI8;
+  const uint64_t sums_bytes = (static_cast<uint64_t>(m) * (w->k / 32) + m) * sizeof(int);
+  // The many-row kernel also takes what the other would have to grow its scratch for while a graph is recorded (the
+  // results are the same bits).
+  if (kq::qgemm_exact_a8_supports(*w, reinterpret_cast<const int8_t*>(xq_dptr), m, ctx->workspace ? ctx->workspace_bytes : 0) &&
+      (kq::qgemm_exact_a8_preferred(*w, m) || (tiled && ctx->capturing && sums_bytes > ctx->idot_sums_bytes))) {
     const kq::LinearTarget target{w, reinterpret_cast<const float*>(bias_dptr), reinterpret_cast<float*>(out_dptr)};
     int n_launched = 0;
     cudaError_t e = kq::launch_qgemm_exact_a8(env_of(ctx), target, reinterpret_cast<const int8_t*>(xq_dptr),
@@ -896,13 +901,11 @@ int kq_linear_a8(kq_ctx* ctx, kq_weight h, uint64_t xq_dptr, uint64_t xs_dptr, u
     ctx->launches += n_launched;
     return KQ_OK;
   }
-  const bool tiled = w->layout == kq::kLayoutTiledI4 || w->layout == kq::kLayoutTiledI8;
   int* row_sum = nullptr;
   int* group_sum = nullptr;
   int launched = 0;
   if (tiled) {
-    const uint64_t need = (static_cast<uint64_t>(m) * (w->k / 32) + m) * sizeof(int);
-    const int rc = grow_scratch(ctx, &ctx->idot_sums, &ctx->idot_sums_bytes, need, "kq_linear_a8");
+    const int rc = grow_scratch(ctx, &ctx->idot_sums, &ctx->idot_sums_bytes, sums_bytes, "kq_linear_a8");
     if (rc != KQ_OK) return rc;
     row_sum = ctx->idot_sums;
     group_sum = ctx->idot_sums + m;

@@ -143,6 +143,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
                                int* launches);
 // ... and the integer-dot form: int8 activations [m, k] with row scales xs (bit-exact contract).
 bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes);
+bool qgemm_exact_a8_preferred(const Weight& w, uint32_t m);  // ... faster here than on the kernels of kq_idot.cu
 cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& target, const int8_t* xq, const float* xs, uint32_t m,
                                   int* launches);
 }  // namespace kq

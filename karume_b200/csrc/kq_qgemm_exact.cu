@@ -1263,18 +1263,23 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
 }
 
 // Integer-dot form: int8 activations xq [m, k] with row scales xs.
-bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes) {
-  // (us, the mma.sync kernel | here)  At most eight rows of a tiled int4 weight run faster there (8 x 4096 -> 65536
-  // 88 | 111: the ascending fma chain over the groups allows no K split).  A tiled int8 one runs faster here, 1 x 4096
-  // -> 4096 41 | 10, 8 x 1536 -> 32768 22 | 18, until its tiles are several waves of CTA pairs, where that kernel
-  // streams and this one starts over: 1 x 1536 -> 65536 24 | 35, -> 151936 45 | 72; from nine rows on, two launches of
-  // it, only with a short k (12 x 256 -> 151936 26 | 48, 12 x 1024 -> 65536 33 | 32; int4 29 | 59, 49 | 44).  The
-  // generic kernel of the untiled layouts (0.09 us per k) only below k = 128.
+bool qgemm_exact_a8_preferred(const Weight& w, uint32_t m) {
+  // (us, the mma.sync kernel | here)  The mma.sync kernel streams a matrix of any size, this one starts over with
+  // every wave of 74 CTA pairs (18,944 channels).
+  //   int4, up to eight rows   the ascending fma chain over the groups allows no K split here, so one wave and no
+  //                            more: 1 x 4096 -> 4096 43 | 29, 8 x 4096 -> 14336 47 | 30, 8 x 1536 -> 1024 14 | 15, but
+  //                            8 x 1024 -> 32768 19 | 23, 8 x 4096 -> 65536 88 | 111
+  //   int8, up to eight rows   1 x 256 -> 4096 7.4 | 4.6, 1 x 4096 -> 4096 41 | 10, 8 x 1536 -> 32768 22 | 18, but
+  //                            1 x 1536 -> 65536 24 | 35, -> 151936 45 | 72
+  //   nine to sixteen          are two launches there, which pay for many waves only with a short k: 12 x 256 ->
+  //                            151936 26 | 48 (int4 29 | 59), 12 x 1024 -> 65536 33 | 32 (int4 49 | 44)
+  //   untiled                  the generic kernel (0.09 us per k) only below k = 128
   const bool many_waves = w.n > 49152, short_k = w.k < 512;
-  if (w.layout == kLayoutTiledI4   ? m <= 8 || (m <= 16 && many_waves && short_k)
-      : w.layout == kLayoutTiledI8 ? many_waves && (m <= 8 || (m <= 16 && short_k))
-                                   : w.k < 128)
-    return false;
+  if (w.layout == kLayoutTiledI4) return m > 16 || (m > 8 ? !(many_waves && short_k) : w.n <= 18944);
+  if (w.layout == kLayoutTiledI8) return m > 16 || !many_waves || (m > 8 && !short_k) || w.k > 65536;  // (its sums end at k = 65536)
+  return w.k >= 128;
+}
+bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes) {
   if (m == 0 || w.k == 0 || !kind_ok(w) || w.k % 16 != 0 || (reinterpret_cast<uintptr_t>(xq) & 15u) != 0) return false;
   if (w.storage == KQ_STORAGE_I8) return true;
   return w.group_size <= kMaxChain && align256(static_cast<uint64_t>(w.k) * 2 * 32) <= workspace_bytes;

@@ -75,7 +75,7 @@ def test_matches_the_f64_oracle(gpu, xdt, storage, group, m, n, k):
 @pytest.mark.parametrize("storage,group,m,n,k", [s for s in SHAPES if s[1] <= 1024] + [("i4", 16, 129, 67, 48), ("i8", 0, 300, 528, 8960),
                          # few rows, on both sides of the lines between this kernel and the mma.sync one
                          ("i8", 0, 3, 64, 32), ("i8", 0, 8, 49152, 96), ("i8", 0, 8, 49168, 96), ("i8", 0, 16, 49168, 448), ("i8", 0, 16, 49168, 512),
-                         ("i4", 32, 8, 144, 512), ("i4", 32, 16, 49168, 448), ("i4", 32, 16, 49168, 512)])
+                         ("i4", 32, 8, 144, 512), ("i4", 32, 1, 18944, 64), ("i4", 32, 8, 18960, 64), ("i4", 32, 16, 49168, 448), ("i4", 32, 16, 49168, 512)])
 def test_integer_dot_is_bit_exact(gpu, storage, group, m, n, k):
     rng = np.random.default_rng(m)
     x = rng.standard_normal((m, k)).astype(np.float32)

@@ -211,3 +211,25 @@ def test_a_graph_keeps_the_scratch_it_was_recorded_with():
     gpu.graph_free(g)
     del filler
     gpu.destroy()
+
+
+@pytest.mark.parametrize("storage,n,k", [("i8", 49168, 512), ("i4", 18960, 256)])
+def test_the_first_call_of_a_context_can_be_recorded(storage, n, k):
+    import torch
+    import karume_b200 as kb
+    gpu = kb.acquire_gpu(0)
+    data, scale = cases.synth_i4(n, k, seed=1) if storage == "i4" else cases.synth_i8(n, k, seed=1)
+    w = gpu.upload_weight(storage, data, scale, (n, k), 32 if storage == "i4" else 0)
+    bias = torch.ones(n, device="cuda")
+    xq, xs = gpu.quantize_rows(torch.randn(2, k, device="cuda"))
+    out = torch.zeros(2, n, device="cuda")
+    torch.cuda.synchronize()
+    gpu.graph_begin()
+    gpu.linear_a8(xq, xs, w, bias, out=out)
+    g = gpu.graph_end()
+    gpu.graph_launch(g)
+    direct = gpu.linear_a8(xq, xs, w, bias)
+    gpu.sync()
+    assert torch.equal(out, direct) and torch.count_nonzero(out)
+    gpu.graph_free(g)
+    gpu.destroy()
