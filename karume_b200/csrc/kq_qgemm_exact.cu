@@ -31,7 +31,8 @@
 // rows the N side (NT <= 256 of them), so a lane of the accumulator is one output channel: its
 // scale and bias are per-lane scalars and a store instruction writes 32 consecutive outputs.
 //
-//   warps 0-7    drain: tcgen05.ld, one fma per sum, then the epilogue
+//   warps 0-7    drain: tcgen05.ld, one fma per sum, then the epilogue (K slices of one tile that form a cluster
+//                add their sums over its shared memory first, in slice order)
 //   warps 8-11   producers: raw packed weights (shared memory) -> integers in the K-major,
 //                128-byte-swizzled tile the MMA reads.  Shared memory to shared memory only: a
 //                global load still in flight when a thread runs its proxy fence would hold the
@@ -79,6 +80,7 @@ constexpr uint32_t kSmemLimit = 227 * 1024;
 constexpr uint32_t kScaleBatch = 8;             // accumulator chains per slot of the scale ring (two slots)
 constexpr uint32_t kTailRowScale = 320, kTailScales = kTailRowScale + kMaxNT * 4;
 constexpr uint32_t kSmemTail = kTailScales + 2 * kScaleBatch * kRows * 4;  // barriers, the tile's row scales, the scale ring
+constexpr uint32_t kMaxClusterSplits = 4;       // K slices that meet in a cluster: two or four (eight CTAs, the portable most)
 constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
 
 struct ExTarget {
@@ -104,6 +106,7 @@ struct ExParams {
   uint32_t stages, stage_bytes, raw_off, raw_bytes, raw_box;
   const float* row_scale;  // [m]: undoes the pre-scale (2^-e), or the activation scale of the integer-dot form; null: 1
   uint32_t splits, ksteps_per_split;
+  uint32_t cluster_splits; // 1, or = splits: the K slices of a tile are one cluster and add their sums over its shared memory
   float* partial;          // [splits][m][n of all weights] raw sums when splits > 1
   uint32_t n_total;
   int* status;
@@ -190,6 +193,12 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+// of another CTA of the cluster (an address of map_to_cta)
+__device__ __forceinline__ uint32_t lds32_cluster(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
 }
 __device__ __forceinline__ void sts64(uint32_t addr, uint2 v) {
@@ -296,7 +305,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 304);
   float* row_scale_s = reinterpret_cast<float*>(tail + kTailRowScale);
   float* scale_ring = reinterpret_cast<float*>(tail + kTailScales);
-  const uint32_t cta_rank = cluster_ctarank();
+  // a cluster is one pair, or the pairs of all K slices of a tile: ranks 2z and 2z + 1 are slice z
+  const uint32_t cluster_rank = cluster_ctarank(), cta_rank = cluster_rank & 1u, pair_rank0 = cluster_rank & ~1u;
   // Tensor memory holds two sets of accumulators, the MMAs fill one while the drain reads the other.  A set is as
   // many chains as fit half of the 512 columns (one of 256 columns, two of 128, four of 64, eight of 32): a
   // hand-over costs about 390 clocks whatever it hands over (24 x 4096 -> 9472: 33 us with one chain of 32 columns each).
@@ -369,7 +379,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       }
     } else {
       const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16;
-      const uint32_t dempty_0 = map_to_cta(dempty, 0);
+      const uint32_t dempty_0 = map_to_cta(dempty, pair_rank0);
       const float* my_scale = scale_ring + quarter * 32u + lane;
       // kBatches x 16 columns per warp, a constant.  A chain of 256 columns takes 883 clocks from one to the next,
       // hand-over included (group 32, binary16: two of them are the k-step of 1,765; 690 at 192 columns, 504 at
@@ -438,24 +448,28 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         case 2: drain_all(std::integral_constant<int, 2>{}); break;
         case 3: drain_all(std::integral_constant<int, 3>{}); break;
         case 4: drain_all(std::integral_constant<int, 4>{}); break;
+        case 5: drain_all(std::integral_constant<int, 5>{}); break;
         case 6: drain_all(std::integral_constant<int, 6>{}); break;
+        case 7: drain_all(std::integral_constant<int, 7>{}); break;
         default: drain_all(std::integral_constant<int, 8>{}); break;
       }
     }
     // ---------------- epilogue ----------------
     const ExTarget tg = p.t[wi];
     const bool row_live = row < tg.n;
+    // the K slices of a cluster meet in slice order, each finishing its share of the columns
+    const uint32_t slices = p.cluster_splits, share0 = slices > 1 ? cols * blockIdx.z / slices : 0u;
+    const uint32_t share1 = slices > 1 ? cols * (blockIdx.z + 1) / slices : cols;
+    if (slices > 1) cluster_sync_all();  // everybody has parked
     const uint32_t mm0 = m0 + col0;
     const uint32_t live_cols = row_live && mm0 < p.m ? min(cols, p.m - mm0) : 0u;
-    if (p.splits == 1) {
+    if (p.splits == 1 || slices > 1) {
       const float bias = row_live ? tg.bias[row] : 0.0f;
       float ws = 1.0f;
       if constexpr (!kGroupScales) ws = row_live ? load_scale_dyn(tg.scale, row, p.scale_f16) : 0.0f;
-      float* dst = tg.out + static_cast<size_t>(mm0) * tg.n + row;
-      const float* res = tg.residual != nullptr ? tg.residual + static_cast<size_t>(mm0) * tg.n + row : nullptr;
-#pragma unroll 4
-      for (uint32_t c = 0; c < live_cols; ++c) {
-        const uint32_t v = lds32(park + c * 128u);
+      float* dst = tg.out + static_cast<size_t>(mm0 + share0) * tg.n + row;
+      const float* res = tg.residual != nullptr ? tg.residual + static_cast<size_t>(mm0 + share0) * tg.n + row : nullptr;
+      auto finish = [&](uint32_t c, uint32_t v) {
         const float rs = row_scale_s[col0 + c];
         float o;
         if constexpr (kMath == kInt8) o = fmaf(__int2float_rn(static_cast<int>(v)), __fmul_rn(rs, ws), bias);
@@ -467,6 +481,31 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         }
         *dst = o;
         dst += tg.n;
+      };
+      if (slices == 1) {
+#pragma unroll 4
+        for (uint32_t c = 0; c < live_cols; ++c) finish(c, lds32(park + c * 128u));
+      } else {
+        const uint32_t last = min(share1, live_cols);
+        uint32_t from[kMaxClusterSplits];
+#pragma unroll
+        for (uint32_t z = 0; z < kMaxClusterSplits; ++z) from[z] = map_to_cta(park, 2u * min(z, slices - 1u) + cta_rank);
+        auto total = [&](auto count, uint32_t c) {
+          uint32_t sum = 0, v[decltype(count)::value];
+#pragma unroll
+          for (uint32_t z = 0; z < decltype(count)::value; ++z) v[z] = lds32_cluster(from[z] + c * 128u);
+#pragma unroll
+          for (uint32_t z = 0; z < decltype(count)::value; ++z)
+            sum = z == 0 ? v[0] : kMath == kInt8 ? sum + v[z] : __float_as_uint(__uint_as_float(sum) + __uint_as_float(v[z]));
+          return sum;
+        };
+        if (slices == 2) {
+#pragma unroll 8
+          for (uint32_t c = share0; c < last; ++c) finish(c, total(std::integral_constant<uint32_t, 2>{}, c));
+        } else {
+#pragma unroll 4
+          for (uint32_t c = share0; c < last; ++c) finish(c, total(std::integral_constant<uint32_t, kMaxClusterSplits>{}, c));
+        }
       }
     } else {
       uint32_t before = 0;
@@ -490,7 +529,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     // order).  Wide tiles of three-part activations leave three stages: a tile's conversion is then part of
     // every third k-step's trip, and the four warps share it.
     const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), full_0 = map_to_cta(full, 0);
+    const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), full_0 = map_to_cta(full, pair_rank0);
     constexpr int kUnroll = kParts == 3 ? 2 : 4;
     const bool shared_stage = stage_warps<kMath>(p.stages) != 1;
     const uint32_t rb0 = shared_stage ? 2u * (warp - kDrainWarps) : 0u, rb1 = shared_stage ? rb0 + 2u : 8u;  // this warp's 16-row blocks
@@ -591,7 +630,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       {
         const uint32_t half_rows = p.nt / 2, b_bytes = half_rows * 128u, raw_bytes = p.raw_bytes;
         const CUtensorMap* w_map = wi == 0 ? &w_map0 : wi == 1 ? &w_map1 : wi == 2 ? &w_map2 : &w_map3;
-        const uint32_t full_0 = map_to_cta(full, 0), raw_off = kW == kI8Rows && kMath == kInt8 ? 0u : p.raw_off;
+        const uint32_t full_0 = map_to_cta(full, pair_rank0), raw_off = kW == kI8Rows && kMath == kInt8 ? 0u : p.raw_off;
         const uint32_t w_row = kTiled ? n0 / 16u : n0, w_step = p.raw_box;  // tensor-map rows and columns of the raw weights
         uint32_t s = 0, phase = 0;
         for (uint32_t ks = 0; ks < ks_count; ++ks) {
@@ -609,6 +648,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       // ---------------- MMA issuer: one thread, nothing converges in its loop ----------------
       {
         const uint32_t idesc = exact_idesc<kMath>(p.nt);
+        const uint32_t pair_mask = 3u << pair_rank0;
         const uint32_t b_step = (p.nt / 2 * 128u) >> 4, stage_step = p.stage_bytes >> 4;
         const uint32_t desc_a0 = static_cast<uint32_t>(umma_desc(tiles)), desc_b0 = static_cast<uint32_t>(umma_desc(tiles + kATile));
         // kSlices: k16 slices per accumulator chain when chains end inside a k-step or with it; 0: longer
@@ -624,7 +664,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           };
           auto chain_ends = [&](bool last) {
             if (++in_set == per_set || last) {
-              commit_both(leader, dfull + (set & 1u) * 8);
+              commit_both(leader, dfull + (set & 1u) * 8, pair_mask);
               ++set;
               in_set = 0;
             }
@@ -662,7 +702,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
                 in_chain = 0;
               }
             }
-            commit_both(leader, this_empty);  // the stage is free, in both CTAs, once these MMAs have read it
+            commit_both(leader, this_empty, pair_mask);  // the stage is free, in both CTAs, once these MMAs have read it
           }
         };
         if (kGroupScales && p.drain16 == 1) issue(std::integral_constant<uint32_t, 1>{});
@@ -750,6 +790,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     }
   }
 
+  if (p.cluster_splits > 1 && warp >= kDrainWarps) cluster_sync_all();  // (the drain warps' barrier in front of their epilogue)
   if (*abort_flag)  // a wait gave up: copies may still be in flight towards this CTA's shared memory
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -960,7 +1001,7 @@ cudaError_t encode_w_map(const void* w, uint32_t rows, uint64_t row_bytes, uint3
 }
 
 template <typename Kernel, typename... Args>
-cudaError_t launch_dependent(Kernel kernel, dim3 grid, uint32_t threads, size_t smem, uint32_t cluster, const LaunchEnv& env, Args... args) {
+cudaError_t launch_dependent(Kernel kernel, dim3 grid, uint32_t threads, size_t smem, dim3 cluster, const LaunchEnv& env, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -973,11 +1014,11 @@ cudaError_t launch_dependent(Kernel kernel, dim3 grid, uint32_t threads, size_t 
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
   }
-  if (cluster > 1) {
+  if (cluster.x > 1) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = cluster;
-    attr[na].val.clusterDim.y = 1;
-    attr[na].val.clusterDim.z = 1;
+    attr[na].val.clusterDim.x = cluster.x;
+    attr[na].val.clusterDim.y = cluster.y;
+    attr[na].val.clusterDim.z = cluster.z;
     ++na;
   }
   cfg.attrs = attr;
@@ -1018,7 +1059,44 @@ cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, uint32_t pairs,
     *configured = true;
   }
   const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + kSmemTail;
-  return launch_dependent(kernel, dim3(pairs * 2, m_tiles, p.splits), kExThreads, smem, 2, env, p, xm, wm[0], wm[1], wm[2], wm[3]);
+  return launch_dependent(kernel, dim3(pairs * 2, m_tiles, p.splits), kExThreads, smem, dim3(2, 1, p.cluster_splits), env, p, xm, wm[0], wm[1], wm[2], wm[3]);
+}
+
+// Pairs (slots[1]) and clusters of two or four pairs that the device holds at once; 0 where it cannot say.  Every form of
+// the kernel fills an SM, so one of them stands for all.
+cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSplits + 1]) {
+  struct Held { bool done; uint32_t clusters[kMaxClusterSplits + 1]; };
+  static PerDevice<Held> held_on;
+  Held* held = held_on.slot();
+  if (held == nullptr) return cudaErrorInvalidDevice;
+  if (!held->done) {
+    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
+    if (e != cudaSuccess) return e;
+    for (uint32_t z = 2; z <= kMaxClusterSplits; z *= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2, 1, z);
+      cfg.blockDim = dim3(kExThreads);
+      cfg.dynamicSmemBytes = kSmemLimit;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 2;
+      attr.val.clusterDim.y = 1;
+      attr.val.clusterDim.z = z;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 0) {
+        (void)cudaGetLastError();
+        n = 0;
+      }
+      held->clusters[z] = static_cast<uint32_t>(n);
+    }
+    held->done = true;
+  }
+  for (uint32_t z = 0; z <= kMaxClusterSplits; ++z) slots[z] = held->clusters[z];
+  slots[1] = static_cast<uint32_t>(std::max(1, env.sm_count / 2));
+  return cudaSuccess;
 }
 
 template <int kW>
@@ -1032,54 +1110,65 @@ cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, uint3
   return cudaErrorInvalidValue;
 }
 
-// Clocks of one k-step, fitted to the difference between k = 4,096 and 12,288 at every tile width (1536
-// channels, one tile; within a third of it, and the choices below are the fastest of a sweep of 13 shapes, 24 to
-// 1,024 rows, within its noise).  The conversion of the weights does not grow with the tile, its copy and the
-// MMAs do; a drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step.
-// Measured at nt = 32, 64, 128, 192, 256:
-//   int4, group 32   binary16 690, 785, 1,010, 1,375, 1,755; f32 805, 1,080, 1,275, 1,520, 1,880
-//   int8, tiled      binary16 475, 535, 650, 690, 775; f32 615, 720, 695, 860, 1,235
-//   int8, rows       binary16 625, 700, 835, 890, 985; f32 1,110, 1,325, 1,415, 1,580, 1,675 (bytes take 9
-//                    instructions for four bf16 integers, 4 for binary16)
-// Three parts above 128 rows leave three stages: a k-step is a third of a stage's whole trip.
+// Clocks of one k-step, from the difference between k = 4,096 and 8,192 with 74 pairs at work (18,944 channels, one
+// tile each; at 1.92 GHz).  The conversion of the weights does not grow with the tile, its copy and the MMAs do; a
+// drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step; the two or three
+// parts of f32 rows cost what their tiles take to arrive, and above 192 rows the power cap.
+// Measured at nt = 32, 64, 96, 128, 160, 192, 224, 256:
+//   int4, group 32   binary16 683, 798, 905, 1,048, 1,275, 1,450, 1,660, 1,750; f32 900, 1,200, 1,320, 1,510, 1,810,
+//                    1,960, 2,370, 2,940
+//   int8, tiled      binary16 535, 632, 632, 711, 764, 836, 950, 1,020 to 1,190; f32 780, 870, 890, 1,110, 1,290, 1,450,
+//                    1,600, 2,070
+//   int8, rows       (k = 4,096 to 12,288, 6 pairs; 32, 64, 128, 192, 256) binary16 625, 700, 835, 890, 985; f32 1,110, 1,325,
+//                    1,415, 1,580, 1,675 (bytes take 9 instructions for four bf16 integers, 4 for binary16)
 uint32_t kstep_clocks(uint32_t nt, int math, uint32_t drains_x4, bool int8_weights) {
   const bool int8 = math == kInt8, bytes_to_bf = int8_weights && (math == kBf1 || math == kBf3);
   const uint32_t parts = parts_of(math);
   const uint32_t mma = 4 * parts * std::max(nt / 2, 48u);
   const uint32_t step = int8 ? 650 + nt : 450 + (bytes_to_bf ? 200 : 0) + 100 * parts + nt + drains_x4 * (nt * 8 / 5 + 20) / 4;
-  const uint32_t trip = parts == 3 && nt > 128 ? nt * 15 / 2 + 100 : 0;
+  const uint32_t fill = parts == 3 ? (nt > 192 ? nt * 10 : 740 + nt * 28 / 5) : parts == 2 ? 640 + nt * 21 / 5 : 0;
   const uint32_t drain = int8 ? 0u : drains_x4 * std::max(nt * 7 / 2 + 60, 330u) / 4;
-  return std::max({mma, step, trip, drain});
+  return std::max({mma, step, fill, drain});
 }
 
-struct Geometry { uint32_t nt, m_tiles, splits; };
+struct Geometry { uint32_t nt, m_tiles, splits, cluster_splits; };
 // Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
-// loads, epilogue) plus its k-steps; a split adds the reduce launch and the partial sums, written and read
-// at 2,200 bytes per clock.  (Priced at 4,000, 1024 x 4096 -> 6144 was cut in two at nt = 256: 174 us, 118 now.)
+// loads, epilogue) plus its k-steps.  Two or four slices may meet in a cluster: no second launch and no partial sums in
+// memory, but 33 clusters of two pairs and 15 of four are all the device holds (74 pairs by themselves), and they start
+// later.  Other slices add the reduce launch and the partial sums, written and read at 2,200 bytes per clock.
+//   (us, with its split launch; reduce launch | cluster)  65 x 1152 -> 3072 group 16, four slices 16.0 | 13.8;
+//   300 x 4096 -> 4096 int8 binary16, two 29.0 | 22.8; 100 x 2048 -> 2048 group 128, four 18.2 | 15.4;
+//   333 x 8960 -> 1536, four, 72 tiles of 128 rows 45.4, 48 of 192 rows 49.3 | 46.6
+// Widths between the powers of two: 804 x 4096 -> 6144 f32 at 160 rows 117, 128 152, 192 123, 256 148.
 Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t ksteps, int math, bool int8_weights, uint32_t drain16,
-                         uint32_t slice_unit, bool may_split, uint32_t sm_pairs, uint64_t partial_room) {
-  Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1};
+                         uint32_t slice_unit, bool may_split, const uint32_t (&slots)[kMaxClusterSplits + 1], uint64_t partial_room) {
+  Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1, 1};
   uint64_t best_cost = ~0ull;
   const uint32_t drains_x4 = std::max(1u, 16 / drain16);  // accumulator chains per k-step, times four
   const uint32_t most = (m + 31) / 32;
   for (uint32_t mt = (m + kMaxNT - 1) / kMaxNT; mt <= most; ++mt) {
     uint32_t nt = ((m + mt - 1) / mt + 31) / 32 * 32;
-    if (nt > 128) nt = (nt + 63) / 64 * 64;
     if ((m + nt - 1) / nt != mt) continue;
     const uint32_t per = kstep_clocks(nt, math, drains_x4, int8_weights);
     for (uint32_t splits = 1; splits <= (may_split ? 16u : 1u); splits *= 2) {
-      if (splits > 1 && (ksteps / splits < 4 || static_cast<uint64_t>(splits) * m * n_total * 4 > partial_room)) break;
+      if (splits > 1 && ksteps / splits < 4) break;
       uint32_t each = (ksteps + splits - 1) / splits;
       each = (each + slice_unit - 1) / slice_unit * slice_unit;
-      const uint64_t waves = (static_cast<uint64_t>(pairs) * mt * splits + sm_pairs - 1) / sm_pairs;
-      uint64_t cost = waves * (5000 + nt * 30 + static_cast<uint64_t>(each) * per);
-      if (splits > 1) cost += 5500 + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = {nt, mt, splits};
+      for (uint32_t in_cluster = 0; in_cluster < 2; ++in_cluster) {
+        if (in_cluster != 0 ? splits == 1 || splits > kMaxClusterSplits || slots[splits] == 0 || (ksteps + each - 1) / each != splits
+                            : splits > 1 && static_cast<uint64_t>(splits) * m * n_total * 4 > partial_room)
+          continue;
+        const uint32_t room = in_cluster != 0 ? slots[splits] * splits : slots[1];
+        const uint64_t waves = (static_cast<uint64_t>(pairs) * mt * splits + room - 1) / room;
+        uint64_t cost = waves * (5000 + nt * 30 + static_cast<uint64_t>(each) * per + (in_cluster != 0 ? 750 * splits : 0));
+        if (splits > 1 && in_cluster == 0) cost += 5500 + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = {nt, mt, splits, in_cluster != 0 ? splits : 1u};
+        }
       }
     }
-    if (mt >= 8 * sm_pairs) break;
+    if (mt >= 8 * slots[1]) break;
   }
   return best;
 }
@@ -1149,11 +1238,15 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   const uint32_t parts = parts_of(math);
   // a K slice is a whole number of int4 accumulator chains (an int8 chain may end anywhere)
   const uint32_t align = i4 && p.drain16 > 4 ? p.drain16 / 4 : 1;
-  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, math, !i4, p.drain16, align, may_split && scratch != nullptr,
-                                       std::max(1, env.sm_count / 2), scratch_bytes);
+  uint32_t slots[kMaxClusterSplits + 1];
+  cudaError_t ce = resident_pairs(env, slots);
+  if (ce != cudaSuccess) return ce;
+  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, math, !i4, p.drain16, align, may_split, slots,
+                                       scratch != nullptr ? scratch_bytes : 0);
   p.nt = geo.nt;
   p.ksteps_per_split = ((p.ksteps + geo.splits - 1) / geo.splits + align - 1) / align * align;
   p.splits = (p.ksteps + p.ksteps_per_split - 1) / p.ksteps_per_split;
+  p.cluster_splits = geo.cluster_splits;
   // stage: weight tile, activation parts, raw weights
   p.raw_bytes = (tiled ? 8 : kRows) * unit;
   p.raw_box = unit / elem;
@@ -1171,7 +1264,7 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   }
   if (e != cudaSuccess) return e;
   if (launches) *launches += 1;
-  if (p.splits > 1) {
+  if (p.splits > p.cluster_splits) {
     for (uint32_t i = 0; i < used; ++i) rp.t[i] = p.t[i];
     rp.count = used;
     rp.m = m;

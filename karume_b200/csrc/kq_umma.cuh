@@ -95,11 +95,11 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t leader, uint32_t tmem_d,
                "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
                ::"r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(idesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHigh), "r"(leader) : "memory");
 }
-// arrives on the barrier at this address in BOTH CTAs of the pair once the MMAs issued so far are done
-__device__ __forceinline__ void commit_both(uint32_t leader, uint32_t bar) {
+// arrives on the barrier at this address in BOTH CTAs of the pair (bits of `ctas`: their cluster ranks) once the MMAs issued so far are done
+__device__ __forceinline__ void commit_both(uint32_t leader, uint32_t bar, uint32_t ctas = 3u) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
                "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-               ::"r"(bar), "h"(static_cast<uint16_t>(3)), "r"(leader) : "memory");
+               ::"r"(bar), "h"(static_cast<uint16_t>(ctas)), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void commit_one(uint32_t leader, uint32_t bar) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"

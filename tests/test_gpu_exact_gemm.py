@@ -95,6 +95,21 @@ def test_integer_dot_is_bit_exact(gpu, storage, group, m, n, k):
     w.free()
 
 
+# K slices that meet in a cluster (two or four, the last one short), next to ragged channels and rows, and tiles of 160 and
+# 224 rows
+@pytest.mark.parametrize("xdt", ["f32", "f16"])
+@pytest.mark.parametrize("storage,group,m,n,k", [("i4", 32, 20, 272, 576), ("i4", 16, 33, 100, 1152), ("i4", 128, 97, 513, 1408),
+                                                 ("i4", 32, 160, 1040, 1088), ("i4", 32, 223, 528, 960), ("i8", 0, 50, 300, 1616),
+                                                 ("i8", 0, 225, 1008, 1120)])
+def test_slices_that_meet_in_a_cluster(gpu, xdt, storage, group, m, n, k):
+    test_matches_the_f64_oracle(gpu, xdt, storage, group, m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(20, 272, 4096), (150, 528, 2176), (97, 259, 1136)])
+def test_integer_sums_that_meet_in_a_cluster(gpu, m, n, k):
+    test_integer_dot_is_bit_exact(gpu, "i8", 0, m, n, k)
+
+
 @pytest.mark.parametrize("m,n,k", [(17, 64, 128), (130, 544, 1536)])
 def test_norm_gate_and_residual_around_it(gpu, m, n, k):
     import torch
