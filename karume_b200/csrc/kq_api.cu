@@ -329,7 +329,7 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
     // Many rows, and not the bf16 GEMM: weights as exact integers on the tensor cores, one launch
     // for all weights of the call.
     int launched = 0;
-    cudaError_t e = kq::launch_qgemm_exact(env, static_cast<int>(count), targets, reinterpret_cast<const void*>(x), x_dtype, m, &launched);
+    cudaError_t e = kq::launch_qgemm_exact(env, static_cast<int>(count), targets, reinterpret_cast<const void*>(x), x_dtype, m, false, &launched);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemm_exact launch");
     ctx->launches += launched;
     return KQ_OK;
@@ -357,7 +357,7 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
     const Weight& w = *targets[i].w;
     if (w.n != 0 && takes_exact_gemm(ctx, 1, &targets[i], x_dtype, m)) {
       int launched = 0;
-      cudaError_t e = kq::launch_qgemm_exact(env, 1, &targets[i], reinterpret_cast<const void*>(x), x_dtype, m, &launched);
+      cudaError_t e = kq::launch_qgemm_exact(env, 1, &targets[i], reinterpret_cast<const void*>(x), x_dtype, m, false, &launched);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemm_exact launch");
       ctx->launches += launched;
       continue;
@@ -1119,6 +1119,26 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
       int launched = 0;
       cudaError_t e = kq::launch_qgemv_i4_xs(env, static_cast<int>(count), probe, reinterpret_cast<const void*>(x_dptr), x_dtype, m, swiglu, &launched);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_i4_xs launch");
+      ctx->launches += launched;
+      return KQ_OK;
+    }
+    // Many rows: the gate in the matmul's epilogue, which writes the output while x may still be read (and takes the
+    // norm into the launch that splits x).
+    const uint64_t x_end = x_dptr + static_cast<uint64_t>(m) * w0->k * dtype_bytes(x_dtype), out_end = out_dptr[0] + static_cast<uint64_t>(m) * w0->n * 4;
+    if (known && swiglu && (out_end <= x_dptr || x_end <= out_dptr[0]) && takes_exact_gemm(ctx, 2, probe, x_dtype, m) &&
+        kq::qgemm_exact_fuses_gate(env_of(ctx), w0->n, m)) {
+      for (uint32_t i = 0; i < 2; ++i) {
+        const int rc = check_linear_args(ctx, probe[i].w, x_dptr, x_dtype, bias_dptr[i], out_dptr[0]);
+        if (rc != KQ_OK) return rc;
+        probe[i].bias = reinterpret_cast<const float*>(bias_dptr[i]);
+        probe[i].out = reinterpret_cast<float*>(out_dptr[0]);
+      }
+      kq::LaunchEnv env = env_of(ctx);
+      env.norm_weight = reinterpret_cast<const float*>(norm_weight_dptr);
+      env.norm_eps = norm_eps;
+      int launched = 0;
+      cudaError_t e = kq::launch_qgemm_exact(env, 2, probe, reinterpret_cast<const void*>(x_dptr), x_dtype, m, true, &launched);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemm_exact launch");
       ctx->launches += launched;
       return KQ_OK;
     }

@@ -139,8 +139,10 @@ cudaError_t launch_qgemm_i4(const LaunchEnv& env, const LinearTarget& target, co
 // storage, weights as exact integers.  All targets of one call share storage, layout, k, group
 // size and scale type.  env.norm_weight (f32 activations) and env.residual (one target) are applied.
 bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, uint64_t workspace_bytes);
+// swiglu: two targets, gate and up, out[0] = silu(gate) * up; worth it where qgemm_exact_fuses_gate says so.
+bool qgemm_exact_fuses_gate(const LaunchEnv& env, uint32_t n, uint32_t m);
 cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,
-                               int* launches);
+                               bool swiglu, int* launches);
 // ... and the integer-dot form: int8 activations [m, k] with row scales xs (bit-exact contract).
 bool qgemm_exact_a8_supports(const Weight& w, const int8_t* xq, uint32_t m, uint64_t workspace_bytes);
 bool qgemm_exact_a8_preferred(const Weight& w, uint32_t m);  // ... faster here than on the kernels of kq_idot.cu

@@ -39,6 +39,9 @@
 //                fence, and with it the stage, for a trip to memory.
 //   warp 12      starts every copy: the activation tile (tensor map), the raw weights (bulk)
 //   warps 14-15  the group scales, a few chains ahead, as f32 into shared memory
+//
+// A gate and its up projection share a tile (64 channels of each per CTA), so that silu(gate) * up is the epilogue:
+// 333 rows of 1536 -> 2 x 8960 took 68 us and the gate's own kernel 11, now 69.
 //   warp 13      tensor memory; in the CTA of cluster rank 0 one thread issues the MMAs
 //                (cta_group::2: the pair shares the activation tile, half from each CTA)
 // Register split (setmaxnreg): 2 x 128 x 184 + 2 x 128 x 72 = 512 x 128.
@@ -78,8 +81,11 @@ constexpr uint32_t kMaxNT = 256;                // activation rows per tile
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kSmemLimit = 227 * 1024;
 constexpr uint32_t kScaleBatch = 8;             // accumulator chains per slot of the scale ring (two slots)
-constexpr uint32_t kTailRowScale = 320, kTailScales = kTailRowScale + kMaxNT * 4;
-constexpr uint32_t kSmemTail = kTailScales + 2 * kScaleBatch * kRows * 4;  // barriers, the tile's row scales, the scale ring
+constexpr uint32_t kOutCols = 8;                // columns a drain warp hands to its epilogue at a time
+constexpr uint32_t kTailScales = 320, kTailRows = kTailScales + 2 * kScaleBatch * kRows * 4;
+// barriers, the scale ring, each drain warp's row factors; where a pair takes several tiles, finished sums on their way out
+__host__ __device__ constexpr uint32_t tail_out(uint32_t nt) { return kTailRows + kDrainWarps * nt / 2 * 4; }
+__host__ __device__ constexpr uint32_t smem_tail(bool multi, uint32_t nt) { return tail_out(nt) + (multi ? kDrainWarps * kOutCols * 128 : 0); }
 constexpr uint32_t kMaxClusterSplits = 4;       // K slices that meet in a cluster: two or four (eight CTAs, the portable most)
 constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
 
@@ -96,6 +102,9 @@ struct ExTarget {
 struct ExParams {
   ExTarget t[kMaxMulti];
   uint32_t count;
+  uint32_t pairs, m_tiles; // column pairs of all weights, row tiles
+  uint32_t multi, resident; // more tiles than pairs the device holds: each of `resident` takes several
+  uint32_t swiglu;         // one output, silu(gate) * up: t[0] is the gate, t[1] up, and a CTA's 128 rows are 64 channels of each
   uint32_t m, k;
   uint32_t ksteps;         // k-steps of 128 bytes (64 binary16 or 128 int8 values)
   uint32_t nt;             // activation rows per tile, a multiple of 32
@@ -285,7 +294,7 @@ __device__ __forceinline__ uint32_t stage_warps(uint32_t stages) {
   return parts_of(kMath) == 3 && stages < kProdWarps ? kProdWarps : 1u;
 }
 
-template <int kW, int kMath>
+template <int kW, int kMath, bool kMulti>
 __global__ void __launch_bounds__(kExThreads, 1)
 qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map0,
                    const __grid_constant__ CUtensorMap w_map1, const __grid_constant__ CUtensorMap w_map2,
@@ -293,6 +302,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   constexpr bool kTiled = kW == kI4Tiled || kW == kI8Tiled;
   constexpr bool kGroupScales = kW == kI4Tiled || kW == kI4Rows;
   constexpr uint32_t kParts = parts_of(kMath);
+  const bool gated = p.swiglu != 0;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t raw_base = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
@@ -303,7 +313,6 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
                  dempty = dfull + 16, sfull = dempty + 16, sempty = sfull + 16;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(tail + 296);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 304);
-  float* row_scale_s = reinterpret_cast<float*>(tail + kTailRowScale);
   float* scale_ring = reinterpret_cast<float*>(tail + kTailScales);
   // a cluster is one pair, or the pairs of all K slices of a tile: ranks 2z and 2z + 1 are slice z
   const uint32_t cluster_rank = cluster_ctarank(), cta_rank = cluster_rank & 1u, pair_rank0 = cluster_rank & ~1u;
@@ -312,18 +321,32 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   // hand-over costs about 390 clocks whatever it hands over (24 x 4096 -> 9472: 33 us with one chain of 32 columns each).
   const uint32_t acc_cols = p.nt <= 32 ? 32u : p.nt <= 64 ? 64u : p.nt <= 128 ? 128u : 256u, per_set = 256u / acc_cols;
 
-  // which weight, which channels, which activation rows, which k-steps
-  const uint32_t pair = blockIdx.x >> 1;
-  uint32_t wi = 0;
+  // kMulti (int8 x int8): a cluster of one pair takes tiles (column pair, row tile, K slice) in turn, and while the drain warps store
+  // a tile's outputs, copies, producers and MMAs are at work on the next (4096 x 2048 -> 8192, 512 tiles on 74 pairs: 111 us
+  // with a cluster per tile, 76 so).  Elsewhere a cluster has one tile: with sums in the drain warps' registers there is
+  // nobody to drain the next one meanwhile (333 x 1536 -> 17920 f32 60 | 66, 1948 x 11264 -> 3088 binary16 group 16 475 | 553).
+  const uint32_t tiles_all = p.pairs * p.m_tiles, tile0 = blockIdx.x >> 1, tile_step = gridDim.x >> 1;  // (kMulti)
+  // (a weight's pointers are read from the parameters where they are used: kept in registers they would spill beside
+  // the drain warps' sums)
+  struct Tile { uint32_t wi, n0, m0, z, ks_begin, ks_count; };  // weight, this CTA's first output channel, first row, K slice and its k-steps
+  auto tile_at = [&](uint32_t t) {
+    Tile r;
+    const uint32_t mt = kMulti ? t / p.pairs : blockIdx.y, pair = kMulti ? t - mt * p.pairs : blockIdx.x >> 1;
+    r.z = kMulti ? 0u : blockIdx.z;
+    r.wi = 0;
+    if (gated) {
+      r.n0 = pair * kRows + cta_rank * (kRows / 2);
+    } else {
 #pragma unroll
-  for (int i = 1; i < kMaxMulti; ++i)
-    if (i < static_cast<int>(p.count) && pair >= p.t[i].pair0) wi = i;
-  // (the weight's pointers are read from the parameters where they are used: kept in registers from
-  // here on they would spill beside the drain warps' sums)
-  const uint32_t n0 = (pair - p.t[wi].pair0) * (2 * kRows) + cta_rank * kRows;  // this CTA's first output channel
-  const uint32_t m0 = blockIdx.y * p.nt;
-  const uint32_t ks_begin = blockIdx.z * p.ksteps_per_split;
-  const uint32_t ks_count = min(ks_begin + p.ksteps_per_split, p.ksteps) - ks_begin;
+      for (int i = 1; i < kMaxMulti; ++i)
+        if (i < static_cast<int>(p.count) && pair >= p.t[i].pair0) r.wi = i;
+      r.n0 = (pair - p.t[r.wi].pair0) * (2 * kRows) + cta_rank * kRows;
+    }
+    r.m0 = mt * p.nt;
+    r.ks_begin = r.z * p.ksteps_per_split;
+    r.ks_count = min(r.ks_begin + p.ksteps_per_split, p.ksteps) - r.ks_begin;
+    return r;
+  };
 
   if (warp == kMmaWarp) {
     if (lane == 0) {
@@ -346,8 +369,6 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   pdl_wait_prior_grid();  // the converted activations come from the launch before
-  for (uint32_t i = threadIdx.x; i < p.nt; i += kExThreads)
-    row_scale_s[i] = p.row_scale != nullptr && m0 + i < p.m ? p.row_scale[m0 + i] : 1.0f;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   cluster_sync_all();  // barriers of both CTAs are initialised
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -361,22 +382,168 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
     const uint32_t quarter = warp & 3u, half = warp >> 2;
     const uint32_t cols = p.nt / 2, col0 = half * cols;  // this warp's share of the tile's activation rows
-    const uint32_t row = n0 + quarter * 32u + lane;      // this lane's output channel
     const uint32_t taddr = tmem + ((quarter * 32u) << 16) + col0;
-    // The finished sums go through this thread's own words of shared memory (the stages are free
-    // then): the stores to `out` can be a short loop, where 128 unrolled copies of it are 24 KB of
-    // instructions that every CTA fetches cold (13 us instead of 3 for 256 x 18944 outputs).
+    // Finished sums leave through shared memory: the stores to `out` are then a short loop, where 128 unrolled copies
+    // of them are 24 KB of instructions that every CTA fetches cold (13 us instead of 3 for 256 x 18944 outputs).  A
+    // CTA's last tile parks them all in the stages, which are free then; before that, eight columns of a warp at a time.
+    const uint32_t out_at = bars + tail_out(p.nt) + warp * (kOutCols * 128u) + lane * 4u;
     const uint32_t park = tiles + warp * (cols * 128u) + lane * 4u;
-    if constexpr (kMath == kInt8) {
-      wait_bounded(dfull, 0, abort_flag, p.status, 23);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-      for (uint32_t b = 0; b * 16u < cols; ++b) {
-        uint32_t v[16];
-        tmem_ld16(taddr + b * 16u, v);
-#pragma unroll
-        for (uint32_t j = 0; j < 16; ++j) sts32(park + (b * 16u + j) * 128u, v[j]);
+    float* row_factor = reinterpret_cast<float*>(tail + kTailRows) + warp * cols;
+    if (p.row_scale == nullptr)
+      for (uint32_t c = lane; c < cols; c += 32u) row_factor[c] = 1.0f;
+    uint32_t set = 0, scale_batch = 0;  // accumulator sets and batches of scales so far, over all tiles
+    uint32_t tile = tile0;
+    do {
+    const Tile at_tile = tile_at(tile);
+    const uint32_t m0 = at_tile.m0, ks_count = at_tile.ks_count;
+    // ---- a tile's columns [8 h, 8 h + 8) of this warp, at `from` in shared memory, to where they go ----
+    // (what belongs to this thread's channel, or to its channel of the gate and of up, is read once a tile)
+    struct Channel { float bias, up_bias, ws, up_ws; };
+    auto channel = [&]() {
+      Channel c = {0.0f, 0.0f, 1.0f, 1.0f};
+      const ExTarget& tg = p.t[at_tile.wi];
+      const uint32_t row = at_tile.n0 + (gated ? quarter & 1u : quarter) * 32u + lane;
+      if (row < tg.n && p.splits == 1) {
+        c.bias = tg.bias[row];
+        if constexpr (!kGroupScales) c.ws = load_scale_dyn(tg.scale, row, p.scale_f16);
+        if (gated) {
+          c.up_bias = p.t[1].bias[row];
+          if constexpr (!kGroupScales) c.up_ws = load_scale_dyn(p.t[1].scale, row, p.scale_f16);
+        }
       }
+      return c;
+    };
+    auto finished = [](uint32_t v, float rs, float ws, float bias) {
+      if constexpr (kMath == kInt8) return fmaf(__int2float_rn(static_cast<int>(v)), __fmul_rn(rs, ws), bias);
+      else if constexpr (kGroupScales) return fmaf(__uint_as_float(v), rs, bias);
+      else return fmaf(__uint_as_float(v) * ws, rs, bias);
+    };
+    auto emit = [&](uint32_t h, const Channel& ch, uint32_t from, uint32_t warp_bytes) {
+      const uint32_t c0 = h * kOutCols, mm0 = m0 + col0 + c0;
+      const ExTarget& tg = p.t[at_tile.wi];
+      if (gated) {
+        // warps 0 and 1 of a column half hold gate rows, 2 and 3 the same rows of up: each takes half of the columns
+        if (kMulti || h == 0) asm volatile("bar.sync %0, 128;" ::"r"(1u + half) : "memory");
+        const uint32_t row = at_tile.n0 + (quarter & 1u) * 32u + lane, first = (quarter >> 1) * (kOutCols / 2);
+        const uint32_t gate_at = from - (quarter >> 1) * 2u * warp_bytes, up_at = gate_at + 2u * warp_bytes;
+        const bool live = row < p.t[0].n;
+        float* dst = p.t[0].out + static_cast<size_t>(mm0 + first) * p.t[0].n + row;
+        float gate[kOutCols / 2], up[kOutCols / 2];
+#pragma unroll
+        for (uint32_t i = 0; i < kOutCols / 2; ++i) {
+          gate[i] = __uint_as_float(lds32(gate_at + (first + i) * 128u));
+          up[i] = __uint_as_float(lds32(up_at + (first + i) * 128u));
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kOutCols / 2; ++i) {
+          const float rs = row_factor[c0 + first + i];
+          if constexpr (!kGroupScales) {
+            gate[i] *= ch.ws;
+            up[i] *= ch.up_ws;
+          }
+          gate[i] = silu_mul(fmaf(gate[i], rs, ch.bias), fmaf(up[i], rs, ch.up_bias));
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kOutCols / 2; ++i, dst += p.t[0].n)
+          if (live && mm0 + first + i < p.m) *dst = gate[i];
+        if (kMulti) asm volatile("bar.sync %0, 128;" ::"r"(1u + half) : "memory");
+        return;
+      }
+      const uint32_t row = at_tile.n0 + quarter * 32u + lane;  // this lane's output channel
+      const bool row_live = row < tg.n;
+      const size_t first = static_cast<size_t>(mm0) * tg.n + row;
+      // (the loads of all columns first: one column at a time is one trip to shared memory after the other)
+      uint32_t v[kOutCols];
+      float o[kOutCols], r[kOutCols];
+#pragma unroll
+      for (uint32_t j = 0; j < kOutCols; ++j) v[j] = lds32(from + j * 128u);
+      const bool add = tg.residual != nullptr;
+#pragma unroll
+      for (uint32_t j = 0; j < kOutCols; ++j)
+        r[j] = add && row_live && mm0 + j < p.m ? tg.residual[first + static_cast<size_t>(j) * tg.n] : 0.0f;
+#pragma unroll
+      for (uint32_t j = 0; j < kOutCols; ++j) {
+        o[j] = finished(v[j], row_factor[c0 + j], ch.ws, ch.bias);
+        if (add) o[j] = __fadd_rn(o[j], r[j]);
+      }
+      float* dst = tg.out + first;
+#pragma unroll
+      for (uint32_t j = 0; j < kOutCols; ++j, dst += tg.n)
+        if (row_live && mm0 + j < p.m) *dst = o[j];
+    };
+    // the factors of this warp's activation rows, into its own words: the warps of a column half may be in different tiles
+    if (p.row_scale != nullptr) {
+      for (uint32_t c = lane; c < cols; c += 32u) row_factor[c] = m0 + col0 + c < p.m ? p.row_scale[m0 + col0 + c] : 1.0f;
+      __syncwarp();
+    }
+    const bool last_tile = !kMulti || tile + tile_step >= tiles_all;
+    // parked sums: the same, all columns (without a gate column by column: 2 us less for 333 x 1536 -> 17920)
+    auto emit_parked = [&]() {
+      const Channel ch = channel();
+      if (kMulti || gated) {
+#pragma unroll 1
+        for (uint32_t h = 0; h * kOutCols < cols; ++h) emit(h, ch, park + h * (kOutCols * 128u), cols * 128u);
+        return;
+      }
+      const ExTarget& tg = p.t[at_tile.wi];
+      const uint32_t row = at_tile.n0 + quarter * 32u + lane, mm0 = m0 + col0;
+      const uint32_t live_cols = row < tg.n && mm0 < p.m ? min(cols, p.m - mm0) : 0u, n = tg.n;
+      if (p.splits == 1) {
+        float* dst = tg.out + static_cast<size_t>(mm0) * n + row;
+        const float* res = tg.residual != nullptr ? tg.residual + static_cast<size_t>(mm0) * n + row : nullptr;
+#pragma unroll 4
+        for (uint32_t c = 0; c < live_cols; ++c) {
+          float o = finished(lds32(park + c * 128u), row_factor[c], ch.ws, ch.bias);
+          if (res != nullptr) {
+            o = __fadd_rn(o, *res);
+            res += n;
+          }
+          *dst = o;
+          dst += n;
+        }
+      } else {
+        uint32_t before = 0;
+#pragma unroll
+        for (int i = 0; i < kMaxMulti; ++i)
+          if (static_cast<uint32_t>(i) < at_tile.wi) before += p.t[i].n;
+        uint32_t* dst = reinterpret_cast<uint32_t*>(p.partial) + (static_cast<size_t>(at_tile.z) * p.m + mm0) * p.n_total + before + row;
+#pragma unroll 4
+        for (uint32_t c = 0; c < live_cols; ++c) {
+          *dst = lds32(park + c * 128u);
+          dst += p.n_total;
+        }
+      }
+    };
+    if constexpr (kMath == kInt8) {
+      wait_bounded(dfull + (set & 1u) * 8, (set >> 1) & 1u, abort_flag, p.status, 23);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t at = taddr + (set & 1u) * kMaxNT;
+      if (kMulti && !last_tile) {
+        const Channel ch = channel();
+#pragma unroll 1
+        for (uint32_t b = 0; b * 16u < cols; ++b) {
+          uint32_t v[16];
+          tmem_ld16(at + b * 16u, v);
+#pragma unroll
+          for (uint32_t hh = 0; hh < 2; ++hh) {
+#pragma unroll
+            for (uint32_t j = 0; j < kOutCols; ++j) sts32(out_at + j * 128u, v[hh * kOutCols + j]);
+            emit(2 * b + hh, ch, out_at, kOutCols * 128u);
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (uint32_t b = 0; b * 16u < cols; ++b) {
+          uint32_t v[16];
+          tmem_ld16(at + b * 16u, v);
+#pragma unroll
+          for (uint32_t j = 0; j < 16; ++j) sts32(park + (b * 16u + j) * 128u, v[j]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      arrive_if(leader, map_to_cta(dempty, pair_rank0) + (set & 1u) * 8);
+      ++set;
     } else {
       const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16;
       const uint32_t dempty_0 = map_to_cta(dempty, pair_rank0);
@@ -392,8 +559,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
 #pragma unroll
           for (int j = 0; j < 16; ++j) acc[b][j] = 0.0f;
 #pragma unroll 1
-        for (uint32_t d0 = 0, set = 0; d0 < drains; d0 += per_set, ++set) {
-          const uint32_t batch = d0 / kScaleBatch, d_end = min(d0 + per_set, drains);  // a set lies inside a batch of scales
+        for (uint32_t d0 = 0; d0 < drains; d0 += per_set, ++set) {
+          const uint32_t batch = scale_batch + d0 / kScaleBatch, d_end = min(d0 + per_set, drains);  // a set lies inside a batch of scales
           if constexpr (kGroupScales) {
             if (d0 % kScaleBatch == 0) wait_bounded(sfull + (batch & 1u) * 8, (batch >> 1) & 1u, abort_flag, p.status, 25);
           }
@@ -436,8 +603,9 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           arrive_if(leader, dempty_0 + (set & 1u) * 8);
-          if (kGroupScales) arrive_if(d_end % kScaleBatch == 0 ? leader : 0u, sempty + (batch & 1u) * 8);
+          if (kGroupScales) arrive_if(d_end % kScaleBatch == 0 || d_end == drains ? leader : 0u, sempty + (batch & 1u) * 8);
         }
+        scale_batch += (drains + kScaleBatch - 1) / kScaleBatch;
 #pragma unroll
         for (int b = 0; b < kBatches; ++b)
 #pragma unroll
@@ -454,27 +622,32 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         default: drain_all(std::integral_constant<int, 8>{}); break;
       }
     }
-    // ---------------- epilogue ----------------
-    const ExTarget tg = p.t[wi];
-    const bool row_live = row < tg.n;
-    // the K slices of a cluster meet in slice order, each finishing its share of the columns
-    const uint32_t slices = p.cluster_splits, share0 = slices > 1 ? cols * blockIdx.z / slices : 0u;
-    const uint32_t share1 = slices > 1 ? cols * (blockIdx.z + 1) / slices : cols;
-    if (slices > 1) cluster_sync_all();  // everybody has parked
-    const uint32_t mm0 = m0 + col0;
-    const uint32_t live_cols = row_live && mm0 < p.m ? min(cols, p.m - mm0) : 0u;
-    if (p.splits == 1 || slices > 1) {
+    if (last_tile && p.cluster_splits == 1) emit_parked();
+    if (!kMulti && p.cluster_splits > 1) {
+      // ---------------- K slices of a cluster: they meet in slice order, each finishing its share of the columns ----------------
+      const ExTarget tg = p.t[at_tile.wi];
+      const uint32_t slices = p.cluster_splits, share0 = cols * at_tile.z / slices, share1 = cols * (at_tile.z + 1) / slices;
+      const uint32_t row = at_tile.n0 + quarter * 32u + lane, mm0 = m0 + col0;
+      const bool row_live = row < tg.n;
+      const uint32_t live_cols = row_live && mm0 < p.m ? min(cols, p.m - mm0) : 0u, last = min(share1, live_cols);
+      cluster_sync_all();  // everybody has parked
       const float bias = row_live ? tg.bias[row] : 0.0f;
-      float ws = 1.0f;
+      [[maybe_unused]] float ws = 1.0f;
       if constexpr (!kGroupScales) ws = row_live ? load_scale_dyn(tg.scale, row, p.scale_f16) : 0.0f;
       float* dst = tg.out + static_cast<size_t>(mm0 + share0) * tg.n + row;
       const float* res = tg.residual != nullptr ? tg.residual + static_cast<size_t>(mm0 + share0) * tg.n + row : nullptr;
-      auto finish = [&](uint32_t c, uint32_t v) {
-        const float rs = row_scale_s[col0 + c];
-        float o;
-        if constexpr (kMath == kInt8) o = fmaf(__int2float_rn(static_cast<int>(v)), __fmul_rn(rs, ws), bias);
-        else if constexpr (kGroupScales) o = fmaf(__uint_as_float(v), rs, bias);
-        else o = fmaf(__uint_as_float(v) * ws, rs, bias);
+      uint32_t from[kMaxClusterSplits];
+#pragma unroll
+      for (uint32_t z = 0; z < kMaxClusterSplits; ++z) from[z] = map_to_cta(park, 2u * min(z, slices - 1u) + cta_rank);
+      auto finish = [&](auto count, uint32_t c) {
+        uint32_t sum = 0, v[decltype(count)::value];
+#pragma unroll
+        for (uint32_t z = 0; z < decltype(count)::value; ++z) v[z] = lds32_cluster(from[z] + c * 128u);
+        const float rs = row_factor[c];
+#pragma unroll
+        for (uint32_t z = 0; z < decltype(count)::value; ++z)
+          sum = z == 0 ? v[0] : kMath == kInt8 ? sum + v[z] : __float_as_uint(__uint_as_float(sum) + __uint_as_float(v[z]));
+        float o = finished(sum, rs, ws, bias);
         if (res != nullptr) {
           o = __fadd_rn(o, *res);
           res += tg.n;
@@ -482,43 +655,15 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         *dst = o;
         dst += tg.n;
       };
-      if (slices == 1) {
-#pragma unroll 4
-        for (uint32_t c = 0; c < live_cols; ++c) finish(c, lds32(park + c * 128u));
-      } else {
-        const uint32_t last = min(share1, live_cols);
-        uint32_t from[kMaxClusterSplits];
-#pragma unroll
-        for (uint32_t z = 0; z < kMaxClusterSplits; ++z) from[z] = map_to_cta(park, 2u * min(z, slices - 1u) + cta_rank);
-        auto total = [&](auto count, uint32_t c) {
-          uint32_t sum = 0, v[decltype(count)::value];
-#pragma unroll
-          for (uint32_t z = 0; z < decltype(count)::value; ++z) v[z] = lds32_cluster(from[z] + c * 128u);
-#pragma unroll
-          for (uint32_t z = 0; z < decltype(count)::value; ++z)
-            sum = z == 0 ? v[0] : kMath == kInt8 ? sum + v[z] : __float_as_uint(__uint_as_float(sum) + __uint_as_float(v[z]));
-          return sum;
-        };
-        if (slices == 2) {
+      if (slices == 2) {
 #pragma unroll 8
-          for (uint32_t c = share0; c < last; ++c) finish(c, total(std::integral_constant<uint32_t, 2>{}, c));
-        } else {
+        for (uint32_t c = share0; c < last; ++c) finish(std::integral_constant<uint32_t, 2>{}, c);
+      } else {
 #pragma unroll 4
-          for (uint32_t c = share0; c < last; ++c) finish(c, total(std::integral_constant<uint32_t, kMaxClusterSplits>{}, c));
-        }
-      }
-    } else {
-      uint32_t before = 0;
-#pragma unroll
-      for (int i = 0; i < kMaxMulti; ++i)
-        if (static_cast<uint32_t>(i) < wi) before += p.t[i].n;
-      uint32_t* dst = reinterpret_cast<uint32_t*>(p.partial) + (static_cast<size_t>(blockIdx.z) * p.m + mm0) * p.n_total + before + row;
-#pragma unroll 4
-      for (uint32_t c = 0; c < live_cols; ++c) {
-        *dst = lds32(park + c * 128u);
-        dst += p.n_total;
+        for (uint32_t c = share0; c < last; ++c) finish(std::integral_constant<uint32_t, kMaxClusterSplits>{}, c);
       }
     }
+    } while (kMulti && (tile += tile_step) < tiles_all);
   } else if (warp < kDrainWarps + kProdWarps) {
     // ---------------- producers ----------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -534,6 +679,10 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     const bool shared_stage = stage_warps<kMath>(p.stages) != 1;
     const uint32_t rb0 = shared_stage ? 2u * (warp - kDrainWarps) : 0u, rb1 = shared_stage ? rb0 + 2u : 8u;  // this warp's 16-row blocks
     uint32_t s = 0, phase = 0;
+    uint32_t tile = tile0;
+    do {
+    const uint32_t ks_count = tile_at(tile).ks_count;
+#pragma unroll 1
     for (uint32_t ks = 0; ks < ks_count; ++ks, s = s + 1 == p.stages ? 0u : s + 1u, phase ^= s == 0 ? 1u : 0u) {
       if (!shared_stage && (s & (kProdWarps - 1u)) != warp - kDrainWarps) continue;
       const uint32_t ready = wait_bounded(rawfull + s * 8, phase, abort_flag, p.status, 21) ? leader : 0u;
@@ -621,6 +770,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       __syncwarp();
       arrive_if(ready, full_0 + s * 8);  // the issuing CTA's barrier
     }
+    } while (kMulti && (tile += tile_step) < tiles_all);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == kCopyWarp) {
@@ -629,19 +779,25 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       // 100 clocks, and a bulk copy per 16-row block, eight of them, 700 - 1000: more than the k-step's MMAs.
       {
         const uint32_t half_rows = p.nt / 2, b_bytes = half_rows * 128u, raw_bytes = p.raw_bytes;
-        const CUtensorMap* w_map = wi == 0 ? &w_map0 : wi == 1 ? &w_map1 : wi == 2 ? &w_map2 : &w_map3;
         const uint32_t full_0 = map_to_cta(full, pair_rank0), raw_off = kW == kI8Rows && kMath == kInt8 ? 0u : p.raw_off;
-        const uint32_t w_row = kTiled ? n0 / 16u : n0, w_step = p.raw_box;  // tensor-map rows and columns of the raw weights
         uint32_t s = 0, phase = 0;
-        for (uint32_t ks = 0; ks < ks_count; ++ks) {
+        uint32_t tile = tile0;
+        do {
+        const Tile at = tile_at(tile);
+        const CUtensorMap* w_map = at.wi == 0 ? &w_map0 : at.wi == 1 ? &w_map1 : at.wi == 2 ? &w_map2 : &w_map3;
+        const uint32_t w_row = kTiled ? at.n0 / 16u : at.n0, w_step = p.raw_box;  // tensor-map rows and columns of the raw weights
+#pragma unroll 1
+        for (uint32_t ks = 0; ks < at.ks_count; ++ks) {
           const uint32_t free = wait_bounded(empty + s * 8, phase ^ 1u, abort_flag, p.status, 20) ? leader : 0u;
-          const uint32_t a_tile = tiles + s * p.stage_bytes, kstep = ks_begin + ks;
+          const uint32_t a_tile = tiles + s * p.stage_bytes, kstep = at.ks_begin + ks;
           expect_tx(cta_rank == 0 ? free : 0u, full + s * 8, kParts * 2u * b_bytes);
           expect_tx(free, rawfull + s * 8, raw_bytes);
           copy_tile_2d(free, a_tile + raw_off, w_map, kstep * w_step, w_row, rawfull + s * 8);
-          copy_tile_3d(free, a_tile + kATile, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), m0 + cta_rank * half_rows, 0, full_0 + s * 8);
+          if (gated) copy_tile_2d(free, a_tile + raw_off + raw_bytes / 2, &w_map1, kstep * w_step, w_row, rawfull + s * 8);
+          copy_tile_3d(free, a_tile + kATile, &x_map, kstep * (kMath == kInt8 ? 128u : 64u), at.m0 + cta_rank * half_rows, 0, full_0 + s * 8);
           if (++s == p.stages) { s = 0; phase ^= 1u; }
         }
+        } while (kMulti && (tile += tile_step) < tiles_all);
       }
       __syncwarp();
     } else if (warp == kMmaWarp && cta_rank == 0) {
@@ -669,6 +825,10 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
               in_set = 0;
             }
           };
+          uint32_t tile = tile0;
+          do {
+          const uint32_t ks_count = tile_at(tile).ks_count;
+#pragma unroll 1
           for (uint32_t ks = 0; ks < ks_count; ++ks) {
             wait_bounded(full + s * 8, phase, abort_flag, p.status, 22);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -681,7 +841,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
 #pragma unroll
             for (uint32_t run = 0; run < 4; run += kRun) {
               const bool starts = kSlices != 0 || in_chain == 0;
-              if (kMath != kInt8 && starts) chain_begins();
+              if (starts) chain_begins();
               const uint32_t dst = tmem + (set & 1u) * kMaxNT + in_set * acc_cols;
 #pragma unroll
               for (uint32_t back = 1; back <= kParts; ++back) {
@@ -704,6 +864,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
             }
             commit_both(leader, this_empty, pair_mask);  // the stage is free, in both CTAs, once these MMAs have read it
           }
+          } while (kMulti && (tile += tile_step) < tiles_all);
         };
         if (kGroupScales && p.drain16 == 1) issue(std::integral_constant<uint32_t, 1>{});
         else if (kGroupScales && p.drain16 == 2) issue(std::integral_constant<uint32_t, 2>{});
@@ -716,12 +877,17 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       // Each of the 64 lanes serves two rows.  A batch is fetched into registers as soon as the one before it has
       // been stored: fetched only once its slot was free, a batch cost two trips to memory and the drain waited
       // for it (4,600 clocks per eight chains; 24 x 4096 -> 9472: 30 us).
-      const uint32_t drains = (ks_count * 4 + p.drain16 - 1) / p.drain16, drain0 = ks_begin * 4 / p.drain16;
-      const ExTarget tg = p.t[wi];
       const uint32_t wl = (warp - kScaleWarp) * 32u + lane;
+      uint32_t batch = 0;
+      uint32_t tile = tile0;
+      do {
+      const Tile at_tile = tile_at(tile);
+      const uint32_t drains = (at_tile.ks_count * 4 + p.drain16 - 1) / p.drain16, drain0 = at_tile.ks_begin * 4 / p.drain16;
       if constexpr (kW == kI4Tiled) {
         // rows 16 (wl / 8) + wl % 8 and + 8: a chunk holds their scales of two groups side by side
-        const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), r = (wl >> 3) * 16u + (wl & 7u), row = n0 + r;
+        const uint32_t unit = raw_unit_bytes<kW, kMath>(p.scale_f16), r = (wl >> 3) * 16u + (wl & 7u);
+        const ExTarget& tg = p.t[gated ? r / (kRows / 2) : at_tile.wi];
+        const uint32_t row = at_tile.n0 + (gated ? r % (kRows / 2) : r);
         const uint8_t* base = tg.w + static_cast<size_t>(row >> 4) * (p.k / kChunkK) * unit + kChunkWeightBytes + (wl & 7u) * (p.scale_f16 ? 8u : 16u);
         float4 v[kScaleBatch / 2];  // {row, group 0 | row + 8, group 0 | row, group 1 | row + 8, group 1}
         auto load = [&](uint32_t d0) {
@@ -742,7 +908,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           }
         };
         load(0);
-        for (uint32_t d0 = 0, batch = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
+        for (uint32_t d0 = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
           if (batch >= 2) wait_bounded(sempty + (batch & 1u) * 8, ((batch >> 1) - 1u) & 1u, abort_flag, p.status, 26);
           float* ring = scale_ring + (batch & 1u) * (kScaleBatch * kRows) + r;
 #pragma unroll
@@ -762,7 +928,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         auto load = [&](uint32_t d0) {
 #pragma unroll
           for (uint32_t rr = 0; rr < 2; ++rr) {
-            const uint32_t row = n0 + wl + rr * 64u;
+            const ExTarget& tg = p.t[gated ? rr : at_tile.wi];
+            const uint32_t row = at_tile.n0 + wl + (gated ? 0u : rr * 64u);
             const uint8_t* base = static_cast<const uint8_t*>(tg.scale) + static_cast<size_t>(row) * p.groups * each;
 #pragma unroll
             for (uint32_t i = 0; i < kScaleBatch; ++i) {
@@ -776,7 +943,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           }
         };
         load(0);
-        for (uint32_t d0 = 0, batch = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
+        for (uint32_t d0 = 0; d0 < drains; d0 += kScaleBatch, ++batch) {
           if (batch >= 2) wait_bounded(sempty + (batch & 1u) * 8, ((batch >> 1) - 1u) & 1u, abort_flag, p.status, 26);
 #pragma unroll
           for (uint32_t rr = 0; rr < 2; ++rr)
@@ -787,6 +954,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           load(d0 + kScaleBatch);
         }
       }
+      } while (kMulti && (tile += tile_step) < tiles_all);
     }
   }
 
@@ -1041,10 +1209,9 @@ bool kind_ok(const Weight& w) {
   }
 }
 
-template <int kW, int kMath>
-cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, uint32_t pairs, uint32_t m_tiles, const CUtensorMap& xm,
-                        const CUtensorMap (&wm)[kMaxMulti]) {
-  auto kernel = qgemm_exact_kernel<kW, kMath>;
+template <int kW, int kMath, bool kMulti>
+cudaError_t launch_form(const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
+  auto kernel = qgemm_exact_kernel<kW, kMath, kMulti>;
   static PerDevice<bool> configured_on;
   bool* configured = configured_on.slot();
   if (configured == nullptr) return cudaErrorInvalidDevice;
@@ -1058,8 +1225,15 @@ cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, uint32_t pairs,
     if (e != cudaSuccess) return e;
     *configured = true;
   }
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + kSmemTail;
-  return launch_dependent(kernel, dim3(pairs * 2, m_tiles, p.splits), kExThreads, smem, dim3(2, 1, p.cluster_splits), env, p, xm, wm[0], wm[1], wm[2], wm[3]);
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + smem_tail(kMulti, p.nt);
+  const dim3 grid = kMulti ? dim3(p.resident * 2) : dim3(p.pairs * 2, p.m_tiles, p.splits);
+  return launch_dependent(kernel, grid, kExThreads, smem, dim3(2, 1, p.cluster_splits), env, p, xm, wm[0], wm[1], wm[2], wm[3]);
+}
+template <int kW, int kMath>
+cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
+  if constexpr (kMath == kInt8)
+    if (p.multi) return launch_form<kW, kMath, true>(env, p, xm, wm);
+  return launch_form<kW, kMath, false>(env, p, xm, wm);
 }
 
 // Pairs (slots[1]) and clusters of two or four pairs that the device holds at once; 0 where it cannot say.  Every form of
@@ -1070,7 +1244,7 @@ cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSp
   Held* held = held_on.slot();
   if (held == nullptr) return cudaErrorInvalidDevice;
   if (!held->done) {
-    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1>;
+    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
     if (e != cudaSuccess) return e;
     for (uint32_t z = 2; z <= kMaxClusterSplits; z *= 2) {
@@ -1100,13 +1274,12 @@ cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSp
 }
 
 template <int kW>
-cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, uint32_t pairs, uint32_t m_tiles, const CUtensorMap& xm,
-                        const CUtensorMap (&wm)[kMaxMulti]) {
-  if (math == kHalf1) return launch_main<kW, kHalf1>(env, p, pairs, m_tiles, xm, wm);
-  if (math == kBf1) return launch_main<kW, kBf1>(env, p, pairs, m_tiles, xm, wm);
+cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
+  if (math == kHalf1) return launch_main<kW, kHalf1>(env, p, xm, wm);
+  if (math == kBf1) return launch_main<kW, kBf1>(env, p, xm, wm);
   constexpr int kF32 = kW == kI8Tiled ? kHalf2 : kBf3;
-  if (math == kF32) return launch_main<kW, kF32>(env, p, pairs, m_tiles, xm, wm);
-  if constexpr (kW == kI8Tiled || kW == kI8Rows) return launch_main<kW, kInt8>(env, p, pairs, m_tiles, xm, wm);
+  if (math == kF32) return launch_main<kW, kF32>(env, p, xm, wm);
+  if constexpr (kW == kI8Tiled || kW == kI8Rows) return launch_main<kW, kInt8>(env, p, xm, wm);
   return cudaErrorInvalidValue;
 }
 
@@ -1190,7 +1363,7 @@ uint32_t chain_of(int math, const Weight& w) {
 
 // x: binary16 (kHalf1), parts already split (kHalf2 / kBf1 / kBf3) or int8 (kInt8).
 cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const float* residual, const void* x, int math,
-                      uint32_t m, uint32_t max_chain, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, int* launches) {
+                      uint32_t m, uint32_t max_chain, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, bool swiglu, int* launches) {
   const Weight& w0 = *targets[0].w;
   const WeightKind kind = kind_of(w0);
   ExParams p = {};
@@ -1210,15 +1383,19 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
     p.t[used] = ExTarget{static_cast<const uint8_t*>(w.data), w.scale, targets[i].bias, targets[i].out, residual, w.n, pairs};
     const uint64_t row_bytes = kind == kI4Tiled ? static_cast<uint64_t>(w.k / kChunkK) * unit
                                : kind == kI8Tiled ? static_cast<uint64_t>(w.k) * 16 : kind == kI4Rows ? w.k / 2 : w.k;
-    cudaError_t e = tiled ? encode_w_map(w.data, w.n / 16, row_bytes, unit, elem, 8, false, &wm[used])
-                          : encode_w_map(w.data, w.n, row_bytes, unit, elem, kRows, kind == kI8Rows && int8, &wm[used]);
+    cudaError_t e = tiled ? encode_w_map(w.data, w.n / 16, row_bytes, unit, elem, swiglu ? 4 : 8, false, &wm[used])
+                          : encode_w_map(w.data, w.n, row_bytes, unit, elem, swiglu ? kRows / 2 : kRows, kind == kI8Rows && int8, &wm[used]);
     if (e != cudaSuccess) return e;
-    pairs += (w.n + 2 * kRows - 1) / (2 * kRows);
-    n_total += w.n;
+    if (!swiglu || used == 0) {
+      const uint32_t wide = swiglu ? kRows : 2 * kRows;  // channels of a pair
+      pairs += (w.n + wide - 1) / wide;
+      n_total += w.n;
+    }
     ++used;
   }
   if (used == 0) return cudaSuccess;
   p.count = used;
+  p.swiglu = swiglu ? 1 : 0;
   p.m = m;
   p.k = w0.k;
   const uint32_t step_k = int8 ? 128 : 64;
@@ -1241,26 +1418,30 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   uint32_t slots[kMaxClusterSplits + 1];
   cudaError_t ce = resident_pairs(env, slots);
   if (ce != cudaSuccess) return ce;
-  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, math, !i4, p.drain16, align, may_split, slots,
+  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, math, !i4, p.drain16, align, may_split && !swiglu, slots,
                                        scratch != nullptr ? scratch_bytes : 0);
   p.nt = geo.nt;
+  p.pairs = pairs;
+  p.m_tiles = geo.m_tiles;
   p.ksteps_per_split = ((p.ksteps + geo.splits - 1) / geo.splits + align - 1) / align * align;
   p.splits = (p.ksteps + p.ksteps_per_split - 1) / p.ksteps_per_split;
   p.cluster_splits = geo.cluster_splits;
+  p.multi = int8 && p.splits == 1 && static_cast<uint64_t>(pairs) * geo.m_tiles > slots[1];
+  p.resident = slots[1];
   // stage: weight tile, activation parts, raw weights
   p.raw_bytes = (tiled ? 8 : kRows) * unit;
   p.raw_box = unit / elem;
   const uint32_t raw_bytes = kind == kI8Rows && int8 ? 0 : p.raw_bytes;  // straight into the weight tile
   p.raw_off = kATile + parts * p.nt / 2 * 128;
   p.stage_bytes = (p.raw_off + raw_bytes + 1023) / 1024 * 1024;
-  p.stages = std::min<uint32_t>(kMaxStages, (kSmemLimit - 1024 - kSmemTail) / p.stage_bytes);
+  p.stages = std::min<uint32_t>(kMaxStages, (kSmemLimit - 1024 - smem_tail(p.multi != 0, p.nt)) / p.stage_bytes);
   cudaError_t e = encode_x_map(x, int8, m, w0.k, parts, p.nt / 2, &xm);
   if (e != cudaSuccess) return e;
   switch (kind) {
-    case kI4Tiled: e = launch_math<kI4Tiled>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
-    case kI4Rows: e = launch_math<kI4Rows>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
-    case kI8Tiled: e = launch_math<kI8Tiled>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
-    default: e = launch_math<kI8Rows>(math, env, p, pairs, geo.m_tiles, xm, wm); break;
+    case kI4Tiled: e = launch_math<kI4Tiled>(math, env, p, xm, wm); break;
+    case kI4Rows: e = launch_math<kI4Rows>(math, env, p, xm, wm); break;
+    case kI8Tiled: e = launch_math<kI8Tiled>(math, env, p, xm, wm); break;
+    default: e = launch_math<kI8Rows>(math, env, p, xm, wm); break;
   }
   if (e != cudaSuccess) return e;
   if (launches) *launches += 1;
@@ -1307,12 +1488,19 @@ bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, ui
   return align256(static_cast<uint64_t>(w0.k) * 2 * parts_of(kBf3) * 16) + 256 <= workspace_bytes;
 }
 
+// A gate and its up projection in one launch, silu(gate) * up written by the epilogue, where the tiles fill half of the
+// device; below that the two are worth cutting along K (the gate's own kernel then follows the matmul).
+bool qgemm_exact_fuses_gate(const LaunchEnv& env, uint32_t n, uint32_t m) {
+  return static_cast<uint64_t>((n + kRows - 1) / kRows) * ((m + kMaxNT - 1) / kMaxNT) * 4 >= static_cast<uint64_t>(env.sm_count);
+}
+
 cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,
-                               int* launches) {
+                               bool swiglu, int* launches) {
   const Weight& w0 = *targets[0].w;
   const uint32_t k = w0.k;
   const bool direct = x_dtype == KQ_F16;  // binary16 rows are the operand
-  if (direct && env.norm_weight != nullptr) return cudaErrorInvalidValue;
+  if ((direct && env.norm_weight != nullptr) || (swiglu && (count != 2 || targets[0].w->n != targets[1].w->n || env.residual != nullptr)))
+    return cudaErrorInvalidValue;
   const int math = direct ? kHalf1 : x_dtype == KQ_BF16 ? kBf1 : kind_of(w0) == kI8Tiled ? kHalf2 : kBf3;
   uint8_t* ws = static_cast<uint8_t*>(env.workspace);
   const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
@@ -1334,7 +1522,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
     const uint8_t* xp = static_cast<const uint8_t*>(x) + static_cast<size_t>(r0) * k * xb;
     cudaError_t e;
     if (direct) {
-      e = run_exact(env, count, t, residual, xp, math, pm, chain_of(math, w0), nullptr, ws, room, true, launches);
+      e = run_exact(env, count, t, residual, xp, math, pm, chain_of(math, w0), nullptr, ws, room, true, swiglu, launches);
     } else {
       float* inv = reinterpret_cast<float*>(ws);
       uint16_t* parts = reinterpret_cast<uint16_t*>(ws + align256(static_cast<uint64_t>(pm) * 4));
@@ -1348,7 +1536,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
       else e = split(split_kernel<float, kHalf2>, reinterpret_cast<const float*>(xp));
       if (e != cudaSuccess) return e;
       if (launches) *launches += 1;
-      e = run_exact(env, count, t, residual, parts, math, pm, chain_of(math, w0), inv, ws + taken, room - taken, true, launches);
+      e = run_exact(env, count, t, residual, parts, math, pm, chain_of(math, w0), inv, ws + taken, room - taken, true, swiglu, launches);
     }
     if (e != cudaSuccess) return e;
   }
@@ -1383,7 +1571,7 @@ cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& targ
   const Weight& w = *target.w;
   uint8_t* ws = static_cast<uint8_t*>(env.workspace);
   const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
-  if (w.storage == KQ_STORAGE_I8) return run_exact(env, 1, &target, nullptr, xq, kInt8, m, kMaxChain, xs, ws, room, true, launches);
+  if (w.storage == KQ_STORAGE_I8) return run_exact(env, 1, &target, nullptr, xq, kInt8, m, kMaxChain, xs, ws, room, true, false, launches);
   // int4: per-group sums as binary16 products (exact), flushed in ascending order: no K slices
   const uint64_t per_row = static_cast<uint64_t>(w.k) * 2;
   uint32_t panel = static_cast<uint32_t>(std::min<uint64_t>(m, room / per_row));
@@ -1398,7 +1586,7 @@ cudaError_t launch_qgemm_exact_a8(const LaunchEnv& env, const LinearTarget& targ
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
     const LinearTarget t{target.w, target.bias, target.out + static_cast<size_t>(r0) * w.n};
-    e = run_exact(env, 1, &t, nullptr, ws, kHalf1, pm, kMaxChain, xs + r0, nullptr, 0, false, launches);
+    e = run_exact(env, 1, &t, nullptr, ws, kHalf1, pm, kMaxChain, xs + r0, nullptr, 0, false, false, launches);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

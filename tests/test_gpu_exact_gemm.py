@@ -110,6 +110,46 @@ def test_integer_sums_that_meet_in_a_cluster(gpu, m, n, k):
     test_integer_dot_is_bit_exact(gpu, "i8", 0, m, n, k)
 
 
+# The gate in the matmul's epilogue (its tiles fill half of the device) and several tiles to a CTA pair: ragged rows and
+# channels, every storage; out on top of x takes the separate kernels
+@pytest.mark.parametrize("storage,group,xdt,m,n,k", [("i4", 32, "f32", 513, 2416, 128), ("i4", 32, "f16", 300, 4752, 64), ("i4", 16, "f32", 270, 2401, 96),
+                                                     ("i8", 0, "f32", 257, 4736, 96), ("i8", 0, "f16", 800, 2440, 80), ("i4", 64, "bf16", 1030, 3333, 192)])
+def test_gate_in_the_epilogue(gpu, storage, group, xdt, m, n, k):
+    import torch
+    rng = np.random.default_rng(m)
+    x = {"f32": lambda v: v, "f16": oracle.round_to_f16, "bf16": oracle.round_to_bf16}[xdt](rng.standard_normal((m, k)).astype(np.float32))
+    norm = (1 + 0.1 * rng.standard_normal(k)).astype(np.float32) if xdt == "f32" else None
+    xn = oracle.rms_norm(x, norm, 1e-5) if xdt == "f32" else x
+    ws, biases, refs = [], [], []
+    for seed in (1, 2):
+        data, scale = cases.synth_i4(n, k, seed=seed, group_size=group) if storage == "i4" else cases.synth_i8(n, k, seed=seed)
+        ws.append(gpu.upload_weight(storage, data, scale, (n, k), group))
+        biases.append(rng.standard_normal(n).astype(np.float32))
+        args = (xn, data, scale.astype(np.float32), biases[-1], n, k)
+        refs.append(oracle.linear_i4(*args, group) if storage == "i4" else oracle.linear_i8(*args))
+    want = (refs[0] / (1 + np.exp(-refs[0].astype(np.float64))) * refs[1]).astype(np.float32)
+    xd = dev(x).to({"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[xdt])
+    out = torch.full((m, n), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    before = gpu.launch_count
+    gpu.linear_fused(xd, ws, [dev(b) for b in biases], [out], norm_weight=dev(norm) if norm is not None else None, eps=1e-5, swiglu=True)
+    gpu.sync()
+    assert gpu.launch_count - before == (1 if xdt == "f16" else 2)
+    rms = float(np.sqrt(np.mean(want.astype(np.float64) ** 2)))
+    rep = oracle.allclose(out.cpu().numpy(), want, atol=1e-5 * max(1.0, rms), rtol=1e-4)
+    assert rep["pass"], rep
+    over = torch.zeros(m * max(n, k), device="cuda")  # x and out share their first bytes
+    xo = over.view(xd.dtype)[: m * k].view(m, k)
+    xo.copy_(xd)
+    torch.cuda.synchronize()
+    gpu.linear_fused(xo, ws, [dev(b) for b in biases], [over[: m * n].view(m, n)], norm_weight=dev(norm) if norm is not None else None, eps=1e-5, swiglu=True)
+    gpu.sync()
+    rep = oracle.allclose(over[: m * n].view(m, n).cpu().numpy(), want, atol=1e-5 * max(1.0, rms), rtol=1e-4)
+    assert rep["pass"], rep
+    for w in ws:
+        w.free()
+
+
 @pytest.mark.parametrize("m,n,k", [(17, 64, 128), (130, 544, 1536)])
 def test_norm_gate_and_residual_around_it(gpu, m, n, k):
     import torch
