@@ -279,6 +279,7 @@ int check_linear_args(kq_ctx* ctx, const Weight* w, uint64_t x, int x_dtype, uin
 // The many-row kernel of kq_qgemm_exact.cu runs this call: more than 16 rows, weights of one kind,
 // and not a case of the bf16 GEMM (bf16 activations on a tiled weight, whose operands are rounded).
 bool takes_exact_gemm(const kq_ctx* ctx, int count, const kq::LinearTarget* targets, int x_dtype, uint32_t m) {
+  if (count == 1 && kq::qgemv_rows_supports(*targets[0].w, m) && kq::qgemv_rows_preferred(*targets[0].w, m)) return false;
   for (int i = 0; i < count; ++i)
     if (kq::qgemm_i4_supports(*targets[i].w, x_dtype, m) || kq::qgemm_i8_supports(*targets[i].w, x_dtype, m)) return false;
   return kq::qgemm_exact_supports(count, targets, m, ctx->workspace ? ctx->workspace_bytes : 0);
@@ -355,6 +356,12 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
   // Everything else: one generic launch per weight.
   for (uint32_t i = 0; i < count; ++i) {
     const Weight& w = *targets[i].w;
+    if (kq::qgemv_rows_supports(w, m) && kq::qgemv_rows_preferred(w, m)) {
+      cudaError_t e = kq::launch_qgemv_rows(env, targets[i], reinterpret_cast<const void*>(x), x_dtype, m);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_rows launch");
+      ctx->launches += 1;
+      continue;
+    }
     if (w.n != 0 && takes_exact_gemm(ctx, 1, &targets[i], x_dtype, m)) {
       int launched = 0;
       cudaError_t e = kq::launch_qgemm_exact(env, 1, &targets[i], reinterpret_cast<const void*>(x), x_dtype, m, false, &launched);

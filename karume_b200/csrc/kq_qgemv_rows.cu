@@ -1,0 +1,323 @@
+// qgemv_rows — the linear for up to sixteen activation rows over weights that keep their row-major packing:
+// int4 of any group size or ragged channel count, int8 with ragged channels (the tiled layouts take groups of 32
+// and whole blocks of sixteen channels; kq_qgemv_i4*.cu, kq_qgemv_i8.cu).
+//
+// Replaces the reference's scalar and small-tile variants for those weights
+// (packages/runtime/src/kernels/gemm-geometry.ts:243-267) and keeps their arithmetic: a weight is dequantised
+// with one f32 multiply and enters an f32 multiply-add with the activation
+// (packages/runtime/src/kernels/gemm.ts:642-718, :922-940).
+//
+// `lanes` threads share two channels' k: 16 bytes of each per step, loaded two steps in front of their use; the
+// activations, up to four rows, lie in shared memory as f32.  Sixteen products are summed from zero and then added to the thread's sum; the threads meet in a shuffle tree and, above a warp, in warp order.
+//
+// What bounds it: instructions.  An int4 weight costs four (unpack, convert, scale) and one per activation row: one row of
+// 1152 -> 60468 (46 MB with f32 scales) 19 us, where the generic kernel and the many-row one took 50; for small
+// matrices the launch and two trips to memory (8064 -> 82: 14.4 us before, 5.6 now).
+#include <type_traits>
+
+#include "kq_common.cuh"
+#include "kq_gemv_core.cuh"
+#include "kq_internal.h"
+
+namespace kq {
+namespace {
+
+constexpr uint32_t kRowsThreads = 256;
+constexpr uint32_t kRowsSmem = 224 * 1024, kRowsMost = 16;  // shared memory for the activations (of four rows at most); rows of a call
+
+struct RowsParams {
+  const uint8_t* w;
+  const void* scale;
+  const float* bias;
+  float* out;
+  const void* x;
+  uint32_t m, n, k;
+  uint32_t steps;       // 16-byte pieces of a channel
+  uint32_t gshift;      // log2 of the group size (int4)
+  uint32_t lanes_log2;  // threads that share two channels
+};
+
+__device__ __forceinline__ uint4 rows_ldg(const uint8_t* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// Eight nibbles u (k ascending) -> u - 8: pairs 1024 + u and 1024 + 16 u as binary16, brought down exactly.
+__device__ __forceinline__ void rows_nibbles(uint32_t w, float (&v)[8]) {
+  const __half2 k1032 = __half2half2(__ushort_as_half(0x6408)), k16th = __half2half2(__ushort_as_half(0x2C00)),
+                km72 = __half2half2(__ushort_as_half(0xD480));
+  const uint32_t w8 = w >> 8;
+  const uint32_t r[4] = {(w & 0x000F000Fu) | 0x64006400u, (w & 0x00F000F0u) | 0x64006400u, (w8 & 0x000F000Fu) | 0x64006400u,
+                         (w8 & 0x00F000F0u) | 0x64006400u};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 p = *reinterpret_cast<const __half2*>(&r[i]);
+    const float2 f = __half22float2((i & 1) ? __hfma2(p, k16th, km72) : __hsub2(p, k1032));
+    v[i] = f.x;
+    v[i + 4] = f.y;
+  }
+}
+// Four bytes -> int8 values: a byte with its sign flipped, under the exponent of 1024, is 1024 + 128 + q.
+__device__ __forceinline__ void rows_bytes(uint32_t w, float* v) {
+  const __half2 k1152 = __half2half2(__ushort_as_half(0x6480));
+  const uint32_t u = w ^ 0x80808080u;
+  const uint32_t r[2] = {__byte_perm(u, 0x64646464u, 0x4140), __byte_perm(u, 0x64646464u, 0x4342)};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float2 f = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&r[i]), k1152));
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+
+template <typename XT, bool kI8, bool kScaleF16, int kRowsX>
+__global__ void __launch_bounds__(kRowsThreads, 2) qgemv_rows_kernel(const RowsParams p) {
+  constexpr uint32_t kPer = kI8 ? 16u : 32u;  // weights of a step
+  constexpr int kEights = kPer / 8;
+  constexpr int kAhead = 2;  // steps of weights in flight besides the one at work
+  __shared__ float part[kRowsThreads / 32][2 * kRowsX];
+  pdl_launch_dependents();
+  const uint32_t m0 = blockIdx.y * kRowsX, live = min(p.m - m0, static_cast<uint32_t>(kRowsX));
+  const uint32_t lanes = 1u << p.lanes_log2, me = threadIdx.x & (lanes - 1u);
+  const uint32_t pair = blockIdx.x * (kRowsThreads >> p.lanes_log2) + (threadIdx.x >> p.lanes_log2);
+  // (threads without a channel, or with one only, read the last channel's; they store nothing)
+  const uint32_t ch[2] = {min(2u * pair, p.n - 1u), min(2u * pair + 1u, p.n - 1u)};
+  const size_t row_bytes = static_cast<size_t>(p.steps) * 16u;
+  const uint8_t* wr[2] = {p.w + ch[0] * row_bytes, p.w + ch[1] * row_bytes};
+  const uint32_t groups = kI8 ? 1u : p.k >> p.gshift;
+
+  struct Piece { uint4 w[2]; float s[2][2]; };
+  auto fetch = [&](uint32_t step) {
+    Piece q;
+    const uint32_t at = min(step, p.steps - 1u);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      q.w[c] = rows_ldg(wr[c] + static_cast<size_t>(at) * 16u);
+      if constexpr (kI8) {
+        q.s[c][0] = q.s[c][1] = 1.0f;
+      } else {
+        const size_t g0 = static_cast<size_t>(ch[c]) * groups + ((at * kPer) >> p.gshift);
+        q.s[c][0] = load_scale<kScaleF16>(p.scale, g0);
+        q.s[c][1] = p.gshift == 4 ? load_scale<kScaleF16>(p.scale, g0 + 1u) : q.s[c][0];
+      }
+    }
+    return q;
+  };
+  Piece ring[kAhead + 1];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) ring[i] = fetch(me + i * lanes);
+  float cs[2] = {1.0f, 1.0f};
+  if constexpr (kI8)
+    for (int c = 0; c < 2; ++c) cs[c] = load_scale<kScaleF16>(p.scale, ch[c]);
+  // nothing the previous kernel writes has been touched so far
+  pdl_wait_prior_grid();
+
+  // Activations -> shared memory as f32, a step's four neighbours of one place side by side over the steps: the threads
+  // of a group, one step apart, then read consecutive 16-byte words (from global memory they are 64 or 128 bytes apart:
+  // 1 x 1152 -> 60468 int4 26 us).  An odd row length keeps the stores off each other's banks.
+  extern __shared__ float4 xs[];
+  const uint32_t row4 = p.steps | 1u;
+  {
+    const XT* x = static_cast<const XT*>(p.x) + static_cast<size_t>(m0) * p.k;
+    const uint32_t eights = p.k / 8u;
+    for (uint32_t i = threadIdx.x; i < kRowsX * eights; i += kRowsThreads) {
+      const uint32_t r = kRowsX == 1 ? 0u : i / eights, at = kRowsX == 1 ? i : i - r * eights, step = at / kEights, e = at % kEights;
+      float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (r < live) load_x8<XT, false>(x + static_cast<size_t>(r) * p.k + at * 8u, v);
+      float4* dst = xs + ((r * kEights + e) * 2u) * row4 + step;
+      dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+      dst[row4] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+  }
+  __syncthreads();
+  float acc[2][kRowsX];
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int r = 0; r < kRowsX; ++r) acc[c][r] = 0.0f;
+  for (uint32_t i0 = 0; i0 * lanes < p.steps; i0 += kAhead + 1)
+#pragma unroll
+  for (uint32_t u = 0; u <= kAhead; ++u) {
+    const uint32_t i = i0 + u;
+    if (i * lanes >= p.steps) break;
+    ring[(u + kAhead) % (kAhead + 1)] = fetch(me + (i + kAhead) * lanes);
+    const Piece& q = ring[u];
+    const uint32_t step = me + i * lanes;
+    if (step < p.steps) {
+      float sum[2][kRowsX];
+#pragma unroll
+      for (int e = 0; e < kEights; ++e) {
+        if (e % 2 == 0) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int r = 0; r < kRowsX; ++r) sum[c][r] = 0.0f;
+        }
+        float wv[2][8];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const uint32_t words[4] = {q.w[c].x, q.w[c].y, q.w[c].z, q.w[c].w};
+          if constexpr (kI8) {
+            rows_bytes(words[2 * e], wv[c]);
+            rows_bytes(words[2 * e + 1], wv[c] + 4);
+          } else {
+            rows_nibbles(words[e], wv[c]);
+          }
+          const float s = kI8 ? cs[c] : q.s[c][e / 2];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) wv[c][j] = __fmul_rn(wv[c][j], s);
+        }
+#pragma unroll
+        for (int r = 0; r < kRowsX; ++r) {
+          {
+            const float4* src = xs + ((r * kEights + e) * 2) * row4 + step;
+            const float4 a = src[0], b = src[row4];
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) sum[c][r] = fmaf(v[j], wv[c][j], sum[c][r]);
+          }
+        }
+        if (e % 2 == 1) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int r = 0; r < kRowsX; ++r) acc[c][r] += sum[c][r];
+        }
+      }
+    }
+  }
+  // the threads of a channel pair meet
+  const uint32_t in_warp = min(lanes, 32u);
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int r = 0; r < kRowsX; ++r)
+      for (uint32_t off = in_warp >> 1; off > 0; off >>= 1) acc[c][r] += __shfl_xor_sync(0xffffffffu, acc[c][r], off);
+  if (lanes > 32u) {
+    if ((threadIdx.x & 31u) == 0)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int r = 0; r < kRowsX; ++r) part[threadIdx.x >> 5][c * kRowsX + r] = acc[c][r];
+    __syncthreads();
+    const uint32_t first = (threadIdx.x >> 5) & ~((lanes >> 5) - 1u);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int r = 0; r < kRowsX; ++r) {
+        float total = 0.0f;
+        for (uint32_t w = 0; w < lanes >> 5; ++w) total += part[first + w][c * kRowsX + r];
+        acc[c][r] = total;
+      }
+  }
+  // thread r of the group stores activation row r (or, of few threads, several)
+#pragma unroll
+  for (int r = 0; r < kRowsX; ++r) {
+    if (static_cast<uint32_t>(r) < live && me == (static_cast<uint32_t>(r) & (lanes - 1u))) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (2u * pair + c < p.n) p.out[static_cast<size_t>(m0 + r) * p.n + 2u * pair + c] = acc[c][r] + p.bias[2u * pair + c];
+    }
+  }
+}
+
+// Bytes of staged activations.
+uint64_t rows_smem(uint32_t steps, uint32_t per, uint32_t rows) { return static_cast<uint64_t>(steps | 1u) * (per / 4u) * rows * 16u; }
+
+template <typename XT, bool kI8, bool kScaleF16, int kRowsX>
+cudaError_t launch_rows(const LaunchEnv& env, const RowsParams& p) {
+  auto kernel = qgemv_rows_kernel<XT, kI8, kScaleF16, kRowsX>;
+  static PerDevice<bool> configured_on;
+  bool* configured = configured_on.slot();
+  if (configured == nullptr) return cudaErrorInvalidDevice;
+  if (!*configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRowsSmem));
+    if (e != cudaSuccess) return e;
+    *configured = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  const uint32_t pairs = (p.n + 1) / 2, per_cta = kRowsThreads >> p.lanes_log2;
+  cfg.gridDim = dim3((pairs + per_cta - 1) / per_cta, (p.m + kRowsX - 1) / kRowsX);
+  cfg.blockDim = dim3(kRowsThreads);
+  cfg.dynamicSmemBytes = rows_smem(p.steps, kI8 ? 16u : 32u, kRowsX);
+  cfg.stream = env.stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = env.overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+template <typename XT, bool kI8, bool kScaleF16>
+cudaError_t launch_rows_m(const LaunchEnv& env, const RowsParams& p) {
+  if (p.m == 1) return launch_rows<XT, kI8, kScaleF16, 1>(env, p);
+  if (p.m == 2) return launch_rows<XT, kI8, kScaleF16, 2>(env, p);
+  return launch_rows<XT, kI8, kScaleF16, 4>(env, p);
+}
+template <typename XT>
+cudaError_t launch_rows_typed(const LaunchEnv& env, const RowsParams& p, bool i8, bool f16s) {
+  if (i8) return f16s ? launch_rows_m<XT, true, true>(env, p) : launch_rows_m<XT, true, false>(env, p);
+  return f16s ? launch_rows_m<XT, false, true>(env, p) : launch_rows_m<XT, false, false>(env, p);
+}
+
+}  // namespace
+
+bool qgemv_rows_supports(const Weight& w, uint32_t m) {
+  return w.layout == kLayoutNative && m >= 1 && m <= kRowsMost && w.n > 0 && w.k > 0 && w.k % (w.storage == KQ_STORAGE_I4 ? 32u : 16u) == 0 &&
+         rows_smem(w.k / (w.storage == KQ_STORAGE_I4 ? 32u : 16u), w.storage == KQ_STORAGE_I4 ? 32u : 16u, m > 2 ? 4u : m) <= kRowsSmem;
+}
+
+// This kernel or the many-row one (kq_qgemm_exact.cu; below its own line the generic kernel, which is behind everywhere
+// by two to seven times), by estimated time in units of 0.01 us.  Here a launch and its trips to memory, then the
+// instructions of a weight for every four activation rows.  There three launches, then whole waves of 74 tiles of 256
+// channels, which few tiles cut along k.  us, there | here, f32 activations:
+//   int4, group 128  1 x 768 -> 36699 23.4 | 8.8, 1 x 1152 -> 60468 50 | 19, 1 x 12288 -> 1490 21.4 | 9.8, 2 x 4096 -> 4090
+//                    17.4 | 11.5, 4 x 768 -> 36699 22.9 | 15.4, 16 x 8064 -> 82 35 | 10.2, but 4 x 12288 -> 1490 21.6 | 25.1,
+//                    8 x 768 -> 36699 23.2 | 28.9
+//   int8             1 x 768 -> 36699 25 | 8.5, 2 x 1152 -> 60468 59 | 26, 1 x 4096 -> 2841 16.7 | 7.8, 16 x 8064 -> 82 15.8 | 8.5, but
+//                    4 x 4096 -> 2841 17.4 | 21.9, 16 x 9984 -> 177 16.0 | 23.7
+bool qgemv_rows_preferred(const Weight& w, uint32_t m) {
+  if (m <= 2) return true;
+  const uint64_t weights = static_cast<uint64_t>(w.n) * w.k, passes = (m + 3) / 4;
+  const uint64_t long_k = (w.k < 4096u ? w.k : 4096u) / (w.storage == KQ_STORAGE_I4 ? 64u : 32u);  // every CTA stages the activations
+  const uint64_t here = 400 + passes * weights * (47 + long_k) / 1000000u;
+  const uint64_t pairs = (w.n + 255) / 256, waves = (pairs + 73) / 74;
+  uint64_t steps = (w.k + 63) / 64;
+  for (uint32_t splits = 2; splits <= 16 && pairs * splits <= 74 && steps >= 8; splits *= 2) steps = (steps + 1) / 2;
+  return here <= 600 + waves * (260 + 47 * steps);
+}
+
+cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const void* x, int x_dtype, uint32_t m) {
+  const Weight& w = *t.w;
+  if (!qgemv_rows_supports(w, m)) return cudaErrorInvalidValue;
+  const bool i8 = w.storage == KQ_STORAGE_I8;
+  RowsParams p = {};
+  p.w = static_cast<const uint8_t*>(w.data);
+  p.scale = w.scale;
+  p.bias = t.bias;
+  p.out = t.out;
+  p.x = x;
+  p.m = m;
+  p.n = w.n;
+  p.k = w.k;
+  p.steps = w.k / (i8 ? 16u : 32u);
+  while (!i8 && (1u << p.gshift) < w.group_size) ++p.gshift;
+  // As few threads to a pair of channels as still give every SM the CTAs it holds (three at most), at least two steps
+  // each: fewer reductions and fewer CTAs that stage the activations.
+  const uint64_t staged = rows_smem(p.steps, i8 ? 16u : 32u, m > 2 ? 4u : m), fit = kRowsSmem / (staged + 1024u);
+  const uint64_t want = static_cast<uint64_t>(env.sm_count) * kRowsThreads * (fit < 1 ? 1 : fit > 3 ? 3 : fit), pairs = (w.n + 1u) / 2u;
+  p.lanes_log2 = 2;
+  while (p.lanes_log2 < 8 && (pairs << p.lanes_log2) < want && (2u << p.lanes_log2) * 2u <= p.steps + 1u) ++p.lanes_log2;
+  const bool f16s = w.scale_dtype == KQ_F16;
+  switch (x_dtype) {
+    case KQ_F32: return launch_rows_typed<float>(env, p, i8, f16s);
+    case KQ_F16: return launch_rows_typed<__half>(env, p, i8, f16s);
+    case KQ_BF16: return launch_rows_typed<__nv_bfloat16>(env, p, i8, f16s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace kq
