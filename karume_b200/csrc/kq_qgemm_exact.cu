@@ -294,7 +294,10 @@ __device__ __forceinline__ uint32_t stage_warps(uint32_t stages) {
   return parts_of(kMath) == 3 && stages < kProdWarps ? kProdWarps : 1u;
 }
 
-template <int kW, int kMath, bool kMulti>
+// What a launch does: a tile to a pair; that, or a tile of a gate and its up projection; several tiles to a pair.
+enum ExForm : int { kPlain, kGate, kSeveral };
+
+template <int kW, int kMath, int kForm>
 __global__ void __launch_bounds__(kExThreads, 1)
 qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map0,
                    const __grid_constant__ CUtensorMap w_map1, const __grid_constant__ CUtensorMap w_map2,
@@ -302,7 +305,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   constexpr bool kTiled = kW == kI4Tiled || kW == kI8Tiled;
   constexpr bool kGroupScales = kW == kI4Tiled || kW == kI4Rows;
   constexpr uint32_t kParts = parts_of(kMath);
-  const bool gated = p.swiglu != 0;
+  constexpr bool kMulti = kForm == kSeveral, kMayGate = kForm == kGate;
+  const bool gated = kMayGate && p.swiglu != 0;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t raw_base = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
@@ -347,6 +351,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     r.ks_count = min(r.ks_begin + p.ksteps_per_split, p.ksteps) - r.ks_begin;
     return r;
   };
+
+  const Tile tile_first = tile_at(tile0);  // (looked up here, in front of the wait for the launch before)
 
   if (warp == kMmaWarp) {
     if (lane == 0) {
@@ -394,7 +400,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     uint32_t set = 0, scale_batch = 0;  // accumulator sets and batches of scales so far, over all tiles
     uint32_t tile = tile0;
     do {
-    const Tile at_tile = tile_at(tile);
+    const Tile at_tile = kMulti ? tile_at(tile) : tile_first;
     const uint32_t m0 = at_tile.m0, ks_count = at_tile.ks_count;
     // ---- a tile's columns [8 h, 8 h + 8) of this warp, at `from` in shared memory, to where they go ----
     // (what belongs to this thread's channel, or to its channel of the gate and of up, is read once a tile)
@@ -681,7 +687,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     uint32_t s = 0, phase = 0;
     uint32_t tile = tile0;
     do {
-    const uint32_t ks_count = tile_at(tile).ks_count;
+    const uint32_t ks_count = kMulti ? tile_at(tile).ks_count : tile_first.ks_count;
 #pragma unroll 1
     for (uint32_t ks = 0; ks < ks_count; ++ks, s = s + 1 == p.stages ? 0u : s + 1u, phase ^= s == 0 ? 1u : 0u) {
       if (!shared_stage && (s & (kProdWarps - 1u)) != warp - kDrainWarps) continue;
@@ -783,7 +789,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         uint32_t s = 0, phase = 0;
         uint32_t tile = tile0;
         do {
-        const Tile at = tile_at(tile);
+        const Tile at = kMulti ? tile_at(tile) : tile_first;
         const CUtensorMap* w_map = at.wi == 0 ? &w_map0 : at.wi == 1 ? &w_map1 : at.wi == 2 ? &w_map2 : &w_map3;
         const uint32_t w_row = kTiled ? at.n0 / 16u : at.n0, w_step = p.raw_box;  // tensor-map rows and columns of the raw weights
 #pragma unroll 1
@@ -827,7 +833,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           };
           uint32_t tile = tile0;
           do {
-          const uint32_t ks_count = tile_at(tile).ks_count;
+          const uint32_t ks_count = kMulti ? tile_at(tile).ks_count : tile_first.ks_count;
 #pragma unroll 1
           for (uint32_t ks = 0; ks < ks_count; ++ks) {
             wait_bounded(full + s * 8, phase, abort_flag, p.status, 22);
@@ -881,7 +887,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       uint32_t batch = 0;
       uint32_t tile = tile0;
       do {
-      const Tile at_tile = tile_at(tile);
+      const Tile at_tile = kMulti ? tile_at(tile) : tile_first;
       const uint32_t drains = (at_tile.ks_count * 4 + p.drain16 - 1) / p.drain16, drain0 = at_tile.ks_begin * 4 / p.drain16;
       if constexpr (kW == kI4Tiled) {
         // rows 16 (wl / 8) + wl % 8 and + 8: a chunk holds their scales of two groups side by side
@@ -1209,9 +1215,9 @@ bool kind_ok(const Weight& w) {
   }
 }
 
-template <int kW, int kMath, bool kMulti>
+template <int kW, int kMath, int kForm>
 cudaError_t launch_form(const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
-  auto kernel = qgemm_exact_kernel<kW, kMath, kMulti>;
+  auto kernel = qgemm_exact_kernel<kW, kMath, kForm>;
   static PerDevice<bool> configured_on;
   bool* configured = configured_on.slot();
   if (configured == nullptr) return cudaErrorInvalidDevice;
@@ -1225,15 +1231,21 @@ cudaError_t launch_form(const LaunchEnv& env, const ExParams& p, const CUtensorM
     if (e != cudaSuccess) return e;
     *configured = true;
   }
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + smem_tail(kMulti, p.nt);
-  const dim3 grid = kMulti ? dim3(p.resident * 2) : dim3(p.pairs * 2, p.m_tiles, p.splits);
+  const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + smem_tail(kForm == kSeveral, p.nt);
+  const dim3 grid = kForm == kSeveral ? dim3(p.resident * 2) : dim3(p.pairs * 2, p.m_tiles, p.splits);
   return launch_dependent(kernel, grid, kExThreads, smem, dim3(2, 1, p.cluster_splits), env, p, xm, wm[0], wm[1], wm[2], wm[3]);
 }
 template <int kW, int kMath>
 cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
-  if constexpr (kMath == kInt8)
-    if (p.multi) return launch_form<kW, kMath, true>(env, p, xm, wm);
-  return launch_form<kW, kMath, false>(env, p, xm, wm);
+  if constexpr (kMath == kInt8) {
+    return p.multi ? launch_form<kW, kMath, kSeveral>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
+  } else {
+    // (a decoder's prompt takes one kernel for all its matmuls: two that take turns cost it 6 us a layer in instructions
+    // fetched again, 692 | 667 us for four layers of 333 rows)
+    constexpr bool kPrompt = kW == kI4Tiled && parts_of(kMath) == 3;
+    if (kPrompt || p.swiglu) return launch_form<kW, kMath, kGate>(env, p, xm, wm);
+    else if constexpr (!kPrompt) return launch_form<kW, kMath, kPlain>(env, p, xm, wm);
+  }
 }
 
 // Pairs (slots[1]) and clusters of two or four pairs that the device holds at once; 0 where it cannot say.  Every form of
@@ -1244,7 +1256,7 @@ cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSp
   Held* held = held_on.slot();
   if (held == nullptr) return cudaErrorInvalidDevice;
   if (!held->done) {
-    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1, false>;
+    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1, kPlain>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
     if (e != cudaSuccess) return e;
     for (uint32_t z = 2; z <= kMaxClusterSplits; z *= 2) {
