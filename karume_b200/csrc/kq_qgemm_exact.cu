@@ -994,7 +994,10 @@ __device__ __forceinline__ Pow2 pow2_row(float amax) {
   r.inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
   return r;
 }
-template <typename XT, int kMath>
+// kHold: a row of up to 2,048 values a unit stays in the threads' registers between the passes; 0: it is read again for
+// each.  (Bound by trips to memory one after the other: three of them were one too many or two.  125 x 11904 -> 5984 78.7 us
+// before, 74.3 now; 257 x 1536 -> 8960 23.3, 22.5; four layers of 333 rows 665, 653.)
+template <typename XT, int kMath, int kHold>
 __global__ void __launch_bounds__(256)
 split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restrict__ parts, float* __restrict__ inv,
              const float* __restrict__ norm_weight, float norm_eps) {
@@ -1004,14 +1007,31 @@ split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restr
   __shared__ float part[8];
   pdl_wait_prior_grid();
   float r_inv = 1.0f;
+  float held[kHold > 0 ? kHold : 1][8];
+  if constexpr (kHold > 0) {
+#pragma unroll
+    for (int h = 0; h < kHold; ++h) {
+      const uint32_t i = threadIdx.x * 8 + h * 2048u;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) held[h][e] = 0.0f;
+      if (i < k) load_x8<XT>(xr + i, held[h]);
+    }
+  }
   if (norm_weight != nullptr) {
     // sum of squares in a fixed order: thread-strided, shuffle tree, warps in order
     float sq = 0.0f;
-    for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
-      float v[8];
-      load_x8<XT>(xr + i, v);
+    if constexpr (kHold > 0) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) sq = fmaf(v[e], v[e], sq);
+      for (int h = 0; h < kHold; ++h)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sq = fmaf(held[h][e], held[h][e], sq);
+    } else {
+      for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
+        float v[8];
+        load_x8<XT>(xr + i, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sq = fmaf(v[e], v[e], sq);
+      }
     }
     sq = warp_sum(sq);
     if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = sq;
@@ -1021,8 +1041,7 @@ split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restr
     r_inv = rsqrtf(total * (1.0f / static_cast<float>(k)) + norm_eps);
     __syncthreads();
   }
-  auto load = [&](uint32_t i, float (&v)[8]) {
-    load_x8<XT>(xr + i, v);
+  auto scaled = [&](uint32_t i, float (&v)[8]) {
     if (norm_weight != nullptr) {
       const float4 w0 = __ldg(reinterpret_cast<const float4*>(norm_weight + i)), w1 = __ldg(reinterpret_cast<const float4*>(norm_weight + i + 4));
       const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
@@ -1031,10 +1050,22 @@ split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restr
     }
   };
   float amax = 0.0f;
-  for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {  // k is a multiple of 16
-    float v[8];
-    load(i, v);
-    amax = fmaxf(amax, absmax8(v));
+  if constexpr (kHold > 0) {
+#pragma unroll
+    for (int h = 0; h < kHold; ++h) {
+      const uint32_t i = threadIdx.x * 8 + h * 2048u;
+      if (i < k) {
+        scaled(i, held[h]);
+        amax = fmaxf(amax, absmax8(held[h]));
+      }
+    }
+  } else {
+    for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {  // k is a multiple of 16
+      float v[8];
+      load_x8<XT>(xr + i, v);
+      scaled(i, v);
+      amax = fmaxf(amax, absmax8(v));
+    }
   }
 #pragma unroll
   for (int offset = 16; offset > 0; offset >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
@@ -1044,9 +1075,7 @@ split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restr
   for (int w = 1; w < 8; ++w) amax = fmaxf(amax, part[w]);
   const Pow2 ps = kIsBf<kMath> ? pow2_row(amax) : pow2_prescale(amax);
   if (threadIdx.x == 0) inv[row] = ps.inv;
-  for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
-    float v[8];
-    load(i, v);
+  auto store = [&](uint32_t i, float (&v)[8]) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= ps.scale;
 #pragma unroll
@@ -1070,6 +1099,20 @@ split_kernel(const XT* __restrict__ x, uint32_t m, uint32_t k, uint16_t* __restr
         v[2 * j + 1] = isinf(f.y) ? 0.0f : v[2 * j + 1] - f.y;
       }
       *reinterpret_cast<uint4*>(parts + (static_cast<size_t>(part) * m + row) * k + i) = o;
+    }
+  };
+  if constexpr (kHold > 0) {
+#pragma unroll
+    for (int h = 0; h < kHold; ++h) {
+      const uint32_t i = threadIdx.x * 8 + h * 2048u;
+      if (i < k) store(i, held[h]);
+    }
+  } else {
+    for (uint32_t i = threadIdx.x * 8; i < k; i += 2048) {
+      float v[8];
+      load_x8<XT>(xr + i, v);
+      scaled(i, v);
+      store(i, v);
     }
   }
   pdl_launch_dependents();
@@ -1540,12 +1583,20 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
       uint16_t* parts = reinterpret_cast<uint16_t*>(ws + align256(static_cast<uint64_t>(pm) * 4));
       const uint64_t taken = align256(static_cast<uint64_t>(pm) * 4) + align256(pm * part_bytes);
       if (taken > room) return cudaErrorMemoryAllocation;
-      auto split = [&](auto kernel, auto* rows) {
-        return launch_dependent(kernel, dim3(pm), 256, 0, 1, env, rows, pm, k, parts, inv, env.norm_weight, env.norm_eps);
+      auto split = [&](auto* rows, auto form) {
+        using XT = std::remove_const_t<std::remove_pointer_t<decltype(rows)>>;
+        constexpr int kForm = decltype(form)::value;
+        auto launch = [&](auto kernel) {
+          return launch_dependent(kernel, dim3(pm), 256, 0, 1, env, rows, pm, k, parts, inv, env.norm_weight, env.norm_eps);
+        };
+        if (k <= 2048) return launch(split_kernel<XT, kForm, 1>);
+        if (k <= 4096) return launch(split_kernel<XT, kForm, 2>);
+        if (k <= 16384) return launch(split_kernel<XT, kForm, 8>);
+        return launch(split_kernel<XT, kForm, 0>);
       };
-      if (math == kBf1) e = split(split_kernel<__nv_bfloat16, kBf1>, reinterpret_cast<const __nv_bfloat16*>(xp));
-      else if (math == kBf3) e = split(split_kernel<float, kBf3>, reinterpret_cast<const float*>(xp));
-      else e = split(split_kernel<float, kHalf2>, reinterpret_cast<const float*>(xp));
+      if (math == kBf1) e = split(reinterpret_cast<const __nv_bfloat16*>(xp), std::integral_constant<int, kBf1>{});
+      else if (math == kBf3) e = split(reinterpret_cast<const float*>(xp), std::integral_constant<int, kBf3>{});
+      else e = split(reinterpret_cast<const float*>(xp), std::integral_constant<int, kHalf2>{});
       if (e != cudaSuccess) return e;
       if (launches) *launches += 1;
       e = run_exact(env, count, t, residual, parts, math, pm, chain_of(math, w0), inv, ws + taken, room - taken, true, swiglu, launches);

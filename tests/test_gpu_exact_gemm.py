@@ -105,6 +105,12 @@ def test_slices_that_meet_in_a_cluster(gpu, xdt, storage, group, m, n, k):
     test_matches_the_f64_oracle(gpu, xdt, storage, group, m, n, k)
 
 
+# Rows whose values stay in the splitting kernel's registers (2,048 a unit, up to eight units), and one beyond that
+@pytest.mark.parametrize("m,n,k", [(17, 40, 2048), (18, 40, 2064), (17, 40, 4112), (17, 24, 16384), (18, 24, 16400)])
+def test_rows_of_any_length_are_split(gpu, m, n, k):
+    test_matches_the_f64_oracle(gpu, "f32", "i8", 0, m, n, k)
+
+
 @pytest.mark.parametrize("m,n,k", [(20, 272, 4096), (150, 528, 2176), (97, 259, 1136)])
 def test_integer_sums_that_meet_in_a_cluster(gpu, m, n, k):
     test_integer_dot_is_bit_exact(gpu, "i8", 0, m, n, k)
