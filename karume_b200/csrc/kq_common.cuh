@@ -134,4 +134,11 @@ __device__ __forceinline__ void pdl_wait_prior_grid() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A barrier of all threads of the cluster.  The aligned form wants every warp converged, which a loop whose lanes leave
+// it at different times, or a load that only some of them do, does not give by itself.
+__device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 }  // namespace kq

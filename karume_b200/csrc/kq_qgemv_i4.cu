@@ -113,9 +113,6 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // K was split over the CTAs of a cluster: every CTA holds its partial sums in `red`
 // ([m][tile_rows] f32 in its own shared memory); after one cluster barrier each CTA adds a

@@ -84,9 +84,6 @@ __device__ __forceinline__ uint2 xs_ldg64(const void* p) {
   asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
-__device__ __forceinline__ void xs_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float xs_ld_rank(uint32_t addr, uint32_t rank) {
   float v;
   asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
@@ -249,7 +246,7 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
             row_factor[threadIdx.x] = rsqrtf(total * (1.0f / static_cast<float>(p.k)) + p.norm_eps);
           }
           if (p.cluster > 1) {
-            xs_cluster_sync();
+            cluster_sync_all();
             if (threadIdx.x < p.m && mine != rank)
               row_factor[threadIdx.x] = xs_ld_rank(static_cast<uint32_t>(__cvta_generic_to_shared(row_factor + threadIdx.x)), mine);
           }
@@ -401,7 +398,7 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
     }
 
     // ---- the cluster's sums meet, in rank order, and leave with the neighbours applied ----
-    if (p.cluster > 1) xs_cluster_sync();
+    if (p.cluster > 1) cluster_sync_all();
     else __syncthreads();
     const uint32_t part_addr = static_cast<uint32_t>(__cvta_generic_to_shared(part));
     const uint32_t outs = units_now * p.m * 16u;
@@ -433,7 +430,7 @@ __global__ void __launch_bounds__(kXsThreads, 1) qgemv_i4_xs_kernel(const XsPara
         p.out[wi][at] = v;
       }
     }
-    if (p.cluster > 1) xs_cluster_sync();  // nobody's sums go away while a peer still reads them
+    if (p.cluster > 1) cluster_sync_all();  // nobody's sums go away while a peer still reads them
     else __syncthreads();
   }
 }

@@ -57,9 +57,6 @@ __device__ __forceinline__ float ld_cluster_f32_8(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ void cluster_sync_all8() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // Stages 32-k chunks [chunk0, chunk0 + chunks) of x.
 //   xs   : [local chunk][active columns][64 B]; inside a column block, 16 B per t = 0..3:
@@ -313,7 +310,7 @@ qgemv_i8_kernel(const Gemv8Params p) {
     }
   }
   if (p.splits == 1) return;
-  cluster_sync_all8();
+  cluster_sync_all();
   const uint32_t rows_here = min(kTileRowsCta, p.n - tile * kTileRowsCta);
   const uint32_t total = rows_here * p.m;
   const uint32_t per_rank = (total + p.splits - 1) / p.splits;
@@ -327,7 +324,7 @@ qgemv_i8_kernel(const Gemv8Params p) {
     const uint32_t row = tile * kTileRowsCta + r;
     p.out[static_cast<size_t>(mm) * p.n + row] = fmaf(load_scale<kScaleF16>(p.scale, row), sum, p.bias[row]);
   }
-  cluster_sync_all8();
+  cluster_sync_all();
 }
 
 template <typename XT, bool kScaleF16, int kCols, int kRB>

@@ -56,9 +56,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // the address of this CTA's shared-memory location `addr` as seen in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   uint32_t r;
