@@ -1261,19 +1261,16 @@ bool kind_ok(const Weight& w) {
 template <int kW, int kMath, int kForm>
 cudaError_t launch_form(const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
   auto kernel = qgemm_exact_kernel<kW, kMath, kForm>;
-  static PerDevice<bool> configured_on;
-  bool* configured = configured_on.slot();
-  if (configured == nullptr) return cudaErrorInvalidDevice;
-  if (!*configured) {
+  static OncePerDevice configured;
+  const cudaError_t ready = configured.run([&]() -> cudaError_t {
     // the register split adds up to 512 x 128: refuse to run a build whose launch holds fewer
     cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
     if (e != cudaSuccess) return e;
     if (fa.numRegs < 128) return cudaErrorInvalidKernelImage;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
-    if (e != cudaSuccess) return e;
-    *configured = true;
-  }
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
+  });
+  if (ready != cudaSuccess) return ready;
   const size_t smem = 1024 + static_cast<size_t>(p.stages) * p.stage_bytes + smem_tail(kForm == kSeveral, p.nt);
   const dim3 grid = kForm == kSeveral ? dim3(p.resident * 2) : dim3(p.pairs * 2, p.m_tiles, p.splits);
   return launch_dependent(kernel, grid, kExThreads, smem, dim3(2, 1, p.cluster_splits), env, p, xm, wm[0], wm[1], wm[2], wm[3]);
@@ -1294,13 +1291,12 @@ cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, const CUtensorM
 // Pairs (slots[1]) and clusters of two or four pairs that the device holds at once; 0 where it cannot say.  Every form of
 // the kernel fills an SM, so one of them stands for all.
 cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSplits + 1]) {
-  struct Held { bool done; uint32_t clusters[kMaxClusterSplits + 1]; };
+  struct Held { uint32_t clusters[kMaxClusterSplits + 1]; };
   static PerDevice<Held> held_on;
-  Held* held = held_on.slot();
-  if (held == nullptr) return cudaErrorInvalidDevice;
-  if (!held->done) {
+  const Held* held = nullptr;
+  const cudaError_t known = held_on.get([](Held& h) -> cudaError_t {
     auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1, kPlain>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
     if (e != cudaSuccess) return e;
     for (uint32_t z = 2; z <= kMaxClusterSplits; z *= 2) {
       cudaLaunchConfig_t cfg = {};
@@ -1319,10 +1315,11 @@ cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSp
         (void)cudaGetLastError();
         n = 0;
       }
-      held->clusters[z] = static_cast<uint32_t>(n);
+      h.clusters[z] = static_cast<uint32_t>(n);
     }
-    held->done = true;
-  }
+    return cudaSuccess;
+  }, &held);
+  if (known != cudaSuccess) return known;
   for (uint32_t z = 0; z <= kMaxClusterSplits; ++z) slots[z] = held->clusters[z];
   slots[1] = static_cast<uint32_t>(std::max(1, env.sm_count / 2));
   return cudaSuccess;

@@ -48,6 +48,7 @@
 // split into binary16 parts, and the inverse is applied to the group's partial sum in f32
 // (kq_gemv_core.cuh: pow2_prescale), so the result does not depend on the magnitude of x.
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "kq_gemv_core.cuh"
@@ -481,8 +482,10 @@ struct ResidencyKey {
   uint32_t ctas;
 };
 uint32_t resident_ctas(const void* kernel, int device, const cudaLaunchConfig_t& cfg, uint32_t splits, int sm_count) {
+  static std::mutex lock;  // the contexts of several threads share the table
   static ResidencyKey cache[64];
   static int cached = 0;
+  std::lock_guard<std::mutex> hold(lock);
   for (int i = 0; i < cached; ++i)
     if (cache[i].kernel == kernel && cache[i].device == device && cache[i].smem == cfg.dynamicSmemBytes &&
         cache[i].splits == splits)
@@ -515,21 +518,20 @@ template <typename XT, bool kScaleF16, int kG, int kD>
 cudaError_t launch_typed_gp_depth(const LaunchEnv& env, GemvParams& p, int count, const LinearTarget* targets,
                                   bool probe_only, uint32_t* ctas_out, uint32_t* capacity_out) {
   auto kernel = qgemv_i4_gp_kernel<XT, kScaleF16, kG, kD>;
-  struct Setup { bool done; uint32_t max_cluster; };
-  static PerDevice<Setup> setup_on;
-  Setup* setup = setup_on.slot();
-  if (setup == nullptr) return cudaErrorInvalidDevice;
-  uint32_t& max_cluster = setup->max_cluster;
-  if (!setup->done) {
-    max_cluster = kMaxCluster;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  static PerDevice<uint32_t> max_cluster_on;
+  const uint32_t* learnt = nullptr;
+  const cudaError_t ready = max_cluster_on.get([&](uint32_t& largest) -> cudaError_t {
+    largest = kMaxCluster;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     if (e != cudaSuccess) return e;
     // few row tiles and a long k (8960 -> 1536): sixteen splits, the largest cluster the device
     // takes with this opt-in, halve each CTA's share again
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) max_cluster = 16;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) largest = 16;
     else (void)cudaGetLastError();
-    setup->done = true;
-  }
+    return cudaSuccess;
+  }, &learnt);
+  if (ready != cudaSuccess) return ready;
+  const uint32_t max_cluster = *learnt;
   constexpr bool kHasLo = !std::is_same<XT, __half>::value;
   constexpr uint32_t kCpg = 8 / kG, kCU = kG / 2;
   constexpr uint32_t kCorrStride = kHasLo ? kCpg / 2 : kCpg;
@@ -941,14 +943,9 @@ template <typename XT, bool kScaleF16, int kTiles, int kRB, int kD>
 cudaError_t launch_typed_wide(const LaunchEnv& env, GemvParams& p, int count, const LinearTarget* targets,
                               int* extra_launches) {
   auto kernel = qgemv_i4_wide_kernel<XT, kScaleF16, kTiles, kRB, kD>;
-  static PerDevice<bool> configured_on;
-  bool* configured = configured_on.slot();
-  if (configured == nullptr) return cudaErrorInvalidDevice;
-  if (!*configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    if (e != cudaSuccess) return e;
-    *configured = true;
-  }
+  static OncePerDevice configured;
+  const cudaError_t ready = configured.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); });
+  if (ready != cudaSuccess) return ready;
   constexpr bool kHasLo = !std::is_same<XT, __half>::value;
   constexpr uint32_t kTileRowsCta = kWarps * kRB * 16;
   uint32_t tiles = 0;

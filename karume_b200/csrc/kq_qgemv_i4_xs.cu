@@ -463,16 +463,16 @@ cudaError_t launch_xs(const LaunchEnv& env, XsParams& p) {
   auto kernel = qgemv_i4_xs_kernel<XT, kScaleF16, kForm>;
   using Shape = XsShape<kForm>;
   constexpr uint32_t kSlabChunks = Shape::slab_chunks;
-  struct Setup { bool done; uint32_t resident[kXsMaxCluster + 1]; };
+  struct Setup { uint32_t resident[kXsMaxCluster + 1]; };
   static PerDevice<Setup> setup_on;
-  Setup* setup = setup_on.slot();
-  if (setup == nullptr) return cudaErrorInvalidDevice;
-  if (!setup->done) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kXsSmem));
+  const Setup* setup = nullptr;
+  const cudaError_t ready = setup_on.get([&](Setup& s) -> cudaError_t {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kXsSmem));
     if (e != cudaSuccess) return e;
-    for (uint32_t c = 1; c <= kXsMaxCluster; ++c) setup->resident[c] = resident_clusters(kernel, c, env.sm_count);
-    setup->done = true;
-  }
+    for (uint32_t c = 1; c <= kXsMaxCluster; ++c) s.resident[c] = resident_clusters(kernel, c, env.sm_count);
+    return cudaSuccess;
+  }, &setup);
+  if (ready != cudaSuccess) return ready;
   // How many CTAs share a row block's k: the cluster size with the shortest longest list of (row block, pass)
   // pairs; a pass costs about two blocks (building the fragments), a cluster about one (its barriers).
   const uint32_t slabs = (p.k / kChunkK + kSlabChunks - 1) / kSlabChunks, per_unit = p.swiglu ? 2u : 1u;

@@ -330,20 +330,19 @@ qgemv_i8_kernel(const Gemv8Params p) {
 template <typename XT, bool kScaleF16, int kCols, int kRB>
 cudaError_t launch_typed8(const LaunchEnv& env, Gemv8Params& p) {
   auto kernel = qgemv_i8_kernel<XT, kScaleF16, kCols, kRB>;
-  struct Setup { bool done; uint32_t max_cluster; };
-  static PerDevice<Setup> setup_on;
-  Setup* setup = setup_on.slot();
-  if (setup == nullptr) return cudaErrorInvalidDevice;
-  uint32_t& max_cluster = setup->max_cluster;
-  if (!setup->done) {
-    max_cluster = kMaxCluster8;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  static PerDevice<uint32_t> max_cluster_on;
+  const uint32_t* learnt = nullptr;
+  const cudaError_t ready = max_cluster_on.get([&](uint32_t& largest) -> cudaError_t {
+    largest = kMaxCluster8;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     if (e != cudaSuccess) return e;
     // few row tiles and a long k: sixteen splits (the largest cluster, by opt-in)
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) max_cluster = 16;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) largest = 16;
     else (void)cudaGetLastError();
-    setup->done = true;
-  }
+    return cudaSuccess;
+  }, &learnt);
+  if (ready != cudaSuccess) return ready;
+  const uint32_t max_cluster = *learnt;
   constexpr bool kHasLo = !std::is_same<XT, __half>::value;
   constexpr uint32_t kTileRowsCta = kWarps8 * kRB * 16;
   const uint32_t tiles = (p.n + kTileRowsCta - 1) / kTileRowsCta;

@@ -230,14 +230,9 @@ uint64_t rows_smem(uint32_t steps, uint32_t per, uint32_t rows) { return static_
 template <typename XT, bool kI8, bool kScaleF16, int kRowsX>
 cudaError_t launch_rows(const LaunchEnv& env, const RowsParams& p) {
   auto kernel = qgemv_rows_kernel<XT, kI8, kScaleF16, kRowsX>;
-  static PerDevice<bool> configured_on;
-  bool* configured = configured_on.slot();
-  if (configured == nullptr) return cudaErrorInvalidDevice;
-  if (!*configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRowsSmem));
-    if (e != cudaSuccess) return e;
-    *configured = true;
-  }
+  static OncePerDevice configured;
+  const cudaError_t ready = configured.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRowsSmem)); });
+  if (ready != cudaSuccess) return ready;
   cudaLaunchConfig_t cfg = {};
   const uint32_t pairs = (p.n + 1) / 2, per_cta = kRowsThreads >> p.lanes_log2;
   cfg.gridDim = dim3((pairs + per_cta - 1) / per_cta, (p.m + kRowsX - 1) / kRowsX);
