@@ -276,10 +276,13 @@ int check_linear_args(kq_ctx* ctx, const Weight* w, uint64_t x, int x_dtype, uin
   return KQ_OK;
 }
 
+// The kernel for row-major packed weights (kq_qgemv_rows.cu) runs this weight: up to 16 rows.
+bool takes_rows_gemv(const Weight& w, uint32_t m) { return kq::qgemv_rows_supports(w, m) && kq::qgemv_rows_preferred(w, m); }
+
 // The many-row kernel of kq_qgemm_exact.cu runs this call: more than 16 rows, weights of one kind,
 // and not a case of the bf16 GEMM (bf16 activations on a tiled weight, whose operands are rounded).
 bool takes_exact_gemm(const kq_ctx* ctx, int count, const kq::LinearTarget* targets, int x_dtype, uint32_t m) {
-  if (count == 1 && kq::qgemv_rows_supports(*targets[0].w, m) && kq::qgemv_rows_preferred(*targets[0].w, m)) return false;
+  if (count == 1 && takes_rows_gemv(*targets[0].w, m)) return false;
   for (int i = 0; i < count; ++i)
     if (kq::qgemm_i4_supports(*targets[i].w, x_dtype, m) || kq::qgemm_i8_supports(*targets[i].w, x_dtype, m)) return false;
   return kq::qgemm_exact_supports(count, targets, m, ctx->workspace ? ctx->workspace_bytes : 0);
@@ -353,10 +356,10 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
     }
     return KQ_OK;
   }
-  // Everything else: one generic launch per weight.
+  // Everything else, weight by weight.
   for (uint32_t i = 0; i < count; ++i) {
     const Weight& w = *targets[i].w;
-    if (kq::qgemv_rows_supports(w, m) && kq::qgemv_rows_preferred(w, m)) {
+    if (takes_rows_gemv(w, m)) {
       cudaError_t e = kq::launch_qgemv_rows(env, targets[i], reinterpret_cast<const void*>(x), x_dtype, m);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_rows launch");
       ctx->launches += 1;
@@ -1100,8 +1103,8 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
   if (m == 0) return KQ_OK;
   DeviceGuard guard(ctx->device);
   // Outside a plan: the same arithmetic as a sequence of kernels — except where the linear takes
-  // the norm and the residual into its own launches (five to sixteen rows on tiled int4 weights,
-  // and the many-row kernel).
+  // the norm and the residual into its own launches (up to sixteen rows on tiled int4 weights or
+  // one row-major weight, and the many-row kernel).
   {
     kq::LinearTarget probe[kq::kMaxMulti];
     bool known = true;
@@ -1151,6 +1154,7 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
     }
     if (known && !reduce && (norm_weight_dptr || residual_dptr) &&
         (kq::qgemv_i4_fuses_neighbours(static_cast<int>(count), probe, x_dtype, m) ||
+         (count == 1 && takes_rows_gemv(*probe[0].w, m)) ||
          takes_exact_gemm(ctx, static_cast<int>(count), probe, x_dtype, m))) {
       int rc;
       if (swiglu) {

@@ -35,6 +35,9 @@ struct RowsParams {
   uint32_t steps;       // 16-byte pieces of a channel
   uint32_t gshift;      // log2 of the group size (int4)
   uint32_t lanes_log2;  // threads that share two channels
+  const float* norm_weight;  // null, or [k]: the f32 activations are rms-normalised as they are staged
+  float norm_eps;
+  const float* residual;  // null, or [m, n] added after the bias (may alias out)
 };
 
 __device__ __forceinline__ uint4 rows_ldg(const uint8_t* p) {
@@ -77,6 +80,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) qgemv_rows_kernel(const RowsP
   constexpr int kEights = kPer / 8;
   constexpr int kAhead = 2;  // steps of weights in flight besides the one at work
   __shared__ float part[kRowsThreads / 32][2 * kRowsX];
+  __shared__ float row_norm[kRowsX];
   pdl_launch_dependents();
   const uint32_t m0 = blockIdx.y * kRowsX, live = min(p.m - m0, static_cast<uint32_t>(kRowsX));
   const uint32_t lanes = 1u << p.lanes_log2, me = threadIdx.x & (lanes - 1u);
@@ -121,10 +125,48 @@ __global__ void __launch_bounds__(kRowsThreads, 2) qgemv_rows_kernel(const RowsP
   {
     const XT* x = static_cast<const XT*>(p.x) + static_cast<size_t>(m0) * p.k;
     const uint32_t eights = p.k / 8u;
+    [[maybe_unused]] const bool norm = std::is_same<XT, float>::value && p.norm_weight != nullptr;
+    if constexpr (std::is_same<XT, float>::value) {
+      if (norm) {
+        // sums of squares in a fixed order: thread-strided, shuffle tree, warps in order
+        float sq[kRowsX];
+#pragma unroll
+        for (int r = 0; r < kRowsX; ++r) sq[r] = 0.0f;
+        for (uint32_t i = threadIdx.x; i < eights; i += kRowsThreads)
+#pragma unroll
+          for (int r = 0; r < kRowsX; ++r) {
+            if (static_cast<uint32_t>(r) >= live) continue;
+            float v[8];
+            load_x8<XT, false>(x + static_cast<size_t>(r) * p.k + i * 8u, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sq[r] = fmaf(v[e], v[e], sq[r]);
+          }
+#pragma unroll
+        for (int r = 0; r < kRowsX; ++r) {
+          sq[r] = warp_sum(sq[r]);
+          if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5][r] = sq[r];
+        }
+        __syncthreads();
+        if (threadIdx.x < kRowsX) {
+          float total = 0.0f;
+          for (uint32_t w = 0; w < kRowsThreads / 32; ++w) total += part[w][threadIdx.x];
+          row_norm[threadIdx.x] = rsqrtf(total * (1.0f / static_cast<float>(p.k)) + p.norm_eps);
+        }
+        __syncthreads();
+      }
+    }
     for (uint32_t i = threadIdx.x; i < kRowsX * eights; i += kRowsThreads) {
       const uint32_t r = kRowsX == 1 ? 0u : i / eights, at = kRowsX == 1 ? i : i - r * eights, step = at / kEights, e = at % kEights;
       float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       if (r < live) load_x8<XT, false>(x + static_cast<size_t>(r) * p.k + at * 8u, v);
+      if constexpr (std::is_same<XT, float>::value) {
+        if (norm) {
+          float wv[8];
+          load_x8<float, false>(p.norm_weight + at * 8u, wv);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(__fmul_rn(v[j], row_norm[r]), wv[j]);
+        }
+      }
       float4* dst = xs + ((r * kEights + e) * 2u) * row4 + step;
       dst[0] = make_float4(v[0], v[1], v[2], v[3]);
       dst[row4] = make_float4(v[4], v[5], v[6], v[7]);
@@ -219,7 +261,12 @@ __global__ void __launch_bounds__(kRowsThreads, 2) qgemv_rows_kernel(const RowsP
     if (static_cast<uint32_t>(r) < live && me == (static_cast<uint32_t>(r) & (lanes - 1u))) {
 #pragma unroll
       for (int c = 0; c < 2; ++c)
-        if (2u * pair + c < p.n) p.out[static_cast<size_t>(m0 + r) * p.n + 2u * pair + c] = acc[c][r] + p.bias[2u * pair + c];
+        if (2u * pair + c < p.n) {
+          const size_t at = static_cast<size_t>(m0 + r) * p.n + 2u * pair + c;
+          float o = __fadd_rn(acc[c][r], p.bias[2u * pair + c]);
+          if (p.residual != nullptr) o = __fadd_rn(o, p.residual[at]);
+          p.out[at] = o;
+        }
     }
   }
 }
@@ -287,7 +334,7 @@ bool qgemv_rows_preferred(const Weight& w, uint32_t m) {
 
 cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const void* x, int x_dtype, uint32_t m) {
   const Weight& w = *t.w;
-  if (!qgemv_rows_supports(w, m)) return cudaErrorInvalidValue;
+  if (!qgemv_rows_supports(w, m) || (env.norm_weight != nullptr && x_dtype != KQ_F32)) return cudaErrorInvalidValue;
   const bool i8 = w.storage == KQ_STORAGE_I8;
   RowsParams p = {};
   p.w = static_cast<const uint8_t*>(w.data);
@@ -299,6 +346,9 @@ cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const
   p.n = w.n;
   p.k = w.k;
   p.steps = w.k / (i8 ? 16u : 32u);
+  p.norm_weight = env.norm_weight;
+  p.norm_eps = env.norm_eps;
+  p.residual = env.residual;
   while (!i8 && (1u << p.gshift) < w.group_size) ++p.gshift;
   // As few threads to a pair of channels as still give every SM the CTAs it holds (three at most), at least two steps
   // each: fewer reductions and fewer CTAs that stage the activations.

@@ -75,3 +75,47 @@ def test_infinities_and_nans_reach_their_channels(gpu):
     assert np.array_equal(got[0], want.astype(np.float32), equal_nan=True)
     assert bool(np.isnan(got[1]).all())
     w.free()
+
+
+# The norm and the residual go into the linear's own launch and need no scratch, so the first call of a context may be a
+# recorded one: rows that take this kernel (one and two rows to a CTA, four, several passes) and some that take the
+# many-row kernel.
+@pytest.mark.parametrize("neighbours", ["norm", "residual", "both"])
+@pytest.mark.parametrize("storage,group,m,n,k", [("i4", 64, 1, 4097, 4096), ("i4", 16, 2, 3001, 4224), ("i8", 0, 1, 3001, 2800), ("i4", 128, 3, 1000, 12288),
+                                                 ("i8", 0, 16, 82, 8064), ("i4", 64, 16, 250, 8192), ("i4", 64, 16, 8191, 768), ("i8", 0, 9, 9001, 1152)])
+def test_norm_and_residual_in_a_first_call_that_is_recorded(storage, group, m, n, k, neighbours):
+    import torch
+    import karume_b200 as kb
+    rng = np.random.default_rng(n)
+    x, bias, res = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (n,), (m, n)))
+    norm = (1 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    xn = x if neighbours == "residual" else oracle.rms_norm(x, norm, 1e-5)
+    if storage == "i4":
+        data, scale = cases.synth_i4(n, k, seed=n, group_size=group)
+        ref = oracle.linear_i4(xn, data, scale.astype(np.float32), bias, n, k, group)
+    else:
+        data, scale = cases.synth_i8(n, k, seed=n)
+        ref = oracle.linear_i8(xn, data, scale.astype(np.float32), bias, n, k)
+    if neighbours != "norm":
+        ref = oracle.add(ref, res)
+    fresh = kb.acquire_gpu(0)
+    fresh.use_stream(torch.cuda.Stream())
+    w = fresh.upload_weight(storage, data, scale, (n, k), group)
+    xd, bd, nd, out = (torch.from_numpy(a).cuda() for a in (x, bias, norm, res))  # the residual is the output buffer
+    kept = out.clone()
+    torch.cuda.synchronize()
+    fresh.graph_begin()
+    fresh.linear_fused(xd, [w], [bd], [out], norm_weight=None if neighbours == "residual" else nd, eps=1e-5 if neighbours != "residual" else 0.0,
+                       residual=None if neighbours == "norm" else out)
+    g = fresh.graph_end()
+    rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
+    for _ in range(2):
+        out.copy_(kept)
+        torch.cuda.synchronize()
+        fresh.graph_launch(g)
+        fresh.sync()
+        rep = oracle.allclose(out.cpu().numpy(), ref, atol=1e-5 * max(1.0, rms), rtol=1e-4)
+        assert rep["pass"], rep
+    fresh.graph_free(g)
+    w.free()
+    fresh.destroy()
