@@ -38,12 +38,12 @@
 //                global load still in flight when a thread runs its proxy fence would hold the
 //                fence, and with it the stage, for a trip to memory.
 //   warp 12      starts every copy: the activation tile (tensor map), the raw weights (bulk)
+//   warp 13      tensor memory; in the first CTA of the pair one thread issues the MMAs
+//                (cta_group::2: the pair shares the activation tile, half from each CTA)
 //   warps 14-15  the group scales, a few chains ahead, as f32 into shared memory
 //
 // A gate and its up projection share a tile (64 channels of each per CTA), so that silu(gate) * up is the epilogue:
 // 333 rows of 1536 -> 2 x 8960 took 68 us and the gate's own kernel 11, now 69.
-//   warp 13      tensor memory; in the CTA of cluster rank 0 one thread issues the MMAs
-//                (cta_group::2: the pair shares the activation tile, half from each CTA)
 // Register split (setmaxnreg): 2 x 128 x 184 + 2 x 128 x 72 = 512 x 128.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets a status word and a CTA-wide abort
@@ -306,6 +306,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   constexpr bool kGroupScales = kW == kI4Tiled || kW == kI4Rows;
   constexpr uint32_t kParts = parts_of(kMath);
   constexpr bool kMulti = kForm == kSeveral, kMayGate = kForm == kGate;
+  static_assert(!kMulti || kMath == kInt8, "only sums that stay in tensor memory leave the drain warps time for another tile");
   const bool gated = kMayGate && p.swiglu != 0;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -325,7 +326,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   // hand-over costs about 390 clocks whatever it hands over (24 x 4096 -> 9472: 33 us with one chain of 32 columns each).
   const uint32_t acc_cols = p.nt <= 32 ? 32u : p.nt <= 64 ? 64u : p.nt <= 128 ? 128u : 256u, per_set = 256u / acc_cols;
 
-  // kMulti (int8 x int8): a cluster of one pair takes tiles (column pair, row tile, K slice) in turn, and while the drain warps store
+  // kMulti (int8 x int8): a cluster of one pair takes tiles (column pair, row tile) in turn, and while the drain warps store
   // a tile's outputs, copies, producers and MMAs are at work on the next (4096 x 2048 -> 8192, 512 tiles on 74 pairs: 111 us
   // with a cluster per tile, 76 so).  Elsewhere a cluster has one tile: with sums in the drain warps' registers there is
   // nobody to drain the next one meanwhile (333 x 1536 -> 17920 f32 60 | 66, 1948 x 11264 -> 3088 binary16 group 16 475 | 553).
@@ -397,12 +398,12 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     float* row_factor = reinterpret_cast<float*>(tail + kTailRows) + warp * cols;
     if (p.row_scale == nullptr)
       for (uint32_t c = lane; c < cols; c += 32u) row_factor[c] = 1.0f;
-    uint32_t set = 0, scale_batch = 0;  // accumulator sets and batches of scales so far, over all tiles
+    uint32_t set = 0;  // accumulator sets so far, over all tiles
     uint32_t tile = tile0;
     do {
     const Tile at_tile = kMulti ? tile_at(tile) : tile_first;
     const uint32_t m0 = at_tile.m0, ks_count = at_tile.ks_count;
-    // ---- a tile's columns [8 h, 8 h + 8) of this warp, at `from` in shared memory, to where they go ----
+    // ---- a tile's columns [8 h, 8 h + 8) of this warp, at `from` in shared memory, to where they go: emit_gate, emit_tile ----
     // (what belongs to this thread's channel, or to its channel of the gate and of up, is read once a tile)
     struct Channel { float bias, up_bias, ws, up_ws; };
     auto channel = [&]() {
@@ -424,58 +425,46 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       else if constexpr (kGroupScales) return fmaf(__uint_as_float(v), rs, bias);
       else return fmaf(__uint_as_float(v) * ws, rs, bias);
     };
-    auto emit = [&](uint32_t h, const Channel& ch, uint32_t from, uint32_t warp_bytes) {
+    // silu(gate) * up of parked sums: warps 0 and 1 of a column half hold gate rows, 2 and 3 the same rows of up; each takes
+    // half of the columns
+    auto emit_gate = [&](uint32_t h, const Channel& ch, uint32_t from, uint32_t warp_bytes) {
+      const uint32_t c0 = h * kOutCols, mm0 = m0 + col0 + c0;
+      const uint32_t row = at_tile.n0 + (quarter & 1u) * 32u + lane, first = (quarter >> 1) * (kOutCols / 2);
+      const uint32_t gate_at = from - (quarter >> 1) * 2u * warp_bytes, up_at = gate_at + 2u * warp_bytes;
+      const bool live = row < p.t[0].n;
+      float* dst = p.t[0].out + static_cast<size_t>(mm0 + first) * p.t[0].n + row;
+      float gate[kOutCols / 2], up[kOutCols / 2];
+#pragma unroll
+      for (uint32_t i = 0; i < kOutCols / 2; ++i) {
+        gate[i] = __uint_as_float(lds32(gate_at + (first + i) * 128u));
+        up[i] = __uint_as_float(lds32(up_at + (first + i) * 128u));
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < kOutCols / 2; ++i) {
+        const float rs = row_factor[c0 + first + i];
+        if constexpr (!kGroupScales) {
+          gate[i] *= ch.ws;
+          up[i] *= ch.up_ws;
+        }
+        gate[i] = silu_mul(fmaf(gate[i], rs, ch.bias), fmaf(up[i], rs, ch.up_bias));
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < kOutCols / 2; ++i, dst += p.t[0].n)
+        if (live && mm0 + first + i < p.m) *dst = gate[i];
+    };
+    // (kMulti: the loads of all columns first, one column at a time is one trip to shared memory after the other)
+    auto emit_tile = [&](uint32_t h, const Channel& ch, uint32_t from) {
       const uint32_t c0 = h * kOutCols, mm0 = m0 + col0 + c0;
       const ExTarget& tg = p.t[at_tile.wi];
-      if (gated) {
-        // warps 0 and 1 of a column half hold gate rows, 2 and 3 the same rows of up: each takes half of the columns
-        if (kMulti || h == 0) asm volatile("bar.sync %0, 128;" ::"r"(1u + half) : "memory");
-        const uint32_t row = at_tile.n0 + (quarter & 1u) * 32u + lane, first = (quarter >> 1) * (kOutCols / 2);
-        const uint32_t gate_at = from - (quarter >> 1) * 2u * warp_bytes, up_at = gate_at + 2u * warp_bytes;
-        const bool live = row < p.t[0].n;
-        float* dst = p.t[0].out + static_cast<size_t>(mm0 + first) * p.t[0].n + row;
-        float gate[kOutCols / 2], up[kOutCols / 2];
-#pragma unroll
-        for (uint32_t i = 0; i < kOutCols / 2; ++i) {
-          gate[i] = __uint_as_float(lds32(gate_at + (first + i) * 128u));
-          up[i] = __uint_as_float(lds32(up_at + (first + i) * 128u));
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < kOutCols / 2; ++i) {
-          const float rs = row_factor[c0 + first + i];
-          if constexpr (!kGroupScales) {
-            gate[i] *= ch.ws;
-            up[i] *= ch.up_ws;
-          }
-          gate[i] = silu_mul(fmaf(gate[i], rs, ch.bias), fmaf(up[i], rs, ch.up_bias));
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < kOutCols / 2; ++i, dst += p.t[0].n)
-          if (live && mm0 + first + i < p.m) *dst = gate[i];
-        if (kMulti) asm volatile("bar.sync %0, 128;" ::"r"(1u + half) : "memory");
-        return;
-      }
       const uint32_t row = at_tile.n0 + quarter * 32u + lane;  // this lane's output channel
       const bool row_live = row < tg.n;
-      const size_t first = static_cast<size_t>(mm0) * tg.n + row;
-      // (the loads of all columns first: one column at a time is one trip to shared memory after the other)
       uint32_t v[kOutCols];
-      float o[kOutCols], r[kOutCols];
 #pragma unroll
       for (uint32_t j = 0; j < kOutCols; ++j) v[j] = lds32(from + j * 128u);
-      const bool add = tg.residual != nullptr;
-#pragma unroll
-      for (uint32_t j = 0; j < kOutCols; ++j)
-        r[j] = add && row_live && mm0 + j < p.m ? tg.residual[first + static_cast<size_t>(j) * tg.n] : 0.0f;
-#pragma unroll
-      for (uint32_t j = 0; j < kOutCols; ++j) {
-        o[j] = finished(v[j], row_factor[c0 + j], ch.ws, ch.bias);
-        if (add) o[j] = __fadd_rn(o[j], r[j]);
-      }
-      float* dst = tg.out + first;
+      float* dst = tg.out + static_cast<size_t>(mm0) * tg.n + row;
 #pragma unroll
       for (uint32_t j = 0; j < kOutCols; ++j, dst += tg.n)
-        if (row_live && mm0 + j < p.m) *dst = o[j];
+        if (row_live && mm0 + j < p.m) *dst = finished(v[j], row_factor[c0 + j], ch.ws, ch.bias);
     };
     // the factors of this warp's activation rows, into its own words: the warps of a column half may be in different tiles
     if (p.row_scale != nullptr) {
@@ -486,9 +475,15 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     // parked sums: the same, all columns (without a gate column by column: 2 us less for 333 x 1536 -> 17920)
     auto emit_parked = [&]() {
       const Channel ch = channel();
-      if (kMulti || gated) {
+      if constexpr (kMulti) {
 #pragma unroll 1
-        for (uint32_t h = 0; h * kOutCols < cols; ++h) emit(h, ch, park + h * (kOutCols * 128u), cols * 128u);
+        for (uint32_t h = 0; h * kOutCols < cols; ++h) emit_tile(h, ch, park + h * (kOutCols * 128u));
+        return;
+      }
+      if (gated) {
+        asm volatile("bar.sync %0, 128;" ::"r"(1u + half) : "memory");  // all warps of the column half have parked
+#pragma unroll 1
+        for (uint32_t h = 0; h * kOutCols < cols; ++h) emit_gate(h, ch, park + h * (kOutCols * 128u), cols * 128u);
         return;
       }
       const ExTarget& tg = p.t[at_tile.wi];
@@ -534,7 +529,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           for (uint32_t hh = 0; hh < 2; ++hh) {
 #pragma unroll
             for (uint32_t j = 0; j < kOutCols; ++j) sts32(out_at + j * 128u, v[hh * kOutCols + j]);
-            emit(2 * b + hh, ch, out_at, kOutCols * 128u);
+            emit_tile(2 * b + hh, ch, out_at);
           }
         }
       } else {
@@ -566,7 +561,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           for (int j = 0; j < 16; ++j) acc[b][j] = 0.0f;
 #pragma unroll 1
         for (uint32_t d0 = 0; d0 < drains; d0 += per_set, ++set) {
-          const uint32_t batch = scale_batch + d0 / kScaleBatch, d_end = min(d0 + per_set, drains);  // a set lies inside a batch of scales
+          const uint32_t batch = d0 / kScaleBatch, d_end = min(d0 + per_set, drains);  // a set lies inside a batch of scales
           if constexpr (kGroupScales) {
             if (d0 % kScaleBatch == 0) wait_bounded(sfull + (batch & 1u) * 8, (batch >> 1) & 1u, abort_flag, p.status, 25);
           }
@@ -609,9 +604,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           arrive_if(leader, dempty_0 + (set & 1u) * 8);
-          if (kGroupScales) arrive_if(d_end % kScaleBatch == 0 || d_end == drains ? leader : 0u, sempty + (batch & 1u) * 8);
+          if (kGroupScales) arrive_if(d_end % kScaleBatch == 0 ? leader : 0u, sempty + (batch & 1u) * 8);
         }
-        scale_batch += (drains + kScaleBatch - 1) / kScaleBatch;
 #pragma unroll
         for (int b = 0; b < kBatches; ++b)
 #pragma unroll
@@ -885,9 +879,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       // for it (4,600 clocks per eight chains; 24 x 4096 -> 9472: 30 us).
       const uint32_t wl = (warp - kScaleWarp) * 32u + lane;
       uint32_t batch = 0;
-      uint32_t tile = tile0;
-      do {
-      const Tile at_tile = kMulti ? tile_at(tile) : tile_first;
+      const Tile at_tile = tile_first;  // (kMulti has no group scales)
       const uint32_t drains = (at_tile.ks_count * 4 + p.drain16 - 1) / p.drain16, drain0 = at_tile.ks_begin * 4 / p.drain16;
       if constexpr (kW == kI4Tiled) {
         // rows 16 (wl / 8) + wl % 8 and + 8: a chunk holds their scales of two groups side by side
@@ -960,7 +952,6 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
           load(d0 + kScaleBatch);
         }
       }
-      } while (kMulti && (tile += tile_step) < tiles_all);
     }
   }
 
@@ -979,7 +970,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
 // ---- f32 and bf16 activations -> parts ----------------------------------------------------------
 // One CTA per row.  [rms_norm ->] a power of two over the whole row -> parts that add up to the value: three
 // bf16 ones of an f32 value, the one of a bf16 value, or two binary16 ones (pow2_prescale); inv[row] = 2^-e
-// undoes the power in the epilogue.  A row is read once from memory and again from the cache.
+// undoes the power in the epilogue.
 //
 // bf16 parts have f32's exponents, so their power of two is only there to keep the sums of up to 1024 products
 // with integers, and those times a group scale, away from both ends of the range: the row's largest value goes
@@ -1283,8 +1274,8 @@ cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, const CUtensorM
     // (a decoder's prompt takes one kernel for all its matmuls: two that take turns cost it 6 us a layer in instructions
     // fetched again, 692 | 667 us for four layers of 333 rows)
     constexpr bool kPrompt = kW == kI4Tiled && parts_of(kMath) == 3;
-    if (kPrompt || p.swiglu) return launch_form<kW, kMath, kGate>(env, p, xm, wm);
-    else if constexpr (!kPrompt) return launch_form<kW, kMath, kPlain>(env, p, xm, wm);
+    if constexpr (kPrompt) return launch_form<kW, kMath, kGate>(env, p, xm, wm);
+    else return p.swiglu ? launch_form<kW, kMath, kGate>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
   }
 }
 
@@ -1524,9 +1515,10 @@ uint64_t align256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
 bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, uint64_t workspace_bytes) {
   if (count < 1 || count > kMaxMulti || m == 0) return false;
   const Weight& w0 = *targets[0].w;
-  // Tiled layouts have GEMVs of their own up to 16 rows.  The untiled ones only have the generic kernel
-  // (one warp per channel), which is faster while the launch is: 13.5 us for anything up to 1 x 4096 ->
-  // 1000, then 26 us for 1 x 4096 -> 4096 int4 (here 22) or 35 us int8 (here 19), and 242 us at 16 rows (here 25).
+  // Tiled layouts have GEMVs of their own up to 16 rows.  A single untiled weight has kq_qgemv_rows.cu, whose line to this
+  // kernel is drawn there; several of them (q|k|v), and rows that it does not hold, come here from the amount of work on
+  // at which the generic kernel (one warp per channel) is behind: 13.5 us for anything up to 1 x 4096 -> 1000, then
+  // 26 us for 1 x 4096 -> 4096 int4 (here 22) or 35 us int8 (here 19), and 242 us at 16 rows (here 25).
   uint64_t work = 0;
   for (int i = 0; i < count; ++i) work += static_cast<uint64_t>(m) * targets[i].w->n * w0.k;
   if (w0.layout != kLayoutNative ? m <= 16 : work < (w0.storage == KQ_STORAGE_I4 ? 12u << 20 : 8u << 20)) return false;
