@@ -28,6 +28,30 @@ __device__ __forceinline__ float dequant_i8(int q, float scale) {
   return __fmul_rn(static_cast<float>(q), scale);
 }
 
+// ---- packed integers -> binary16, exact ------------------------------------------
+// Nibbles u of a word as pairs (k, k + 4), k = 0..3, of u - 8.  (w & 0x000F000F) | 0x6400.. is the pair 1024 + u of
+// nibbles 0 and 4; (w & 0x00F000F0) | 0x6400.. the pair 1024 + 16 u of nibbles 1 and 5, brought down by one exact fused
+// multiply-add.
+__device__ __forceinline__ void nibble_pairs(uint32_t w, __half2 (&h)[4]) {
+  const __half2 k1032 = __half2half2(__ushort_as_half(0x6408)), k16th = __half2half2(__ushort_as_half(0x2C00)),
+                km72 = __half2half2(__ushort_as_half(0xD480));
+  const uint32_t w8 = w >> 8;
+  const uint32_t r[4] = {(w & 0x000F000Fu) | 0x64006400u, (w & 0x00F000F0u) | 0x64006400u, (w8 & 0x000F000Fu) | 0x64006400u,
+                         (w8 & 0x00F000F0u) | 0x64006400u};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 v = *reinterpret_cast<const __half2*>(&r[i]);
+    h[i] = (i & 1) ? __hfma2(v, k16th, km72) : __hsub2(v, k1032);
+  }
+}
+// Bytes q + 128 of a word as pairs (k, k + 1) of q: a byte under the exponent of 1024 is 1024 + byte.
+__device__ __forceinline__ void byte_pairs(uint32_t w, __half2 (&h)[2]) {
+  const __half2 k1152 = __half2half2(__ushort_as_half(0x6480));
+  const uint32_t r[2] = {__byte_perm(w, 0x64646464u, 0x4140), __byte_perm(w, 0x64646464u, 0x4342)};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) h[i] = __hsub2(*reinterpret_cast<const __half2*>(&r[i]), k1152);
+}
+
 // Companion scale -> f32.  binary16 widens exactly, subnormals included
 // (packages/runtime/src/format/f16.ts:23-36); the build never enables flush-to-zero.
 template <bool kF16>

@@ -128,22 +128,13 @@ __device__ __forceinline__ float load_scale_dyn(const void* base, size_t index, 
 // ---- integers -> binary16 or bf16 ------------------------------------------------------------
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) { return (a & mask) | bits; }
 
-// 8 nibbles u (k ascending) -> 8 binary16 values u - 8, exact.  (w & 0x000F000F) | 0x6400.. is
-// the pair 1024 + u of nibbles 0 and 4; (w & 0x00F000F0) | 0x6400.. the pair 1024 + 16 u of
-// nibbles 1 and 5, brought down by one exact fused multiply-add.
+// 8 nibbles u (k ascending) -> 8 binary16 values u - 8, exact.
 __device__ __forceinline__ uint4 nibbles_to_half(uint32_t w) {
-  const __half2 k1032 = __half2half2(__ushort_as_half(0x6408)), k16th = __half2half2(__ushort_as_half(0x2C00)),
-                km72 = __half2half2(__ushort_as_half(0xD480));
-  const uint32_t w8 = w >> 8;
-  uint32_t r[4] = {and_or(w, 0x000F000Fu, 0x64006400u), and_or(w, 0x00F000F0u, 0x64006400u),
-                   and_or(w8, 0x000F000Fu, 0x64006400u), and_or(w8, 0x00F000F0u, 0x64006400u)};
   __half2 h[4];
+  nibble_pairs(w, h);
+  uint32_t r[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __half2 v = *reinterpret_cast<const __half2*>(&r[i]);
-    h[i] = (i & 1) ? __hfma2(v, k16th, km72) : __hsub2(v, k1032);
-    r[i] = *reinterpret_cast<const uint32_t*>(&h[i]);
-  }
+  for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const uint32_t*>(&h[i]);
   return make_uint4(__byte_perm(r[0], r[1], 0x5410), __byte_perm(r[2], r[3], 0x5410), __byte_perm(r[0], r[1], 0x7632),
                     __byte_perm(r[2], r[3], 0x7632));
 }
@@ -167,12 +158,11 @@ __device__ __forceinline__ uint4 nibbles_to_operand(uint32_t w) {
   else return nibbles_to_half(w);
 }
 
-// 4 bytes q + 128 -> 4 binary16 values q, exact: a byte under the exponent of 1024 is 1024 + byte.
+// 4 bytes q + 128 -> 4 binary16 values q, exact.
 __device__ __forceinline__ uint2 bytes_to_half(uint32_t w) {
-  const __half2 k1152 = __half2half2(__ushort_as_half(0x6480));
-  uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
-  const __half2 ha = __hsub2(*reinterpret_cast<const __half2*>(&a), k1152), hb = __hsub2(*reinterpret_cast<const __half2*>(&b), k1152);
-  return make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
+  __half2 h[2];
+  byte_pairs(w, h);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&h[0]), *reinterpret_cast<const uint32_t*>(&h[1]));
 }
 // ... -> 4 bf16 values q, exact.  With b = q + 128 under the exponent of 128 the seven low bits of b read as
 // 128 + (b & 127); the top bit, which would reach into the exponent, is taken out and says what to subtract:

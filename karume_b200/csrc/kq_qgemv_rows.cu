@@ -46,29 +46,23 @@ __device__ __forceinline__ uint4 rows_ldg(const uint8_t* p) {
   return v;
 }
 
-// Eight nibbles u (k ascending) -> u - 8: pairs 1024 + u and 1024 + 16 u as binary16, brought down exactly.
+// The weights of a word as f32, k ascending.
 __device__ __forceinline__ void rows_nibbles(uint32_t w, float (&v)[8]) {
-  const __half2 k1032 = __half2half2(__ushort_as_half(0x6408)), k16th = __half2half2(__ushort_as_half(0x2C00)),
-                km72 = __half2half2(__ushort_as_half(0xD480));
-  const uint32_t w8 = w >> 8;
-  const uint32_t r[4] = {(w & 0x000F000Fu) | 0x64006400u, (w & 0x00F000F0u) | 0x64006400u, (w8 & 0x000F000Fu) | 0x64006400u,
-                         (w8 & 0x00F000F0u) | 0x64006400u};
+  __half2 h[4];
+  nibble_pairs(w, h);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const __half2 p = *reinterpret_cast<const __half2*>(&r[i]);
-    const float2 f = __half22float2((i & 1) ? __hfma2(p, k16th, km72) : __hsub2(p, k1032));
+    const float2 f = __half22float2(h[i]);
     v[i] = f.x;
     v[i + 4] = f.y;
   }
 }
-// Four bytes -> int8 values: a byte with its sign flipped, under the exponent of 1024, is 1024 + 128 + q.
 __device__ __forceinline__ void rows_bytes(uint32_t w, float* v) {
-  const __half2 k1152 = __half2half2(__ushort_as_half(0x6480));
-  const uint32_t u = w ^ 0x80808080u;
-  const uint32_t r[2] = {__byte_perm(u, 0x64646464u, 0x4140), __byte_perm(u, 0x64646464u, 0x4342)};
+  __half2 h[2];
+  byte_pairs(w ^ 0x80808080u, h);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const float2 f = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&r[i]), k1152));
+    const float2 f = __half22float2(h[i]);
     v[2 * i] = f.x;
     v[2 * i + 1] = f.y;
   }
