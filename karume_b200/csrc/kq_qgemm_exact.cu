@@ -58,6 +58,7 @@
 #include <type_traits>
 
 #include "kq_common.cuh"
+#include "kq_exact_geometry.h"
 #include "kq_gemv_core.cuh"
 #include "kq_internal.h"
 #include "kq_umma.cuh"
@@ -66,18 +67,15 @@ namespace kq {
 namespace {
 
 using namespace umma;
+using namespace exact;
 
 enum WeightKind : int { kI4Tiled = 0, kI4Rows = 1, kI8Tiled = 2, kI8Rows = 3 };
-// one binary16 part or two, one bf16 part or three, or int8 x int8
-enum MathKind : int { kHalf1, kHalf2, kBf1, kBf3, kInt8 };
 template <int kMath>
 constexpr bool kIsBf = kMath == kBf1 || kMath == kBf3;
-__host__ __device__ constexpr uint32_t parts_of(int math) { return math == kBf3 ? 3u : math == kHalf2 ? 2u : 1u; }
 
 constexpr int kDrainWarps = 8, kProdWarps = 4, kCopyWarp = 12, kMmaWarp = 13, kScaleWarp = 14, kExThreads = 512;
 constexpr uint32_t kRows = 128;                 // output channels per CTA
 constexpr uint32_t kATile = kRows * 128;        // 16 KB: 128 rows x 128 bytes of k
-constexpr uint32_t kMaxNT = 256;                // activation rows per tile
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kSmemLimit = 227 * 1024;
 constexpr uint32_t kScaleBatch = 8;             // accumulator chains per slot of the scale ring (two slots)
@@ -86,7 +84,6 @@ constexpr uint32_t kTailScales = 320, kTailRows = kTailScales + 2 * kScaleBatch 
 // barriers, the scale ring, each drain warp's row factors; where a pair takes several tiles, finished sums on their way out
 __host__ __device__ constexpr uint32_t tail_out(uint32_t nt) { return kTailRows + kDrainWarps * nt / 2 * 4; }
 __host__ __device__ constexpr uint32_t smem_tail(bool multi, uint32_t nt) { return tail_out(nt) + (multi ? kDrainWarps * kOutCols * 128 : 0); }
-constexpr uint32_t kMaxClusterSplits = 4;       // K slices that meet in a cluster: two or four (eight CTAs, the portable most)
 constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
 
 struct ExTarget {
@@ -1316,84 +1313,6 @@ cudaError_t launch_math(int math, const LaunchEnv& env, const ExParams& p, const
   return cudaErrorInvalidValue;
 }
 
-// Clocks of one k-step, from the difference between k = 4,096 and 8,192 with 74 pairs at work (18,944 channels, one
-// tile each; at 1.92 GHz).  The conversion of the weights does not grow with the tile, its copy and the MMAs do; a
-// drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step; the two or three
-// parts of f32 rows cost what their tiles take to arrive, and above 192 rows the power cap.
-// Measured at nt = 32, 64, 96, 128, 160, 192, 224, 256:
-//   int4, group 32   binary16 683, 798, 905, 1,048, 1,275, 1,450, 1,660, 1,750; f32 900, 1,200, 1,320, 1,510, 1,810,
-//                    1,960, 2,370, 2,940
-//   int8, tiled      binary16 535, 632, 632, 711, 764, 836, 950, 1,020 to 1,190; f32 780, 870, 890, 1,110, 1,290, 1,450,
-//                    1,600, 2,070
-//   int8, rows       (k = 4,096 to 12,288, 6 pairs; 32, 64, 128, 192, 256) binary16 625, 700, 835, 890, 985; f32 1,110, 1,325,
-//                    1,415, 1,580, 1,675 (bytes take 9 instructions for four bf16 integers, 4 for binary16)
-uint32_t kstep_clocks(uint32_t nt, int math, uint32_t drains_x4, bool int8_weights) {
-  const bool int8 = math == kInt8, bytes_to_bf = int8_weights && (math == kBf1 || math == kBf3);
-  const uint32_t parts = parts_of(math);
-  const uint32_t mma = 4 * parts * std::max(nt / 2, 48u);
-  const uint32_t step = int8 ? 650 + nt : 450 + (bytes_to_bf ? 200 : 0) + 100 * parts + nt + drains_x4 * (nt * 8 / 5 + 20) / 4;
-  const uint32_t fill = parts == 3 ? (nt > 192 ? nt * 10 : 740 + nt * 28 / 5) : parts == 2 ? 640 + nt * 21 / 5 : 0;
-  const uint32_t drain = int8 ? 0u : drains_x4 * std::max(nt * 7 / 2 + 60, 330u) / 4;
-  return std::max({mma, step, fill, drain});
-}
-
-struct Geometry { uint32_t nt, m_tiles, splits, cluster_splits; };
-// Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
-// loads, epilogue) plus its k-steps.  Two or four slices may meet in a cluster: no second launch and no partial sums in
-// memory, but 33 clusters of two pairs and 15 of four are all the device holds (74 pairs by themselves), and they start
-// later.  Other slices add the reduce launch and the partial sums, written and read at 2,200 bytes per clock.
-//   (us, with its split launch; reduce launch | cluster)  65 x 1152 -> 3072 group 16, four slices 16.0 | 13.8;
-//   300 x 4096 -> 4096 int8 binary16, two 29.0 | 22.8; 100 x 2048 -> 2048 group 128, four 18.2 | 15.4;
-//   333 x 8960 -> 1536, four, 72 tiles of 128 rows 45.4, 48 of 192 rows 49.3 | 46.6
-// Widths between the powers of two: 804 x 4096 -> 6144 f32 at 160 rows 117, 128 152, 192 123, 256 148.
-Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, uint32_t ksteps, int math, bool int8_weights, uint32_t drain16,
-                         uint32_t slice_unit, bool may_split, const uint32_t (&slots)[kMaxClusterSplits + 1], uint64_t partial_room) {
-  Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1, 1};
-  uint64_t best_cost = ~0ull;
-  const uint32_t drains_x4 = std::max(1u, 16 / drain16);  // accumulator chains per k-step, times four
-  const uint32_t most = (m + 31) / 32;
-  for (uint32_t mt = (m + kMaxNT - 1) / kMaxNT; mt <= most; ++mt) {
-    uint32_t nt = ((m + mt - 1) / mt + 31) / 32 * 32;
-    if ((m + nt - 1) / nt != mt) continue;
-    const uint32_t per = kstep_clocks(nt, math, drains_x4, int8_weights);
-    for (uint32_t splits = 1; splits <= (may_split ? 16u : 1u); splits *= 2) {
-      if (splits > 1 && ksteps / splits < 4) break;
-      uint32_t each = (ksteps + splits - 1) / splits;
-      each = (each + slice_unit - 1) / slice_unit * slice_unit;
-      for (uint32_t in_cluster = 0; in_cluster < 2; ++in_cluster) {
-        if (in_cluster != 0 ? splits == 1 || splits > kMaxClusterSplits || slots[splits] == 0 || (ksteps + each - 1) / each != splits
-                            : splits > 1 && static_cast<uint64_t>(splits) * m * n_total * 4 > partial_room)
-          continue;
-        const uint32_t room = in_cluster != 0 ? slots[splits] * splits : slots[1];
-        const uint64_t waves = (static_cast<uint64_t>(pairs) * mt * splits + room - 1) / room;
-        uint64_t cost = waves * (5000 + nt * 30 + static_cast<uint64_t>(each) * per + (in_cluster != 0 ? 750 * splits : 0));
-        if (splits > 1 && in_cluster == 0) cost += 5500 + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
-        if (cost < best_cost) {
-          best_cost = cost;
-          best = {nt, mt, splits, in_cluster != 0 ? splits : 1u};
-        }
-      }
-    }
-    if (mt >= 8 * slots[1]) break;
-  }
-  return best;
-}
-
-// Most k of an accumulator chain.  Each of a chain's accumulations truncates (half a unit of 2^-24 on average, all the
-// same way), while the sums of the drain round to nearest.  Relative error against f64 (2-norm, k = 4,096), and us for
-// 300 x 4096 -> 4090 int8, with chains of 64, 128, 256 and 1,024:
-//   f32, three parts        1.3, 2.7, 6.0, 26e-7   50, 47, 46, 46
-//   f32, two parts (tiled)  1.7, 2.5, 4.8, 21e-7   (1024 x 4096 -> 4096) 68, 63, 61.5, 60
-//   binary16, int8 weights  1.6, 1.5, 2.3, 9.7e-7  32, 30, 29, 29
-//   bf16, int8 weights      1.1, 1.0, 1.1, 3.3e-7  44, 42, 41, 40
-//   binary16, int4 weights  1.5, 1.1, 0.9, 2.1e-7  (300 x 8192 -> 4000) 52, 47, 45, 43
-// An f32 multiply-add per weight is 2.1e-7 from f64 there, the int8 GEMV 8 to 13e-7: each is kept below the path it
-// stands in for.
-uint32_t chain_of(int math, const Weight& w) {
-  if (math == kBf3) return 64;
-  return math == kHalf1 && w.storage == KQ_STORAGE_I8 ? 128 : 256;
-}
-
 // x: binary16 (kHalf1), parts already split (kHalf2 / kBf1 / kBf3) or int8 (kInt8).
 cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const float* residual, const void* x, int math,
                       uint32_t m, uint32_t max_chain, const float* row_scale, void* scratch, uint64_t scratch_bytes, bool may_split, bool swiglu, int* launches) {
@@ -1431,13 +1350,12 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   p.swiglu = swiglu ? 1 : 0;
   p.m = m;
   p.k = w0.k;
-  const uint32_t step_k = int8 ? 128 : 64;
-  p.ksteps = (w0.k + step_k - 1) / step_k;
   p.scale_f16 = w0.scale_dtype == KQ_F16;
   const bool i4 = kind == kI4Tiled || kind == kI4Rows;
-  const uint32_t group = i4 ? w0.group_size : max_chain;
-  const uint32_t chain = std::min(group, max_chain);
-  p.drain16 = chain / 16;
+  const Steps steps = steps_of(w0.k, math, i4 ? w0.group_size : 0, max_chain);
+  const uint32_t group = i4 ? w0.group_size : max_chain, chain = steps.drain16 * 16;
+  p.ksteps = steps.ksteps;
+  p.drain16 = steps.drain16;
   p.drains_per_group_shift = 0;
   while ((chain << p.drains_per_group_shift) < group) ++p.drains_per_group_shift;
   p.groups = i4 ? w0.k / w0.group_size : ~0u;
@@ -1446,17 +1364,15 @@ cudaError_t run_exact(const LaunchEnv& env, int count, const LinearTarget* targe
   p.status = env.status;
   p.partial = static_cast<float*>(scratch);
   const uint32_t parts = parts_of(math);
-  // a K slice is a whole number of int4 accumulator chains (an int8 chain may end anywhere)
-  const uint32_t align = i4 && p.drain16 > 4 ? p.drain16 / 4 : 1;
   uint32_t slots[kMaxClusterSplits + 1];
   cudaError_t ce = resident_pairs(env, slots);
   if (ce != cudaSuccess) return ce;
-  const Geometry geo = choose_geometry(m, n_total, pairs, p.ksteps, math, !i4, p.drain16, align, may_split && !swiglu, slots,
+  const Geometry geo = choose_geometry(m, n_total, pairs, steps, math, !i4, may_split && !swiglu, slots,
                                        scratch != nullptr ? scratch_bytes : 0);
   p.nt = geo.nt;
   p.pairs = pairs;
   p.m_tiles = geo.m_tiles;
-  p.ksteps_per_split = ((p.ksteps + geo.splits - 1) / geo.splits + align - 1) / align * align;
+  p.ksteps_per_split = ((p.ksteps + geo.splits - 1) / geo.splits + steps.slice_unit - 1) / steps.slice_unit * steps.slice_unit;
   p.splits = (p.ksteps + p.ksteps_per_split - 1) / p.ksteps_per_split;
   p.cluster_splits = geo.cluster_splits;
   p.multi = int8 && p.splits == 1 && static_cast<uint64_t>(pairs) * geo.m_tiles > slots[1];
@@ -1556,7 +1472,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
     const uint8_t* xp = static_cast<const uint8_t*>(x) + static_cast<size_t>(r0) * k * xb;
     cudaError_t e;
     if (direct) {
-      e = run_exact(env, count, t, residual, xp, math, pm, chain_of(math, w0), nullptr, ws, room, true, swiglu, launches);
+      e = run_exact(env, count, t, residual, xp, math, pm, chain_of(math, w0.storage == KQ_STORAGE_I8), nullptr, ws, room, true, swiglu, launches);
     } else {
       float* inv = reinterpret_cast<float*>(ws);
       uint16_t* parts = reinterpret_cast<uint16_t*>(ws + align256(static_cast<uint64_t>(pm) * 4));
@@ -1578,7 +1494,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
       else e = split(reinterpret_cast<const float*>(xp), std::integral_constant<int, kHalf2>{});
       if (e != cudaSuccess) return e;
       if (launches) *launches += 1;
-      e = run_exact(env, count, t, residual, parts, math, pm, chain_of(math, w0), inv, ws + taken, room - taken, true, swiglu, launches);
+      e = run_exact(env, count, t, residual, parts, math, pm, chain_of(math, w0.storage == KQ_STORAGE_I8), inv, ws + taken, room - taken, true, swiglu, launches);
     }
     if (e != cudaSuccess) return e;
   }

@@ -135,3 +135,16 @@ def synth_i8(n, k, seed=0):
     s = (np.abs(rng.standard_normal(n).astype(np.float32)) * np.float32(0.02 / 127)).astype(np.float16)
     s[s == 0] = np.float16(6e-8)
     return q, s
+
+
+# ---- shapes of the many-row kernel by the form they take (tests/test_exact_geometry.py holds them to it) ----
+
+# (activations, storage, group, m, n, k, rows a tile, K slices that meet in a cluster); "i8": the integer-dot form
+EXACT_SLICED = [("f16", "i4", 16, 65, 6240, 576, 96, 2), ("f16", "i4", 32, 385, 1040, 1728, 160, 4), ("f32", "i4", 32, 681, 272, 1728, 128, 4),
+                ("f32", "i4", 32, 135, 6224, 832, 160, 2), ("f32", "i4", 32, 195, 2880, 2496, 224, 4), ("f32", "i8", 0, 203, 2848, 1984, 224, 4),
+                ("f16", "i8", 0, 521, 848, 2496, 192, 4), ("f16", "i8", 0, 494, 1296, 3520, 256, 4),
+                ("i8", "i8", 0, 26, 64, 1344, 32, 2), ("i8", "i8", 0, 531, 272, 2368, 96, 4), ("i8", "i8", 0, 135, 2848, 3456, 160, 4),
+                ("i8", "i8", 0, 168, 4176, 3200, 192, 2)]
+# (m, n, k) of int8 x int8 calls with more tiles than the device holds pairs: one and several row tiles, the last one ragged,
+# tiled and row-major weights, one k-step and more than the pipeline has stages
+EXACT_RESIDENT = [(300, 9488, 128), (250, 19008, 160), (520, 9481, 400), (777, 5003, 1168), (1000, 8192, 1056)]

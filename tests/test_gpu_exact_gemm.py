@@ -95,8 +95,7 @@ def test_integer_dot_is_bit_exact(gpu, storage, group, m, n, k):
     w.free()
 
 
-# K slices that meet in a cluster (two or four, the last one short), next to ragged channels and rows, and tiles of 160 and
-# 224 rows
+# K slices that meet in a cluster (two or four, the last one short), next to ragged channels and rows, on tiles of 32 and 64 rows
 @pytest.mark.parametrize("xdt", ["f32", "f16"])
 @pytest.mark.parametrize("storage,group,m,n,k", [("i4", 32, 20, 272, 576), ("i4", 16, 33, 100, 1152), ("i4", 128, 97, 513, 1408),
                                                  ("i4", 32, 160, 1040, 1088), ("i4", 32, 223, 528, 960), ("i8", 0, 50, 300, 1616),
@@ -116,8 +115,137 @@ def test_integer_sums_that_meet_in_a_cluster(gpu, m, n, k):
     test_integer_dot_is_bit_exact(gpu, "i8", 0, m, n, k)
 
 
-# The gate in the matmul's epilogue (its tiles fill half of the device) and several tiles to a CTA pair: ragged rows and
-# channels, every storage; out on top of x takes the separate kernels
+# ... and on tiles of 32 to 256 rows; no launch adds the slices
+@pytest.mark.parametrize("xdt,storage,group,m,n,k,nt,slices", [s for s in cases.EXACT_SLICED if s[0] != "i8"])
+def test_slices_of_wide_tiles_meet_in_a_cluster(gpu, xdt, storage, group, m, n, k, nt, slices):
+    before = gpu.launch_count
+    test_matches_the_f64_oracle(gpu, xdt, storage, group, m, n, k)
+    repacked = 1 if group in (0, 32) and n % 16 == 0 and k % (32 if storage == "i8" else 64) == 0 else 0
+    assert gpu.launch_count - before - repacked == 2 * (1 if xdt == "f16" else 2)
+
+
+def test_residual_and_several_weights_of_slices_in_a_cluster(gpu):
+    import torch
+    rng = np.random.default_rng(5)
+    xdt, storage, group, m, n, k, _, _ = cases.EXACT_SLICED[3]
+    x, res = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    norm, bias = (1 + 0.1 * rng.standard_normal(k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    data, scale = cases.synth_i4(n, k, seed=n)
+    w = gpu.upload_weight(storage, data, scale, (n, k), group)
+    out = dev(res)  # the residual is the output buffer
+    before = gpu.launch_count
+    gpu.linear_fused(dev(x), [w], [dev(bias)], [out], norm_weight=dev(norm), eps=1e-5, residual=out)
+    gpu.sync()
+    assert gpu.launch_count - before == 2
+    want = oracle.add(oracle.linear_i4(oracle.rms_norm(x, norm, 1e-5), data, scale.astype(np.float32), bias, n, k, group), res)
+    rep = oracle.allclose(out.cpu().numpy(), want, atol=1e-5 * float(np.sqrt(np.mean(want.astype(np.float64) ** 2))), rtol=1e-4)
+    assert rep["pass"], rep
+    w.free()
+    # 512, 256 and 272 channels are the column pairs of the 1,040 of this case
+    xdt, storage, group, m, n, k, _, _ = cases.EXACT_SLICED[1]
+    x = oracle.round_to_f16(rng.standard_normal((m, k)).astype(np.float32))
+    ws, biases, wants = [], [], []
+    for each in (512, 256, n - 768):
+        data, scale = cases.synth_i4(each, k, seed=each)
+        ws.append(gpu.upload_weight(storage, data, scale, (each, k), group))
+        biases.append(rng.standard_normal(each).astype(np.float32))
+        wants.append(oracle.linear_i4(x, data, scale.astype(np.float32), biases[-1], each, k, group))
+    before = gpu.launch_count
+    outs = gpu.linear_multi(dev(x).to(torch.float16), ws, [dev(b) for b in biases])
+    gpu.sync()
+    assert gpu.launch_count - before == 1
+    for got, want in zip(outs, wants):
+        rep = oracle.allclose(got.cpu().numpy(), want, atol=1e-5 * max(1.0, float(np.sqrt(np.mean(want.astype(np.float64) ** 2)))), rtol=1e-4)
+        assert rep["pass"], rep
+    for w in ws:
+        w.free()
+
+
+@pytest.mark.parametrize("m,n,k,nt,slices", [s[3:] for s in cases.EXACT_SLICED if s[0] == "i8"])
+def test_integer_sums_of_wide_tiles_meet_in_a_cluster(gpu, m, n, k, nt, slices):
+    before = gpu.launch_count
+    test_integer_dot_is_bit_exact(gpu, "i8", 0, m, n, k)
+    assert gpu.launch_count - before == 3  # the weight's repacking, the quantiser, the matmul
+
+
+# A resident pair takes several tiles in turn: bit for bit on every channel of the rows at the edges of the row tiles (of the
+# multiples of 32 that they may have)
+@pytest.mark.parametrize("m,n,k", cases.EXACT_RESIDENT)
+def test_several_tiles_to_a_pair_are_bit_exact(gpu, m, n, k):
+    rng = np.random.default_rng(m)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    data, scale = cases.synth_i8(n, k, seed=n)
+    rows = sorted({r for edge in range(0, m + 32, 32) for r in (edge - 1, edge) if 0 <= r < m} | {m - 1})
+    want = np.asarray(oracle.linear_w8a8(x[rows], data, scale.astype(np.float32), bias), np.float32)
+    w = gpu.upload_weight("i8", data, scale, (n, k), 0)
+    xq, xs = gpu.quantize_rows(dev(x))
+    outs = [gpu.linear_a8(xq, xs, w, dev(bias)) for _ in range(2)]
+    gpu.sync()
+    got = outs[0].cpu().numpy()
+    assert np.array_equal(got[rows].view(np.uint32), want.view(np.uint32))
+    assert np.array_equal(got.view(np.uint32), outs[1].cpu().numpy().view(np.uint32))
+    w.free()
+
+
+def test_every_form_behind_the_other_in_a_recording(gpu):
+    """Launches that overlap (each starts while the one before ends) replay with the bits of the same calls one at a time: a
+    gated pair, slices in a cluster that read its output, several tiles to a pair, and few rows over row-major weights."""
+    import torch
+    rng = np.random.default_rng(9)
+    m, k, n, n8 = 300, 256, 4752, 9488
+    gate, up = (gpu.upload_weight("i4", *cases.synth_i4(n, k, seed=s), (n, k), 32) for s in (1, 2))
+    w8 = gpu.upload_weight("i8", *cases.synth_i8(n8, n, seed=3), (n8, n), 0)
+    down = gpu.upload_weight("i4", *cases.synth_i4(1056, n, seed=4, group_size=16), (1056, n), 16)
+    few = gpu.upload_weight("i4", *cases.synth_i4(4097, 1056, seed=5, group_size=16), (4097, 1056), 16)
+    x, norm = dev(rng.standard_normal((m, k)).astype(np.float32)), dev((1 + 0.1 * rng.standard_normal(k)).astype(np.float32))
+    zero = torch.zeros(16384, device="cuda")
+    xq, xs = gpu.quantize_rows(dev(rng.standard_normal((m, n)).astype(np.float32)))
+    gpu.sync()
+
+    def step(into, fence):
+        act, y, z, last = into
+        gpu.linear_fused(x, [gate, up], [zero[:n], zero[:n]], [act], norm_weight=norm, eps=1e-5, swiglu=True)
+        fence()
+        gpu.linear(act, down, zero[:1056], out=y)
+        fence()
+        gpu.linear_a8(xq, xs, w8, zero[:n8], out=z)
+        fence()
+        gpu.linear(y[:3], few, zero[:4097], out=last)
+        fence()
+
+    def outputs():
+        return [torch.zeros(s, device="cuda") for s in ((m, n), (m, 1056), (m, n8), (3, 4097))]
+
+    stream = torch.cuda.Stream()
+    gpu.use_stream(stream)
+    gpu.set_overlap(True)
+    try:
+        with torch.cuda.stream(stream):
+            want, got = outputs(), outputs()
+            torch.cuda.synchronize()
+            step(want, gpu.sync)
+            step(got, lambda: None)
+            gpu.sync()
+            assert all(torch.equal(a, b) for a, b in zip(want, got))
+            gpu.graph_begin()
+            step(got, lambda: None)
+            g = gpu.graph_end()
+            for _ in range(3):
+                for t in got:
+                    t.zero_()
+                gpu.graph_launch(g)
+                gpu.sync()
+                assert all(torch.equal(a, b) for a, b in zip(want, got))
+            gpu.graph_free(g)
+    finally:
+        gpu.use_stream(torch.cuda.current_stream())
+    for w in (gate, up, w8, down, few):
+        w.free()
+
+
+# The gate in the matmul's epilogue (its tiles fill half of the device): ragged rows and channels, every storage; out on top
+# of x takes the separate kernels
 @pytest.mark.parametrize("storage,group,xdt,m,n,k", [("i4", 32, "f32", 513, 2416, 128), ("i4", 32, "f16", 300, 4752, 64), ("i4", 16, "f32", 270, 2401, 96),
                                                      ("i8", 0, "f32", 257, 4736, 96), ("i8", 0, "f16", 800, 2440, 80), ("i4", 64, "bf16", 1030, 3333, 192)])
 def test_gate_in_the_epilogue(gpu, storage, group, xdt, m, n, k):
