@@ -286,8 +286,10 @@ KQ_API int kq_add(kq_ctx* ctx, uint64_t a_dptr, uint64_t b_dptr, uint64_t out_dp
  *                     outputs are added across the connected ranks (as kq_linear_reduce), then
  *                     the bias and the residual are added, the same bits on every rank
  *   residual_dptr     0, or f32 [m, n] (count == 1); may be the same buffer as out_dptr[0]
- * out must not alias x.  Called directly it runs as separate kernels (norm, linears, gate or
- * add).  Recorded into a fused plan (kq_plan_begin .. kq_plan_end) the persistent kernel does
+ * out must not alias x.  Called directly, up to sixteen rows on tiled int4 weights are one launch; one
+ * row-major weight at few rows takes the norm and the residual into its launch, the many-row kernel the norm
+ * into the launch that converts x and the residual, or the gate where its tiles fill half of the device, into
+ * its epilogue; anything else runs as separate kernels (norm, linears, gate or add).  Recorded into a fused plan (kq_plan_begin .. kq_plan_end) the persistent kernel does
  * the norm while it stages the activations and the gate / exchange / residual in the epilogue
  * of the matmul, so gate and up never travel through HBM; that needs the plan's paired kernel
  * (at most two f32 / bf16 rows or four binary16 rows, n a multiple of 32 except for the gate

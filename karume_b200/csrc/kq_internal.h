@@ -76,11 +76,12 @@ struct LaunchEnv {
   const float* residual = nullptr;
 };
 
-// Generic kernels: any shape the storage contract allows, native layout.
-// Up to sixteen rows over row-major packed weights (kq_qgemv_rows.cu).
+// Up to sixteen rows over row-major packed weights (kq_qgemv_rows.cu); env.norm_weight (f32 activations) and env.residual
+// are applied.
 bool qgemv_rows_supports(const Weight& w, uint32_t m);
 bool qgemv_rows_preferred(const Weight& w, uint32_t m);
 cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const void* x, int x_dtype, uint32_t m);
+// Generic kernels: any shape the storage contract allows, native layout.
 cudaError_t launch_linear_generic(const LaunchEnv& env, const Weight& w, const void* x, int x_dtype,
                                   const float* bias, float* out, uint32_t m);
 cudaError_t launch_dequant(const LaunchEnv& env, const Weight& w, float* out);
