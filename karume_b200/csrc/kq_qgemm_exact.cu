@@ -81,9 +81,11 @@ constexpr uint32_t kSmemLimit = 227 * 1024;
 constexpr uint32_t kScaleBatch = 8;             // accumulator chains per slot of the scale ring (two slots)
 constexpr uint32_t kOutCols = 8;                // columns a drain warp hands to its epilogue at a time
 constexpr uint32_t kTailScales = 320, kTailRows = kTailScales + 2 * kScaleBatch * kRows * 4;
-// barriers, the scale ring, each drain warp's row factors; where a pair takes several tiles, finished sums on their way out
+// Barriers, the scale ring, the row factors; where a pair takes several tiles each drain warp has row factors of its own
+// (the warps of a column half may be in different tiles), and finished sums on their way out.  (A copy for each warp in
+// every form cost binary16 tiles of 256 rows one of six stages: 1225 x 2816 -> 7424 group 128 69.7 us, 65.1 without.)
 __host__ __device__ constexpr uint32_t tail_out(uint32_t nt) { return kTailRows + kDrainWarps * nt / 2 * 4; }
-__host__ __device__ constexpr uint32_t smem_tail(bool multi, uint32_t nt) { return tail_out(nt) + (multi ? kDrainWarps * kOutCols * 128 : 0); }
+__host__ __device__ constexpr uint32_t smem_tail(bool multi, uint32_t nt) { return multi ? tail_out(nt) + kDrainWarps * kOutCols * 128 : kTailRows + nt * 4; }
 constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
 
 struct ExTarget {
@@ -382,9 +384,15 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     // CTA's last tile parks them all in the stages, which are free then; before that, eight columns of a warp at a time.
     const uint32_t out_at = bars + tail_out(p.nt) + warp * (kOutCols * 128u) + lane * 4u;
     const uint32_t park = tiles + warp * (cols * 128u) + lane * 4u;
-    float* row_factor = reinterpret_cast<float*>(tail + kTailRows) + warp * cols;
-    if (p.row_scale == nullptr)
-      for (uint32_t c = lane; c < cols; c += 32u) row_factor[c] = 1.0f;
+    float* row_factor = reinterpret_cast<float*>(tail + kTailRows) + (kMulti ? warp * cols : col0);
+    // the factors of activation rows c, c + step, .. of this warp's columns
+    auto row_factors = [&](uint32_t first_row, uint32_t c, uint32_t step) {
+      for (; c < cols; c += step) row_factor[c] = p.row_scale != nullptr && first_row + c < p.m ? p.row_scale[first_row + c] : 1.0f;
+    };
+    if constexpr (!kMulti) {  // one tile: the four warps of a column half share them
+      row_factors(blockIdx.y * p.nt + col0, quarter * 32u + lane, 128u);
+      asm volatile("bar.sync %0, 128;" ::"r"(1u + half) : "memory");
+    }
     uint32_t set = 0;  // accumulator sets so far, over all tiles
     uint32_t tile = tile0;
     do {
@@ -453,9 +461,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
       for (uint32_t j = 0; j < kOutCols; ++j, dst += tg.n)
         if (row_live && mm0 + j < p.m) *dst = finished(v[j], row_factor[c0 + j], ch.ws, ch.bias);
     };
-    // the factors of this warp's activation rows, into its own words: the warps of a column half may be in different tiles
-    if (p.row_scale != nullptr) {
-      for (uint32_t c = lane; c < cols; c += 32u) row_factor[c] = m0 + col0 + c < p.m ? p.row_scale[m0 + col0 + c] : 1.0f;
+    if constexpr (kMulti) {
+      row_factors(m0 + col0, lane, 32u);
       __syncwarp();
     }
     const bool last_tile = !kMulti || tile + tile_step >= tiles_all;
