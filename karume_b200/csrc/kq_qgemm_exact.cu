@@ -83,7 +83,7 @@ constexpr uint32_t kOutCols = 8;                // columns a drain warp hands to
 constexpr uint32_t kTailScales = 320, kTailRows = kTailScales + 2 * kScaleBatch * kRows * 4;
 // Barriers, the scale ring, the row factors; where a pair takes several tiles each drain warp has row factors of its own
 // (the warps of a column half may be in different tiles), and finished sums on their way out.  (A copy for each warp in
-// every form cost binary16 tiles of 256 rows one of six stages: 1225 x 2816 -> 7424 group 128 69.7 us, 65.1 without.)
+// every form cost binary16 tiles of 256 rows one of six stages: 1225 x 2816 -> 7424 group 128 69.7 us, TBD without.)
 __host__ __device__ constexpr uint32_t tail_out(uint32_t nt) { return kTailRows + kDrainWarps * nt / 2 * 4; }
 __host__ __device__ constexpr uint32_t smem_tail(bool multi, uint32_t nt) { return multi ? tail_out(nt) + kDrainWarps * kOutCols * 128 : kTailRows + nt * 4; }
 constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
@@ -283,8 +283,10 @@ __device__ __forceinline__ uint32_t stage_warps(uint32_t stages) {
   return parts_of(kMath) == 3 && stages < kProdWarps ? kProdWarps : 1u;
 }
 
-// What a launch does: a tile to a pair; that, or a tile of a gate and its up projection; several tiles to a pair.
-enum ExForm : int { kPlain, kGate, kSeveral };
+// What a launch does: a tile to a pair; K slices of a tile to a cluster; either, or a tile of a gate and its up projection;
+// several tiles to a pair.  (Code that a launch does not run still costs it, in instructions fetched cold around those that
+// it does: with the slices' in the plain form 20 x 4224 -> 112 binary16 9.7 us, 9.2 without, 24 x 4096 -> 256 11.3, 10.8.)
+enum ExForm : int { kPlain, kSliced, kGate, kSeveral };
 
 template <int kW, int kMath, int kForm>
 __global__ void __launch_bounds__(kExThreads, 1)
@@ -294,7 +296,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
   constexpr bool kTiled = kW == kI4Tiled || kW == kI8Tiled;
   constexpr bool kGroupScales = kW == kI4Tiled || kW == kI4Rows;
   constexpr uint32_t kParts = parts_of(kMath);
-  constexpr bool kMulti = kForm == kSeveral, kMayGate = kForm == kGate;
+  constexpr bool kMulti = kForm == kSeveral, kMayGate = kForm == kGate, kMaySlice = kForm == kSliced || kForm == kGate;
   static_assert(!kMulti || kMath == kInt8, "only sums that stay in tensor memory leave the drain warps time for another tile");
   const bool gated = kMayGate && p.swiglu != 0;
   extern __shared__ uint8_t smem_raw[];
@@ -616,8 +618,8 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
         default: drain_all(std::integral_constant<int, 8>{}); break;
       }
     }
-    if (last_tile && p.cluster_splits == 1) emit_parked();
-    if (!kMulti && p.cluster_splits > 1) {
+    if (last_tile && (!kMaySlice || p.cluster_splits == 1)) emit_parked();
+    if (kMaySlice && p.cluster_splits > 1) {
       // ---------------- K slices of a cluster: they meet in slice order, each finishing its share of the columns ----------------
       const ExTarget tg = p.t[at_tile.wi];
       const uint32_t slices = p.cluster_splits, share0 = cols * at_tile.z / slices, share1 = cols * (at_tile.z + 1) / slices;
@@ -949,7 +951,7 @@ qgemm_exact_kernel(const ExParams p, const __grid_constant__ CUtensorMap x_map, 
     }
   }
 
-  if (p.cluster_splits > 1 && warp >= kDrainWarps) cluster_sync_all();  // (the drain warps' barrier in front of their epilogue)
+  if (kMaySlice && p.cluster_splits > 1 && warp >= kDrainWarps) cluster_sync_all();  // (the drain warps' barrier in front of their epilogue)
   if (*abort_flag)  // a wait gave up: copies may still be in flight towards this CTA's shared memory
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1263,13 +1265,15 @@ cudaError_t launch_form(const LaunchEnv& env, const ExParams& p, const CUtensorM
 template <int kW, int kMath>
 cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, const CUtensorMap& xm, const CUtensorMap (&wm)[kMaxMulti]) {
   if constexpr (kMath == kInt8) {
-    return p.multi ? launch_form<kW, kMath, kSeveral>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
+    return p.multi ? launch_form<kW, kMath, kSeveral>(env, p, xm, wm)
+           : p.cluster_splits > 1 ? launch_form<kW, kMath, kSliced>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
   } else {
     // (a decoder's prompt takes one kernel for all its matmuls: two that take turns cost it 6 us a layer in instructions
     // fetched again, 692 | 667 us for four layers of 333 rows)
     constexpr bool kPrompt = kW == kI4Tiled && parts_of(kMath) == 3;
     if constexpr (kPrompt) return launch_form<kW, kMath, kGate>(env, p, xm, wm);
-    else return p.swiglu ? launch_form<kW, kMath, kGate>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
+    else return p.swiglu ? launch_form<kW, kMath, kGate>(env, p, xm, wm)
+                : p.cluster_splits > 1 ? launch_form<kW, kMath, kSliced>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
   }
 }
 
@@ -1280,7 +1284,7 @@ cudaError_t resident_pairs(const LaunchEnv& env, uint32_t (&slots)[kMaxClusterSp
   static PerDevice<Held> held_on;
   const Held* held = nullptr;
   const cudaError_t known = held_on.get([](Held& h) -> cudaError_t {
-    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1, kPlain>;
+    auto kernel = qgemm_exact_kernel<kI4Tiled, kHalf1, kSliced>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
     if (e != cudaSuccess) return e;
     for (uint32_t z = 2; z <= kMaxClusterSplits; z *= 2) {
