@@ -21,11 +21,13 @@ KQ_EXACT_FN uint32_t parts_of(int math) { return math == kBf3 ? 3u : math == kHa
 constexpr uint32_t kMaxNT = 256;           // activation rows per tile
 constexpr uint32_t kMaxClusterSplits = 4;  // K slices that meet in a cluster: two or four (eight CTAs, the portable most)
 
-// Clocks of one k-step, from the difference between k = 4,096 and 8,192 with 74 pairs at work (18,944 channels, one
-// tile each; at 1.92 GHz).  The conversion of the weights does not grow with the tile, its copy and the MMAs do; a
+// Clocks of one k-step.  The conversion of the weights does not grow with the tile, its copy and the MMAs do; a
 // drain costs its 32 to 256 fmas, 330 clocks at least, and is hidden until it alone fills the step; the two or three
-// parts of f32 rows cost what their tiles take to arrive, and above 192 rows the power cap.
-// Measured at nt = 32, 64, 96, 128, 160, 192, 224, 256:
+// parts of f32 rows cost what their tiles take to arrive, and above 192 rows the power cap, the more of it the more pairs
+// are at work: int4 group 32 f32, between k = 1,536 and 14,336, at 160, 192, 224, 256 rows 1,650, 1,590, 1,820, 1,910 on
+// 37 pairs, 1,780, 1,760, 2,230, 2,340 on 64, 1,970, 1,940, 2,410, 2,520 on 74.  The price above 192 rows is that of calls
+// whose last wave is not full (at 10 clocks a row 2048 x 14336 -> 4096 went from two waves of 256 rows, 543 us, to three of
+// 160, 591).  Measured with 74 pairs between k = 4,096 and 8,192, at 1.92 GHz, nt = 32, 64, 96, 128, 160, 192, 224, 256:
 //   int4, group 32   binary16 683, 798, 905, 1,048, 1,275, 1,450, 1,660, 1,750; f32 900, 1,200, 1,320, 1,510, 1,810,
 //                    1,960, 2,370, 2,940
 //   int8, tiled      binary16 535, 632, 632, 711, 764, 836, 950, 1,020 to 1,190; f32 780, 870, 890, 1,110, 1,290, 1,450,
@@ -37,7 +39,7 @@ inline uint32_t kstep_clocks(uint32_t nt, int math, uint32_t drains_x4, bool int
   const uint32_t parts = parts_of(math);
   const uint32_t mma = 4 * parts * std::max(nt / 2, 48u);
   const uint32_t step = int8 ? 650 + nt : 450 + (bytes_to_bf ? 200 : 0) + 100 * parts + nt + drains_x4 * (nt * 8 / 5 + 20) / 4;
-  const uint32_t fill = parts == 3 ? (nt > 192 ? nt * 10 : 740 + nt * 28 / 5) : parts == 2 ? 640 + nt * 21 / 5 : 0;
+  const uint32_t fill = parts == 3 ? (nt > 192 ? nt * 35 / 4 : 740 + nt * 28 / 5) : parts == 2 ? 640 + nt * 21 / 5 : 0;
   const uint32_t drain = int8 ? 0u : drains_x4 * std::max(nt * 7 / 2 + 60, 330u) / 4;
   return std::max({mma, step, fill, drain});
 }
@@ -54,7 +56,10 @@ struct Geometry { uint32_t nt, m_tiles, splits, cluster_splits; };
 // Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
 // loads, epilogue) plus its k-steps.  Two or four slices may meet in a cluster: no second launch and no partial sums in
 // memory, but 33 clusters of two pairs and 15 of four are all the device holds (74 pairs by themselves), and they start
-// later.  Other slices add the reduce launch and the partial sums, written and read at 2,200 bytes per clock.
+// later and wait for one another (priced at 750 clocks a slice, 153 x 1152 -> 5280 int8 binary16 went from 63 tiles, 11.3 us,
+// to 21 clusters, 14.1).  Other slices add the reduce launch and the partial sums, written and read at 2,200 bytes per clock.
+// The prices are those that come closest over 242 shapes (17 to 2,048 rows, all storages and activations) of which up to
+// eighteen cuts each were timed: 0.5 % behind the fastest in the mean, more than 5 % on eight of them.
 //   (us, with its split launch; reduce launch | cluster)  65 x 1152 -> 3072 group 16, four slices 16.0 | 13.8;
 //   300 x 4096 -> 4096 int8 binary16, two 29.0 | 22.8; 100 x 2048 -> 2048 group 128, four 18.2 | 15.4;
 //   333 x 8960 -> 1536, four, 72 tiles of 128 rows 45.4, 48 of 192 rows 49.3 | 46.6
@@ -80,8 +85,8 @@ inline Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, co
           continue;
         const uint32_t room = in_cluster != 0 ? slots[splits] * splits : slots[1];
         const uint64_t waves = (static_cast<uint64_t>(pairs) * mt * splits + room - 1) / room;
-        uint64_t cost = waves * (5000 + nt * 30 + static_cast<uint64_t>(each) * per + (in_cluster != 0 ? 750 * splits : 0));
-        if (splits > 1 && in_cluster == 0) cost += 5500 + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
+        uint64_t cost = waves * (6000 + nt * 30 + static_cast<uint64_t>(each) * per + (in_cluster != 0 ? 2500 : 0));
+        if (splits > 1 && in_cluster == 0) cost += 4400 + 140 * splits + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
         if (cost < best_cost) {
           best_cost = cost;
           best = {nt, mt, splits, in_cluster != 0 ? splits : 1u};

@@ -285,7 +285,7 @@ __device__ __forceinline__ uint32_t stage_warps(uint32_t stages) {
 
 // What a launch does: a tile to a pair; K slices of a tile to a cluster; either, or a tile of a gate and its up projection;
 // several tiles to a pair.  (Code that a launch does not run still costs it, in instructions fetched cold around those that
-// it does: with the slices' in the plain form 20 x 4224 -> 112 binary16 9.7 us, 9.2 without, 24 x 4096 -> 256 11.3, 10.8.)
+// it does: with the slices' in the plain form 24 x 9472 -> 4096 binary16 20.5 us, 20.0 without, 39 x 4736 -> 1920 bf16 14.4, 13.9.)
 enum ExForm : int { kPlain, kSliced, kGate, kSeveral };
 
 template <int kW, int kMath, int kForm>

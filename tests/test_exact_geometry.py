@@ -49,3 +49,16 @@ def test_the_shapes_of_the_resident_pair_tests_are_more_tiles_than_pairs(program
     shapes = [("i8", "i8", 0, m, n, k) for m, n, k in cases.EXACT_RESIDENT]
     for (_, _, _, m, n, k), (nt, tiles, slices, _) in zip(shapes, cut(program, shapes), strict=True):
         assert slices == 1 and (n + 255) // 256 * tiles > 74, (m, n, k, nt, tiles, slices)
+
+
+# Cuts that were timed against their neighbours, with those that came within 3 % of the fastest: (rows a tile, slices, slices
+# in a cluster)
+MEASURED = [(("f32", "i4", 32, 2048, 4096, 14336), {(256, 1, 1)}), (("f32", "i4", 32, 1905, 4608, 1600), {(256, 1, 1)}),
+            (("f16", "i8", 0, 153, 5280, 1152), {(64, 1, 1)}), (("f16", "i4", 32, 675, 432, 640), {(32, 1, 1)}),
+            (("f32", "i4", 32, 1788, 400, 640), {(64, 1, 1)}), (("f16", "i4", 64, 422, 832, 640), {(32, 1, 1)}),
+            (("f32", "i4", 32, 804, 6144, 4096), {(160, 1, 1)}), (("f16", "i4", 32, 87, 1152, 1792), {(32, 4, 4)})]
+
+
+def test_measured_shapes_are_cut_as_was_fastest(program):
+    for (shape, fast), (nt, _, slices, in_cluster) in zip(MEASURED, cut(program, [s for s, _ in MEASURED]), strict=True):
+        assert (nt, slices, in_cluster) in fast, (shape, nt, slices, in_cluster)
