@@ -24,7 +24,7 @@ TORCH_OUT = os.path.join(HERE, "_kqtorch.so")  # the Python calls on torch tenso
 
 SOURCES = ["kq_api.cu", "kq_generic.cu", "kq_qgemv_i4.cu", "kq_qgemv_i4_xs.cu", "kq_qgemv_i4_tc.cu", "kq_qgemv_rows.cu", "kq_plan.cu", "kq_qgemm_i4.cu", "kq_qgemm_exact.cu", "kq_qgemv_i8.cu",
            "kq_comm.cu", "kq_idot.cu", "kq_fused_ops.cu", "kq_container.cu"]
-HEADERS = ["kq_common.cuh", "kq_gemv_core.cuh", "kq_umma.cuh", "kq_gemm_stream.h", "kq_internal.h", "kq_per_device.h", "kq_exact_geometry.h", os.path.join("..", "..", "include", "kq.h")]
+HEADERS = ["kq_common.cuh", "kq_gemv_core.cuh", "kq_umma.cuh", "kq_gemm_stream.h", "kq_internal.h", "kq_per_device.h", "kq_exact_geometry.h", "kq_rows_line.h", os.path.join("..", "..", "include", "kq.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

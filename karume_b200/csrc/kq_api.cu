@@ -277,12 +277,14 @@ int check_linear_args(kq_ctx* ctx, const Weight* w, uint64_t x, int x_dtype, uin
 }
 
 // The kernel for row-major packed weights (kq_qgemv_rows.cu) runs this weight: up to 16 rows.
-bool takes_rows_gemv(const Weight& w, uint32_t m) { return kq::qgemv_rows_supports(w, m) && kq::qgemv_rows_preferred(w, m); }
+bool takes_rows_gemv(const kq::LaunchEnv& env, const kq::LinearTarget& t, int x_dtype, uint32_t m) {
+  return kq::qgemv_rows_supports(*t.w, m) && kq::qgemv_rows_preferred(env, t, x_dtype, m);
+}
 
 // The many-row kernel of kq_qgemm_exact.cu runs this call: more than 16 rows, weights of one kind,
 // and not a case of the bf16 GEMM (bf16 activations on a tiled weight, whose operands are rounded).
-bool takes_exact_gemm(const kq_ctx* ctx, int count, const kq::LinearTarget* targets, int x_dtype, uint32_t m) {
-  if (count == 1 && takes_rows_gemv(*targets[0].w, m)) return false;
+bool takes_exact_gemm(kq_ctx* ctx, int count, const kq::LinearTarget* targets, int x_dtype, uint32_t m) {
+  if (count == 1 && takes_rows_gemv(env_of(ctx), targets[0], x_dtype, m)) return false;
   for (int i = 0; i < count; ++i)
     if (kq::qgemm_i4_supports(*targets[i].w, x_dtype, m) || kq::qgemm_i8_supports(*targets[i].w, x_dtype, m)) return false;
   return kq::qgemm_exact_supports(count, targets, m, ctx->workspace ? ctx->workspace_bytes : 0);
@@ -359,7 +361,7 @@ int run_linear(kq_ctx* ctx, uint32_t count, const kq_weight* handles, uint64_t x
   // Everything else, weight by weight.
   for (uint32_t i = 0; i < count; ++i) {
     const Weight& w = *targets[i].w;
-    if (takes_rows_gemv(w, m)) {
+    if (takes_rows_gemv(env, targets[i], x_dtype, m)) {
       cudaError_t e = kq::launch_qgemv_rows(env, targets[i], reinterpret_cast<const void*>(x), x_dtype, m);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qgemv_rows launch");
       ctx->launches += 1;
@@ -1152,9 +1154,12 @@ int kq_linear_fused(kq_ctx* ctx, uint32_t count, const kq_weight* w, uint64_t x_
       ctx->launches += launched;
       return KQ_OK;
     }
+    kq::LaunchEnv with_neighbours = env_of(ctx);
+    with_neighbours.norm_weight = reinterpret_cast<const float*>(norm_weight_dptr);
+    with_neighbours.residual = reinterpret_cast<const float*>(residual_dptr);
     if (known && !reduce && (norm_weight_dptr || residual_dptr) &&
         (kq::qgemv_i4_fuses_neighbours(static_cast<int>(count), probe, x_dtype, m) ||
-         (count == 1 && takes_rows_gemv(*probe[0].w, m)) ||
+         (count == 1 && takes_rows_gemv(with_neighbours, probe[0], x_dtype, m)) ||
          takes_exact_gemm(ctx, static_cast<int>(count), probe, x_dtype, m))) {
       int rc;
       if (swiglu) {

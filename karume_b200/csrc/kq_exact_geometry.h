@@ -52,7 +52,7 @@ inline Steps steps_of(uint32_t k, int math, uint32_t group, uint32_t max_chain) 
   return Steps{(k + step_k - 1) / step_k, drain16, group != 0 && drain16 > 4 ? drain16 / 4 : 1};
 }
 
-struct Geometry { uint32_t nt, m_tiles, splits, cluster_splits; };
+struct Geometry { uint32_t nt, m_tiles, splits, cluster_splits; uint64_t clocks; };  // clocks: what it is expected to take
 // Tile width and K slices by estimated time: whole waves of pairs, each a fixed cost (tile fill, first
 // loads, epilogue) plus its k-steps.  Two or four slices may meet in a cluster: no second launch and no partial sums in
 // memory, but 33 clusters of two pairs and 15 of four are all the device holds (74 pairs by themselves), and they start
@@ -67,7 +67,7 @@ struct Geometry { uint32_t nt, m_tiles, splits, cluster_splits; };
 inline Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, const Steps& of, int math, bool int8_weights, bool may_split,
                                 const uint32_t (&slots)[kMaxClusterSplits + 1], uint64_t partial_room) {
   const uint32_t ksteps = of.ksteps, drain16 = of.drain16, slice_unit = of.slice_unit;
-  Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1, 1};
+  Geometry best = {kMaxNT, (m + kMaxNT - 1) / kMaxNT, 1, 1, 0};
   uint64_t best_cost = ~0ull;
   const uint32_t drains_x4 = std::max(1u, 16 / drain16);  // accumulator chains per k-step, times four
   const uint32_t most = (m + 31) / 32;
@@ -89,7 +89,7 @@ inline Geometry choose_geometry(uint32_t m, uint32_t n_total, uint32_t pairs, co
         if (splits > 1 && in_cluster == 0) cost += 4400 + 140 * splits + static_cast<uint64_t>(m) * n_total * (2 * splits + 1) * 4 / 2200;
         if (cost < best_cost) {
           best_cost = cost;
-          best = {nt, mt, splits, in_cluster != 0 ? splits : 1u};
+          best = {nt, mt, splits, in_cluster != 0 ? splits : 1u, cost};
         }
       }
     }

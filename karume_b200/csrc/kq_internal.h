@@ -79,7 +79,7 @@ struct LaunchEnv {
 // Up to sixteen rows over row-major packed weights (kq_qgemv_rows.cu); env.norm_weight (f32 activations) and env.residual
 // are applied.
 bool qgemv_rows_supports(const Weight& w, uint32_t m);
-bool qgemv_rows_preferred(const Weight& w, uint32_t m);
+bool qgemv_rows_preferred(const LaunchEnv& env, const LinearTarget& t, int x_dtype, uint32_t m);  // ... faster than what else runs this call
 cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const void* x, int x_dtype, uint32_t m);
 // Generic kernels: any shape the storage contract allows, native layout.
 cudaError_t launch_linear_generic(const LaunchEnv& env, const Weight& w, const void* x, int x_dtype,
@@ -131,6 +131,7 @@ cudaError_t launch_qgemm_i4(const LaunchEnv& env, const LinearTarget& target, co
 // storage, weights as exact integers.  All targets of one call share storage, layout, k, group
 // size and scale type.  env.norm_weight (f32 activations) and env.residual (one target) are applied.
 bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, uint64_t workspace_bytes);
+uint64_t qgemm_exact_clocks(const LaunchEnv& env, const Weight& w, int x_dtype, uint32_t m);  // what its tiles are expected to take
 // swiglu: two targets, gate and up, out[0] = silu(gate) * up; worth it where qgemm_exact_fuses_gate says so.
 bool qgemm_exact_fuses_gate(const LaunchEnv& env, uint32_t n, uint32_t m);
 cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarget* targets, const void* x, int x_dtype, uint32_t m,

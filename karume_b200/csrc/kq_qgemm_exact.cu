@@ -43,7 +43,7 @@
 //   warps 14-15  the group scales, a few chains ahead, as f32 into shared memory
 //
 // A gate and its up projection share a tile (64 channels of each per CTA), so that silu(gate) * up is the epilogue:
-// 333 rows of 1536 -> 2 x 8960 took 68 us and the gate's own kernel 11, now 69.
+// 333 rows of 1536 -> 2 x 8960, norm included, 66.7 us with the gate in a kernel of its own, 61.4 so.
 // Register split (setmaxnreg): 2 x 128 x 184 + 2 x 128 x 72 = 512 x 128.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets a status word and a CTA-wide abort
@@ -1235,6 +1235,7 @@ WeightKind kind_of(const Weight& w) {
   if (w.layout == kLayoutTiledI8) return kI8Tiled;
   return w.storage == KQ_STORAGE_I4 ? kI4Rows : kI8Rows;
 }
+int math_of(int x_dtype, const Weight& w) { return x_dtype == KQ_F16 ? kHalf1 : x_dtype == KQ_BF16 ? kBf1 : kind_of(w) == kI8Tiled ? kHalf2 : kBf3; }
 // The packed rows of the untiled layouts are read through a tensor map: 16-byte row strides.
 bool kind_ok(const Weight& w) {
   switch (kind_of(w)) {
@@ -1449,6 +1450,15 @@ bool qgemm_exact_supports(int count, const LinearTarget* targets, uint32_t m, ui
   return align256(static_cast<uint64_t>(w0.k) * 2 * parts_of(kBf3) * 16) + 256 <= workspace_bytes;
 }
 
+uint64_t qgemm_exact_clocks(const LaunchEnv& env, const Weight& w, int x_dtype, uint32_t m) {
+  const bool int8_weights = w.storage == KQ_STORAGE_I8;
+  const int math = math_of(x_dtype, w);
+  uint32_t slots[kMaxClusterSplits + 1];
+  if (resident_pairs(env, slots) != cudaSuccess) return 0;
+  return choose_geometry(m, w.n, (w.n + 2 * kRows - 1) / (2 * kRows), steps_of(w.k, math, int8_weights ? 0 : w.group_size, chain_of(math, int8_weights)), math,
+                         int8_weights, true, slots, env.workspace != nullptr ? env.workspace_bytes : 0).clocks;
+}
+
 // A gate and its up projection in one launch, silu(gate) * up written by the epilogue, where the tiles fill half of the
 // device; below that the two are worth cutting along K (the gate's own kernel then follows the matmul).
 bool qgemm_exact_fuses_gate(const LaunchEnv& env, uint32_t n, uint32_t m) {
@@ -1462,7 +1472,7 @@ cudaError_t launch_qgemm_exact(const LaunchEnv& env, int count, const LinearTarg
   const bool direct = x_dtype == KQ_F16;  // binary16 rows are the operand
   if ((direct && env.norm_weight != nullptr) || (swiglu && (count != 2 || targets[0].w->n != targets[1].w->n || env.residual != nullptr)))
     return cudaErrorInvalidValue;
-  const int math = direct ? kHalf1 : x_dtype == KQ_BF16 ? kBf1 : kind_of(w0) == kI8Tiled ? kHalf2 : kBf3;
+  const int math = math_of(x_dtype, w0);
   uint8_t* ws = static_cast<uint8_t*>(env.workspace);
   const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
   // row panels whose split activations take at most three quarters of the scratch (the rest: partial sums, which

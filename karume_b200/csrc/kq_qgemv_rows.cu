@@ -12,18 +12,22 @@
 //
 // What bounds it: instructions.  An int4 weight costs four (unpack, convert, scale) and one per activation row: one row of
 // 1152 -> 60468 (46 MB with f32 scales) 19 us, where the generic kernel and the many-row one took 50; for small
-// matrices the launch and two trips to memory (8064 -> 82: 14.4 us before, 5.6 now).
+// matrices the launch and two trips to memory (8064 -> 82: 12.8 us before, 5.2 now).
 #include <type_traits>
 
 #include "kq_common.cuh"
 #include "kq_gemv_core.cuh"
 #include "kq_internal.h"
+#include "kq_rows_line.h"
 
 namespace kq {
 namespace {
 
-constexpr uint32_t kRowsThreads = 256;
-constexpr uint32_t kRowsSmem = 224 * 1024, kRowsMost = 16;  // shared memory for the activations (of four rows at most); rows of a call
+constexpr uint32_t kRowsThreads = rows::kThreads, kRowsSmem = rows::kSmem;
+
+rows::Call rows_call(const Weight& w, uint32_t m, int sm_count) {
+  return rows::Call{w.storage == KQ_STORAGE_I4, w.n, w.k, m, static_cast<uint32_t>(sm_count)};
+}
 
 struct RowsParams {
   const uint8_t* w;
@@ -119,47 +123,43 @@ __global__ void __launch_bounds__(kRowsThreads, 2) qgemv_rows_kernel(const RowsP
   {
     const XT* x = static_cast<const XT*>(p.x) + static_cast<size_t>(m0) * p.k;
     const uint32_t eights = p.k / 8u;
-    [[maybe_unused]] const bool norm = std::is_same<XT, float>::value && p.norm_weight != nullptr;
-    if constexpr (std::is_same<XT, float>::value) {
-      if (norm) {
-        // sums of squares in a fixed order: thread-strided, shuffle tree, warps in order
-        float sq[kRowsX];
+    const bool norm = std::is_same<XT, float>::value && p.norm_weight != nullptr;
+    if (norm) {
+      // sums of squares in a fixed order: thread-strided, shuffle tree, warps in order
+      float sq[kRowsX];
 #pragma unroll
-        for (int r = 0; r < kRowsX; ++r) sq[r] = 0.0f;
-        for (uint32_t i = threadIdx.x; i < eights; i += kRowsThreads)
-#pragma unroll
-          for (int r = 0; r < kRowsX; ++r) {
-            if (static_cast<uint32_t>(r) >= live) continue;
-            float v[8];
-            load_x8<XT, false>(x + static_cast<size_t>(r) * p.k + i * 8u, v);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sq[r] = fmaf(v[e], v[e], sq[r]);
-          }
+      for (int r = 0; r < kRowsX; ++r) sq[r] = 0.0f;
+      for (uint32_t i = threadIdx.x; i < eights; i += kRowsThreads)
 #pragma unroll
         for (int r = 0; r < kRowsX; ++r) {
-          sq[r] = warp_sum(sq[r]);
-          if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5][r] = sq[r];
+          if (static_cast<uint32_t>(r) >= live) continue;
+          float v[8];
+          load_x8<XT, false>(x + static_cast<size_t>(r) * p.k + i * 8u, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) sq[r] = fmaf(v[e], v[e], sq[r]);
         }
-        __syncthreads();
-        if (threadIdx.x < kRowsX) {
-          float total = 0.0f;
-          for (uint32_t w = 0; w < kRowsThreads / 32; ++w) total += part[w][threadIdx.x];
-          row_norm[threadIdx.x] = rsqrtf(total * (1.0f / static_cast<float>(p.k)) + p.norm_eps);
-        }
-        __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kRowsX; ++r) {
+        sq[r] = warp_sum(sq[r]);
+        if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5][r] = sq[r];
       }
+      __syncthreads();
+      if (threadIdx.x < kRowsX) {
+        float total = 0.0f;
+        for (uint32_t w = 0; w < kRowsThreads / 32; ++w) total += part[w][threadIdx.x];
+        row_norm[threadIdx.x] = rsqrtf(total * (1.0f / static_cast<float>(p.k)) + p.norm_eps);
+      }
+      __syncthreads();
     }
     for (uint32_t i = threadIdx.x; i < kRowsX * eights; i += kRowsThreads) {
       const uint32_t r = kRowsX == 1 ? 0u : i / eights, at = kRowsX == 1 ? i : i - r * eights, step = at / kEights, e = at % kEights;
       float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       if (r < live) load_x8<XT, false>(x + static_cast<size_t>(r) * p.k + at * 8u, v);
-      if constexpr (std::is_same<XT, float>::value) {
-        if (norm) {
-          float wv[8];
-          load_x8<float, false>(p.norm_weight + at * 8u, wv);
+      if (norm) {
+        float wv[8];
+        load_x8<float, false>(p.norm_weight + at * 8u, wv);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(__fmul_rn(v[j], row_norm[r]), wv[j]);
-        }
+        for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(__fmul_rn(v[j], row_norm[r]), wv[j]);
       }
       float4* dst = xs + ((r * kEights + e) * 2u) * row4 + step;
       dst[0] = make_float4(v[0], v[1], v[2], v[3]);
@@ -265,9 +265,6 @@ __global__ void __launch_bounds__(kRowsThreads, 2) qgemv_rows_kernel(const RowsP
   }
 }
 
-// Bytes of staged activations.
-uint64_t rows_smem(uint32_t steps, uint32_t per, uint32_t rows) { return static_cast<uint64_t>(steps | 1u) * (per / 4u) * rows * 16u; }
-
 template <typename XT, bool kI8, bool kScaleF16, int kRowsX>
 cudaError_t launch_rows(const LaunchEnv& env, const RowsParams& p) {
   auto kernel = qgemv_rows_kernel<XT, kI8, kScaleF16, kRowsX>;
@@ -278,7 +275,7 @@ cudaError_t launch_rows(const LaunchEnv& env, const RowsParams& p) {
   const uint32_t pairs = (p.n + 1) / 2, per_cta = kRowsThreads >> p.lanes_log2;
   cfg.gridDim = dim3((pairs + per_cta - 1) / per_cta, (p.m + kRowsX - 1) / kRowsX);
   cfg.blockDim = dim3(kRowsThreads);
-  cfg.dynamicSmemBytes = rows_smem(p.steps, kI8 ? 16u : 32u, kRowsX);
+  cfg.dynamicSmemBytes = rows::staged_bytes(rows::Call{!kI8, p.n, p.k, p.m, 1});
   cfg.stream = env.stream;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -301,29 +298,13 @@ cudaError_t launch_rows_typed(const LaunchEnv& env, const RowsParams& p, bool i8
 
 }  // namespace
 
-bool qgemv_rows_supports(const Weight& w, uint32_t m) {
-  return w.layout == kLayoutNative && m >= 1 && m <= kRowsMost && w.n > 0 && w.k > 0 && w.k % (w.storage == KQ_STORAGE_I4 ? 32u : 16u) == 0 &&
-         rows_smem(w.k / (w.storage == KQ_STORAGE_I4 ? 32u : 16u), w.storage == KQ_STORAGE_I4 ? 32u : 16u, m > 2 ? 4u : m) <= kRowsSmem;
-}
-
-// This kernel or the many-row one (kq_qgemm_exact.cu; below its own line the generic kernel, which is behind everywhere
-// by two to seven times), by estimated time in units of 0.01 us.  Here a launch and its trips to memory, then the
-// instructions of a weight for every four activation rows.  There three launches, then whole waves of 74 tiles of 256
-// channels, which few tiles cut along k.  us, there | here, f32 activations:
-//   int4, group 128  1 x 768 -> 36699 23.4 | 8.8, 1 x 1152 -> 60468 50 | 19, 1 x 12288 -> 1490 21.4 | 9.8, 2 x 4096 -> 4090
-//                    17.4 | 11.5, 4 x 768 -> 36699 22.9 | 15.4, 16 x 8064 -> 82 35 | 10.2, but 4 x 12288 -> 1490 21.6 | 25.1,
-//                    8 x 768 -> 36699 23.2 | 28.9
-//   int8             1 x 768 -> 36699 25 | 8.5, 2 x 1152 -> 60468 59 | 26, 1 x 4096 -> 2841 16.7 | 7.8, 16 x 8064 -> 82 15.8 | 8.5, but
-//                    4 x 4096 -> 2841 17.4 | 21.9, 16 x 9984 -> 177 16.0 | 23.7
-bool qgemv_rows_preferred(const Weight& w, uint32_t m) {
-  if (m <= 2) return true;
-  const uint64_t weights = static_cast<uint64_t>(w.n) * w.k, passes = (m + 3) / 4;
-  const uint64_t long_k = (w.k < 4096u ? w.k : 4096u) / (w.storage == KQ_STORAGE_I4 ? 64u : 32u);  // every CTA stages the activations
-  const uint64_t here = 400 + passes * weights * (47 + long_k) / 1000000u;
-  const uint64_t pairs = (w.n + 255) / 256, waves = (pairs + 73) / 74;
-  uint64_t steps = (w.k + 63) / 64;
-  for (uint32_t splits = 2; splits <= 16 && pairs * splits <= 74 && steps >= 8; splits *= 2) steps = (steps + 1) / 2;
-  return here <= 600 + waves * (260 + 47 * steps);
+bool qgemv_rows_supports(const Weight& w, uint32_t m) { return w.layout == kLayoutNative && rows::supports(rows_call(w, m, 1)); }
+bool qgemv_rows_preferred(const LaunchEnv& env, const LinearTarget& t, int x_dtype, uint32_t m) {
+  const rows::Call call = rows_call(*t.w, m, env.sm_count);
+  const uint64_t room = env.workspace != nullptr ? env.workspace_bytes : 0;
+  if (qgemm_exact_supports(1, &t, m, room)) return rows::preferred(call, rows::estimate_many_row(qgemm_exact_clocks(env, *t.w, x_dtype, m), x_dtype == KQ_F16));
+  const int neighbours = (env.norm_weight != nullptr) + (env.residual != nullptr);  // kernels of their own beside the generic one
+  return rows::preferred(call, rows::estimate_generic(call) + neighbours * rows::kNeighbour);
 }
 
 cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const void* x, int x_dtype, uint32_t m) {
@@ -344,12 +325,7 @@ cudaError_t launch_qgemv_rows(const LaunchEnv& env, const LinearTarget& t, const
   p.norm_eps = env.norm_eps;
   p.residual = env.residual;
   while (!i8 && (1u << p.gshift) < w.group_size) ++p.gshift;
-  // As few threads to a pair of channels as still give every SM the CTAs it holds (three at most), at least two steps
-  // each: fewer reductions and fewer CTAs that stage the activations.
-  const uint64_t staged = rows_smem(p.steps, i8 ? 16u : 32u, m > 2 ? 4u : m), fit = kRowsSmem / (staged + 1024u);
-  const uint64_t want = static_cast<uint64_t>(env.sm_count) * kRowsThreads * (fit < 1 ? 1 : fit > 3 ? 3 : fit), pairs = (w.n + 1u) / 2u;
-  p.lanes_log2 = 2;
-  while (p.lanes_log2 < 8 && (pairs << p.lanes_log2) < want && (2u << p.lanes_log2) * 2u <= p.steps + 1u) ++p.lanes_log2;
+  p.lanes_log2 = rows::lanes_log2(rows_call(w, m, env.sm_count));
   const bool f16s = w.scale_dtype == KQ_F16;
   switch (x_dtype) {
     case KQ_F32: return launch_rows_typed<float>(env, p, i8, f16s);
