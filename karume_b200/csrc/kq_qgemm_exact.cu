@@ -1270,11 +1270,11 @@ cudaError_t launch_main(const LaunchEnv& env, const ExParams& p, const CUtensorM
            : p.cluster_splits > 1 ? launch_form<kW, kMath, kSliced>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
   } else {
     // (a decoder's prompt takes one kernel for all its matmuls: two that take turns cost it 6 us a layer in instructions
-    // fetched again, 692 | 667 us for four layers of 333 rows)
+    // fetched again, 692 | 667 us for four layers of 333 rows.  Up to 512 channels are none of a decoder's: 20 x 64 -> 256 7.9
+    // us in the prompt's form, 7.2 in the plain one, 64 x 6144 -> 128 16.0, 15.3)
     constexpr bool kPrompt = kW == kI4Tiled && parts_of(kMath) == 3;
-    if constexpr (kPrompt) return launch_form<kW, kMath, kGate>(env, p, xm, wm);
-    else return p.swiglu ? launch_form<kW, kMath, kGate>(env, p, xm, wm)
-                : p.cluster_splits > 1 ? launch_form<kW, kMath, kSliced>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
+    if (p.swiglu || (kPrompt && p.pairs > 2)) return launch_form<kW, kMath, kGate>(env, p, xm, wm);
+    return p.cluster_splits > 1 ? launch_form<kW, kMath, kSliced>(env, p, xm, wm) : launch_form<kW, kMath, kPlain>(env, p, xm, wm);
   }
 }
 
