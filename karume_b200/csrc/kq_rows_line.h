@@ -51,7 +51,8 @@ inline double estimate(const Call& c) {
   if (c.i4) {
     const uint64_t resident = std::min<uint64_t>(2, kSmem / (staged_bytes(c) + 1024u)), at_once = std::max<uint64_t>(1, c.sm_count * std::max<uint64_t>(1, resident));
     const double waves = ctas <= at_once ? 1.0 : 0.5 * ((ctas + at_once - 1) / at_once + static_cast<double>(ctas) / at_once);
-    return 33 + 0.021 * x * k + waves * (212 + 0.0198 * x * k + 0.352 * x * k * std::max<uint64_t>(1, resident) / lanes) + 14.6 * mega;
+    const double trips = 212 + (waves - 1.0) * std::min(212.0, 80 + k / 4);  // a wave's own; those of a short k overlap the next one's
+    return 33 + 0.021 * x * k + trips + waves * (0.0198 * x * k + 0.352 * x * k * std::max<uint64_t>(1, resident) / lanes) + 14.6 * mega;
   }
   return 226 + 0.013 * x * k + mega * (0.7 + 7.6 * x) + 0.82 * x * k / lanes + static_cast<double>(ctas) / c.sm_count * (45 + 0.0123 * x * k);
 }

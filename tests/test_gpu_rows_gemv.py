@@ -1,6 +1,7 @@
 """Up to sixteen rows over row-major packed weights (kq_qgemv_rows.cu): every storage, activation type and number of
 rows at the edges of its steps, groups of threads and passes, against the f64 oracle; a value's arithmetic is an f32
-multiply and multiply-adds, sixteen to a chain, so 1e-5 of the result's rms and 1e-4 relative hold with a wide margin."""
+multiply and multiply-adds, sixteen to a chain, so 1e-5 of the result's rms and 1e-4 relative hold with a wide margin.
+The smallest shapes stay on the generic kernel (kq_rows_line.h), in one launch as well."""
 import numpy as np
 import pytest
 
@@ -59,9 +60,18 @@ def test_matches_the_f64_oracle(gpu, storage, group, n, k, m, xdt):
     w.free()
 
 
-def test_infinities_and_nans_reach_their_channels(gpu):
+# Groups of sixteen, two scales to a step, and odd channel counts on rows long enough for this kernel
+@pytest.mark.parametrize("xdt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 16])
+@pytest.mark.parametrize("storage,group,n,k", [("i4", 16, 35, 4128), ("i4", 64, 1, 8192), ("i8", 0, 3, 8208)])
+def test_long_rows_of_few_channels(gpu, storage, group, n, k, m, xdt):
+    test_matches_the_f64_oracle(gpu, storage, group, n, k, m, xdt)
+
+
+@pytest.mark.parametrize("k", [96, 4128])
+def test_infinities_and_nans_reach_their_channels(gpu, k):
     import torch
-    n, k = 35, 96
+    n = 35
     data, scale = cases.synth_i4(n, k, seed=1, group_size=16)
     w = gpu.upload_weight("i4", data, scale, (n, k), 16)
     x = np.zeros((2, k), np.float32)
